@@ -831,6 +831,7 @@ int createImpl(const xpbi_scene_desc* scenes, uint32_t nScenes, xpbi_sim** out) 
   for (const SceneHost& h : s->sc) b.maxSceneN = std::max<uint32_t>(b.maxSceneN, (uint32_t)h.n);
   b.scanTiles = scan_tiles(b.C);
   const size_t n = std::max<size_t>(b.N, 1);
+  b.planeN = (uint32_t)((n + 3) & ~size_t(3));
 #define A(ptr, cnt)                               \
   do {                                            \
     rc = alloc(s, &(ptr), (cnt));                 \
@@ -869,6 +870,8 @@ int createImpl(const xpbi_scene_desc* scenes, uint32_t nScenes, xpbi_sim** out) 
   A(b.nbrP, (size_t)kNbrCap * n);
   A(b.nbrPCount, n);
   A(b.xc, n);
+  A(b.posP, 3 * (size_t)b.planeN);
+  A(b.xcP, 3 * (size_t)b.planeN);
   A(b.pbfRec, n);
   A(b.lamOut, n);
   A(b.lamPrev, n);

@@ -104,6 +104,15 @@ struct PV {
   float4 p, v;
 };
 
+// The predicted position of slot i for the PBF passes: the record their pair
+// loops gather and the coordinate planes pbfA's candidate walk reads.
+__device__ __forceinline__ void storeXc(const Bufs& b, uint32_t i, V3 xc, float w) {
+  b.xc[i] = make_float4(xc.x, xc.y, xc.z, w);
+  b.xcP[i] = xc.x;
+  b.xcP[i + b.planeN] = xc.y;
+  b.xcP[i + 2 * (size_t)b.planeN] = xc.z;
+}
+
 template <class T>
 __device__ __forceinline__ T ldg(const T* p) {
   return __ldg(p);
@@ -260,24 +269,60 @@ __device__ __forceinline__ V3 laneSum(V3 v) {
   return v3(laneSum<G>(v.x), laneSum<G>(v.y), laneSum<G>(v.z));
 }
 
-// Records, in stencil order, the candidates j != i of the rows around `x`
-// whose test(j) holds: list entry j | water bit from flag(j).
-template <class Test>
-__device__ __forceinline__ uint32_t recordCandidates(const SceneDev& S, const uint32_t* __restrict__ cellStart, V3 x,
-                                                     uint32_t i, uint32_t* __restrict__ out, Test&& test) {
-  uint32_t cnt = 0;
+// Visits, in stencil order, the candidates j != i of the rows around `x`
+// whose point in the coordinate planes P (P.x, P.y, P.z of slot j) lies
+// within sqrt(s2) of `c`: hit(j).
+//
+// A walk tests ~216 candidates for ~33 hits and is bound by the L1 data pipe
+// and by issue, so its inner loop does nothing but test: four candidates per
+// step from three 16-byte loads (aligned down to the planes' groups of four;
+// 12 bytes per candidate through the L1 pipe, not the 16 of a position
+// record), their distances two per packed instruction with the bound as the
+// sums' start value, each sign shifted into a mask of up to 32 candidates.
+// The candidates before the row's start and past its end are masked off (the
+// planes are padded), and a second loop over the set bits does a hit's work.
+struct Planes {
+  const float *x, *y, *z;
+};
+__device__ __forceinline__ Planes planesOf(const float* p, uint32_t stride) {
+  return Planes{p, p + stride, p + 2 * (size_t)stride};
+}
+template <class Hit>
+__device__ __forceinline__ void walkCandidates(const SceneDev& S, const uint32_t* __restrict__ cellStart, V3 x,
+                                               uint32_t i, Planes P, V3 c, float s2, Hit&& hit) {
+  const F2 cx = f2(-c.x, -c.x), cy = f2(-c.y, -c.y), cz = f2(-c.z, -c.z), ns2 = f2(-s2, -s2);
   forRows(S, cellStart, x, [&](uint32_t beg, uint32_t end) {
-#pragma unroll 4
-    for (uint32_t j = beg; j < end; ++j) {
-      uint32_t e;
-      const bool ok = test(j, e) && j != i;
-      // past the capacity the last slot is overwritten: such a list is
-      // marked as overflowed and never read
-      if (ok) out[min(cnt, kNbrCap - 1u)] = e;
-      cnt += ok ? 1u : 0u;
+#pragma unroll 1
+    for (uint32_t b0 = beg & ~3u; b0 < end; b0 += 32u) {
+      const uint32_t n = min(32u, end - b0);
+      uint32_t mask = 0;
+#pragma unroll 1
+      for (uint32_t t = 0; t < n; t += 4u) {
+        const ulonglong2 X = ldg(reinterpret_cast<const ulonglong2*>(P.x + b0 + t));
+        const ulonglong2 Y = ldg(reinterpret_cast<const ulonglong2*>(P.y + b0 + t));
+        const ulonglong2 Z = ldg(reinterpret_cast<const ulonglong2*>(P.z + b0 + t));
+        const F2 dx0 = add2(X.x, cx), dy0 = add2(Y.x, cy), dz0 = add2(Z.x, cz);
+        const F2 dx1 = add2(X.y, cx), dy1 = add2(Y.y, cy), dz1 = add2(Z.y, cz);
+        const F2 r0 = fma2(dz0, dz0, fma2(dy0, dy0, fma2(dx0, dx0, ns2)));
+        const F2 r1 = fma2(dz1, dz1, fma2(dy1, dy1, fma2(dx1, dx1, ns2)));
+        mask = __funnelshift_l((uint32_t)r0, mask, 1);
+        mask = __funnelshift_l((uint32_t)(r0 >> 32), mask, 1);
+        mask = __funnelshift_l((uint32_t)r1, mask, 1);
+        mask = __funnelshift_l((uint32_t)(r1 >> 32), mask, 1);
+      }
+      // candidate t of the chunk -> bit 31 - t
+      mask <<= 32u - ((n + 3u) & ~3u);
+      mask &= 0xffffffffu << (32u - n);
+      if (b0 < beg) mask &= 0xffffffffu >> (beg - b0);
+      if (i - b0 < 32u) mask &= ~(0x80000000u >> (i - b0));
+#pragma unroll 1
+      while (mask) {
+        const uint32_t t = (uint32_t)__clz((int)mask);
+        mask &= ~(0x80000000u >> t);
+        hit(b0 + t);
+      }
     }
   });
-  return cnt;
 }
 
 // A += V_b (v_b - v_i) g_b^T, the constraint sweep's velocity sum, with every
@@ -983,11 +1028,13 @@ __device__ __forceinline__ void computeL(const Bufs& b) {
   const float4 pi = posS[i];
   const V3 xi = xyz(pi);
   const float s2 = S.support2;
-  const uint32_t cnt = recordCandidates(S, b.cellStart, xi, i, listOf(b.nbr, i), [&](uint32_t j, uint32_t& e) {
-    const float4 p = ldg(posS + j);
-    const V3 d = xi - xyz(p);
-    e = j | (__float_as_uint(p.w) & kWaterBit);  // the water flag is the sign bit of pos.w
-    return dot(d, d) < s2;
+  uint32_t cnt = 0;
+  uint32_t* __restrict__ out = listOf(b.nbr, i);
+  walkCandidates(S, b.cellStart, xi, i, planesOf(b.posP, b.planeN), xi, s2, [&](uint32_t j) {
+    // past the capacity the last slot is overwritten: such a list is marked
+    // as overflowed and never read; the water flag is the sign bit of pos.w
+    out[min(cnt, kNbrCap - 1u)] = j | (__float_as_uint(ldg(&posS[j].w)) & kWaterBit);
+    ++cnt;
   });
   b.nbrCount[i] = cnt <= kNbrCap ? cnt : kNbrOverflow;
   // no pass of the substep reads a water particle's correction (every
@@ -1276,7 +1323,7 @@ __global__ void __launch_bounds__(kBlock, kMinB) k_solveB(Bufs b, int k, const f
       velOut[i] = vi4;
       if (writeXc) {
         const V3 xc = xyz(pi) + S.dt * xyz(vi4);
-        b.xc[i] = make_float4(xc.x, xc.y, xc.z, pi.w);
+        storeXc(b, i, xc, pi.w);
       }
     }
     return;
@@ -1384,7 +1431,7 @@ __global__ void __launch_bounds__(kBlock, kMinB) k_solveB(Bufs b, int k, const f
   velOut[i] = make_float4(v.x, v.y, v.z, vi4.w);
   if (writeXc) {
     const V3 xc = xi + S.dt * v;
-    b.xc[i] = make_float4(xc.x, xc.y, xc.z, pi.w);
+    storeXc(b, i, xc, pi.w);
   }
 }
 
@@ -1412,7 +1459,7 @@ __device__ __forceinline__ void solveBActiveSlot(const Bufs& b, int k, float4* _
     if (writeXc) {
       const float4 vi4 = vel[i];
       const V3 xc = xyz(pi) + S.dt * xyz(vi4);
-      b.xc[i] = make_float4(xc.x, xc.y, xc.z, pi.w);
+      storeXc(b, i, xc, pi.w);
     }
     return;
   }
@@ -1422,7 +1469,7 @@ __device__ __forceinline__ void solveBActiveSlot(const Bufs& b, int k, float4* _
     if (writeXc) {
       const float4 vi4 = vel[i];
       const V3 xc = xyz(pi) + S.dt * xyz(vi4);
-      b.xc[i] = make_float4(xc.x, xc.y, xc.z, pi.w);
+      storeXc(b, i, xc, pi.w);
     }
     return;
   }
@@ -1438,7 +1485,7 @@ __device__ __forceinline__ void solveBActiveSlot(const Bufs& b, int k, float4* _
       if (writeXc) {
         const float4 vi4 = vel[i];
         const V3 xc = xyz(pi) + S.dt * xyz(vi4);
-        b.xc[i] = make_float4(xc.x, xc.y, xc.z, pi.w);
+        storeXc(b, i, xc, pi.w);
       }
       return;
     }
@@ -1530,7 +1577,7 @@ __device__ __forceinline__ void solveBActiveSlot(const Bufs& b, int k, float4* _
   vel[i] = make_float4(v.x, v.y, v.z, vi4.w);
   if (writeXc) {
     const V3 xc = xi + S.dt * v;
-    b.xc[i] = make_float4(xc.x, xc.y, xc.z, pi.w);
+    storeXc(b, i, xc, pi.w);
   }
   const V3 dvel = v - xyz(vi4);
   const float dv2 = dot(dvel, dvel);
@@ -1619,22 +1666,16 @@ __global__ void XPBI_LB_PBF k_pbfA(Bufs b, int k, int flags) {
   }
   const V3 xci = xyz(xcS[i]);
   const float s2 = S.support2;
-  // the water flag is the sign bit of xc.w (the sorted pos.w)
-  const uint32_t cnt =
-      iWater ? recordCandidates(S, b.cellStart, xyz(pi), i, listOf(b.nbrP, i),
-                                [&](uint32_t j, uint32_t& e) {  // water pairs with everything
-                                  const float4 c = ldg(xcS + j);
-                                  const V3 d = xci - xyz(c);
-                                  e = j | (__float_as_uint(c.w) & kWaterBit);
-                                  return dot(d, d) < s2;
-                                })
-             : recordCandidates(S, b.cellStart, xyz(pi), i, listOf(b.nbrP, i),
-                                [&](uint32_t j, uint32_t& e) {  // a solid with water only
-                                  const float4 c = ldg(xcS + j);
-                                  const V3 d = xci - xyz(c);
-                                  e = j | kWaterBit;
-                                  return waterW(c.w) && dot(d, d) < s2;
-                                });
+  // water pairs with everything, a solid with water only (the water flag is
+  // the sign bit of xc.w, the sorted pos.w)
+  uint32_t cnt = 0;
+  uint32_t* __restrict__ out = listOf(b.nbrP, i);
+  walkCandidates(S, b.cellStart, xyz(pi), i, planesOf(b.xcP, b.planeN), xci, s2, [&](uint32_t j) {
+    const uint32_t flag = __float_as_uint(ldg(&xcS[j].w)) & kWaterBit;
+    if (!iWater && flag == 0u) return;
+    out[min(cnt, kNbrCap - 1u)] = j | flag;
+    ++cnt;
+  });
   const uint32_t stored = cnt <= kNbrCap ? cnt : kNbrOverflow;
   b.nbrPCount[i] = stored;
   if (!iWater) {
@@ -1891,7 +1932,7 @@ __global__ void k_predict(Bufs b, const float4* __restrict__ vel) {
   const SceneDev& S = *ctxOf(b, i).scene;
   const float4 pi = b.posS[i];
   const V3 xc = xyz(pi) + S.dt * xyz(vel[i]);
-  b.xc[i] = make_float4(xc.x, xc.y, xc.z, pi.w);
+  storeXc(b, i, xc, pi.w);
 }
 __global__ void k_copy_vel(uint32_t n, const float4* __restrict__ src, float4* __restrict__ dst) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;

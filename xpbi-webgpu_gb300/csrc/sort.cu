@@ -255,6 +255,9 @@ __global__ void __launch_bounds__(kThreads) k_reorder(Bufs b, int keepLam) {
   if (pp.w > 0.f) mi = min((uint32_t)pp.w, 7u);
   const bool water = b.mats[S.matBase + mi].kind == kKindWater;
   b.posS[s] = make_float4(pp.x, pp.y, pp.z, water ? -pp.w : pp.w);
+  b.posP[s] = pp.x;
+  b.posP[s + b.planeN] = pp.y;
+  b.posP[s + 2 * (size_t)b.planeN] = pp.z;
   M3 F = loadM(b.F, b.N, i);
   storeM(b.FS, b.N, s, F);
   float Vn = S.V0 * clampf(det(F), 0.1f, 10.f);

@@ -105,6 +105,8 @@ struct Bufs {
   float* F;             // [9][N] current F, plane (3c+r) holds F[c][r]
   float* state;         // [N] current plastic state
   float4* posS;         // [N] sorted positions
+  float* posP;          // [3][planeN] the sorted positions as coordinate planes (candidate walks)
+  float* xcP;           // [3][planeN] the predicted positions likewise
   float4* velS[2];      // [N] Jacobi ping-pong velocities
   float* FS;            // [9][N] sorted F
   float* stateS;        // [N] sorted plastic state
@@ -172,6 +174,7 @@ struct Bufs {
   int* err;             // [1] device error word
   unsigned long long* waitProbe;  // [1] a descriptor nothing publishes (xpbi_test_wait_expiry)
   uint32_t N, C, S;
+  uint32_t planeN;      // plane stride: N rounded up to whole groups of four
   uint32_t maxSceneN;   // particles of the largest scene
   uint32_t scanTiles;
 };

@@ -39,6 +39,34 @@ __device__ __forceinline__ V3 vlog(V3 v) { return {logf(v.x), logf(v.y), logf(v.
 __device__ __forceinline__ V3 vexp(V3 v) { return {expf(v.x), expf(v.y), expf(v.z)}; }
 __device__ __forceinline__ V3 vsqrt(V3 v) { return {sqrtf(v.x), sqrtf(v.y), sqrtf(v.z)}; }
 
+// Two f32 lanes in one 64-bit register pair (sm_100's packed add / multiply /
+// fused multiply-add, each lane rounded like the scalar operation): the
+// neighbour passes are issue-bound, and these do two candidates' or two
+// neighbours' arithmetic per instruction.
+typedef unsigned long long F2;
+__device__ __forceinline__ F2 f2(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float lo2(F2 a) { return __uint_as_float((uint32_t)a); }
+__device__ __forceinline__ float hi2(F2 a) { return __uint_as_float((uint32_t)(a >> 32)); }
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
 // Column-major 3x3, c[j] = column j (WGSL mat3x3f).
 struct M3 {
   V3 c[3];
