@@ -213,6 +213,15 @@ void buildSceneDev(const SceneHost& s, uint32_t sceneIdx, SceneDev& d, MatDev* m
     }
   }
   d.invH = 1.f / h;
+  // The pair sums form t = 1 - r halfInvH and multiply by gradC once, after
+  // the loop. The rounding of halfInvH (up to 6e-8) shifts t^3 the same way
+  // for every neighbour — by 5.5 times as much over a lattice's neighbours
+  // weighted as in sum t^3 r^2, the moment of every gradient sum — so gradC
+  // takes that shift out again.
+  const double half = 0.5 / (double)h;
+  d.halfInvH = (float)half;
+  d.gradC = (float)(-5.0 * 21.0 / (16.0 * 3.14159265 * (double)h * h * h * h * h) *
+                    (1.0 + 5.5 * ((double)d.halfInvH / half - 1.0)));
   d.invW0 = 1.f / fmaxf(d.w0, 1e-12f);
   d.alphaT = (1.f / d.V0) / (dt * dt);
   d.minD = 0.75f * h;
@@ -237,6 +246,7 @@ void buildSceneDev(const SceneHost& s, uint32_t sceneIdx, SceneDev& d, MatDev* m
     M.p3 = wf(q, 7);
     M.boundFriction = wf(q, 12);
     M.mass = wf(q, 13);
+    M.invMass = 1.f / M.mass;
     M.massPerDensity = M.density != 0.f ? M.mass / M.density : 0.f;
   }
   // PBF pairs weight by the water particle's mass / density; with one water
@@ -638,7 +648,7 @@ cudaError_t enqueueSubstep(xpbi_sim* s, const Schedule& sch, cudaStream_t st, Re
   // the velocity-free sums are read by the one-lane constraint sweeps; with
   // features (the learned solve, or features logged) the same pass also
   // stores iteration 0's constraint and the network's features
-  launch_computeL(b, sch.lanes == 1 || sch.features, sch.features, st);
+  launch_computeL(b, sch.features, st);
   R.mark(st, "computeL");
   if (sch.mode == 1) {
     mlp_forward(b.feat, b.N, b.netBlob, b.netOut, nullptr, s->netErr, st, true);
@@ -865,9 +875,9 @@ int createImpl(const xpbi_scene_desc* scenes, uint32_t nScenes, xpbi_sim** out) 
   b.tileStatus = ctl + 1;
   A(b.bigList, n / 64 + 2);
   A(b.sceneOf, n);
-  A(b.nbr, (size_t)kNbrCap * n);
+  A(b.nbr, (size_t)kNbrCap * ((n + 31) & ~size_t(31)));  // whole warps of interleaved lists
   A(b.nbrCount, n);
-  A(b.nbrP, (size_t)kNbrCap * n);
+  A(b.nbrP, (size_t)kNbrCap * ((n + 31) & ~size_t(31)));
   A(b.nbrPCount, n);
   A(b.xc, n);
   A(b.posP, 3 * (size_t)b.planeN);
@@ -1409,7 +1419,7 @@ int xpbi_autotune(xpbi_sim* sim, int32_t iterations, int32_t has_water, int32_t 
     launch_scan(b, st);
     launch_scatter(b, st);
     launch_reorder(b, false, st);
-    launch_computeL(b, true, false, st);
+    launch_computeL(b, false, st);
     cudaMemsetAsync(b.done, 0, sizeof(int) * b.S, st);  // no scene counts as converged here
     cudaMemsetAsync(b.solidDisp, 0, sizeof(uint32_t) * 2 * b.S, st);
     // iteration 0 of each variant from lambda = 0, then solveB on its record

@@ -38,6 +38,13 @@ namespace xpbi {
 namespace {
 
 constexpr int kThreads = 128;
+#ifndef A_AHEAD
+#define A_AHEAD false
+#endif
+#ifndef L_AHEAD
+#define L_AHEAD false
+#endif
+
 
 // Launch bounds of the stencil kernels: defining XPBI_MINB_<KERNEL> at build
 // time asks the register allocator for that many resident CTAs per SM
@@ -46,7 +53,7 @@ constexpr int kThreads = 128;
 #ifdef XPBI_MINB_COMPUTEL
 #define XPBI_LB_COMPUTEL __launch_bounds__(kThreads, XPBI_MINB_COMPUTEL)
 #else
-#define XPBI_LB_COMPUTEL XPBI_LB_DEFAULT
+#define XPBI_LB_COMPUTEL __launch_bounds__(kThreads, 8)
 #endif
 // computeL with the stored constraint and features (the learned solve) at
 // 7 CTAs per SM (72 registers): 1.36 ms per 4M-particle substep against
@@ -65,10 +72,10 @@ constexpr int kThreads = 128;
 // within 1% on the 256-scene batch, the snowball and the sand column; for
 // solveB the allocator's choice (80 registers) beat every cap. The 64- and
 // 256-thread shapes keep an entry's occupancy with other block sizes.
-constexpr int kSolveAMinB[kSolveAVariants] = {8, 6, 5, 7, 14, 4};
-constexpr int kSolveABlock[kSolveAVariants] = {128, 128, 128, 128, 64, 256};
-constexpr int kSolveBMinB[kSolveBVariants] = {0, 7, 5, 0, 0};
-constexpr int kSolveBBlock[kSolveBVariants] = {128, 128, 128, 64, 256};
+constexpr int kSolveAMinB[kSolveAVariants] = {8, 9, 10, 7, 16, 6};
+constexpr int kSolveABlock[kSolveAVariants] = {128, 128, 128, 128, 64, 128};
+constexpr int kSolveBMinB[kSolveBVariants] = {9, 8, 7, 10, 6};
+constexpr int kSolveBBlock[kSolveBVariants] = {128, 128, 128, 128, 128};
 #ifdef XPBI_MINB_PBF
 #define XPBI_LB_PBF __launch_bounds__(kThreads, XPBI_MINB_PBF)
 #else
@@ -142,114 +149,220 @@ __device__ __forceinline__ void forRows(const SceneDev& S, const uint32_t* __res
   }
 }
 
-// A particle's list occupies kNbrCap consecutive words (16-byte aligned) and
-// is read four entries per load, one load ahead; the gather of entry k+1 is
-// issued before the body of entry k runs.
+// Neighbour lists. The lists of 32 consecutive slots (a warp's) are
+// interleaved by groups of four entries: group q of slot i is one 16-byte
+// load at nbrGroups(i)[32 q], and the 32 lanes' loads are contiguous. The
+// entries of slot i's own phase (solid or water), the only ones most passes
+// visit, come first in stencil order, padded to whole groups with i itself —
+// whose distance is 0, so that it adds nothing to a gradient sum and no loop
+// tests for its end; computeL puts the other phase's entries at the far end.
+// (The list loads are plain ones: computeL and pbfA read what they have just
+// written.)
+constexpr uint32_t kGroupStride = 32u;
+__device__ __forceinline__ uint4* nbrGroups(uint32_t* base, uint32_t i) {
+  return reinterpret_cast<uint4*>(base) + (size_t)(i >> 5) * (kNbrCap / 4u * 32u) + (i & 31u);
+}
+__device__ __forceinline__ uint32_t* nbrEntry(uint32_t* base, uint32_t i, uint32_t e) {
+  return reinterpret_cast<uint32_t*>(nbrGroups(base, i) + kGroupStride * (e >> 2)) + (e & 3u);
+}
 __device__ __forceinline__ uint32_t lane4(const uint4& q, uint32_t s) {
   return s == 0u ? q.x : (s == 1u ? q.y : (s == 2u ? q.z : q.w));
 }
+// the count word: entries of the slot's own phase, of the other one
+__device__ __forceinline__ uint32_t sameCount(uint32_t c) { return c & 0xffu; }
+__device__ __forceinline__ uint32_t otherCount(uint32_t c) { return c >> 8; }
 
-// kRaw: gather() receives the raw entry (index | water bit), e.g. to skip
-// the loads of entries the body ignores.
-template <bool kRaw = false, class Gather, class Body>
-__device__ __forceinline__ void forList(const uint32_t* __restrict__ list, uint32_t cnt, Gather&& gather,
-                                        Body&& body) {
-  if (cnt == 0) return;
-  const uint4* __restrict__ L = reinterpret_cast<const uint4*>(list);
-  uint4 cur = __ldg(L);
-  uint4 nxt = cnt > 4u ? __ldg(L + 1) : cur;
-  uint32_t e = cur.x;
-  auto d = gather(kRaw ? e : e & ~kWaterBit);
+// Two neighbours at a time over `groups` groups: body(j0, j1, d0, d1) with
+// d = gather(j). The gathers of a pair are issued before the arithmetic of
+// the pair before it, the list's groups one group ahead.
+template <class Gather, class Body>
+__device__ __forceinline__ void forPairs(const uint4* L, uint32_t groups, Gather&& gather, Body&& body) {
+  if (groups == 0u) return;
+  uint4 cur = *(L);
+  uint4 nxt = *(L + kGroupStride * min(1u, groups - 1u));
+  auto a0 = gather(cur.x), a1 = gather(cur.y);
+#pragma unroll 1
+  for (uint32_t q = 1u; q < groups; ++q) {
+    const auto b0 = gather(cur.z), b1 = gather(cur.w);
+    const uint4 nn = *(L + kGroupStride * min(q + 1u, groups - 1u));
+    body(cur.x, cur.y, a0, a1);
+    a0 = gather(nxt.x);
+    a1 = gather(nxt.y);
+    body(cur.z, cur.w, b0, b1);
+    cur = nxt;
+    nxt = nn;
+  }
+  const auto b0 = gather(cur.z), b1 = gather(cur.w);
+  body(cur.x, cur.y, a0, a1);
+  body(cur.z, cur.w, b0, b1);
+}
+
+// One entry at a time: body(j, d) with d = gather(j), the gather of an entry
+// issued before the arithmetic of the one before it (kAhead).
+#ifndef EACH_AHEAD
+#define EACH_AHEAD 0
+#endif
+template <bool kAhead = true, class Gather, class Body>
+__device__ __forceinline__ void forSingles(const uint4* L, uint32_t groups, Gather&& gather, Body&& body) {
+  if (groups == 0u) return;
+  uint4 cur = *(L);
+  if constexpr (kAhead) {
+    uint4 nxt = *(L + kGroupStride * min(1u, groups - 1u));
+    auto d = gather(cur.x);
+#pragma unroll 1
+    for (uint32_t q = 1u; q <= groups; ++q) {
+      auto e = gather(cur.y);
+      body(cur.x, d);
+      d = gather(cur.z);
+      body(cur.y, e);
+      e = gather(cur.w);
+      body(cur.z, d);
+      const uint4 nn = *(L + kGroupStride * min(q + 1u, groups - 1u));
+      d = gather(nxt.x);
+      body(cur.w, e);
+      cur = nxt;
+      nxt = nn;
+    }
+  } else {
+#pragma unroll 1
+    for (uint32_t q = 1u; q <= groups; ++q) {
+      const uint4 nxt = *(L + kGroupStride * min(q, groups - 1u));
+      body(cur.x, gather(cur.x));
+      body(cur.y, gather(cur.y));
+      body(cur.z, gather(cur.z));
+      body(cur.w, gather(cur.w));
+      cur = nxt;
+    }
+  }
+}
+template <class Gather, class Body>
+__device__ __forceinline__ void forEach(const uint4* L, uint32_t cnt, Gather&& gather, Body&& body) {
+  if (cnt == 0u) return;
+  uint4 cur = *(L);
+  uint4 nxt = cnt > 4u ? *(L + kGroupStride) : cur;
+  auto d = gather(cur.x);
 #pragma unroll 1
   for (uint32_t k = 1; k < cnt; ++k) {
     const uint32_t sl = k & 3u;
     if (sl == 0u) {
       cur = nxt;
-      if (k + 4u < cnt) nxt = __ldg(L + (k >> 2) + 1);
+      if (k + 4u < cnt) nxt = *(L + kGroupStride * ((k >> 2) + 1u));
     }
-    const uint32_t en = lane4(cur, sl);
-    auto dn = gather(kRaw ? en : en & ~kWaterBit);
-    body(e & ~kWaterBit, (e & kWaterBit) != 0u, d);
-    e = en;
+    auto dn = gather(lane4(cur, sl));
+    body(d);
     d = dn;
   }
-  body(e & ~kWaterBit, (e & kWaterBit) != 0u, d);
+  body(d);
 }
 
-__device__ __forceinline__ uint32_t* listOf(uint32_t* base, uint32_t i) { return base + (size_t)i * kNbrCap; }
+// The same without gathers in flight over a pair's arithmetic (records of
+// many registers).
+template <class Gather, class Body>
+__device__ __forceinline__ void forPairsNow(const uint4* L, uint32_t groups, Gather&& gather, Body&& body) {
+  if (groups == 0u) return;
+  uint4 cur = *(L);
+#pragma unroll 1
+  for (uint32_t q = 1u; q <= groups; ++q) {
+    const uint4 nxt = *(L + kGroupStride * min(q, groups - 1u));
+    body(cur.x, cur.y, gather(cur.x), gather(cur.y));
+    body(cur.z, cur.w, gather(cur.z), gather(cur.w));
+    cur = nxt;
+  }
+}
 
-// Keeps every recorded neighbour.
-struct KeepAll {
-  __device__ __forceinline__ bool operator()(uint32_t) const { return true; }
-};
-
-// In-support neighbours of slot i in stencil order: body(j, jIsWater, data).
-// keep(entry) (index | water bit) false: the body will ignore that neighbour,
-// so its data is not loaded (the body receives a zero-initialised value).
-template <class Gather, class Body, class Keep = KeepAll>
-__device__ __forceinline__ void forNbrs(const Bufs& b, const Ctx& cx, uint32_t i, V3 xi, Gather&& gather,
-                                        Body&& body, Keep keep = Keep{}) {
-  const uint32_t cnt = b.nbrCount[i];
-  if (cnt != kNbrOverflow) {
-    forList<true>(listOf(b.nbr, i), cnt,
-                  [&](uint32_t e) {
-                    using T = decltype(gather(0u));
-                    return keep(e) ? gather(e & ~kWaterBit) : T{};
-                  },
-                  body);
+// Slot i's neighbours of its own phase, two at a time, over the recorded
+// list, or by the stencil walk if it overflowed (each neighbour then paired
+// with i itself).
+//
+// Several lanes per slot (small scenes): the G lanes of slot i are
+// consecutive in the warp; lane `lane` visits the pairs p with p % G == lane
+// (on the walk every G-th candidate of each row) and accumulates a partial
+// sum; laneSum adds them over the group.
+template <int G, bool kAhead = true, class Gather, class Body>
+__device__ __forceinline__ void forSame(const Bufs& b, const Ctx& cx, uint32_t i, V3 xi, bool iWater, uint32_t lane,
+                                        Gather&& gather, Body&& body) {
+  static_assert(G == 1 || G == 2 || G == 4, "one, two or four lanes per slot");
+  const uint32_t c = b.nbrCount[i];
+  if (c != kNbrOverflow) {
+    const uint4* L = nbrGroups(b.nbr, i);
+    if constexpr (G == 1) {
+      if constexpr (kAhead)
+        forPairs(L, (sameCount(c) + 3u) >> 2, gather, body);
+      else
+        forPairsNow(L, (sameCount(c) + 3u) >> 2, gather, body);
+    } else {
+      const uint32_t pairs = (sameCount(c) + 1u) >> 1;
+#pragma unroll 2
+      for (uint32_t p = lane; p < pairs; p += G) {
+        const uint2 e = *(reinterpret_cast<const uint2*>(L + kGroupStride * (p >> 1)) + (p & 1u));
+        body(e.x, e.y, gather(e.x), gather(e.y));
+      }
+    }
   } else {
     const SceneDev& S = *cx.scene;
+    const auto self = gather(i);
     forRows(S, b.cellStart, xi, [&](uint32_t beg, uint32_t end) {
 #pragma unroll 1
-      for (uint32_t j = beg; j < end; ++j) {
+      for (uint32_t j = beg + lane; j < end; j += G) {
         if (j == i) continue;
         const float4 pj = ldg(b.posS + j);
         const V3 d = xi - xyz(pj);
-        if (dot(d, d) < S.support2) body(j, waterW(pj.w), gather(j));
+        if (dot(d, d) < S.support2 && waterW(pj.w) == iWater) body(j, i, gather(j), self);
       }
     });
   }
 }
 
-// Several lanes per slot (small scenes): the G lanes of slot i are
-// consecutive in the warp; lane `lane` visits the list entries k with
-// k % G == lane (each group of four entries is one load, shared by the
-// lanes), or on the overflow walk every G-th candidate of each row. Each
-// lane accumulates a partial sum; laneSum adds them over the group.
-template <int G, class Gather, class Body, class Keep = KeepAll>
-__device__ __forceinline__ void forNbrsLanes(const Bufs& b, const Ctx& cx, uint32_t i, V3 xi, uint32_t lane,
-                                             Gather&& gather, Body&& body, Keep keep = Keep{}) {
-  static_assert(G == 1 || G == 2 || G == 4, "one, two or four lanes per slot");
-  if constexpr (G == 1) {
-    (void)lane;
-    forNbrs(b, cx, i, xi, gather, body, keep);
-  } else {
-    const uint32_t cnt = b.nbrCount[i];
-    if (cnt != kNbrOverflow) {
-      const uint4* __restrict__ L = reinterpret_cast<const uint4*>(listOf(b.nbr, i));
-      const uint32_t groups = (cnt + 3u) >> 2;
-#pragma unroll 1
-      for (uint32_t q = 0; q < groups; ++q) {
-        const uint4 grp = __ldg(L + q);
-#pragma unroll
-        for (uint32_t s = lane; s < 4u; s += G) {
-          const uint32_t e = lane4(grp, s);
-          if (4u * q + s < cnt && keep(e)) body(e & ~kWaterBit, (e & kWaterBit) != 0u, gather(e & ~kWaterBit));
-        }
-      }
+// A solid's solid neighbours one at a time.
+template <int G, bool kAhead, class Gather, class Body>
+__device__ __forceinline__ void forSameSingles(const Bufs& b, const Ctx& cx, uint32_t i, V3 xi, uint32_t lane,
+                                               Gather&& gather, Body&& body) {
+  const uint32_t c = b.nbrCount[i];
+  if (c != kNbrOverflow) {
+    const uint4* L = nbrGroups(b.nbr, i);
+    if constexpr (G == 1) {
+      forSingles<kAhead>(L, (sameCount(c) + 3u) >> 2, gather, body);
     } else {
-      const SceneDev& S = *cx.scene;
-      forRows(S, b.cellStart, xi, [&](uint32_t beg, uint32_t end) {
-#pragma unroll 1
-        for (uint32_t j = beg + lane; j < end; j += G) {
-          if (j == i) continue;
-          const float4 pj = ldg(b.posS + j);
-          const V3 d = xi - xyz(pj);
-          if (dot(d, d) < S.support2) body(j, waterW(pj.w), gather(j));
-        }
-      });
+      const uint32_t pairs = (sameCount(c) + 1u) >> 1;
+#pragma unroll 2
+      for (uint32_t p = lane; p < pairs; p += G) {
+        const uint2 e = *(reinterpret_cast<const uint2*>(L + kGroupStride * (p >> 1)) + (p & 1u));
+        const auto d0 = gather(e.x), d1 = gather(e.y);
+        body(e.x, d0);
+        body(e.y, d1);
+      }
     }
+  } else {
+    const SceneDev& S = *cx.scene;
+    forRows(S, b.cellStart, xi, [&](uint32_t beg, uint32_t end) {
+#pragma unroll 1
+      for (uint32_t j = beg + lane; j < end; j += G) {
+        if (j == i) continue;
+        const float4 pj = ldg(b.posS + j);
+        const V3 d = xi - xyz(pj);
+        if (dot(d, d) < S.support2 && !waterW(pj.w)) body(j, gather(j));
+      }
+    });
   }
+}
+
+// The radial factor of the kernel gradient of two neighbours at offsets
+// (dx, dy, dz): gradW = c g (dx, dy, dz) with c = S.gradC = -5 sigW / h^2 and
+// g = t^3, t = 1 - r / (2 h). (The Wendland gradient's q / (h r) is 1 / h^2,
+// so neither a division by r nor a test for r = 0 is left; neighbours are
+// within the support, so t is not negative beyond rounding.)
+__device__ __forceinline__ float sqrtFast(float x) {
+  float y;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// t = 1 - r / (2 h) from r^2
+__device__ __forceinline__ F2 falloff2(const SceneDev& S, F2 r2) {
+  return fma2(f2(sqrtFast(lo2(r2)), sqrtFast(hi2(r2))), f2(-S.halfInvH, -S.halfInvH), f2(1.f, 1.f));
+}
+__device__ __forceinline__ F2 radial2(const SceneDev& S, F2 r2) {
+  const F2 t = falloff2(S, r2);
+  return mul2(mul2(t, t), t);
 }
 
 template <int G>
@@ -268,6 +381,8 @@ template <int G>
 __device__ __forceinline__ V3 laneSum(V3 v) {
   return v3(laneSum<G>(v.x), laneSum<G>(v.y), laneSum<G>(v.z));
 }
+// both halves of a packed sum
+__device__ __forceinline__ float sum2(F2 a) { return lo2(a) + hi2(a); }
 
 // Visits, in stencil order, the candidates j != i of the rows around `x`
 // whose point in the coordinate planes P (P.x, P.y, P.z of slot j) lies
@@ -325,86 +440,145 @@ __device__ __forceinline__ void walkCandidates(const SceneDev& S, const uint32_t
   });
 }
 
-// A += V_b (v_b - v_i) g_b^T, the constraint sweep's velocity sum, with every
-// rounding explicit: solveA's sweep and computeL's (which stores iteration
-// 0's constraint for it) form the same bits whatever the compiler would
-// fuse around them.
-__device__ __forceinline__ void addVelSum(M3& A, const float4& vb, V3 vi, V3 g) {
-  const float dx = __fmul_rn(__fsub_rn(vb.x, vi.x), vb.w);
-  const float dy = __fmul_rn(__fsub_rn(vb.y, vi.y), vb.w);
-  const float dz = __fmul_rn(__fsub_rn(vb.z, vi.z), vb.w);
-  const float gc[3] = {g.x, g.y, g.z};
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    A.c[c].x = __fmaf_rn(dx, gc[c], A.c[c].x);
-    A.c[c].y = __fmaf_rn(dy, gc[c], A.c[c].y);
-    A.c[c].z = __fmaf_rn(dz, gc[c], A.c[c].z);
-  }
+// The offsets of two neighbours from xi and what the sums weigh them by:
+// (dx, dy, dz) = xi - x_b, w = V_b g (dx, dy, dz), so that V_b gradW_b = c w.
+struct Pair {
+  F2 dx, dy, dz, wx, wy, wz;
+};
+__device__ __forceinline__ Pair pairOf(const SceneDev& S, V3 xi, const PV& p, const PV& q) {
+  Pair r;
+  r.dx = f2(xi.x - p.p.x, xi.x - q.p.x);
+  r.dy = f2(xi.y - p.p.y, xi.y - q.p.y);
+  r.dz = f2(xi.z - p.p.z, xi.z - q.p.z);
+  const F2 s = mul2(radial2(S, fma2(r.dz, r.dz, fma2(r.dy, r.dy, mul2(r.dx, r.dx)))), f2(p.v.w, q.v.w));
+  r.wx = mul2(r.dx, s);
+  r.wy = mul2(r.dy, s);
+  r.wz = mul2(r.dz, s);
+  return r;
 }
+
+// A += (v_b - v_i) w_b^T for two neighbours: the velocity sum of the
+// constraint sweeps, sum V_b (v_b - v_i) gradW_b^T without its factor c. Even
+// and odd neighbours add up in the two halves. solveA's sweep and computeL's
+// (which stores iteration 0's constraint for it) run these same operations,
+// every one with its rounding fixed, so they form the same bits.
+struct VelSum {
+  F2 a[9];
+  __device__ __forceinline__ VelSum() {
+#pragma unroll
+    for (int k = 0; k < 9; ++k) a[k] = 0ull;
+  }
+  __device__ __forceinline__ void add(const Pair& r, V3 vi, const float4& v0, const float4& v1) {
+    const F2 vx = f2(v0.x - vi.x, v1.x - vi.x), vy = f2(v0.y - vi.y, v1.y - vi.y), vz = f2(v0.z - vi.z, v1.z - vi.z);
+    a[0] = fma2(vx, r.wx, a[0]);
+    a[1] = fma2(vy, r.wx, a[1]);
+    a[2] = fma2(vz, r.wx, a[2]);
+    a[3] = fma2(vx, r.wy, a[3]);
+    a[4] = fma2(vy, r.wy, a[4]);
+    a[5] = fma2(vz, r.wy, a[5]);
+    a[6] = fma2(vx, r.wz, a[6]);
+    a[7] = fma2(vy, r.wz, a[7]);
+    a[8] = fma2(vz, r.wz, a[8]);
+  }
+  // the sum over the slot's lanes, with the factor c
+  template <int G>
+  __device__ __forceinline__ M3 total(float c) const {
+    M3 m;
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      m.c[k] = v3(__fmul_rn(laneSum<G>(__fadd_rn(lo2(a[3 * k]), hi2(a[3 * k]))), c),
+                  __fmul_rn(laneSum<G>(__fadd_rn(lo2(a[3 * k + 1]), hi2(a[3 * k + 1]))), c),
+                  __fmul_rn(laneSum<G>(__fadd_rn(lo2(a[3 * k + 2]), hi2(a[3 * k + 2]))), c));
+    return m;
+  }
+};
 
 // ---------------------------------------------------------------- computeL
 // L of slot i (simkernels.js:198-220) over its recorded neighbours: the
-// SVD pseudo-inverse of sum V_b (grad W_b) (x_b - x_i)^T. For a solid
-// (kSolid) the same sweep also forms the sums of the constraint passes that
-// no velocity enters — s = sum V_b g_b, P = sum (V_b^2 / m_b) g_b g_b^T and
-// the solid neighbour count, over the solid neighbours in list order — and
-// stores them in sgP for every iteration of the substep. With kVel (a solid,
-// at the velocities iteration 0 starts from) the sweep also forms that
-// iteration's velocity sum Av = sum V_b (v_b - v_i) g_b^T over the solid
-// neighbours in list order — the constraint sweep's own expression — and
-// hands the sums and L to the caller.
-struct SweepSums {
-  M3 Av, L;
-  V3 sg;
-  float p00, p11, p22, p01, p02, p12, cnt;
-};
+// SVD pseudo-inverse of sum V_b (grad W_b) (x_b - x_i)^T, which is symmetric
+// (the gradient points along the offset). For a solid (kSolid) the same sweep
+// also forms the sums of the constraint passes that no velocity enters —
+// s = sum V_b g_b, P = sum (V_b^2 / m_b) g_b g_b^T and the solid neighbour
+// count, over the solid neighbours — and stores them in sgP for every
+// iteration of the substep. With kVel (a solid, at the velocities iteration 0
+// starts from) the sweep also forms that iteration's velocity sum
+// Av = sum V_b (v_b - v_i) g_b^T — the constraint sweep's own operations.
 template <bool kSolid, bool kVel = false>
-__device__ __forceinline__ void bonetLok(const Bufs& b, const Ctx& cx, uint32_t i, V3 xi, SweepSums* out = nullptr) {
+__device__ __forceinline__ void bonetLok(const Bufs& b, const Ctx& cx, uint32_t i, V3 xi, M3* velSum = nullptr) {
   static_assert(kSolid || !kVel, "the velocity sum is a solid's");
   const SceneDev& S = *cx.scene;
   const float4* __restrict__ posS = b.posS;
   const float4* __restrict__ velIn = b.velS[0];  // V^n (.w), which no pass changes; with kVel also v
-  M3 A = mzero(), Av = mzero();
-  V3 sg = splat(0.f);
   V3 vi = splat(0.f);
   if constexpr (kVel) vi = xyz(velIn[i]);
-  float p00 = 0.f, p11 = 0.f, p22 = 0.f, p01 = 0.f, p02 = 0.f, p12 = 0.f, cnt = 0.f;
-  forNbrs(b, cx, i, xi, [&](uint32_t j) { return PV{ldg(posS + j), ldg(velIn + j)}; },
-          [&](uint32_t, bool water, const PV& d) {
-            const V3 pb = xyz(d.p);
-            const V3 g = gradWFast(S, xi - pb);
-            const V3 r = pb - xi;
-            // A += V_b g r^T with every rounding explicit, so the two
-            // instances (with and without the sums below) form the same L
-            const float Vb0 = d.v.w;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-              A.c[c].x = __fmaf_rn(__fmul_rn(g.x, r[c]), Vb0, A.c[c].x);
-              A.c[c].y = __fmaf_rn(__fmul_rn(g.y, r[c]), Vb0, A.c[c].y);
-              A.c[c].z = __fmaf_rn(__fmul_rn(g.z, r[c]), Vb0, A.c[c].z);
-            }
-            if (kSolid && !water) {
-              if constexpr (kVel) addVelSum(Av, d.v, vi, g);
-              const float Vb = d.v.w;
-              sg = sg + g * Vb;
-              const float c = Vb * Vb / cx.mats[matOfW(d.p.w)].mass;
-              const V3 cg = g * c;
-              p00 += cg.x * g.x;
-              p11 += cg.y * g.y;
-              p22 += cg.z * g.z;
-              p01 += cg.x * g.y;
-              p02 += cg.x * g.z;
-              p12 += cg.y * g.z;
-              cnt += 1.f;
-            }
-          });
+  VelSum Av;
+  // sum w dx^T (symmetric) over every neighbour; s and P / c^2 over the solid ones
+  F2 a00 = 0ull, a11 = 0ull, a22 = 0ull, a01 = 0ull, a02 = 0ull, a12 = 0ull;
+  F2 sx = 0ull, sy = 0ull, sz = 0ull;
+  F2 p00 = 0ull, p11 = 0ull, p22 = 0ull, p01 = 0ull, p02 = 0ull, p12 = 0ull;
+  float cnt = 0.f;
+  auto gather = [&](uint32_t j) { return PV{ldg(posS + j), ldg(velIn + j)}; };
+  auto addA = [&](const Pair& r) {
+    a00 = fma2(r.wx, r.dx, a00);
+    a11 = fma2(r.wy, r.dy, a11);
+    a22 = fma2(r.wz, r.dz, a22);
+    a01 = fma2(r.wx, r.dy, a01);
+    a02 = fma2(r.wx, r.dz, a02);
+    a12 = fma2(r.wy, r.dz, a12);
+  };
+  forSame<1, L_AHEAD>(b, cx, i, xi, !kSolid, 0u, gather, [&](uint32_t j0, uint32_t j1, const PV& d0, const PV& d1) {
+    const Pair r = pairOf(S, xi, d0, d1);
+    addA(r);
+    if constexpr (kSolid) {
+      if constexpr (kVel) Av.add(r, vi, d0.v, d1.v);
+      sx = add2(sx, r.wx);
+      sy = add2(sy, r.wy);
+      sz = add2(sz, r.wz);
+      const F2 m = f2(cx.mats[matOfW(d0.p.w)].invMass, cx.mats[matOfW(d1.p.w)].invMass);
+      const F2 ux = mul2(r.wx, m), uy = mul2(r.wy, m), uz = mul2(r.wz, m);
+      p00 = fma2(ux, r.wx, p00);
+      p11 = fma2(uy, r.wy, p11);
+      p22 = fma2(uz, r.wz, p22);
+      p01 = fma2(ux, r.wy, p01);
+      p02 = fma2(ux, r.wz, p02);
+      p12 = fma2(uy, r.wz, p12);
+      cnt += (j0 != i ? 1.f : 0.f) + (j1 != i ? 1.f : 0.f);
+    }
+  });
+  // the other phase's neighbours enter L alone
+  const uint32_t c = b.nbrCount[i];
+  if (c != kNbrOverflow) {
+    const uint32_t other = (otherCount(c) + 3u) >> 2;
+    if (other)
+      forPairs(nbrGroups(b.nbr, i) + kGroupStride * (kNbrCap / 4u - other), other, gather,
+               [&](uint32_t, uint32_t, const PV& d0, const PV& d1) { addA(pairOf(S, xi, d0, d1)); });
+  } else {
+    const PV self = gather(i);
+    forRows(S, b.cellStart, xi, [&](uint32_t beg, uint32_t end) {
+#pragma unroll 1
+      for (uint32_t j = beg; j < end; ++j) {
+        if (j == i) continue;
+        const float4 pj = ldg(posS + j);
+        const V3 d = xi - xyz(pj);
+        if (dot(d, d) < S.support2 && waterW(pj.w) == kSolid) addA(pairOf(S, xi, gather(j), self));
+      }
+    });
+  }
+  const float gc = S.gradC;
+  const V3 sg = v3(sum2(sx) * gc, sum2(sy) * gc, sum2(sz) * gc);
+  const float c2 = gc * gc;
+  const float q00 = sum2(p00) * c2, q11 = sum2(p11) * c2, q22 = sum2(p22) * c2;
+  const float q01 = sum2(p01) * c2, q02 = sum2(p02) * c2, q12 = sum2(p12) * c2;
   if constexpr (kSolid) {
     float4* __restrict__ R = b.sgP + i;
     const size_t N = b.N;
     R[0] = make_float4(sg.x, sg.y, sg.z, cnt);
-    R[N] = make_float4(p00, p11, p22, p01);
-    R[2 * N] = make_float4(p02, p12, 0.f, 0.f);
+    R[N] = make_float4(q00, q11, q22, q01);
+    R[2 * N] = make_float4(q02, q12, 0.f, 0.f);
   }
+  // x_b - x_i = -(dx, dy, dz)
+  const float b01 = -gc * sum2(a01), b02 = -gc * sum2(a02), b12 = -gc * sum2(a12);
+  const M3 A = {{v3(-gc * sum2(a00), b01, b02), v3(b01, -gc * sum2(a11), b12), v3(b02, b12, -gc * sum2(a22))}};
   const SVD s = svd3Fast(A);
   const float tol = 0.2f;
   V3 inv = splat(0.f);
@@ -413,7 +587,7 @@ __device__ __forceinline__ void bonetLok(const Bufs& b, const Ctx& cx, uint32_t 
   if (fabsf(s.sig.z) > tol) inv.z = __frcp_rn(s.sig.z);
   const M3 L = diagMul(s.V, inv, s.U);
   storeM(b.L, b.N, i, L);
-  if constexpr (kVel) *out = SweepSums{Av, L, sg, p00, p11, p22, p01, p02, p12, cnt};
+  if constexpr (kVel) *velSum = Av.total<1>(gc);
 }
 // The water particles' L of the last substep, from the same positions,
 // neighbour lists and V^n as k_computeL would have used.
@@ -441,28 +615,16 @@ __device__ __forceinline__ void storeSp(const Bufs& b, uint32_t i, const M3& m, 
   b.SpSelf[i] = make_float4(self.x, self.y, self.z, 0.f);
 }
 
-// Solid neighbours only: water entries are skipped before their data loads.
-struct SolidOnly {
-  __device__ __forceinline__ bool operator()(uint32_t e) const { return (e & kWaterBit) == 0u; }
-};
-
-// velocityGradient (simkernels.js:224-245) over the neighbour list.
+// velocityGradient (simkernels.js:224-245) of a solid over its solid neighbours.
 __device__ __forceinline__ M3 velocityGradient(const Bufs& b, const Ctx& cx, uint32_t i, V3 xi, V3 vi,
                                                const float4* __restrict__ velIn) {
   const SceneDev& S = *cx.scene;
   const float4* __restrict__ posS = b.posS;
   // sum dv_b (L g_b)^T = (sum dv_b g_b^T) L^T: L applied once, after the loop
-  M3 A = mzero();
-  forNbrs(
-      b, cx, i, xi, [&](uint32_t j) { return PV{ldg(posS + j), ldg(velIn + j)}; },
-      [&](uint32_t, bool water, const PV& d) {
-        if (water) return;
-        const V3 g = gradWFast(S, xi - xyz(d.p));
-        const V3 dv = (xyz(d.v) - vi) * d.v.w;
-        A = madd(A, M3{{dv * g.x, dv * g.y, dv * g.z}});
-      },
-      SolidOnly{});
-  return mul(A, transpose(loadM(b.L, b.N, i)));
+  VelSum A;
+  forSame<1>(b, cx, i, xi, false, 0u, [&](uint32_t j) { return PV{ldg(posS + j), ldg(velIn + j)}; },
+             [&](uint32_t, uint32_t, const PV& d0, const PV& d1) { A.add(pairOf(S, xi, d0, d1), vi, d0.v, d1.v); });
+  return mul(A.total<1>(S.gradC), transpose(loadM(b.L, b.N, i)));
 }
 
 // ---------------------------------------------------------------- solveA
@@ -494,107 +656,60 @@ struct Constraint {
 // (Compiled once, not inlined: solveA and computeL with features run the
 // same instructions, so iteration 0's stored constraint is bit for bit the
 // one solveA would evaluate; inlined, the compiler fuses multiplies and adds
-// differently in each kernel.)
-__device__ __noinline__ Constraint constraintFromSums(const SceneDev& S, const M3& A, V3 sg, float p00, float p11,
-                                                     float p22, float p01, float p02, float p12, float cnt,
-                                                     const M3& Li, const M3& Fn, const MatDev& m, float st);
+// differently in each kernel. The slot's L, F and sums are loaded in here,
+// not handed over through the stack.)
+struct TailIn {
+  const float *L, *F;
+  const float4* sgP;
+  uint32_t N, i;
+};
+__device__ __noinline__ Constraint constraintTail(M3 A, TailIn in, const SceneDev* S, const MatDev* m, float st);
 
 template <int NL = 1>
 __device__ __forceinline__ Constraint evalConstraint(const Bufs& b, const Ctx& cx, uint32_t i, float4 pi,
-                                                     const float4* __restrict__ velIn, const MatDev& m, float st,
+                                                     const float4* __restrict__ velIn, const MatDev* m, float st,
                                                      uint32_t lane = 0) {
   const SceneDev& S = *cx.scene;
   const float4* __restrict__ posS = b.posS;
   const V3 xi = xyz(pi);
   const V3 vi = xyz(velIn[i]);
-  // The sums run over the raw kernel gradients g_b; the correction L is
+  // The sum runs over the raw kernel gradients g_b; the correction L is
   // applied once afterwards: with gt_b = L g_b,
   //   G = sum dv_b gt_b^T = A L^T,  s = L sum V_b g_b,  Q = L P L^T,
   // A = sum dv_b g_b^T, P = sum (V_b^2 / m_b) g_b g_b^T (same terms, the L
-  // products factored out of the pair loop).
-  M3 A = mzero();
-  V3 sg = splat(0.f);
-  float p00 = 0.f, p11 = 0.f, p22 = 0.f, p01 = 0.f, p02 = 0.f, p12 = 0.f, cnt = 0.f;
-  if constexpr (NL == 1) {
-    // s, P and the count do not depend on the velocities: computeL formed
-    // them in the same order, so the sweep only accumulates A
-    forNbrs(
-        b, cx, i, xi, [&](uint32_t j) { return PV{ldg(posS + j), ldg(velIn + j)}; },
-        [&](uint32_t, bool water, const PV& d) {
-          if (water) return;
-          addVelSum(A, d.v, vi, gradWFast(S, xi - xyz(d.p)));
-        },
-        SolidOnly{});
-    const float4* __restrict__ R = b.sgP + i;
-    const size_t N = b.N;
-    const float4 r0 = R[0], r1 = R[N], r2 = R[2 * N];
-    sg = xyz(r0);
-    cnt = r0.w;
-    p00 = r1.x;
-    p11 = r1.y;
-    p22 = r1.z;
-    p01 = r1.w;
-    p02 = r2.x;
-    p12 = r2.y;
-  } else {
-    forNbrsLanes<NL>(
-        b, cx, i, xi, lane, [&](uint32_t j) { return PV{ldg(posS + j), ldg(velIn + j)}; },
-        [&](uint32_t, bool water, const PV& d) {
-          if (water) return;
-          const V3 g = gradWFast(S, xi - xyz(d.p));
-          const float Vb = d.v.w;
-          addVelSum(A, d.v, vi, g);
-          sg = sg + g * Vb;
-          const float c = Vb * Vb / cx.mats[matOfW(d.p.w)].mass;
-          const V3 cg = g * c;
-          p00 += cg.x * g.x;
-          p11 += cg.y * g.y;
-          p22 += cg.z * g.z;
-          p01 += cg.x * g.y;
-          p02 += cg.x * g.z;
-          p12 += cg.y * g.z;
-          cnt += 1.f;
-        },
-        SolidOnly{});
-  }
-  if constexpr (NL > 1) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) A.c[c] = laneSum<NL>(A.c[c]);
-    sg = laneSum<NL>(sg);
-    p00 = laneSum<NL>(p00);
-    p11 = laneSum<NL>(p11);
-    p22 = laneSum<NL>(p22);
-    p01 = laneSum<NL>(p01);
-    p02 = laneSum<NL>(p02);
-    p12 = laneSum<NL>(p12);
-    cnt = laneSum<NL>(cnt);
-    if (lane != 0) return Constraint{};  // lane 0 finishes the slot
-  }
-  return constraintFromSums(S, A, sg, p00, p11, p22, p01, p02, p12, cnt, loadM(b.L, b.N, i), loadM(b.FS, b.N, i), m,
-                            st);
+  // products factored out of the pair loop). s, P and the count do not depend
+  // on the velocities: computeL formed them, so the sweep only accumulates A.
+  VelSum A;
+  forSame<NL, A_AHEAD>(b, cx, i, xi, false, lane, [&](uint32_t j) { return PV{ldg(posS + j), ldg(velIn + j)}; },
+              [&](uint32_t, uint32_t, const PV& d0, const PV& d1) { A.add(pairOf(S, xi, d0, d1), vi, d0.v, d1.v); });
+  const M3 At = A.template total<NL>(S.gradC);
+  if (NL > 1 && lane != 0) return Constraint{};  // lane 0 finishes the slot
+  return constraintTail(At, TailIn{b.L, b.FS, b.sgP, b.N, i}, cx.scene, m, st);
 }
 
-// The per-particle part of the constraint from the sweep's sums (A = sum dv
-// g^T, s = sum V g, P = sum (V^2/m) g g^T over the solid neighbours in list
-// order, their count), the slot's correction L and its F.
-__device__ __noinline__ Constraint constraintFromSums(const SceneDev& S, const M3& A, V3 sg, float p00, float p11,
-                                                     float p22, float p01, float p02, float p12, float cnt,
-                                                     const M3& Li, const M3& Fn, const MatDev& m, float st) {
-  const M3 LiT = transpose(Li);
-  const M3 G = mul(A, LiT);
-  const V3 sv = mul(Li, sg);
-  const M3 Qm = mul(mul(Li, M3{{v3(p00, p01, p02), v3(p01, p11, p12), v3(p02, p12, p22)}}), LiT);
-  const float q00 = Qm.c[0].x, q11 = Qm.c[1].y, q22 = Qm.c[2].z;
-  const float q01 = Qm.c[1].x, q02 = Qm.c[2].x, q12 = Qm.c[2].y;
-  Constraint out;
-  out.nNbr = cnt;
-  const M3 Ftr = mul(madd(mident(), mscale(G, S.dt)), Fn);
+// The per-particle part of the constraint from the sweep's sum A = sum dv g^T:
+// with s = sum V g and P = sum (V^2/m) g g^T over the solid neighbours
+// (computeL's sums), the slot's correction L and its F. With G = A L^T and
+// M = (dC/dF) F^nT, GL = M L gives every contraction directly:
+//   sgrad = -M L s = -GL s,  <M^T M, L P L^T> = <GL^T GL, P>,  <M, A L^T> = <GL, A>.
+__device__ __noinline__ Constraint constraintTail(M3 A, TailIn in, const SceneDev* Sp, const MatDev* mp, float st) {
+  const SceneDev& S = *Sp;
+  const MatDev& m = *mp;
+  const M3 Li = loadM(in.L, in.N, in.i), Fn = loadM(in.F, in.N, in.i);
+  const float4* __restrict__ R = in.sgP + in.i;
+  const float hard = hardening(m, st);
+  const float mu = m.mu * hard, lam = m.lam * hard;
+  const M3 Ftr = madd(Fn, mscale(mul(mul(A, transpose(Li)), Fn), S.dt));
   const SVD sd = svd3Fast(Ftr);
+  Constraint out;
   out.logSigTr = vlog(safeSig(sd.sig));
   float stOut;
-  const V3 sig = returnMap(sd.sig, m, st, S.dt, stOut);
-  const float psi = stvkPsi(sig, m.mu, m.lam);
-  out.C = sqrtf(fmaxf(2.f * psi, 0.f));
+  const Mapped mp2 = returnMap(sd.sig, out.logSigTr, m, mu, lam, st, S.dt, stOut);
+  const V3 e = mp2.e;
+  const float tr = e.x + e.y + e.z;
+  out.C = sqrtf(fmaxf(2.f * stvkPsi(e, mu, lam), 0.f));
+  const float4 r0 = R[0];
+  out.nNbr = r0.w;
   if (out.C < 1e-7f) {
     out.C = 0.f;
     out.denom = 0.f;
@@ -603,17 +718,19 @@ __device__ __noinline__ Constraint constraintFromSums(const SceneDev& S, const M
     out.sgrad = splat(0.f);
     return out;
   }
-  const V3 dpsi = stvkDPsi(sig, m.mu, m.lam);
-  const M3 Pk = diagMul(sd.U, dpsi * __frcp_rn(out.C), sd.V);
-  const M3 Mm = mul(Pk, transpose(Fn));
-  out.GL = mul(Mm, Li);
-  out.sgrad = -mul(Mm, sv);
-  // <M^T M, Q> = sum over column pairs (a, b) of (M_a . M_b) Q_ab
-  const V3 c0 = Mm.c[0], c1 = Mm.c[1], c2 = Mm.c[2];
-  const float denomN = dot(c0, c0) * q00 + dot(c1, c1) * q11 + dot(c2, c2) * q22 +
-                       2.f * (dot(c0, c1) * q01 + dot(c0, c2) * q02 + dot(c1, c2) * q12);
+  const V3 s = safeSig(mp2.sig);
+  const V3 dC = v3((2.f * mu * e.x + lam * tr) / (s.x * out.C), (2.f * mu * e.y + lam * tr) / (s.y * out.C),
+                   (2.f * mu * e.z + lam * tr) / (s.z * out.C));
+  const M3 Pk = diagMul(sd.U, dC, sd.V);
+  out.GL = mul(mul(Pk, transpose(Fn)), Li);
+  const float4 r1 = R[in.N], r2 = R[2 * (size_t)in.N];
+  out.sgrad = -mul(out.GL, xyz(r0));
+  // <GL^T GL, P> = sum over column pairs (a, b) of (GL_a . GL_b) P_ab
+  const V3 c0 = out.GL.c[0], c1 = out.GL.c[1], c2 = out.GL.c[2];
+  const float denomN = dot(c0, c0) * r1.x + dot(c1, c1) * r1.y + dot(c2, c2) * r1.z +
+                       2.f * (dot(c0, c1) * r1.w + dot(c0, c2) * r2.x + dot(c1, c2) * r2.y);
   out.denom = denomN + dot(out.sgrad, out.sgrad) / m.mass;
-  out.cdot = dot(Mm.c[0], G.c[0]) + dot(Mm.c[1], G.c[1]) + dot(Mm.c[2], G.c[2]);
+  out.cdot = dot(c0, A.c[0]) + dot(c1, A.c[1]) + dot(c2, A.c[2]);
   return out;
 }
 
@@ -702,22 +819,21 @@ __device__ __forceinline__ void countWarp(uint32_t* ctr) {
   if ((threadIdx.x & 31u) == (unsigned)(__ffs(m) - 1)) atomicAdd(ctr, (uint32_t)__popc(m));
 }
 
-// flag[j] = 1 for every solid neighbour j of slot i (list order; the stencil
-// walk for an overflowed list). Plain byte stores: concurrent writers store
-// the same value.
+// flag[j] = 1 for every solid neighbour j of the solid slot i. Plain byte
+// stores: concurrent writers store the same value.
 __device__ __forceinline__ void markSolidNbrs(const Bufs& b, const Ctx& cx, uint32_t i, V3 xi,
                                               uint8_t* __restrict__ flag) {
-  const uint32_t cnt = b.nbrCount[i];
-  if (cnt != kNbrOverflow) {
-    const uint4* __restrict__ L = reinterpret_cast<const uint4*>(listOf(b.nbr, i));
-    const uint32_t groups = (cnt + 3u) >> 2;
+  const uint32_t c = b.nbrCount[i];
+  if (c != kNbrOverflow) {
+    const uint4* L = nbrGroups(b.nbr, i);
+    const uint32_t cnt = sameCount(c);
 #pragma unroll 1
-    for (uint32_t q = 0; q < groups; ++q) {
-      const uint4 g = __ldg(L + q);
+    for (uint32_t q = 0; 4u * q < cnt; ++q) {
+      const uint4 g = *(L + kGroupStride * q);
 #pragma unroll
       for (uint32_t t = 0; t < 4u; ++t) {
         const uint32_t e = lane4(g, t);
-        if (4u * q + t < cnt && !(e & kWaterBit)) flag[e] = 1;
+        if (e != i) flag[e] = 1;
       }
     }
   } else {
@@ -859,8 +975,7 @@ __global__ void __launch_bounds__(kBlock, kMinB) k_solveA(Bufs b, int k, const f
   }
   const uint32_t mi = matOfW(pi.w);
   const float st = b.stateS[i];
-  const MatDev m = hardenedMat(cx.mats[mi], st);
-  const Constraint c = evalConstraint<G>(b, cx, i, pi, velIn, m, st, lane);
+  const Constraint c = evalConstraint<G>(b, cx, i, pi, velIn, cx.mats + mi, st, lane);
   if (G > 1 && lane != 0) return;
   solveAUpdate<kTrack>(b, cx, i, pi, velIn, mi, c, k, warm0, measure, act);
 }
@@ -946,8 +1061,7 @@ __global__ void __launch_bounds__(kBlock, kMinB) k_solveA_list(Bufs b, int k, co
     recordSolidDisp(b, i, k, S.dt * length(xyz(velIn[i])));
     const uint32_t mi = matOfW(pi.w);
     const float st = b.stateS[i];
-    const MatDev m = hardenedMat(cx.mats[mi], st);
-    const Constraint c = evalConstraint<1>(b, cx, i, pi, velIn, m, st, 0);
+    const Constraint c = evalConstraint<1>(b, cx, i, pi, velIn, cx.mats + mi, st, 0);
     solveAUpdate<true>(b, cx, i, pi, velIn, mi, c, k, false, false, true);
   }
   (void)flags;
@@ -987,7 +1101,7 @@ __global__ void __launch_bounds__(kThreads) k_solveA_stored(Bufs b, const float4
 //   8-14 material kind one-hot
 //   15   log10(mu) - 4.5
 __device__ __forceinline__ void fillFeatures(float (&f)[kFeat], const SceneDev& S, const Constraint& c, float lamPrev,
-                                             uint32_t kind, const MatDev& m) {
+                                             uint32_t kind, float mu) {
   const float aT = S.alphaT;
   f[0] = c.logSigTr.x;
   f[1] = c.logSigTr.y;
@@ -999,7 +1113,7 @@ __device__ __forceinline__ void fillFeatures(float (&f)[kFeat], const SceneDev& 
   f[7] = c.nNbr * (1.f / 32.f);
 #pragma unroll
   for (uint32_t q = 0; q < 7u; ++q) f[8 + q] = kind == q ? 1.f : 0.f;  // constant indices: f stays in registers
-  f[15] = log10f(fmaxf(m.mu, 1e-6f)) - 4.5f;
+  f[15] = log10f(fmaxf(mu, 1e-6f)) - 4.5f;
 }
 __device__ __forceinline__ void storeFeatures(const Bufs& b, uint32_t i, const float (&f)[kFeat]) {
   float4* out = reinterpret_cast<float4*>(b.feat + (size_t)i * kFeat);
@@ -1015,9 +1129,8 @@ __device__ __forceinline__ void storeFeatures(const Bufs& b, uint32_t i, const f
 // k_solveA_stored here, with the network's features (fillFeatures; zeros
 // for water and for scenes without iterations), without a second sweep of
 // every solid's neighbours.
-template <bool kSums, bool kFeatures>
+template <bool kFeatures>
 __device__ __forceinline__ void computeL(const Bufs& b) {
-  static_assert(kSums || !kFeatures, "the features need the sums");
   // blocks run last to first: the pass starts where the reorder ended, on
   // slots whose data is still in L2
   const uint32_t i = (gridDim.x - 1u - blockIdx.x) * blockDim.x + threadIdx.x;
@@ -1028,15 +1141,24 @@ __device__ __forceinline__ void computeL(const Bufs& b) {
   const float4 pi = posS[i];
   const V3 xi = xyz(pi);
   const float s2 = S.support2;
-  uint32_t cnt = 0;
-  uint32_t* __restrict__ out = listOf(b.nbr, i);
+  // own phase from the front, the other one from the back (the water flag is
+  // the sign bit of pos.w); a list past the capacity is marked as overflowed
+  // and never read, its last entries land anywhere in it
+  uint32_t same = 0, other = 0;
   walkCandidates(S, b.cellStart, xi, i, planesOf(b.posP, b.planeN), xi, s2, [&](uint32_t j) {
-    // past the capacity the last slot is overwritten: such a list is marked
-    // as overflowed and never read; the water flag is the sign bit of pos.w
-    out[min(cnt, kNbrCap - 1u)] = j | (__float_as_uint(ldg(&posS[j].w)) & kWaterBit);
-    ++cnt;
+    const bool own = ((__float_as_uint(ldg(&posS[j].w)) ^ __float_as_uint(pi.w)) & kWaterBit) == 0u;
+    const uint32_t e = own ? same : ~other;
+    *nbrEntry(b.nbr, i, e & (kNbrCap - 1u)) = j;
+    same += own ? 1u : 0u;
+    other += own ? 0u : 1u;
   });
-  b.nbrCount[i] = cnt <= kNbrCap ? cnt : kNbrOverflow;
+  const uint32_t same4 = (same + 3u) & ~3u, other4 = (other + 3u) & ~3u;
+  const bool fits = same4 + other4 <= kNbrCap;
+  if (fits) {
+    for (uint32_t e = same; e < same4; ++e) *nbrEntry(b.nbr, i, e) = i;
+    for (uint32_t e = other; e < other4; ++e) *nbrEntry(b.nbr, i, kNbrCap - 1u - e) = i;
+  }
+  b.nbrCount[i] = fits ? same | other << 8 : kNbrOverflow;
   // no pass of the substep reads a water particle's correction (every
   // velocity gradient is a solid's): k_computeL_water forms it when the state
   // is read
@@ -1045,28 +1167,24 @@ __device__ __forceinline__ void computeL(const Bufs& b) {
 #pragma unroll
     for (int q = 0; q < kFeat; ++q) f[q] = 0.f;
     if (!waterW(pi.w)) {
-      SweepSums w;
-      bonetLok<true, true>(b, cx, i, xi, &w);
+      M3 Av;
+      bonetLok<true, true>(b, cx, i, xi, &Av);
       if (S.iterations > 0) {
         const uint32_t mi = matOfW(pi.w);
         const float st = b.stateS[i];
-        const MatDev m = hardenedMat(cx.mats[mi], st);
-        const Constraint c = constraintFromSums(S, w.Av, w.sg, w.p00, w.p11, w.p22, w.p01, w.p02, w.p12, w.cnt, w.L,
-                                                loadM(b.FS, b.N, i), m, st);
+        const MatDev& m = cx.mats[mi];
+        const Constraint c = constraintTail(Av, TailIn{b.L, b.FS, b.sgP, b.N, i}, cx.scene, &m, st);
         storeConstraint(b, i, c);
-        fillFeatures(f, S, c, b.lamPrev[i], cx.mats[mi].kind, m);
+        fillFeatures(f, S, c, b.lamPrev[i], m.kind, m.mu * hardening(m, st));
       }
     }
     storeFeatures(b, i, f);
   } else {
-    if (!waterW(pi.w)) bonetLok<kSums>(b, cx, i, xi);
+    if (!waterW(pi.w)) bonetLok<true>(b, cx, i, xi);
   }
 }
-template <bool kSums>
-__global__ void XPBI_LB_COMPUTEL k_computeL(Bufs b) {
-  computeL<kSums, false>(b);
-}
-__global__ void XPBI_LB_COMPUTEL_FEATURES k_computeL_features(Bufs b) { computeL<true, true>(b); }
+__global__ void XPBI_LB_COMPUTEL k_computeL(Bufs b) { computeL<false>(b); }
+__global__ void XPBI_LB_COMPUTEL_FEATURES k_computeL_features(Bufs b) { computeL<true>(b); }
 
 // lambda_warm = previous multiplier + network output / alphaT (the network
 // predicts alphaT times the increment over the previous substep's multiplier)
@@ -1291,6 +1409,32 @@ __device__ __forceinline__ V3 applyBoundary(const SceneDev& S, V3 xcIn, V3 vIn, 
 struct SBData {
   float4 r0, r1, r2;  // a neighbour's dlam G L columns with its position in .w (the record's first planes)
 };
+__device__ __forceinline__ SBData gatherSp(const float4* __restrict__ R, size_t N) {
+  return SBData{ldg(R), ldg(R + N), ldg(R + 2 * N)};
+}
+
+// sum over the neighbours b of S_b g_b (S_b = dlam G L of b, the kernel
+// gradient at x_b - x_i without its factor c). Every rounding is explicit, so
+// that solveB and its active-set form add the same bits. add returns the
+// squared distance.
+struct ImpulseSum {
+  V3 dv = V3{0.f, 0.f, 0.f};
+  __device__ __forceinline__ float add(const SceneDev& S, V3 xi, const SBData& d) {
+    const float dx = __fsub_rn(d.r0.w, xi.x), dy = __fsub_rn(d.r1.w, xi.y), dz = __fsub_rn(d.r2.w, xi.z);
+    const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+    const float t = __fmaf_rn(sqrtFast(r2), -S.halfInvH, 1.f);
+    const float g = __fmul_rn(__fmul_rn(t, t), t);
+    const float wx = __fmul_rn(dx, g), wy = __fmul_rn(dy, g), wz = __fmul_rn(dz, g);
+    dv.x = __fmaf_rn(d.r0.x, wx, __fmaf_rn(d.r1.x, wy, __fmaf_rn(d.r2.x, wz, dv.x)));
+    dv.y = __fmaf_rn(d.r0.y, wx, __fmaf_rn(d.r1.y, wy, __fmaf_rn(d.r2.y, wz, dv.y)));
+    dv.z = __fmaf_rn(d.r0.z, wx, __fmaf_rn(d.r1.z, wy, __fmaf_rn(d.r2.z, wz, dv.z)));
+    return r2;
+  }
+  // k sum + self
+  __device__ __forceinline__ V3 total(float k, V3 self) const {
+    return v3(__fmaf_rn(dv.x, k, self.x), __fmaf_rn(dv.y, k, self.y), __fmaf_rn(dv.z, k, self.z));
+  }
+};
 
 // ---------------------------------------------------------------- solveB
 // Constraint dv gather + contact correction + boundaries (simkernels.js:315-366).
@@ -1334,7 +1478,6 @@ __global__ void __launch_bounds__(kBlock, kMinB) k_solveB(Bufs b, int k, const f
   V3 dv = splat(0.f), corr = splat(0.f);
   if (!waterW(pi.w)) {
     const size_t N = b.N;
-    if (G == 1) dv = xyz(b.SpSelf[i]);
     const float Vi = vi4.w;
     const V3 xci = xi + S.dt * xyz(vi4);
     const float minD = S.minD;
@@ -1350,14 +1493,11 @@ __global__ void __launch_bounds__(kBlock, kMinB) k_solveB(Bufs b, int k, const f
                          __uint_as_float(__ldg(b.solidDisp + (size_t)(k & 1) * b.S + (cx.scene - b.scenes)))) *
                         1.01f;
     const float reach2 = reach * reach;
-    auto body = [&](uint32_t j, bool water, const SBData& d) {
-      if (water) return;
-      const V3 pb = v3(d.r0.w, d.r1.w, d.r2.w);
-      const M3 Sb = {{xyz(d.r0), xyz(d.r1), xyz(d.r2)}};
-      const V3 dxp = pb - xi;
-      dv = dv + Vi * mul(Sb, gradWFast(S, dxp));
-      if (!(dot(dxp, dxp) < reach2)) return;
-      const float4 r3 = ldg(Sp + 3 * b.N + j);
+    ImpulseSum sum;
+    auto body = [&](uint32_t j, const SBData& d) {
+      const float r2 = sum.add(S, xi, d);
+      if (!(r2 < reach2) || j == i) return;
+      const float4 r3 = ldg(Sp + 3 * N + j);
       const V3 dxc = xci - xyz(r3);
       const float d2 = dot(dxc, dxc);
       if (d2 < minD * minD && d2 > 1e-18f) {
@@ -1368,57 +1508,14 @@ __global__ void __launch_bounds__(kBlock, kMinB) k_solveB(Bufs b, int k, const f
         corr = corr + dxc * (rinv * ((minD - dist) * w));
       }
     };
-    const uint32_t cnt = b.nbrCount[i];
-    if (G > 1 && cnt != kNbrOverflow) {
-      // lane `lane` takes the entries k % G == lane, skipping water ones
-      const uint4* __restrict__ L = reinterpret_cast<const uint4*>(listOf(b.nbr, i));
-      const uint32_t groups = (cnt + 3u) >> 2;
-#pragma unroll 1
-      for (uint32_t q = 0; q < groups; ++q) {
-        const uint4 grp = __ldg(L + q);
-#pragma unroll
-        for (uint32_t s = lane; s < 4u; s += G) {
-          const uint32_t e = lane4(grp, s);
-          if (4u * q + s < cnt && !(e & kWaterBit)) {
-            const float4* R = Sp + e;
-            body(e, false, SBData{ldg(R), ldg(R + N), ldg(R + 2 * N)});
-          }
-        }
-      }
-    } else if (G == 1 && cnt != kNbrOverflow) {
-      // water neighbours are skipped before their record is loaded
-      forList<true>(listOf(b.nbr, i), cnt,
-                    [&](uint32_t e) {
-                      SBData d;
-                      if (e & kWaterBit) {
-                        d.r0 = d.r1 = d.r2 = make_float4(0.f, 0.f, 0.f, 0.f);
-                      } else {
-                        const float4* R = Sp + e;
-                        d.r0 = ldg(R);
-                        d.r1 = ldg(R + N);
-                        d.r2 = ldg(R + 2 * N);
-                      }
-                      return d;
-                    },
-                    [&](uint32_t j, bool water, const SBData& d) { body(j, water, d); });
-    } else {
-      forRows(S, b.cellStart, xi, [&](uint32_t beg, uint32_t end) {
-#pragma unroll 1
-        for (uint32_t j = beg + lane; j < end; j += G) {
-          if (j == i) continue;
-          const float4 pj = ldg(posS + j);
-          const V3 d = xi - xyz(pj);
-          if (dot(d, d) < S.support2 && !waterW(pj.w)) {
-            const float4* R = Sp + j;
-            body(j, false, SBData{ldg(R), ldg(R + N), ldg(R + 2 * N)});
-          }
-        }
-      });
-    }
+    forSameSingles<G, EACH_AHEAD>(b, cx, i, xi, lane, [&](uint32_t j) { return gatherSp(Sp + j, N); }, body);
+    const V3 self = xyz(b.SpSelf[i]);
+    const float k = Vi * S.gradC;
     if constexpr (G > 1) {
-      dv = laneSum<G>(dv) + xyz(b.SpSelf[i]);
+      sum.dv = laneSum<G>(sum.dv);
       corr = laneSum<G>(corr);
     }
+    dv = sum.total(k, self);
   }
   if (G > 1 && lane != 0) return;
   if (track) b.rc[i] = dot(corr, corr);
@@ -1521,31 +1618,29 @@ __device__ __forceinline__ void solveBActiveSlot(const Bufs& b, int k, float4* _
         corr = corr + dxc * (rinv * ((minD - dist) * w));
       }
     };
+    ImpulseSum sum;
     auto visit = [&](uint32_t j) {
       const bool jImp = !skip || b.imp[j] == stamp;
       if (jImp) {
         const float4* R = Sp + j;
         const float4 r0 = ldg(R), r1 = ldg(R + N), r2 = ldg(R + 2 * N);
-        const V3 pb = v3(r0.w, r1.w, r2.w);
-        const M3 Sb = {{xyz(r0), xyz(r1), xyz(r2)}};
-        const V3 dxp = pb - xi;
-        dv = dv + Vi * mul(Sb, gradWFast(S, dxp));
-        if (changed && dot(dxp, dxp) < reach2) contact(ldg(Sp + 3 * N + j));
+        const float d2 = sum.add(S, xi, SBData{r0, r1, r2});
+        if (changed && d2 < reach2) contact(ldg(Sp + 3 * N + j));
       } else if (changed) {
         contact(ldg(Sp + 3 * N + j));
       }
     };
-    const uint32_t cnt = b.nbrCount[i];
-    if (cnt != kNbrOverflow) {
-      const uint4* __restrict__ L = reinterpret_cast<const uint4*>(listOf(b.nbr, i));
-      const uint32_t groups = (cnt + 3u) >> 2;
+    const uint32_t c = b.nbrCount[i];
+    if (c != kNbrOverflow) {
+      const uint4* L = nbrGroups(b.nbr, i);
+      const uint32_t cnt = sameCount(c);
 #pragma unroll 1
-      for (uint32_t q = 0; q < groups; ++q) {
-        const uint4 g = __ldg(L + q);
+      for (uint32_t q = 0; 4u * q < cnt; ++q) {
+        const uint4 g = *(L + kGroupStride * q);
 #pragma unroll
         for (uint32_t t = 0; t < 4u; ++t) {
           const uint32_t e = lane4(g, t);
-          if (4u * q + t < cnt && !(e & kWaterBit)) visit(e);
+          if (e != i) visit(e);
         }
       }
     } else {
@@ -1559,6 +1654,7 @@ __device__ __forceinline__ void solveBActiveSlot(const Bufs& b, int k, float4* _
         }
       });
     }
+    dv = sum.total(Vi * S.gradC, dv);
     if (changed) {
       const float c2 = dot(corr, corr);
       b.rc[i] = c2;
@@ -1669,13 +1765,16 @@ __global__ void XPBI_LB_PBF k_pbfA(Bufs b, int k, int flags) {
   // water pairs with everything, a solid with water only (the water flag is
   // the sign bit of xc.w, the sorted pos.w)
   uint32_t cnt = 0;
-  uint32_t* __restrict__ out = listOf(b.nbrP, i);
-  walkCandidates(S, b.cellStart, xyz(pi), i, planesOf(b.xcP, b.planeN), xci, s2, [&](uint32_t j) {
-    const uint32_t flag = __float_as_uint(ldg(&xcS[j].w)) & kWaterBit;
-    if (!iWater && flag == 0u) return;
-    out[min(cnt, kNbrCap - 1u)] = j | flag;
+  auto record = [&](uint32_t j) {
+    *nbrEntry(b.nbrP, i, min(cnt, kNbrCap - 1u)) = j;
     ++cnt;
-  });
+  };
+  if (iWater)
+    walkCandidates(S, b.cellStart, xyz(pi), i, planesOf(b.xcP, b.planeN), xci, s2, record);
+  else
+    walkCandidates(S, b.cellStart, xyz(pi), i, planesOf(b.xcP, b.planeN), xci, s2, [&](uint32_t j) {
+      if (waterW(ldg(&xcS[j].w))) record(j);
+    });
   const uint32_t stored = cnt <= kNbrCap ? cnt : kNbrOverflow;
   b.nbrPCount[i] = stored;
   if (!iWater) {
@@ -1689,7 +1788,7 @@ __global__ void XPBI_LB_PBF k_pbfA(Bufs b, int k, int flags) {
   float rho = m.mass * S.w00;
   V3 gradSum = splat(0.f);
   float grad2 = 0.f;
-  auto body = [&](uint32_t, bool, const float4& c) {
+  auto body = [&](const float4& c) {
     const V3 dxv = xci - xyz(c);
     const float r2 = dot(dxv, dxv);
     const float mb = cx.mats[matOfW(c.w)].mass;
@@ -1699,7 +1798,7 @@ __global__ void XPBI_LB_PBF k_pbfA(Bufs b, int k, int flags) {
     grad2 = grad2 + dot(g, g);
   };
   if (stored != kNbrOverflow) {
-    forList(listOf(b.nbrP, i), stored, [&](uint32_t j) { return ldg(xcS + j); }, body);
+    forEach(nbrGroups(b.nbrP, i), stored, [&](uint32_t j) { return ldg(xcS + j); }, body);
   } else {
     forRows(S, b.cellStart, xyz(pi), [&](uint32_t beg, uint32_t end) {
 #pragma unroll 1
@@ -1707,7 +1806,7 @@ __global__ void XPBI_LB_PBF k_pbfA(Bufs b, int k, int flags) {
         if (j == i) continue;
         const float4 c = ldg(xcS + j);
         const V3 d = xci - xyz(c);
-        if (dot(d, d) < s2) body(j, waterW(c.w), c);
+        if (dot(d, d) < s2) body(c);
       }
     });
   }
@@ -1755,8 +1854,8 @@ __global__ void XPBI_LB_PBF k_pbfB(Bufs b, int k, const float4* velIn, float4* v
     const float sCorr = -S.sCorrK * (x2 * x2);
     dp = dp + (li + lb + sCorr) * spikyGradFast(S, dxv, r2) * mpd;
   };
-  auto body = [&](uint32_t, bool jWater, const PBData& d) {
-    const MatDev& mw = jWater ? cx.mats[matOfW(d.c.w)] : mWi;  // a water material
+  auto body = [&](const PBData& d) {
+    const MatDev& mw = waterW(d.c.w) ? cx.mats[matOfW(d.c.w)] : mWi;  // a water material
     term(xyz(d.c), d.lb, mw.massPerDensity);
   };
   const uint32_t cnt = b.nbrPCount[i];
@@ -1764,10 +1863,10 @@ __global__ void XPBI_LB_PBF k_pbfB(Bufs b, int k, const float4* velIn, float4* v
     // one water material: every pair weighs by its mass / density, and one
     // gather of pbfA's record (predicted position, multiplier) serves a pair
     const float mpd = S.waterMpd;
-    forList(listOf(b.nbrP, i), cnt, [&](uint32_t j) { return ldg(b.pbfRec + j); },
-            [&](uint32_t, bool, const float4& r) { term(xyz(r), r.w, mpd); });
+    forEach(nbrGroups(b.nbrP, i), cnt, [&](uint32_t j) { return ldg(b.pbfRec + j); },
+            [&](const float4& r) { term(xyz(r), r.w, mpd); });
   } else if (cnt != kNbrOverflow) {
-    forList(listOf(b.nbrP, i), cnt, gather, body);
+    forEach(nbrGroups(b.nbrP, i), cnt, gather, body);
   } else {
     forRows(S, b.cellStart, xyz(pi), [&](uint32_t beg, uint32_t end) {
 #pragma unroll 1
@@ -1777,7 +1876,7 @@ __global__ void XPBI_LB_PBF k_pbfB(Bufs b, int k, const float4* velIn, float4* v
         const bool jWater = waterW(c.w);
         if (!(iWater || jWater)) continue;
         const V3 d = xci - xyz(c);
-        if (dot(d, d) < S.support2) body(j, jWater, gather(j));
+        if (dot(d, d) < S.support2) body(gather(j));
       }
     });
   }
@@ -1814,15 +1913,21 @@ __global__ void XPBI_LB_UPDATE k_xsph(Bufs b, const float4* __restrict__ velIn,
   const float4 vi4 = velIn[i];
   const V3 vi = xyz(vi4);
   const bool iWater = waterW(pi.w);
-  V3 acc = splat(0.f);
-  forNbrs(
-      b, cx, i, xi, [&](uint32_t j) { return PV{ldg(posS + j), ldg(velIn + j)}; },
-      [&](uint32_t, bool jWater, const PV& d) {
-        if (jWater != iWater) return;
-        const V3 dxv = xi - xyz(d.p);
-        acc = acc + d.v.w * (xyz(d.v) - vi) * kernelWFast(S, dot(dxv, dxv));
-      },
-      [iWater](uint32_t e) { return ((e & kWaterBit) != 0u) == iWater; });  // same phase only
+  // W = sigW t^4 (2 q + 1) with t = 1 - q / 2, so 2 q + 1 = 5 - 4 t
+  F2 ax = 0ull, ay = 0ull, az = 0ull;
+  forSame<1>(b, cx, i, xi, iWater, 0u, [&](uint32_t j) { return PV{ldg(posS + j), ldg(velIn + j)}; },
+             [&](uint32_t, uint32_t, const PV& d0, const PV& d1) {
+               const F2 dx = f2(xi.x - d0.p.x, xi.x - d1.p.x), dy = f2(xi.y - d0.p.y, xi.y - d1.p.y),
+                        dz = f2(xi.z - d0.p.z, xi.z - d1.p.z);
+               const F2 r2 = fma2(dz, dz, fma2(dy, dy, mul2(dx, dx)));
+               const F2 t = falloff2(S, r2);
+               const F2 t2 = mul2(t, t);
+               const F2 w = mul2(mul2(mul2(t2, t2), fma2(t, f2(-4.f, -4.f), f2(5.f, 5.f))), f2(d0.v.w, d1.v.w));
+               ax = fma2(w, f2(d0.v.x - vi.x, d1.v.x - vi.x), ax);
+               ay = fma2(w, f2(d0.v.y - vi.y, d1.v.y - vi.y), ay);
+               az = fma2(w, f2(d0.v.z - vi.z, d1.v.z - vi.z), az);
+             });
+  const V3 acc = v3(sum2(ax), sum2(ay), sum2(az)) * S.sigW;
   float c = S.xsphC;
   if (iWater) c = S.xsphC * 10.f;
   const V3 v = vi + c * acc;
@@ -1839,10 +1944,11 @@ __global__ void XPBI_LB_UPDATE k_xsph(Bufs b, const float4* __restrict__ velIn,
 // 4M-particle substep, the same bits).
 __device__ __noinline__ M3 plasticUpdate(const SceneDev& S, const M3& gradV, const M3& F0, const MatDev& m, float st,
                                          float& stOut) {
-  const M3 Ftr = mul(madd(mident(), mscale(gradV, S.dt)), F0);
+  const M3 Ftr = madd(F0, mscale(mul(gradV, F0), S.dt));
   const SVD sv = svd3Fast(Ftr);
-  const V3 sig = returnMap(sv.sig, m, st, S.dt, stOut);
-  return diagMul(sv.U, safeSig(sig), sv.V);
+  const float hard = hardening(m, st);
+  const Mapped mp = returnMap(sv.sig, vlog(safeSig(sv.sig)), m, m.mu * hard, m.lam * hard, st, S.dt, stOut);
+  return diagMul(sv.U, safeSig(mp.sig), sv.V);
 }
 __global__ void XPBI_LB_UPDATE k_updateF_integrate(Bufs b, const float4* __restrict__ velIn) {
   // blocks run last to first: the pass starts where xsph ended, on
@@ -1858,7 +1964,7 @@ __global__ void XPBI_LB_UPDATE k_updateF_integrate(Bufs b, const float4* __restr
   M3 Fn = loadM(b.FS, b.N, i);
   float stOut = st;
   if (!waterW(pi.w)) {
-    const MatDev m = hardenedMat(cx.mats[mi], st);
+    const MatDev& m = cx.mats[mi];
     const M3 gradV = velocityGradient(b, cx, i, xyz(pi), xyz(vi4), velIn);
     Fn = plasticUpdate(S, gradV, Fn, m, st, stOut);
   }
@@ -1944,13 +2050,11 @@ inline unsigned gridOf(uint32_t n, int block) { return (unsigned)((n + (uint32_t
 
 }  // namespace
 
-void launch_computeL(const Bufs& b, bool sums, bool features, cudaStream_t st) {
+void launch_computeL(const Bufs& b, bool features, cudaStream_t st) {
   if (features)
     k_computeL_features<<<grid(b.N), kThreads, 0, st>>>(b);
-  else if (sums)
-    k_computeL<true><<<grid(b.N), kThreads, 0, st>>>(b);
   else
-    k_computeL<false><<<grid(b.N), kThreads, 0, st>>>(b);
+    k_computeL<<<grid(b.N), kThreads, 0, st>>>(b);
 }
 void launch_computeL_water(const Bufs& b, cudaStream_t st) { k_computeL_water<<<grid(b.N), kThreads, 0, st>>>(b); }
 template <int V>

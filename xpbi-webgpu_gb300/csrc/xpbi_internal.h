@@ -74,6 +74,8 @@ struct SceneDev {
   float vmaxCFL;            // 0.45 support / dt           simkernels.js:535
   float dvCap;              // 0.2 support / dt            simkernels.js:361
   float invH;               // 1 / h
+  float gradC;              // -5 sigW / h^2: grad W = gradC (1 - r / 2h)^3 dx
+  float halfInvH;           // 1 / (2 h)
   float invW0;              // 1 / max(w0, 1e-12)          simkernels.js:466
   int iterations;           // XPBI Jacobi iterations this substep (an early-stopped solve's cap)
   int pbfIterations;        // PBF passes (first k iterations)
@@ -93,7 +95,7 @@ struct MatDev {
   float p0, p1, p2, p3;
   float boundFriction, mass;
   float massPerDensity;     // mass / density (host f32, the same IEEE quotient as on the device)
-  float pad;
+  float invMass;            // 1 / mass
 };
 
 // Device buffers of one handle. "Current" arrays hold the state between
@@ -128,10 +130,11 @@ struct Bufs {
   unsigned long long* tileStatus;  // [tiles] look-back descriptors (after the two words)
   uint32_t* bigList;               // [N/64 + 2] crowded cells (> 64 members)
   uint16_t* sceneOf;    // [N] scene of each particle slot (static)
-  uint32_t* nbr;        // [N][kNbrCap] in-support neighbours, stencil order: index | water << 31
-  uint32_t* nbrCount;   // [N] list length, kNbrOverflow if it did not fit
-  uint32_t* nbrP;       // [N][kNbrCap] predicted-position neighbours of the current PBF pass
-  uint32_t* nbrPCount;  // [N]
+  uint32_t* nbr;        // [ceil(N / 32)][kNbrCap / 4][32][4] in-support neighbours: own phase from the front in
+                        //   stencil order, the other phase from the back
+  uint32_t* nbrCount;   // [N] own-phase entries | other-phase entries << 8, kNbrOverflow if they did not fit
+  uint32_t* nbrP;       // the same layout: predicted-position neighbours of the current PBF pass
+  uint32_t* nbrPCount;  // [N] entries, kNbrOverflow if they did not fit
   float4* xc;           // [N] predicted positions x + dt v of the current PBF pass, w = pos.w
   float4* pbfRec;       // [N] the same predicted position with the pass's PBF multiplier in .w (written by pbfA)
   // solver instrumentation and warm start
@@ -189,9 +192,8 @@ void launch_warm_from_prev(const Bufs& b, cudaStream_t st);
 uint32_t scan_tiles(uint32_t cells);
 
 // ---- launchers (solve.cu) ----
-// sums: also form the solids' velocity-free constraint sums (sgP);
 // features: also iteration 0's constraint (cons0) and the network features
-void launch_computeL(const Bufs& b, bool sums, bool features, cudaStream_t st);
+void launch_computeL(const Bufs& b, bool features, cudaStream_t st);
 // the water particles' L of the last substep (computeL forms the solids' only)
 void launch_computeL_water(const Bufs& b, cudaStream_t st);
 void launch_solveA(const Bufs& b, int k, const float4* velIn, int flags, int variant, int lanes, cudaStream_t st);

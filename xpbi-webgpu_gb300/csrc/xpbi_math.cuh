@@ -105,57 +105,11 @@ __device__ __forceinline__ void storeM(float* __restrict__ P, uint32_t N, uint32
 }
 
 // ----------------------------------------------------------------- SPH kernels
-// Wendland C2, support 2h (common.js:63-79). sigW is the precomputed
-// 21/(16 pi h^3).
-__device__ __forceinline__ float kernelW(const SceneDev& S, float r) {
-  float q = r / S.h;
-  if (q >= 2.f) return 0.f;
-  float t = 1.f - 0.5f * q;
-  return S.sigW * t * t * t * t * (2.f * q + 1.f);
-}
-__device__ __forceinline__ V3 kernelGradW(const SceneDev& S, V3 dxv) {
-  float r = length(dxv);
-  float q = r / S.h;
-  if (q >= 2.f || r < 1e-9f) return splat(0.f);
-  float t = 1.f - 0.5f * q;
-  float dwdq = S.sigW * (-5.f * q) * t * t * t;
-  return dxv * (dwdq / (S.h * r));
-}
-// PBF kernels with H = support (common.js:81-94).
-__device__ __forceinline__ float kernelPoly6(const SceneDev& S, float r) {
-  float H = S.support;
-  if (r >= H) return 0.f;
-  float x = H * H - r * r;
-  return S.poly6C * x * x * x;
-}
-__device__ __forceinline__ V3 kernelSpikyGrad(const SceneDev& S, V3 dxv) {
-  float H = S.support;
-  float r = length(dxv);
-  if (r >= H || r < 1e-9f) return splat(0.f);
-  float t = H - r;
-  return dxv * (S.spikyC * t * t / r);
-}
-
-// Same kernels with the square root and the divisions by h and r replaced
-// by one reciprocal square root and multiplications by the precomputed 1/h:
-// a few ulp from the WGSL expressions, far below the parity tolerance.
-// r < 1e-9 (the reference's zero-distance guard) is r^2 < 1e-18.
-__device__ __forceinline__ V3 gradWFast(const SceneDev& S, V3 dxv) {
-  const float r2 = dot(dxv, dxv);
-  if (r2 < 1e-18f) return splat(0.f);
-  const float rinv = rsqrtf(r2);
-  const float q = r2 * rinv * S.invH;
-  if (q >= 2.f) return splat(0.f);
-  const float t = 1.f - 0.5f * q;
-  const float dwdq = S.sigW * (-5.f * q) * t * t * t;
-  return dxv * (dwdq * S.invH * rinv);
-}
-__device__ __forceinline__ float kernelWFast(const SceneDev& S, float r2) {
-  const float q = r2 > 0.f ? r2 * rsqrtf(r2) * S.invH : 0.f;
-  if (q >= 2.f) return 0.f;
-  const float t = 1.f - 0.5f * q;
-  return S.sigW * t * t * t * t * (2.f * q + 1.f);
-}
+// The Wendland C2 kernel and its gradient (support 2h, common.js:63-79) are
+// formed in the pair loops of solve.cu. PBF kernels with H = support
+// (common.js:81-94), with the square root and the division by r replaced by
+// one reciprocal square root; r < 1e-9 (the reference's zero-distance guard)
+// is r^2 < 1e-18.
 // poly6 from the squared distance: H^2 - r^2 with r^2 taken directly
 __device__ __forceinline__ float poly6Fast(const SceneDev& S, float r2) {
   if (r2 >= S.support2) return 0.f;
@@ -190,44 +144,6 @@ __device__ __forceinline__ uint32_t cellIndex(const SceneDev& S, int x, int y, i
 }
 
 // ----------------------------------------------------------------- svd3
-// Jacobi eigen-decomposition of F^T F, 6 sweeps (common.js:105-184).
-template <int p, int q>
-__device__ __forceinline__ void jacobiRot(M3& S, M3& V) {
-  float Spq = S.c[q][p];
-  float Spp = S.c[p][p];
-  float Sqq = S.c[q][q];
-  if (fabsf(Spq) < 1e-12f) return;
-  float tau = (Sqq - Spp) / (2.f * Spq);
-  float t;
-  if (tau >= 0.f) t = 1.f / (tau + sqrtf(1.f + tau * tau));
-  else t = 1.f / (tau - sqrtf(1.f + tau * tau));
-  float c = 1.f / sqrtf(1.f + t * t);
-  float s = t * c;
-  M3 Sn = S;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    float Skp = S.c[p][k], Skq = S.c[q][k];
-    Sn.c[p][k] = c * Skp - s * Skq;
-    Sn.c[q][k] = s * Skp + c * Skq;
-  }
-  M3 S2 = Sn;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    float Spk = Sn.c[k][p], Sqk = Sn.c[k][q];
-    S2.c[k][p] = c * Spk - s * Sqk;
-    S2.c[k][q] = s * Spk + c * Sqk;
-  }
-  S = S2;
-  M3 Vn = V;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    float Vkp = V.c[p][k], Vkq = V.c[q][k];
-    Vn.c[p][k] = c * Vkp - s * Vkq;
-    Vn.c[q][k] = s * Vkp + c * Vkq;
-  }
-  V = Vn;
-}
-
 struct SVD {
   M3 U;
   V3 sig;
@@ -237,99 +153,64 @@ struct SVD {
 __device__ __forceinline__ void swapf(float& a, float& b) { float t = a; a = b; b = t; }
 __device__ __forceinline__ void swapv(V3& a, V3& b) { V3 t = a; a = b; b = t; }
 
-__device__ __forceinline__ SVD svd3(const M3& F) {
-  M3 S = mul(transpose(F), F);
-  M3 V = mident();
-#pragma unroll 1
-  for (int sweep = 0; sweep < 6; ++sweep) {
-    jacobiRot<0, 1>(S, V);
-    jacobiRot<0, 2>(S, V);
-    jacobiRot<1, 2>(S, V);
-  }
-  V3 sig = v3(sqrtf(fmaxf(S.c[0].x, 0.f)), sqrtf(fmaxf(S.c[1].y, 0.f)), sqrtf(fmaxf(S.c[2].z, 0.f)));
-  V3 a0 = V.c[0], a1 = V.c[1], a2 = V.c[2];
-  if (sig.x < sig.y) { swapf(sig.x, sig.y); swapv(a0, a1); }
-  if (sig.x < sig.z) { swapf(sig.x, sig.z); swapv(a0, a2); }
-  if (sig.y < sig.z) { swapf(sig.y, sig.z); swapv(a1, a2); }
-  if (dot(cross(a0, a1), a2) < 0.f) a2 = -a2;
-  SVD out;
-  out.V = {{a0, a1, a2}};
-  V3 u0, u1;
-  const float eps = 1e-8f;
-  if (sig.x > eps) u0 = normalize(mul(F, a0));
-  else u0 = v3(1.f, 0.f, 0.f);
-  if (sig.y > eps) {
-    V3 Fv1 = mul(F, a1);
-    u1 = Fv1 - dot(Fv1, u0) * u0;
-    float l = length(u1);
-    if (l > eps) u1 = u1 / l;
-    else u1 = normalize(cross(v3(0.f, 1.f, 0.f), u0) + splat(1e-4f));
-  } else {
-    V3 a = cross(u0, v3(0.f, 1.f, 0.f));
-    if (length(a) < 1e-4f) a = cross(u0, v3(1.f, 0.f, 0.f));
-    u1 = normalize(a);
-  }
-  V3 u2 = cross(u0, u1);
-  if (det(F) < 0.f) sig.z = -sig.z;
-  out.U = {{u0, u1, u2}};
-  out.sig = sig;
-  return out;
-}
-
-// The same Jacobi sweeps with approximate reciprocal, reciprocal square
-// root and division (MUFU based). Rotation angles differ from the IEEE
-// version by a few ulp; the decomposition converges to the same U, sigma, V
-// to ~1e-6 and the products used downstream (U diag V^T) agree to rounding.
-template <int p, int q>
-__device__ __forceinline__ void jacobiRotFast(M3& S, M3& V) {
-  const float Spq = S.c[q][p];
-  const float Spp = S.c[p][p];
-  const float Sqq = S.c[q][q];
-  if (fabsf(Spq) < 1e-12f) return;
-  const float tau = __fdividef(Sqq - Spp, 2.f * Spq);
+// One Jacobi rotation of the symmetric S = [d0 d1 d2; off-diagonals], zeroing
+// the off-diagonal `apq` of the axes p, q (diagonals dp, dq; the other two
+// off-diagonals arp, arq), with V's columns vp, vq rotated along. The
+// diagonals change by t apq exactly, so only the two remaining off-diagonals
+// and V are rotated (a full two-sided product is twice the work). MUFU based:
+// the angle is off by a few ulp, which the rotation's own orthogonality to
+// rounding does not depend on.
+__device__ __forceinline__ void jacobiRotSym(float& dp, float& dq, float& apq, float& arp, float& arq, V3& vp,
+                                             V3& vq) {
+  if (fabsf(apq) < 1e-12f) return;
+  const float tau = __fdividef(dq - dp, 2.f * apq);
   const float h2 = 1.f + tau * tau;
   const float root = h2 * rsqrtf(h2);
   const float t = __fdividef(1.f, tau >= 0.f ? tau + root : tau - root);
   const float c = rsqrtf(1.f + t * t);
   const float s = t * c;
-  M3 Sn = S;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const float Skp = S.c[p][k], Skq = S.c[q][k];
-    Sn.c[p][k] = c * Skp - s * Skq;
-    Sn.c[q][k] = s * Skp + c * Skq;
-  }
-  M3 S2 = Sn;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const float Spk = Sn.c[k][p], Sqk = Sn.c[k][q];
-    S2.c[k][p] = c * Spk - s * Sqk;
-    S2.c[k][q] = s * Spk + c * Sqk;
-  }
-  S = S2;
-  M3 Vn = V;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const float Vkp = V.c[p][k], Vkq = V.c[q][k];
-    Vn.c[p][k] = c * Vkp - s * Vkq;
-    Vn.c[q][k] = s * Vkp + c * Vkq;
-  }
-  V = Vn;
+  dp -= t * apq;
+  dq += t * apq;
+  apq = 0.f;
+  const float x = arp, y = arq;
+  arp = c * x - s * y;
+  arq = s * x + c * y;
+  const V3 p = vp, q = vq;
+  vp = c * p - s * q;
+  vq = s * p + c * q;
 }
 
-__device__ __forceinline__ V3 normalizeFast(V3 a) { return a * rsqrtf(dot(a, a)); }
+// 1 / sqrt(d): the MUFU's value after one Newton step
+__device__ __forceinline__ float rsqrtNewton(float d) {
+  const float r = rsqrtf(d);
+  return r * fmaf(-0.5f * d * r, r, 1.5f);
+}
+__device__ __forceinline__ V3 normalizeFast(V3 a) { return a * rsqrtNewton(dot(a, a)); }
+// A vector whose length is 1 up to rounding, with the error's first order taken off
+__device__ __forceinline__ V3 renormalize(V3 a) { return a * fmaf(-0.5f, dot(a, a), 1.5f); }
 
+// SVD by Jacobi sweeps of F^T F (common.js:105-184, at most its six). The
+// sweeps end once every off-diagonal is below 4e-9 of the trace: a rotation
+// of what is left would change S = F^T F by less than a tenth of the rounding
+// its entries carry (6e-8 of the trace), and a warp of strained particles
+// gets there in three sweeps or four.
 __device__ __forceinline__ SVD svd3Fast(const M3& F) {
-  M3 S = mul(transpose(F), F);
-  M3 V = mident();
+  float s00 = dot(F.c[0], F.c[0]), s11 = dot(F.c[1], F.c[1]), s22 = dot(F.c[2], F.c[2]);
+  float s01 = dot(F.c[0], F.c[1]), s02 = dot(F.c[0], F.c[2]), s12 = dot(F.c[1], F.c[2]);
+  V3 a0 = v3(1.f, 0.f, 0.f), a1 = v3(0.f, 1.f, 0.f), a2 = v3(0.f, 0.f, 1.f);
+  const float small = 4e-9f * (s00 + s11 + s22);
 #pragma unroll 1
   for (int sweep = 0; sweep < 6; ++sweep) {
-    jacobiRotFast<0, 1>(S, V);
-    jacobiRotFast<0, 2>(S, V);
-    jacobiRotFast<1, 2>(S, V);
+    if (fmaxf(fmaxf(fabsf(s01), fabsf(s02)), fabsf(s12)) <= small) break;
+    jacobiRotSym(s00, s11, s01, s02, s12, a0, a1);
+    jacobiRotSym(s00, s22, s02, s01, s12, a0, a2);
+    jacobiRotSym(s11, s22, s12, s01, s02, a1, a2);
   }
-  V3 sig = v3(sqrtf(fmaxf(S.c[0].x, 0.f)), sqrtf(fmaxf(S.c[1].y, 0.f)), sqrtf(fmaxf(S.c[2].z, 0.f)));
-  V3 a0 = V.c[0], a1 = V.c[1], a2 = V.c[2];
+  // the approximate cosines leave V's columns a few ulp off length 1
+  a0 = renormalize(a0);
+  a1 = renormalize(a1);
+  a2 = renormalize(a2);
+  V3 sig = v3(sqrtf(fmaxf(s00, 0.f)), sqrtf(fmaxf(s11, 0.f)), sqrtf(fmaxf(s22, 0.f)));
   if (sig.x < sig.y) { swapf(sig.x, sig.y); swapv(a0, a1); }
   if (sig.x < sig.z) { swapf(sig.x, sig.z); swapv(a0, a2); }
   if (sig.y < sig.z) { swapf(sig.y, sig.z); swapv(a1, a2); }
@@ -344,7 +225,7 @@ __device__ __forceinline__ SVD svd3Fast(const M3& F) {
     const V3 Fv1 = mul(F, a1);
     u1 = Fv1 - dot(Fv1, u0) * u0;
     const float l2 = dot(u1, u1);
-    if (l2 > eps * eps) u1 = u1 * rsqrtf(l2);
+    if (l2 > eps * eps) u1 = u1 * rsqrtNewton(l2);
     else u1 = normalizeFast(cross(v3(0.f, 1.f, 0.f), u0) + splat(1e-4f));
   } else {
     V3 a = cross(u0, v3(0.f, 1.f, 0.f));
@@ -367,56 +248,62 @@ __device__ __forceinline__ M3 diagMul(const M3& U, V3 d, const M3& V) {
 // ----------------------------------------------------------------- StVK-Hencky
 // common.js:186-201
 __device__ __forceinline__ V3 safeSig(V3 s) { return vclamp(s, 1e-3f, 1e3f); }
-__device__ __forceinline__ float stvkPsi(V3 sig, float mu, float lam) {
-  V3 e = vlog(safeSig(sig));
+// energy from the logs e of the clamped singular values; its gradient is
+// (2 mu e + lam tr e) / safeSig(sig)
+__device__ __forceinline__ float stvkPsi(V3 e, float mu, float lam) {
   float tr = e.x + e.y + e.z;
   return mu * dot(e, e) + 0.5f * lam * tr * tr;
 }
-__device__ __forceinline__ V3 stvkDPsi(V3 sig, float mu, float lam) {
-  V3 s = safeSig(sig);
-  V3 e = vlog(s);
-  float tr = e.x + e.y + e.z;
-  return (2.f * mu * e + splat(lam * tr)) / s;
-}
 
 // ----------------------------------------------------------------- return maps
-// Drucker-Prager (common.js:205-221)
-__device__ __forceinline__ V3 rmDruckerPrager(V3 sig, const MatDev& m) {
+// A return map's result: the singular values and the logs of their clamped
+// values (safeSig), which the energy and its gradient take. The maps that work
+// on the logs (Drucker-Prager, von Mises) hand them on, not the rounded log of
+// a rounded exponential.
+struct Mapped {
+  V3 sig, e;
+};
+__device__ __forceinline__ Mapped mappedLog(V3 e) {
+  const V3 s = vexp(e);
+  // log(clamp(exp e)) = clamp(e): the bounds are the logs of safeSig's
+  return Mapped{s, vclamp(e, -6.90775528f, 6.90775528f)};
+}
+__device__ __forceinline__ Mapped mappedSig(V3 s) { return Mapped{s, vlog(safeSig(s))}; }
+// Drucker-Prager (common.js:205-221); e0 = log(safeSig(sig))
+__device__ __forceinline__ Mapped rmDruckerPrager(V3 sig, V3 e0, const MatDev& m, float mu, float lam) {
   float alpha = m.p0, coh = m.p1;
-  V3 e = vlog(safeSig(sig)) - splat(coh);
+  V3 e = e0 - splat(coh);
   float tr = e.x + e.y + e.z;
   V3 dev = e - splat(tr / 3.f);
   float dn = length(dev);
-  if (dn < 1e-9f || tr > 0.f) return vexp(splat(coh));
-  float dg = dn + alpha * (3.f * m.lam + 2.f * m.mu) / (2.f * m.mu) * tr;
-  if (dg <= 0.f) return sig;
+  if (dn < 1e-9f || tr > 0.f) return mappedLog(splat(coh));
+  float dg = dn + alpha * (3.f * lam + 2.f * mu) / (2.f * mu) * tr;
+  if (dg <= 0.f) return Mapped{sig, e0};
   V3 en = e - (dg / dn) * dev;
-  return vexp(en + splat(coh));
+  return mappedLog(en + splat(coh));
 }
 // Von Mises (common.js:223-234)
-__device__ __forceinline__ V3 rmVonMises(V3 sig, const MatDev& m) {
+__device__ __forceinline__ Mapped rmVonMises(V3 sig, V3 e, const MatDev& m, float mu) {
   float sigY = m.p0;
-  V3 e = vlog(safeSig(sig));
   float tr = e.x + e.y + e.z;
   V3 dev = e - splat(tr / 3.f);
   float dn = length(dev);
-  float dg = dn - sigY / (2.f * m.mu);
-  if (dg <= 0.f || dn < 1e-9f) return sig;
-  V3 en = e - (dg / dn) * dev;
-  return vexp(en);
+  float dg = dn - sigY / (2.f * mu);
+  if (dg <= 0.f || dn < 1e-9f) return Mapped{sig, e};
+  return mappedLog(e - (dg / dn) * dev);
 }
 // Herschel-Bulkley, b-bar-e form with bisection (common.js:236-280)
-__device__ __forceinline__ V3 rmHerschelBulkley(V3 sig, const MatDev& m, float dt) {
+__device__ __forceinline__ V3 rmHerschelBulkley(V3 sig, const MatDev& m, float mu, float dt) {
   float sigY = m.p0, hexp = m.p1, eta = m.p2;
   V3 s3 = safeSig(sig);
   float J = s3.x * s3.y * s3.z;
   V3 bbar = s3 * s3 * powf(J, (float)(-2.0 / 3.0));
   float trb = bbar.x + bbar.y + bbar.z;
   V3 devb = bbar - splat(trb / 3.f);
-  float sPre = m.mu * length(devb);
+  float sPre = mu * length(devb);
   float sY = (float)0.816496580927726 * sigY;  // sqrt(2/3)
   if (sPre <= sY || sPre < 1e-12f) return sig;
-  float muT = (trb / 3.f) * m.mu;
+  float muT = (trb / 3.f) * mu;
   float sNew;
   if (fabsf(hexp - 1.f) < 1e-3f || eta < 1e-9f) {
     sNew = sPre - (sPre - sY) / (1.f + eta / (2.f * muT * dt));
@@ -440,9 +327,9 @@ __device__ __forceinline__ V3 rmHerschelBulkley(V3 sig, const MatDev& m, float d
   return vsqrt(bNew) * powf(J, (float)(1.0 / 3.0));
 }
 // NACC, b^E form with fracture-friendly hardening (common.js:287-364)
-__device__ __forceinline__ V3 rmNACC(V3 sig, const MatDev& m, float alphaIn, float& alphaOut) {
-  float beta = m.p1, xi = m.p2, Mf = m.p3, mu = m.mu;
-  float kappa = (float)(2.0 / 3.0) * mu + m.lam;
+__device__ __forceinline__ V3 rmNACC(V3 sig, const MatDev& m, float mu, float lam, float alphaIn, float& alphaOut) {
+  float beta = m.p1, xi = m.p2, Mf = m.p3;
+  float kappa = (float)(2.0 / 3.0) * mu + lam;
   float alpha = alphaIn;
   V3 s3 = safeSig(sig);
   float Jtr = s3.x * s3.y * s3.z;
@@ -504,33 +391,29 @@ __device__ __forceinline__ V3 rmNACC(V3 sig, const MatDev& m, float alphaIn, flo
   alphaOut = alpha;
   return outSig;
 }
-// Snow hardening of mu, lambda (common.js:366-375)
-__device__ __forceinline__ MatDev hardenedMat(const MatDev& m, float state) {
-  MatDev mm = m;
-  if (m.kind == kKindSnow) {
-    float s = expf(fminf(m.p2 * (1.f - state), 5.f));
-    mm.mu = m.mu * s;
-    mm.lam = m.lam * s;
-  }
-  return mm;
+// Snow hardening of mu, lambda (common.js:366-375): the factor on both
+__device__ __forceinline__ float hardening(const MatDev& m, float state) {
+  return m.kind == kKindSnow ? expf(fminf(m.p2 * (1.f - state), 5.f)) : 1.f;
 }
-// Dispatch on the material kind (common.js:377-396)
-__device__ __forceinline__ V3 returnMap(V3 sig, const MatDev& m, float state, float dt, float& stateOut) {
+// Dispatch on the material kind (common.js:377-396) with the (hardened) mu,
+// lambda; e = log(safeSig(sig)).
+__device__ __forceinline__ Mapped returnMap(V3 sig, V3 e, const MatDev& m, float mu, float lam, float state, float dt,
+                                            float& stateOut) {
   stateOut = state;
   switch (m.kind) {
-    case 1u: return rmDruckerPrager(sig, m);
-    case 2u: return rmNACC(sig, m, state, stateOut);
-    case 3u: return rmVonMises(sig, m);
-    case 4u: return rmHerschelBulkley(sig, m, dt);
+    case 1u: return rmDruckerPrager(sig, e, m, mu, lam);
+    case 2u: return mappedSig(rmNACC(sig, m, mu, lam, state, stateOut));
+    case 3u: return rmVonMises(sig, e, m, mu);
+    case 4u: return mappedSig(rmHerschelBulkley(sig, m, mu, dt));
     case 5u: {
       V3 sNew = v3(clampf(sig.x, 1.f - m.p0, 1.f + m.p1), clampf(sig.y, 1.f - m.p0, 1.f + m.p1),
                    clampf(sig.z, 1.f - m.p0, 1.f + m.p1));
       float jOld = sig.x * sig.y * sig.z;
       float jNew = sNew.x * sNew.y * sNew.z;
       stateOut = clampf(state * jOld / fmaxf(jNew, 1e-6f), 0.2f, 2.f);
-      return sNew;
+      return mappedSig(sNew);
     }
-    default: return sig;
+    default: return Mapped{sig, e};
   }
 }
 
