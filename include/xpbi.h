@@ -289,9 +289,9 @@ int xpbi_set_solver(xpbi_sim* sim, int32_t mode, float rel_tol, float contact_re
  * applies a contact correction only above the same share of the contact
  * budget; a particle's velocity is updated only if it was re-evaluated or a
  * neighbour's impulse reaches it. A velocity change counts as a move if its
- * square exceeds share * rel_tol^2 times the mean squared velocity change of
- * iteration 0 (smaller ones shift a neighbour's residual by about its settle
- * threshold or less). Settled particles hold about `share` of each budget,
+ * square exceeds share * rel_tol^2 / 4 times the mean squared velocity change
+ * of iteration 0 (smaller ones shift a neighbour's residual by less than its
+ * settle threshold). Settled particles hold about `share` of each budget,
  * and the scene stops once the residual sums over all particles (the
  * settled ones with their last values) are within tolerance; with
  * track_residual the final state's residuals are re-measured over every

@@ -271,8 +271,8 @@ __device__ __forceinline__ void forPairsNow(const uint4* L, uint32_t groups, Gat
 }
 
 // Slot i's neighbours of its own phase, two at a time, over the recorded
-// list, or by the stencil walk if it overflowed (each neighbour then paired
-// with i itself).
+// list, or by the stencil walk if it overflowed (a last odd neighbour is
+// paired with i itself).
 //
 // Several lanes per slot (small scenes): the G lanes of slot i are
 // consecutive in the warp; lane `lane` visits the pairs p with p % G == lane
@@ -300,16 +300,23 @@ __device__ __forceinline__ void forSame(const Bufs& b, const Ctx& cx, uint32_t i
     }
   } else {
     const SceneDev& S = *cx.scene;
-    const auto self = gather(i);
+    uint32_t first = i;  // a neighbour waiting for its partner
     forRows(S, b.cellStart, xi, [&](uint32_t beg, uint32_t end) {
 #pragma unroll 1
       for (uint32_t j = beg + lane; j < end; j += G) {
         if (j == i) continue;
         const float4 pj = ldg(b.posS + j);
         const V3 d = xi - xyz(pj);
-        if (dot(d, d) < S.support2 && waterW(pj.w) == iWater) body(j, i, gather(j), self);
+        if (!(dot(d, d) < S.support2) || waterW(pj.w) != iWater) continue;
+        if (first == i) {
+          first = j;
+        } else {
+          body(first, j, gather(first), gather(j));
+          first = i;
+        }
       }
     });
+    if (first != i) body(first, i, gather(first), gather(i));
   }
 }
 
@@ -808,10 +815,10 @@ __device__ __forceinline__ void recordSolidDisp(const Bufs& b, uint32_t i, int k
 // the marking. The per-slot thresholds (formed once the
 // iteration-0 sums are known) give each settled slot an equal share of
 // asShare times the scene's residual budget, so settled slots alone can
-// never hold the scene above its tolerance. The velocity scale is the same
-// share of tol^2 times the mean squared velocity change of iteration 0: a
-// change below it moves a neighbour's residual by about that neighbour's
-// settle threshold or less, so the kept residuals are exact where nothing
+// never hold the scene above its tolerance. The velocity scale is a quarter
+// of that share of tol^2 times the mean squared velocity change of iteration
+// 0: a change below it moves a neighbour's residual by less than that
+// neighbour's settle threshold, so the kept residuals are exact where nothing
 // moved and otherwise off by at most that much (a tracked solve re-measures
 // the final state over every slot).
 __device__ __forceinline__ void countWarp(uint32_t* ctr) {
@@ -1354,10 +1361,12 @@ __global__ void __launch_bounds__(kResidThreads) k_resid(Bufs b, int k, int warm
     const double share = (double)S.asShare / (double)max(S.nSolid, 1u);
     b.thr[3 * s] = (float)(share * tol * tol * ta0);
     b.thr[3 * s + 1] = (float)(share * tolC * tolC * tac);
-    // a velocity change at the scale the converged solve still makes (the
-    // tolerance times iteration 0's) moves a neighbour's residual by about
-    // its own settle threshold: smaller ones do not count as moved
-    b.thr[3 * s + 2] = (float)(share * tol * tol * tav);
+    // a velocity change at half the scale the converged solve still makes
+    // (the tolerance times iteration 0's) moves a neighbour's residual by
+    // less than its own settle threshold: smaller ones do not count as moved.
+    // (At the whole scale, changes that add up over the iterations left one
+    // particle of a 50k dam breach stale by more than the tolerance.)
+    b.thr[3 * s + 2] = (float)(0.25 * share * tol * tol * tav);
   }
   if (tol > 0.0 && ta <= tol * tol * b.c0[s] && tac <= tolC * tolC * b.cc0[s] && !(warm && k == 0)) b.done[s] = 1;
   b.itersUsed[s] = k + 1;

@@ -153,31 +153,30 @@ struct SVD {
 __device__ __forceinline__ void swapf(float& a, float& b) { float t = a; a = b; b = t; }
 __device__ __forceinline__ void swapv(V3& a, V3& b) { V3 t = a; a = b; b = t; }
 
-// One Jacobi rotation of the symmetric S = [d0 d1 d2; off-diagonals], zeroing
-// the off-diagonal `apq` of the axes p, q (diagonals dp, dq; the other two
-// off-diagonals arp, arq), with V's columns vp, vq rotated along. The
-// diagonals change by t apq exactly, so only the two remaining off-diagonals
-// and V are rotated (a full two-sided product is twice the work). MUFU based:
-// the angle is off by a few ulp, which the rotation's own orthogonality to
-// rounding does not depend on.
-__device__ __forceinline__ void jacobiRotSym(float& dp, float& dq, float& apq, float& arp, float& arq, V3& vp,
-                                             V3& vq) {
-  if (fabsf(apq) < 1e-12f) return;
-  const float tau = __fdividef(dq - dp, 2.f * apq);
+// One Jacobi rotation of two columns bp, bq of F V (squared lengths np, nq)
+// that makes them orthogonal, V's columns vp, vq rotated along; nothing if
+// they are already, to rounding, or one is negligible against the other.
+// `more`: another sweep is needed (a sweep of angles below 2e-4 leaves
+// columns orthogonal to their square). MUFU based: the angle is off by a few
+// ulp.
+__device__ __forceinline__ void jacobiRot(V3& bp, V3& bq, float& np, float& nq, V3& vp, V3& vq, bool& more) {
+  const float g = dot(bp, bq);
+  if (g * g <= 1e-14f * (np * nq)) return;
+  const float tau = __fdividef(nq - np, 2.f * g);
+  if (!(fabsf(tau) < 1e9f)) return;
   const float h2 = 1.f + tau * tau;
   const float root = h2 * rsqrtf(h2);
   const float t = __fdividef(1.f, tau >= 0.f ? tau + root : tau - root);
+  more |= fabsf(t) > 2e-4f;
   const float c = rsqrtf(1.f + t * t);
   const float s = t * c;
-  dp -= t * apq;
-  dq += t * apq;
-  apq = 0.f;
-  const float x = arp, y = arq;
-  arp = c * x - s * y;
-  arq = s * x + c * y;
-  const V3 p = vp, q = vq;
-  vp = c * p - s * q;
-  vq = s * p + c * q;
+  np -= t * g;
+  nq += t * g;
+  const V3 b = bp, v = vp;
+  bp = c * b - s * bq;
+  bq = s * b + c * bq;
+  vp = c * v - s * vq;
+  vq = s * v + c * vq;
 }
 
 // 1 / sqrt(d): the MUFU's value after one Newton step
@@ -186,44 +185,53 @@ __device__ __forceinline__ float rsqrtNewton(float d) {
   return r * fmaf(-0.5f * d * r, r, 1.5f);
 }
 __device__ __forceinline__ V3 normalizeFast(V3 a) { return a * rsqrtNewton(dot(a, a)); }
-// A vector whose length is 1 up to rounding, with the error's first order taken off
-__device__ __forceinline__ V3 renormalize(V3 a) { return a * fmaf(-0.5f, dot(a, a), 1.5f); }
 
-// SVD by Jacobi sweeps of F^T F (common.js:105-184, at most its six). The
-// sweeps end once every off-diagonal is below 4e-9 of the trace: a rotation
-// of what is left would change S = F^T F by less than a tenth of the rounding
-// its entries carry (6e-8 of the trace), and a warp of strained particles
-// gets there in three sweeps or four.
+// SVD with the reference's conventions (common.js:105-184: sigma descending,
+// the last one negative if det F < 0, U and V rotations) by one-sided Jacobi
+// sweeps: the columns of F V are made orthogonal instead of diagonalising
+// F^T F, so the squared condition number of F never enters (a singular value
+// keeps its relative accuracy) and F V hands over U sigma. The sweeps, at most
+// the reference's six, end once their angles are small: three for a warp of
+// strained particles.
 __device__ __forceinline__ SVD svd3Fast(const M3& F) {
-  float s00 = dot(F.c[0], F.c[0]), s11 = dot(F.c[1], F.c[1]), s22 = dot(F.c[2], F.c[2]);
-  float s01 = dot(F.c[0], F.c[1]), s02 = dot(F.c[0], F.c[2]), s12 = dot(F.c[1], F.c[2]);
+  V3 b0 = F.c[0], b1 = F.c[1], b2 = F.c[2];
   V3 a0 = v3(1.f, 0.f, 0.f), a1 = v3(0.f, 1.f, 0.f), a2 = v3(0.f, 0.f, 1.f);
-  const float small = 4e-9f * (s00 + s11 + s22);
+  float n0 = dot(b0, b0), n1 = dot(b1, b1), n2 = dot(b2, b2);
 #pragma unroll 1
   for (int sweep = 0; sweep < 6; ++sweep) {
-    if (fmaxf(fmaxf(fabsf(s01), fabsf(s02)), fabsf(s12)) <= small) break;
-    jacobiRotSym(s00, s11, s01, s02, s12, a0, a1);
-    jacobiRotSym(s00, s22, s02, s01, s12, a0, a2);
-    jacobiRotSym(s11, s22, s12, s01, s02, a1, a2);
+    bool more = false;
+    jacobiRot(b0, b1, n0, n1, a0, a1, more);
+    jacobiRot(b0, b2, n0, n2, a0, a2, more);
+    jacobiRot(b1, b2, n1, n2, a1, a2, more);
+    if (!more) break;
   }
-  // the approximate cosines leave V's columns a few ulp off length 1
-  a0 = renormalize(a0);
-  a1 = renormalize(a1);
-  a2 = renormalize(a2);
-  V3 sig = v3(sqrtf(fmaxf(s00, 0.f)), sqrtf(fmaxf(s11, 0.f)), sqrtf(fmaxf(s22, 0.f)));
-  if (sig.x < sig.y) { swapf(sig.x, sig.y); swapv(a0, a1); }
-  if (sig.x < sig.z) { swapf(sig.x, sig.z); swapv(a0, a2); }
-  if (sig.y < sig.z) { swapf(sig.y, sig.z); swapv(a1, a2); }
-  if (dot(cross(a0, a1), a2) < 0.f) a2 = -a2;
+  // the approximate cosines leave V's columns, and F V's with them, a few ulp
+  // off length 1: the first order of that off both
+  const float k0 = fmaf(-0.5f, dot(a0, a0), 1.5f), k1 = fmaf(-0.5f, dot(a1, a1), 1.5f),
+              k2 = fmaf(-0.5f, dot(a2, a2), 1.5f);
+  a0 = a0 * k0;
+  a1 = a1 * k1;
+  a2 = a2 * k2;
+  b0 = b0 * k0;
+  b1 = b1 * k1;
+  b2 = b2 * k2;
+  V3 sig = v3(sqrtf(dot(b0, b0)), sqrtf(dot(b1, b1)), sqrtf(dot(b2, b2)));
+  if (sig.x < sig.y) { swapf(sig.x, sig.y); swapv(a0, a1); swapv(b0, b1); }
+  if (sig.x < sig.z) { swapf(sig.x, sig.z); swapv(a0, a2); swapv(b0, b2); }
+  if (sig.y < sig.z) { swapf(sig.y, sig.z); swapv(a1, a2); swapv(b1, b2); }
+  if (dot(cross(a0, a1), a2) < 0.f) {
+    a2 = -a2;
+    b2 = -b2;
+  }
+  if (dot(cross(b0, b1), b2) < 0.f) sig.z = -sig.z;  // det F (V is a rotation)
   SVD out;
   out.V = {{a0, a1, a2}};
   V3 u0, u1;
   const float eps = 1e-8f;
-  if (sig.x > eps) u0 = normalizeFast(mul(F, a0));
+  if (sig.x > eps) u0 = normalizeFast(b0);
   else u0 = v3(1.f, 0.f, 0.f);
   if (sig.y > eps) {
-    const V3 Fv1 = mul(F, a1);
-    u1 = Fv1 - dot(Fv1, u0) * u0;
+    u1 = b1 - dot(b1, u0) * u0;
     const float l2 = dot(u1, u1);
     if (l2 > eps * eps) u1 = u1 * rsqrtNewton(l2);
     else u1 = normalizeFast(cross(v3(0.f, 1.f, 0.f), u0) + splat(1e-4f));
@@ -233,7 +241,6 @@ __device__ __forceinline__ SVD svd3Fast(const M3& F) {
     u1 = normalizeFast(a);
   }
   const V3 u2 = cross(u0, u1);
-  if (det(F) < 0.f) sig.z = -sig.z;
   out.U = {{u0, u1, u2}};
   out.sig = sig;
   return out;
