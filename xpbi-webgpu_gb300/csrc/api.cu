@@ -252,13 +252,18 @@ void buildSceneDev(const SceneHost& s, uint32_t sceneIdx, SceneDev& d, MatDev* m
   // PBF pairs weight by the water particle's mass / density; with one water
   // material it is a scene constant
   d.waterMpd = 0.f;
-  int nWater = 0;
+  int nWater = 0, nOther = 0;
   for (uint32_t i = 0; i < s.nMats && i < (uint32_t)kMaxMats; ++i)
     if (md[i].kind == kKindWater) {
       ++nWater;
       d.waterMpd = md[i].massPerDensity;
+      d.massW = md[i].mass;
+    } else {
+      ++nOther;
+      d.massS = md[i].mass;
     }
   if (nWater != 1) d.waterMpd = 0.f;
+  d.twoMasses = nWater == 1 && nOther <= 1 ? 1 : 0;
 }
 
 int validateScene(const xpbi_scene_desc* d) {

@@ -168,9 +168,11 @@ __device__ __forceinline__ uint32_t* nbrEntry(uint32_t* base, uint32_t i, uint32
 __device__ __forceinline__ uint32_t lane4(const uint4& q, uint32_t s) {
   return s == 0u ? q.x : (s == 1u ? q.y : (s == 2u ? q.z : q.w));
 }
-// the count word: entries of the slot's own phase, of the other one
+// the count word: entries of the slot's own phase, of the other one, and for
+// a solid whether its 27 cells hold no water (never set on an overflow)
 __device__ __forceinline__ uint32_t sameCount(uint32_t c) { return c & 0xffu; }
-__device__ __forceinline__ uint32_t otherCount(uint32_t c) { return c >> 8; }
+__device__ __forceinline__ uint32_t otherCount(uint32_t c) { return (c >> 8) & 0xffu; }
+__device__ __forceinline__ bool dryCount(uint32_t c) { return (c >> 16) == 1u; }
 
 // Two neighbours at a time over `groups` groups: body(j0, j1, d0, d1) with
 // d = gather(j). The gathers of a pair are issued before the arithmetic of
@@ -235,26 +237,6 @@ __device__ __forceinline__ void forSingles(const uint4* L, uint32_t groups, Gath
     }
   }
 }
-template <class Gather, class Body>
-__device__ __forceinline__ void forEach(const uint4* L, uint32_t cnt, Gather&& gather, Body&& body) {
-  if (cnt == 0u) return;
-  uint4 cur = *(L);
-  uint4 nxt = cnt > 4u ? *(L + kGroupStride) : cur;
-  auto d = gather(cur.x);
-#pragma unroll 1
-  for (uint32_t k = 1; k < cnt; ++k) {
-    const uint32_t sl = k & 3u;
-    if (sl == 0u) {
-      cur = nxt;
-      if (k + 4u < cnt) nxt = *(L + kGroupStride * ((k >> 2) + 1u));
-    }
-    auto dn = gather(lane4(cur, sl));
-    body(d);
-    d = dn;
-  }
-  body(d);
-}
-
 // The same without gathers in flight over a pair's arithmetic (records of
 // many registers).
 template <class Gather, class Body>
@@ -1165,7 +1147,23 @@ __device__ __forceinline__ void computeL(const Bufs& b) {
     for (uint32_t e = same; e < same4; ++e) *nbrEntry(b.nbr, i, e) = i;
     for (uint32_t e = other; e < other4; ++e) *nbrEntry(b.nbr, i, kNbrCap - 1u - e) = i;
   }
-  b.nbrCount[i] = fits ? same | other << 8 : kNbrOverflow;
+  uint32_t dry = 0u;
+  if (S.hasWater && !waterW(pi.w) && fits) {  // for the PBF passes
+    const I3 cc = cellCoord(S, xi);
+    dry = 1u;
+#pragma unroll
+    for (int dz = -1; dz <= 1; ++dz)
+#pragma unroll
+      for (int dy = -1; dy <= 1; ++dy)
+#pragma unroll
+        for (int dx = -1; dx <= 1; ++dx) {
+          const int x = cc.x + dx, y = cc.y + dy, z = cc.z + dz;
+          if (x >= 0 && x < S.dims[0] && y >= 0 && y < S.dims[1] && z >= 0 && z < S.dims[2] &&
+              __ldg(b.cellWater + S.cellBase + cellIndex(S, x, y, z)) != 0)
+            dry = 0u;
+        }
+  }
+  b.nbrCount[i] = fits ? same | other << 8 | dry << 16 : kNbrOverflow;
   // no pass of the substep reads a water particle's correction (every
   // velocity gradient is a solid's): k_computeL_water forms it when the state
   // is read
@@ -1733,6 +1731,30 @@ __device__ __forceinline__ bool pbfActive(const SceneDev& S, int k) {
   return S.hasWater && k < S.pbfUntil;
 }
 
+// The PBF pair sums, two predicted neighbours per packed instruction: offset,
+// r^2, the poly6 argument x = H^2 - r^2 cubed, and the radial factor of the
+// spiky gradient, t^2 / r with t = H - r (0 below r = 1e-9, the reference's
+// zero-distance guard). The kernels' constants multiply the sums after the
+// loop.
+struct PbfPair {
+  F2 dx, dy, dz, x3, f;
+};
+__device__ __forceinline__ float invDist(float r2) { return r2 < 1e-18f ? 0.f : rsqrtf(r2); }
+__device__ __forceinline__ PbfPair pbfPair(const SceneDev& S, V3 c, const float4& p, const float4& q) {
+  PbfPair r;
+  r.dx = f2(c.x - p.x, c.x - q.x);
+  r.dy = f2(c.y - p.y, c.y - q.y);
+  r.dz = f2(c.z - p.z, c.z - q.z);
+  const F2 r2 = fma2(r.dz, r.dz, fma2(r.dy, r.dy, mul2(r.dx, r.dx)));
+  const F2 minus = f2(-1.f, -1.f);
+  const F2 x = fma2(r2, minus, f2(S.support2, S.support2));
+  r.x3 = mul2(mul2(x, x), x);
+  const F2 rinv = f2(invDist(lo2(r2)), invDist(hi2(r2)));
+  const F2 t = fma2(mul2(r2, rinv), minus, f2(S.support, S.support));
+  r.f = mul2(mul2(t, t), rinv);
+  return r;
+}
+
 // ---------------------------------------------------------------- pbfA
 // PBF density multiplier (simkernels.js:407-439). Walks the stencil around
 // the current cell with predicted positions and records, in order, the
@@ -1747,27 +1769,15 @@ __global__ void XPBI_LB_PBF k_pbfA(Bufs b, int k, int flags) {
   const float4* __restrict__ xcS = b.xc;
   const float4 pi = b.posS[i];
   const bool iWater = waterW(pi.w);
-  if (!iWater) {
-    // a solid only pairs with water here; candidates come from its 27 cells,
-    // so with no water particle in them there is nothing to record
-    const I3 cc = cellCoord(S, xyz(pi));
-    bool near = false;
-#pragma unroll
-    for (int dz = -1; dz <= 1; ++dz)
-#pragma unroll
-      for (int dy = -1; dy <= 1; ++dy)
-#pragma unroll
-        for (int dx = -1; dx <= 1; ++dx) {
-          const int x = cc.x + dx, y = cc.y + dy, z = cc.z + dz;
-          if (x >= 0 && x < S.dims[0] && y >= 0 && y < S.dims[1] && z >= 0 && z < S.dims[2])
-            near |= __ldg(b.cellWater + S.cellBase + cellIndex(S, x, y, z)) != 0;
-        }
-    if (!near) {
+  if (!iWater && dryCount(b.nbrCount[i])) {
+    // a solid only pairs with water here; its candidates come from its 27
+    // cells, and computeL found no water particle in them: nothing to record
+    // in any pass of the substep (no water particle pairs with it either)
+    if (k == 0) {
       b.nbrPCount[i] = 0u;
       b.pbfLam[i] = 0.f;
-      b.pbfRec[i] = make_float4(0.f, 0.f, 0.f, 0.f);  // no PBF pair reads it
-      return;
     }
+    return;
   }
   const V3 xci = xyz(xcS[i]);
   const float s2 = S.support2;
@@ -1785,6 +1795,8 @@ __global__ void XPBI_LB_PBF k_pbfA(Bufs b, int k, int flags) {
       if (waterW(ldg(&xcS[j].w))) record(j);
     });
   const uint32_t stored = cnt <= kNbrCap ? cnt : kNbrOverflow;
+  if (stored != kNbrOverflow)  // whole groups
+    for (uint32_t e = cnt; e & 3u; ++e) *nbrEntry(b.nbrP, i, e) = i;
   b.nbrPCount[i] = stored;
   if (!iWater) {
     b.pbfLam[i] = 0.f;
@@ -1794,20 +1806,34 @@ __global__ void XPBI_LB_PBF k_pbfA(Bufs b, int k, int flags) {
   const MatDev& m = cx.mats[matOfW(pi.w)];
   const float rho0 = m.density;
   const float invRho0 = __frcp_rn(rho0);
-  float rho = m.mass * S.w00;
-  V3 gradSum = splat(0.f);
-  float grad2 = 0.f;
-  auto body = [&](const float4& c) {
-    const V3 dxv = xci - xyz(c);
-    const float r2 = dot(dxv, dxv);
-    const float mb = cx.mats[matOfW(c.w)].mass;
-    rho = rho + mb * poly6Fast(S, r2);
-    const V3 g = spikyGradFast(S, dxv, r2) * (mb * invRho0);
-    gradSum = gradSum + g;
-    grad2 = grad2 + dot(g, g);
+  // sums of m_b x^3, m_b f dx and their squares; a padding entry (i itself)
+  // and, on the stencil walk, the second of each pair weigh 0
+  F2 rho = 0ull, gx = 0ull, gy = 0ull, gz = 0ull, g2 = 0ull;
+  auto add = [&](const float4& p, const float4& q, F2 mass) {
+    const PbfPair r = pbfPair(S, xci, p, q);
+    rho = fma2(r.x3, mass, rho);
+    const F2 f = mul2(r.f, mass);
+    const F2 ux = mul2(r.dx, f), uy = mul2(r.dy, f), uz = mul2(r.dz, f);
+    gx = add2(gx, ux);
+    gy = add2(gy, uy);
+    gz = add2(gz, uz);
+    g2 = fma2(ux, ux, fma2(uy, uy, fma2(uz, uz, g2)));
   };
+  auto massOf = [&](float w) { return cx.mats[matOfW(w)].mass; };
+  auto gather = [&](uint32_t j) { return ldg(xcS + j); };
   if (stored != kNbrOverflow) {
-    forEach(nbrGroups(b.nbrP, i), stored, [&](uint32_t j) { return ldg(xcS + j); }, body);
+    const uint4* L = nbrGroups(b.nbrP, i);
+    const uint32_t groups = (stored + 3u) >> 2;
+    if (S.twoMasses) {  // one water and at most one solid material: the sign of xc.w tells a neighbour's mass
+      const float mW = S.massW, mS = S.massS;
+      forPairsNow(L, groups, gather, [&](uint32_t j0, uint32_t j1, const float4& p, const float4& q) {
+        add(p, q, f2(j0 == i ? 0.f : (waterW(p.w) ? mW : mS), j1 == i ? 0.f : (waterW(q.w) ? mW : mS)));
+      });
+    } else {
+      forPairsNow(L, groups, gather, [&](uint32_t j0, uint32_t j1, const float4& p, const float4& q) {
+        add(p, q, f2(j0 == i ? 0.f : massOf(p.w), j1 == i ? 0.f : massOf(q.w)));
+      });
+    }
   } else {
     forRows(S, b.cellStart, xyz(pi), [&](uint32_t beg, uint32_t end) {
 #pragma unroll 1
@@ -1815,20 +1841,18 @@ __global__ void XPBI_LB_PBF k_pbfA(Bufs b, int k, int flags) {
         if (j == i) continue;
         const float4 c = ldg(xcS + j);
         const V3 d = xci - xyz(c);
-        if (dot(d, d) < s2) body(c);
+        if (dot(d, d) < s2) add(c, c, f2(massOf(c.w), 0.f));
       }
     });
   }
-  const float C = fmaxf(rho * invRho0 - 1.f, 0.f);
-  const float lam = -C / (grad2 + dot(gradSum, gradSum) + S.pbfEps);
+  const float k6 = S.poly6C, kg = S.spikyC * invRho0;
+  const V3 gradSum = v3(sum2(gx), sum2(gy), sum2(gz)) * kg;
+  const float dens = m.mass * S.w00 + k6 * sum2(rho);
+  const float C = fmaxf(dens * invRho0 - 1.f, 0.f);
+  const float lam = -C / (kg * kg * sum2(g2) + dot(gradSum, gradSum) + S.pbfEps);
   b.pbfLam[i] = lam;
   b.pbfRec[i] = make_float4(xci.x, xci.y, xci.z, lam);
 }
-
-struct PBData {
-  float4 c;
-  float lb;
-};
 
 // ---------------------------------------------------------------- pbfB
 // PBF position correction with s_corr (simkernels.js:441-477) over pbfA's
@@ -1841,54 +1865,57 @@ __global__ void XPBI_LB_PBF k_pbfB(Bufs b, int k, const float4* velIn, float4* v
   const Ctx cx = ctxOf(b, i);
   const SceneDev& S = *cx.scene;
   const float4 vi4 = velIn[i];
-  if (!pbfActive(S, k) || ((flags & kRerun) && !b.rerun[sceneIndex(b, cx)])) {
+  const uint32_t cnt = b.nbrPCount[i];
+  const float4 pi = b.posS[i];
+  const bool iWater = waterW(pi.w);
+  // no pass, or a solid without pairs: nothing moves it
+  if (!pbfActive(S, k) || ((flags & kRerun) && !b.rerun[sceneIndex(b, cx)]) || (cnt == 0u && !iWater)) {
     velOut[i] = vi4;
     return;
   }
   const float4* __restrict__ xcS = b.xc;
-  const float* __restrict__ lam = b.pbfLam;
-  const float4 pi = b.posS[i];
   const uint32_t mi = matOfW(pi.w);
   const V3 xci = xyz(xcS[i]);
-  V3 dp = splat(0.f);
-  const float li = lam[i];
-  const bool iWater = waterW(pi.w);
+  const float li = b.pbfLam[i];
   const MatDev& mWi = cx.mats[mi];
-  auto gather = [&](uint32_t j) { return PBData{ldg(xcS + j), ldg(lam + j)}; };
-  auto term = [&](V3 xcb, float lb, float mpd) {
-    const V3 dxv = xci - xcb;
-    const float r2 = dot(dxv, dxv);
-    const float x = poly6Fast(S, r2) * S.invW0;
-    const float x2 = x * x;
-    const float sCorr = -S.sCorrK * (x2 * x2);
-    dp = dp + (li + lb + sCorr) * spikyGradFast(S, dxv, r2) * mpd;
+  // sum of (lambda_i + lambda_b + s_corr) mpd_b f dx, s_corr = -k (W / W0)^4
+  F2 px = 0ull, py = 0ull, pz = 0ull;
+  const float rel = S.poly6C * S.invW0, nk = -S.sCorrK;
+  auto add = [&](const float4& p, const float4& q, F2 lb, F2 mpd) {
+    const PbfPair r = pbfPair(S, xci, p, q);
+    const F2 w = mul2(r.x3, f2(rel, rel));
+    const F2 w2 = mul2(w, w);
+    const F2 s = mul2(mul2(fma2(mul2(w2, w2), f2(nk, nk), add2(lb, f2(li, li))), r.f), mpd);
+    px = fma2(r.dx, s, px);
+    py = fma2(r.dy, s, py);
+    pz = fma2(r.dz, s, pz);
   };
-  auto body = [&](const PBData& d) {
-    const MatDev& mw = waterW(d.c.w) ? cx.mats[matOfW(d.c.w)] : mWi;  // a water material
-    term(xyz(d.c), d.lb, mw.massPerDensity);
-  };
-  const uint32_t cnt = b.nbrPCount[i];
+  // a pair weighs by its water particle's mass / density
+  auto mpdOf = [&](float w) { return waterW(w) ? cx.mats[matOfW(w)].massPerDensity : mWi.massPerDensity; };
   if (cnt != kNbrOverflow && S.waterMpd > 0.f) {
     // one water material: every pair weighs by its mass / density, and one
     // gather of pbfA's record (predicted position, multiplier) serves a pair
-    const float mpd = S.waterMpd;
-    forEach(nbrGroups(b.nbrP, i), cnt, [&](uint32_t j) { return ldg(b.pbfRec + j); },
-            [&](const float4& r) { term(xyz(r), r.w, mpd); });
+    const F2 mpd = f2(S.waterMpd, S.waterMpd);
+    forPairsNow(nbrGroups(b.nbrP, i), (cnt + 3u) >> 2, [&](uint32_t j) { return ldg(b.pbfRec + j); },
+                [&](uint32_t, uint32_t, const float4& p, const float4& q) { add(p, q, f2(p.w, q.w), mpd); });
   } else if (cnt != kNbrOverflow) {
-    forEach(nbrGroups(b.nbrP, i), cnt, gather, body);
+    forPairsNow(nbrGroups(b.nbrP, i), (cnt + 3u) >> 2, [&](uint32_t j) { return ldg(xcS + j); },
+                [&](uint32_t j0, uint32_t j1, const float4& p, const float4& q) {
+                  add(p, q, f2(ldg(b.pbfLam + j0), ldg(b.pbfLam + j1)), f2(mpdOf(p.w), mpdOf(q.w)));
+                });
   } else {
     forRows(S, b.cellStart, xyz(pi), [&](uint32_t beg, uint32_t end) {
 #pragma unroll 1
       for (uint32_t j = beg; j < end; ++j) {
         if (j == i) continue;
         const float4 c = ldg(xcS + j);
-        const bool jWater = waterW(c.w);
-        if (!(iWater || jWater)) continue;
+        if (!(iWater || waterW(c.w))) continue;
         const V3 d = xci - xyz(c);
-        if (dot(d, d) < S.support2) body(gather(j));
+        if (dot(d, d) < S.support2) add(c, c, f2(ldg(b.pbfLam + j), 0.f), f2(mpdOf(c.w), 0.f));
       }
     });
   }
+  const V3 dp = v3(sum2(px), sum2(py), sum2(pz)) * S.spikyC;
   const float scale = iWater ? 1.f : 0.5f;
   V3 v = xyz(vi4) + dp * (scale / S.dt);
   // active set: a water particle's boundary, which the next solveB would

@@ -85,6 +85,8 @@ struct SceneDev {
   float residTol;           // early stop at |r_k| <= residTol |C(v_pred)|; <= 0: never
   float residTolC;          // ... and |contact_k| <= residTolC |contact_0|
   float waterMpd;           // mass / density of the scene's one water material; 0: none or several
+  int twoMasses;            // one water and at most one solid material: their masses
+  float massW, massS;
   uint32_t nSolid;          // solid particles of the scene
   float asShare;            // active set: share of the residual budget settled particles may hold (0: off)
 };
