@@ -656,7 +656,7 @@ cudaError_t enqueueSubstep(xpbi_sim* s, const Schedule& sch, cudaStream_t st, Re
   launch_computeL(b, sch.features, st);
   R.mark(st, "computeL");
   if (sch.mode == 1) {
-    mlp_forward(b.feat, b.N, b.netBlob, b.netOut, nullptr, s->netErr, st, true);
+    mlp_forward(b.feat, b.N, b.netBlob, b.netOut, s->netErr, st, true);
     R.mark(st, "network");
     launch_warm_from_net(b, st);
     R.mark(st, "warmstart");
@@ -979,7 +979,7 @@ int createImpl(const xpbi_scene_desc* scenes, uint32_t nScenes, xpbi_sim** out) 
             cudaMemset(b.cellStart, 0, 4 * ((size_t)b.C + 4)) == cudaSuccess;
   if (!ok) return bail(fail(XPBI_ERR_CUDA, "initial upload failed"));
   // sets the network kernel's shared-memory attribute outside any capture
-  if (mlp_forward(nullptr, 0, nullptr, nullptr, nullptr, nullptr, s->stream) != cudaSuccess)
+  if (mlp_forward(nullptr, 0, nullptr, nullptr, nullptr, s->stream) != cudaSuccess)
     return bail(fail(XPBI_ERR_CUDA, "network kernel attribute"));
   rc = upload(s);
   if (rc != XPBI_OK) return bail(rc);

@@ -14,11 +14,12 @@ namespace xpbi {
 int mlp_param_count();
 size_t mlp_blob_bytes();
 void mlp_pack(const float* dParams, void* dBlob, cudaStream_t st);
-cudaError_t mlp_forward(const float* dX, uint32_t rows, const void* dBlob, float* dY, float* dZ, int* dErr,
-                        cudaStream_t st, bool skipZero);
-cudaError_t mlp_grad(const float* dX, const float* dT, uint32_t rows, const void* dBlob, float* dY, float* dZ,
-                     float* dPartial, float* dSq, float* dGrad, float* dLoss, int* dErr, cudaStream_t st);
-void mlp_adam(float* dW, const float* dG, float* dM, float* dV, float lr, int step, cudaStream_t st);
+size_t mlp_partial_floats(uint32_t rows);
+cudaError_t mlp_grad(const float* dX, const float* dT, uint32_t rows, const void* dBlob, float* dPartial, float* dSq,
+                     float* dGrad, float* dLoss, int* dErr, cudaStream_t st);
+cudaError_t mlp_train_step(const float* dX, const float* dT, uint32_t rows, float* dW, float* dM, float* dV,
+                           void* dBlob, float* dPartial, float* dSq, float* dLoss, float lr, int step, int* dErr,
+                           cudaStream_t st);
 int setError(int code, const std::string& msg);
 }  // namespace xpbi
 
@@ -75,7 +76,7 @@ int xpbi_mlp_forward(const float* X, uint32_t rows, const float* params, float* 
   MLP_CK(cudaMemcpy(dP, params, sizeof(float) * P, cudaMemcpyHostToDevice));
   MLP_CK(cudaMemset(dE, 0, sizeof(int)));
   mlp_pack(dP, dB, 0);
-  MLP_CK(mlp_forward(dX, rows, dB, dY, nullptr, dE, 0, false));
+  MLP_CK(mlp_forward(dX, rows, dB, dY, dE, 0, false));
   MLP_CK(cudaDeviceSynchronize());
   int rc = deviceErr(dE);
   if (rc) return rc;
@@ -93,21 +94,19 @@ int xpbi_mlp_grad(const float* X, const float* T, uint32_t rows, const float* pa
   float* dT = s.get<float>(rows);
   float* dP = s.get<float>(P);
   void* dB = s.get<uint8_t>(mlp_blob_bytes());
-  float* dY = s.get<float>(rows);
-  float* dZ = s.get<float>((size_t)rows * 64 * 3);
-  float* dPart = s.get<float>((size_t)tiles * P);
+  float* dPart = s.get<float>(mlp_partial_floats(rows));
   float* dSq = s.get<float>(tiles);
   float* dG = s.get<float>(P);
   float* dL = s.get<float>(1);
   int* dE = s.get<int>(1);
-  if (!dX || !dT || !dP || !dB || !dY || !dZ || !dPart || !dSq || !dG || !dL || !dE)
+  if (!dX || !dT || !dP || !dB || !dPart || !dSq || !dG || !dL || !dE)
     return setError(XPBI_ERR_OOM, "cudaMalloc failed");
   MLP_CK(cudaMemcpy(dX, X, sizeof(float) * rows * 16, cudaMemcpyHostToDevice));
   MLP_CK(cudaMemcpy(dT, T, sizeof(float) * rows, cudaMemcpyHostToDevice));
   MLP_CK(cudaMemcpy(dP, params, sizeof(float) * P, cudaMemcpyHostToDevice));
   MLP_CK(cudaMemset(dE, 0, sizeof(int)));
   mlp_pack(dP, dB, 0);
-  MLP_CK(mlp_grad(dX, dT, rows, dB, dY, dZ, dPart, dSq, dG, dL, dE, 0));
+  MLP_CK(mlp_grad(dX, dT, rows, dB, dPart, dSq, dG, dL, dE, 0));
   MLP_CK(cudaDeviceSynchronize());
   int rc = deviceErr(dE);
   if (rc) return rc;
@@ -133,14 +132,11 @@ int xpbi_mlp_train(const float* X, const float* T, uint32_t rows, float* params,
   float* dM = s.get<float>(P);
   float* dV = s.get<float>(P);
   void* dB = s.get<uint8_t>(mlp_blob_bytes());
-  float* dY = s.get<float>(batch);
-  float* dZ = s.get<float>((size_t)batch * 64 * 3);
-  float* dPart = s.get<float>((size_t)tiles * P);
+  float* dPart = s.get<float>(mlp_partial_floats(batch));
   float* dSq = s.get<float>(tiles);
-  float* dG = s.get<float>(P);
   float* dL = s.get<float>(steps > 0 ? steps : 1);
   int* dE = s.get<int>(1);
-  if (!dX || !dT || !dW || !dM || !dV || !dB || !dY || !dZ || !dPart || !dSq || !dG || !dL || !dE)
+  if (!dX || !dT || !dW || !dM || !dV || !dB || !dPart || !dSq || !dL || !dE)
     return setError(XPBI_ERR_OOM, "cudaMalloc failed");
   MLP_CK(cudaMemcpy(dX, X, sizeof(float) * rows * 16, cudaMemcpyHostToDevice));
   MLP_CK(cudaMemcpy(dT, T, sizeof(float) * rows, cudaMemcpyHostToDevice));
@@ -148,12 +144,12 @@ int xpbi_mlp_train(const float* X, const float* T, uint32_t rows, float* params,
   MLP_CK(cudaMemset(dM, 0, sizeof(float) * P));
   MLP_CK(cudaMemset(dV, 0, sizeof(float) * P));
   MLP_CK(cudaMemset(dE, 0, sizeof(int)));
+  mlp_pack(dW, dB, 0);
   uint32_t off = 0;
   for (int t = 0; t < steps; ++t) {
     if (off + batch > rows) off = 0;
-    mlp_pack(dW, dB, 0);
-    MLP_CK(mlp_grad(dX + (size_t)off * 16, dT + off, batch, dB, dY, dZ, dPart, dSq, dG, dL + t, dE, 0));
-    mlp_adam(dW, dG, dM, dV, lr, t + 1, 0);
+    MLP_CK(mlp_train_step(dX + (size_t)off * 16, dT + off, batch, dW, dM, dV, dB, dPart, dSq, dL + t, lr, t + 1, dE,
+                          0));
     off += batch;
   }
   MLP_CK(cudaDeviceSynchronize());

@@ -9,21 +9,20 @@
 // of the next layer's A tile. The 64 -> 1 output layer is a per-thread dot
 // product in FP32.
 //
-// Training (hand-written backward):
-//   forward stores the pre-activations z1..z3 (f32) and the output;
-//   backward forms dy = 2 (y - t) / B, dz3 = (dy w4) * silu'(z3), and the
-//   activation gradients dh2 = dz3 W3, dh1 = dz2 W2 on the tensor cores
-//   (A = bf16 dz, B = W^T tiles); weight gradients dW = dz^T h are FP32
-//   SIMT reductions over the CTA's rows into per-CTA partials, summed in a
-//   fixed order afterwards; Adam updates FP32 master weights, which are then
-//   repacked as BF16 tiles.
+// Training (hand-written backward), one kernel per step and tile of 128 rows:
+//   the forward pass keeps the activations and silu' on chip; backward forms
+//   dy = 2 (y - t) / B, dz3 = (dy w4) * silu'(z3), and the activation gradients
+//   dh2 = dz3 W3, dh1 = dz2 W2 on the tensor cores (A = bf16 dz, B = W^T
+//   tiles); weight gradients dW = dz^T h are FP32 sums over the CTA's rows into
+//   per-CTA partials. A second kernel adds the partials in a fixed order,
+//   applies Adam to the FP32 master weights and repacks them as BF16 tiles.
 //
 // Every mbarrier wait is bounded; on expiry the kernel raises an error bit,
 // stops issuing work and still releases its TMEM.
 #include <cuda_bf16.h>
 
 #include "tc.cuh"
-#include "xpbi_internal.h"
+#include "xpbi_math.cuh"
 
 namespace xpbi {
 
@@ -56,9 +55,9 @@ constexpr uint32_t sW3 = sW2 + kHid * kHid * 2;
 constexpr uint32_t sF32 = sW3 + kHid * kHid * 2;
 constexpr uint32_t kFwdSmem = sF32 + (4 * kHid + 4) * 4;
 
-// SiLU z * sigmoid(z) with the MUFU exponential and reciprocal (a few ulp)
+// The sigmoid with the MUFU exponential and reciprocal (a few ulp): training's
+// SiLU is z sigm(z), its derivative sigm(z) (1 + z (1 - sigm(z))).
 __device__ __forceinline__ float sigm(float z) { return __fdividef(1.f, 1.f + __expf(-z)); }
-__device__ __forceinline__ float silu(float z) { return z * sigm(z); }
 // SiLU for inference: z sigmoid(z) = h + h tanh(h) with h = z / 2 and the
 // MUFU tanh (one special-function op instead of an exponential and a
 // reciprocal). Its ~5e-4 relative error lies below the bf16 rounding every
@@ -72,49 +71,48 @@ __device__ __forceinline__ float siluFast(float z) {
   const float h = 0.5f * z;
   return fmaf(h, tanhMufu(h), h);
 }
-__device__ __forceinline__ float dsilu(float z) {
-  const float s = sigm(z);
-  return s * (1.f + z * (1.f - s));
-}
 
-// f32 params -> packed blob
-__global__ void k_mlp_pack(const float* __restrict__ p, uint8_t* __restrict__ blob) {
-  for (int t = threadIdx.x; t < kHid * kHid; t += blockDim.x) {
-    const int r = t / kHid, k = t % kHid;  // W[out=r][in=k]
-    *reinterpret_cast<__nv_bfloat16*>(blob + bW2 + tc::coreOffset(r, k, kHid)) = __float2bfloat16_rn(p[oW2 + t]);
-    *reinterpret_cast<__nv_bfloat16*>(blob + bW3 + tc::coreOffset(r, k, kHid)) = __float2bfloat16_rn(p[oW3 + t]);
-    // transposed tiles: row = in, col = out
-    *reinterpret_cast<__nv_bfloat16*>(blob + bW2T + tc::coreOffset(k, r, kHid)) = __float2bfloat16_rn(p[oW2 + t]);
-    *reinterpret_cast<__nv_bfloat16*>(blob + bW3T + tc::coreOffset(k, r, kHid)) = __float2bfloat16_rn(p[oW3 + t]);
-  }
-  for (int t = threadIdx.x; t < kHid * kIn; t += blockDim.x) {
-    const int r = t / kIn, k = t % kIn;
-    *reinterpret_cast<__nv_bfloat16*>(blob + bW1 + tc::coreOffset(r, k, kIn)) = __float2bfloat16_rn(p[oW1 + t]);
-  }
+// One f32 parameter into the packed blob.
+__device__ __forceinline__ void packParam(uint8_t* __restrict__ blob, int q, float v) {
+  auto tile = [&](uint32_t base, int r, int k, int K) {
+    *reinterpret_cast<__nv_bfloat16*>(blob + base + tc::coreOffset(r, k, K)) = __float2bfloat16_rn(v);
+  };
   float* f = reinterpret_cast<float*>(blob + bF32);
-  for (int t = threadIdx.x; t < kHid; t += blockDim.x) {
-    f[t] = p[oB1 + t];
-    f[kHid + t] = p[oB2 + t];
-    f[2 * kHid + t] = p[oB3 + t];
-    f[3 * kHid + t] = __bfloat162float(__float2bfloat16_rn(p[oW4 + t]));
+  if (q < oB1) {
+    tile(bW1, q / kIn, q % kIn, kIn);  // W[out][in]
+  } else if (q < oW2) {
+    f[q - oB1] = v;
+  } else if (q < oB2) {
+    const int t = q - oW2;
+    tile(bW2, t / kHid, t % kHid, kHid);
+    tile(bW2T, t % kHid, t / kHid, kHid);  // row = in, col = out
+  } else if (q < oW3) {
+    f[kHid + q - oB2] = v;
+  } else if (q < oB3) {
+    const int t = q - oW3;
+    tile(bW3, t / kHid, t % kHid, kHid);
+    tile(bW3T, t % kHid, t / kHid, kHid);
+  } else if (q < oW4) {
+    f[2 * kHid + q - oB3] = v;
+  } else if (q < oB4) {
+    f[3 * kHid + q - oW4] = __bfloat162float(__float2bfloat16_rn(v));
+  } else {
+    f[4 * kHid] = v;
   }
-  if (threadIdx.x == 0) f[4 * kHid] = p[oB4];
 }
-
-struct FwdOut {
-  float* y;        // [rows] network output
-  float* z;        // [3][rows][64] pre-activations (training) or null
-};
+__global__ void k_mlp_pack(const float* __restrict__ p, uint8_t* __restrict__ blob) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q < kParams) packParam(blob, q, p[q]);
+}
 
 // Forward over `rows` feature rows X[rows][16] (f32).
 __global__ void __launch_bounds__(kRows) k_mlp_fwd(const float* __restrict__ X, uint32_t rows,
-                                                   const uint8_t* __restrict__ blob, FwdOut out, int* err,
-                                                   int skipZero) {
+                                                   const uint8_t* __restrict__ blob, float* __restrict__ y_out,
+                                                   int* err, int skipZero) {
   extern __shared__ __align__(1024) uint8_t sm[];
   __shared__ __align__(8) uint64_t bar;
   __shared__ uint32_t tbase;
   const int tid = threadIdx.x, warp = tid >> 5;
-  const bool infer = out.z == nullptr;  // no pre-activations kept: inference
   // weights -> shared memory (straight copy of the packed tiles)
   {
     const uint4* src = reinterpret_cast<const uint4*>(blob);
@@ -168,7 +166,7 @@ __global__ void __launch_bounds__(kRows) k_mlp_fwd(const float* __restrict__ X, 
     // the solver's tiles of water particles (all-zero feature rows) need no
     // prediction: their output is defined as 0
     if (skipZero && !__syncthreads_or(active)) {
-      if (row < rows) out.y[row] = 0.f;
+      if (row < rows) y_out[row] = 0.f;
       continue;
     }
     float y = F[4 * kHid];
@@ -202,30 +200,22 @@ __global__ void __launch_bounds__(kRows) k_mlp_fwd(const float* __restrict__ X, 
         tc::ld16(tRow + 16 * c, z);
 #pragma unroll
         for (int j = 0; j < 16; ++j) z[j] += bias[16 * c + j];
-        if (out.z != nullptr && row < rows) {
-          float4* zr = reinterpret_cast<float4*>(out.z + ((size_t)layer * rows + row) * kHid + 16 * c);
-#pragma unroll
-          for (int q = 0; q < 4; ++q) zr[q] = make_float4(z[4 * q], z[4 * q + 1], z[4 * q + 2], z[4 * q + 3]);
-        }
         if (layer < 2) {
 #pragma unroll
           for (int h8 = 0; h8 < 2; ++h8) {
             __align__(16) __nv_bfloat16 h[8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              const float a = z[8 * h8 + e];
-              h[e] = __float2bfloat16_rn(infer ? siluFast(a) : silu(a));
-            }
+            for (int e = 0; e < 8; ++e) h[e] = __float2bfloat16_rn(siluFast(z[8 * h8 + e]));
             *reinterpret_cast<uint4*>(sm + sA + tc::coreOffset(tid, 16 * c + 8 * h8, kHid)) =
                 *reinterpret_cast<uint4*>(h);
           }
         } else {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) y += (infer ? siluFast(z[j]) : silu(z[j])) * w4[16 * c + j];
+          for (int j = 0; j < 16; ++j) y += siluFast(z[j]) * w4[16 * c + j];
         }
       }
     }
-    if (ok && row < rows) out.y[row] = y;
+    if (ok && row < rows) y_out[row] = y;
   }
   tc::fenceBeforeSync();
   __syncthreads();
@@ -233,195 +223,397 @@ __global__ void __launch_bounds__(kRows) k_mlp_fwd(const float* __restrict__ X, 
   if (warp == 0) tc::tmemDealloc(tmem, 64);
 }
 
-// Backward over one batch: per-CTA weight-gradient partials and the squared
-// error. Shared memory: A tile (bf16 dz, 16 KB), W3T, W2T (8 KB each), the
-// CTA's dz and h rows in f32 (2 x 32 KB) and the f32 vectors.
-constexpr uint32_t bA = 0;
-constexpr uint32_t bW3Ts = bA + kRows * kHid * 2;
-constexpr uint32_t bW2Ts = bW3Ts + kHid * kHid * 2;
-constexpr uint32_t bDZ = bW2Ts + kHid * kHid * 2;     // f32 [128][64]
-constexpr uint32_t bH = bDZ + kRows * kHid * 4;       // f32 [128][64]
-constexpr uint32_t bFv = bH + kRows * kHid * 4;
-constexpr uint32_t bRed = bFv + (4 * kHid + 4) * 4;   // f32 [128] scratch
-constexpr uint32_t kBwdSmem = bRed + kRows * 4;
+// One training step's forward and backward over a tile of 128 rows per CTA:
+// per-CTA weight-gradient partials and the squared error.
+//
+// 256 threads: thread (row, half) holds 32 of its row's 64 columns, so a
+// warp's lanes are the TMEM lanes of its quadrant. The activations h1, h2 (the
+// bf16 values the next layer sees, as f32) and the derivatives silu'(z1),
+// silu'(z2) stay in shared memory between the passes, rows padded to 68 floats
+// so that 16-byte accesses of a row per lane meet every bank once. The weight
+// gradients dW = dz^T h are f32 products (dz is not rounded): four groups of
+// 64 threads take 32 rows each, 8 x 8 outputs per thread in packed f32x2, and
+// the four sums are added in a fixed order. One CTA per SM; a step is bound by
+// the chain of layers and the weight gradients' shared-memory reads. (8192
+// rows: 20 us against 159 us for the forward and backward kernels it
+// replaces, whose per-thread arrays lived in local memory.)
+constexpr int kStepThreads = 256;
+constexpr int kLd = 68;  // row stride of the f32 buffers
+constexpr uint32_t tA = 0;                              // A tile, bf16
+constexpr uint32_t tW = tA + kRows * kHid * 2;          // W1 W2 W3 W2T W3T as in the blob
+constexpr uint32_t tF = tW + bF32;                      // f32 vectors
+constexpr uint32_t tH1 = tF + (4 * kHid + 4) * 4;
+constexpr uint32_t kBuf = kRows * kLd * 4;
+constexpr uint32_t tH2 = tH1 + kBuf, tD1 = tH2 + kBuf, tD2 = tD1 + kBuf, tDZ = tD2 + kBuf;
+constexpr uint32_t tRed = tDZ + kBuf;                   // [2][128] and [4][64] f32 scratch
+constexpr uint32_t kStepSmem = tRed + 512 * 4;
+static_assert(kStepSmem <= 227 * 1024, "one CTA's shared memory");
+static_assert(tH1 % 16 == 0 && bF32 % 16 == 0, "16-byte aligned buffers");
+constexpr int kPartStride = (kParams + 31) & ~31;       // floats per CTA's partial
 
-// SIMT weight-gradient partial: G[j][i] = sum_r dz[r][j] * h[r][i] over the
-// CTA's valid rows (h has `nin` columns, stride kHid).
-__device__ __forceinline__ void wgradPartial(const float* dz, const float* h, int nin, int nvalid, float* outW,
-                                             float* outB) {
-  for (int p = threadIdx.x; p < kHid * nin; p += kRows) {
-    const int j = p / nin, i = p % nin;
-    float acc = 0.f;
-    for (int r = 0; r < nvalid; ++r) acc += dz[r * kHid + j] * h[r * kHid + i];
-    outW[p] = acc;
+// Column sums of v[c] over the warp's 32 lanes: lane c returns column c's, in
+// 31 exchanges (each halves the columns a lane still adds up).
+__device__ __forceinline__ float columnSums(float (&v)[32]) {
+  const uint32_t lane = threadIdx.x & 31u;
+#pragma unroll
+  for (int w = 16; w > 0; w >>= 1) {
+    const bool up = (lane & (uint32_t)w) != 0u;
+#pragma unroll
+    for (int c = 0; c < w; ++c) {
+      const float give = up ? v[c] : v[c + w];
+      const float keep = up ? v[c + w] : v[c];
+      v[c] = keep + __shfl_xor_sync(0xffffffffu, give, w);
+    }
   }
-  for (int j = threadIdx.x; j < kHid; j += kRows) {
-    float acc = 0.f;
-    for (int r = 0; r < nvalid; ++r) acc += dz[r * kHid + j];
-    outB[j] = acc;
+  return v[0];
+}
+
+// out[j * nin + i] = sum over the CTA's rows of dz[r][j] h[r][i], h with
+// nin = 64 columns. The group partials go through `scratch0` (groups 0, 1) and
+// `scratch1` (2, 3), which may be dz and h themselves.
+__device__ __forceinline__ void wgrad64(const float* dz, const float* h, float* scratch0, float* scratch1,
+                                        float* __restrict__ out) {
+  const int tid = threadIdx.x, grp = tid >> 6, u = tid & 63, j0 = (u >> 3) * 8, i0 = (u & 7) * 4;
+  F2 acc[8][4];
+#pragma unroll
+  for (int a = 0; a < 8; ++a)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) acc[a][q] = 0ull;
+#pragma unroll 2
+  for (int r = grp * 32; r < grp * 32 + 32; ++r) {
+    const float4 d0 = *reinterpret_cast<const float4*>(dz + r * kLd + j0);
+    const float4 d1 = *reinterpret_cast<const float4*>(dz + r * kLd + j0 + 4);
+    const ulonglong2 h0 = *reinterpret_cast<const ulonglong2*>(h + r * kLd + i0);
+    const ulonglong2 h1 = *reinterpret_cast<const ulonglong2*>(h + r * kLd + i0 + 32);
+    const float d[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
+#pragma unroll
+    for (int a = 0; a < 8; ++a) {
+      const F2 dd = f2(d[a], d[a]);
+      acc[a][0] = fma2(dd, h0.x, acc[a][0]);
+      acc[a][1] = fma2(dd, h0.y, acc[a][1]);
+      acc[a][2] = fma2(dd, h1.x, acc[a][2]);
+      acc[a][3] = fma2(dd, h1.y, acc[a][3]);
+    }
+  }
+  __syncthreads();  // every read of dz and h is done
+  float* mine = (grp < 2 ? scratch0 : scratch1) + (grp & 1) * kHid * kHid;
+#pragma unroll
+  for (int a = 0; a < 8; ++a) {
+    *reinterpret_cast<ulonglong2*>(mine + (j0 + a) * kHid + i0) = make_ulonglong2(acc[a][0], acc[a][1]);
+    *reinterpret_cast<ulonglong2*>(mine + (j0 + a) * kHid + i0 + 32) = make_ulonglong2(acc[a][2], acc[a][3]);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < kHid * kHid / 4 / kStepThreads; ++q) {
+    const int o = (q * kStepThreads + tid) * 4;
+    const float4 a = *reinterpret_cast<const float4*>(scratch0 + o);
+    const float4 b = *reinterpret_cast<const float4*>(scratch0 + kHid * kHid + o);
+    const float4 c = *reinterpret_cast<const float4*>(scratch1 + o);
+    const float4 d = *reinterpret_cast<const float4*>(scratch1 + kHid * kHid + o);
+    *reinterpret_cast<float4*>(out + o) = make_float4((a.x + b.x) + (c.x + d.x), (a.y + b.y) + (c.y + d.y),
+                                                      (a.z + b.z) + (c.z + d.z), (a.w + b.w) + (c.w + d.w));
   }
 }
 
-__global__ void __launch_bounds__(kRows) k_mlp_bwd(const float* __restrict__ X, const float* __restrict__ T,
-                                                   uint32_t rows, const uint8_t* __restrict__ blob,
-                                                   const float* __restrict__ Y, const float* __restrict__ Z,
-                                                   float* __restrict__ partial, float* __restrict__ sqerr, int* err) {
+__global__ void __launch_bounds__(kStepThreads) k_mlp_step(const float* __restrict__ X, const float* __restrict__ T,
+                                                           uint32_t rows, const uint8_t* __restrict__ blob,
+                                                           float* __restrict__ partial, float* __restrict__ sqerr,
+                                                           int* err) {
   extern __shared__ __align__(1024) uint8_t sm[];
   __shared__ __align__(8) uint64_t bar;
   __shared__ uint32_t tbase;
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, half = warp >> 2;
+  const int r = (warp & 3) * 32 + lane;  // row within the tile
+  const int c0 = half * 32;              // first of this thread's columns
+  const uint32_t row = blockIdx.x * kRows + r;
+  const bool valid = row < rows;
+  float* const F = reinterpret_cast<float*>(sm + tF);
+  float* const H1 = reinterpret_cast<float*>(sm + tH1);
+  float* const H2 = reinterpret_cast<float*>(sm + tH2);
+  float* const D1 = reinterpret_cast<float*>(sm + tD1);
+  float* const D2 = reinterpret_cast<float*>(sm + tD2);
+  float* const DZ = reinterpret_cast<float*>(sm + tDZ);
+  float* const red = reinterpret_cast<float*>(sm + tRed);
+  float* const P = partial + (size_t)blockIdx.x * kPartStride;
   {
-    const uint4* src = reinterpret_cast<const uint4*>(blob + bW2T);
-    uint4* d3 = reinterpret_cast<uint4*>(sm + bW3Ts);
-    uint4* d2 = reinterpret_cast<uint4*>(sm + bW2Ts);
-    const uint32_t n = kHid * kHid * 2 / 16;
-    for (uint32_t q = tid; q < n; q += kRows) {
-      d2[q] = src[q];       // W2T
-      d3[q] = src[n + q];   // W3T
-    }
+    const uint4* src = reinterpret_cast<const uint4*>(blob);
+    uint4* dst = reinterpret_cast<uint4*>(sm + tW);
+    for (uint32_t q = tid; q < bF32 / 16u; q += kStepThreads) dst[q] = src[q];
     const float* fs = reinterpret_cast<const float*>(blob + bF32);
-    float* fd = reinterpret_cast<float*>(sm + bFv);
-    for (uint32_t q = tid; q < 4 * kHid + 1; q += kRows) fd[q] = fs[q];
+    for (uint32_t q = tid; q < 4 * kHid + 1; q += kStepThreads) F[q] = fs[q];
   }
   if (warp == 0) tc::tmemAlloc(&tbase, 64);
   if (tid == 0) tc::mbarInit(&bar, 1);
+  // the inputs as bf16, 8 columns per thread
+  {
+    __align__(16) __nv_bfloat16 x[8];
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+    if (valid) {
+      const float4* xr = reinterpret_cast<const float4*>(X + (size_t)row * kIn + 8 * half);
+      a = __ldg(xr);
+      b = __ldg(xr + 1);
+    }
+    const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int e = 0; e < 8; ++e) x[e] = __float2bfloat16_rn(v[e]);
+    *reinterpret_cast<uint4*>(sm + tA + tc::coreOffset(r, 8 * half, kIn)) = *reinterpret_cast<uint4*>(x);
+  }
+  const float target = valid ? T[row] : 0.f;
+  tc::fenceProxyAsync();
   tc::fenceBeforeSync();
   __syncthreads();
   tc::fenceAfterSync();
   const uint32_t tmem = tbase;
-  const uint32_t tRow = tmem + ((uint32_t)(warp * 32) << 16);
-  const float* Fv = reinterpret_cast<const float*>(sm + bFv);
-  float* dz = reinterpret_cast<float*>(sm + bDZ);
-  float* h = reinterpret_cast<float*>(sm + bH);
-  float* red = reinterpret_cast<float*>(sm + bRed);
-  const uint32_t aAddr = tc::smemAddr(sm + bA);
+  const uint32_t tRow = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0;
+  const uint32_t aAddr = tc::smemAddr(sm + tA);
   constexpr uint32_t idesc = tc::idescBf16F32(kRows, kHid);
-  const uint32_t tile = blockIdx.x;
-  const uint32_t row = tile * kRows + tid;
-  const bool valid = row < rows;
-  const int nvalid = (int)min((uint32_t)kRows, rows - tile * kRows);
-  float* P = partial + (size_t)blockIdx.x * kParams;
-  auto zAt = [&](int layer, int j) { return valid ? Z[((size_t)layer * rows + row) * kHid + j] : 0.f; };
-  // dy and the squared error
-  float dy = 0.f;
-  if (valid) {
-    const float e = Y[row] - T[row];
-    dy = 2.f * e / (float)rows;
-    red[tid] = e * e;
-  } else {
-    red[tid] = 0.f;
-  }
-  // h3 (f32) and dz3
-  float dzr[kHid];
-  {
-    const float* w4 = Fv + 3 * kHid;
-#pragma unroll 4
-    for (int j = 0; j < kHid; ++j) {
-      const float z3 = zAt(2, j);
-      h[tid * kHid + j] = valid ? silu(z3) : 0.f;
-      dzr[j] = valid ? dy * w4[j] * dsilu(z3) : 0.f;
-    }
-  }
-  __syncthreads();
-  // w4, b4 gradients
-  for (int j = tid; j < kHid; j += kRows) {
-    float acc = 0.f;
-    for (int r = 0; r < nvalid; ++r) {
-      const float e = Y[tile * kRows + r] - T[tile * kRows + r];
-      acc += 2.f * e / (float)rows * h[r * kHid + j];
-    }
-    P[oW4 + j] = acc;
-  }
-  if (tid == 0) {
-    float acc = 0.f, se = 0.f;
-    for (int r = 0; r < nvalid; ++r) {
-      acc += 2.f * (Y[tile * kRows + r] - T[tile * kRows + r]) / (float)rows;
-      se += red[r];
-    }
-    P[oB4] = acc;
-    sqerr[blockIdx.x] = se;
-  }
-  bool ok = true;
-  // layers 3 and 2: dz (f32) -> dW, db; dh_prev = dz W (tensor cores); dz_prev
-  for (int layer = 2; layer >= 1 && ok; --layer) {
-    __syncthreads();
-#pragma unroll 4
-    for (int j = 0; j < kHid; ++j) {
-      dz[tid * kHid + j] = dzr[j];
-      h[tid * kHid + j] = valid ? __bfloat162float(__float2bfloat16_rn(silu(zAt(layer - 1, j)))) : 0.f;
-    }
-#pragma unroll
-    for (int c = 0; c < kHid / 8; ++c) {
-      __align__(16) __nv_bfloat16 hb[8];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) hb[e] = __float2bfloat16_rn(dzr[8 * c + e]);
-      *reinterpret_cast<uint4*>(sm + bA + tc::coreOffset(tid, 8 * c, kHid)) = *reinterpret_cast<uint4*>(hb);
-    }
-    tc::fenceProxyAsync();
-    tc::fenceBeforeSync();
-    __syncthreads();
+  uint32_t phase = 0;
+  // D = A B^T on the tensor cores; every thread has fenced and synchronised
+  auto issue = [&](uint32_t wOffset, uint32_t K) {
     if (tid == 0) {
-      tc::fenceAfterSync();
-      const uint32_t wAddr = tc::smemAddr(sm + (layer == 2 ? bW3Ts : bW2Ts));
-      for (uint32_t ks = 0; ks < kHid / 16; ++ks)
-        tc::mma(tmem, tc::smemDesc(aAddr + ks * 256, 128, 1024), tc::smemDesc(wAddr + ks * 256, 128, 1024), idesc,
+      const uint32_t wAddr = tc::smemAddr(sm + tW + wOffset), sbo = (K / 8) * 128;
+      for (uint32_t ks = 0; ks < K / 16; ++ks)
+        tc::mma(tmem, tc::smemDesc(aAddr + ks * 256, 128, sbo), tc::smemDesc(wAddr + ks * 256, 128, sbo), idesc,
                 ks > 0);
       tc::commit(&bar);
     }
-    const int oW = layer == 2 ? oW3 : oW2, oB = layer == 2 ? oB3 : oB2;
-    wgradPartial(dz, h, kHid, nvalid, P + oW, P + oB);
-    if (!tc::mbarWait(&bar, (uint32_t)(2 - layer), kSpin)) {
-      if (tid == 0) atomicOr(err, kErrMma);
-      ok = false;
-    }
+  };
+  // no barrier is skipped when a wait expires: the error word says so, and the
+  // CTA goes on to release its TMEM
+  auto await = [&]() {
+    if (!tc::mbarWait(&bar, phase, kSpin) && tid == 0) atomicOr(err, kErrMma);
+    phase ^= 1u;
     tc::fenceAfterSync();
-    float dh[kHid];
-#pragma unroll
-    for (int c = 0; c < kHid / 16; ++c) tc::ld16(tRow + 16 * c, dh + 16 * c);
-#pragma unroll 4
-    for (int j = 0; j < kHid; ++j) dzr[j] = valid ? dh[j] * dsilu(zAt(layer - 1, j)) : 0.f;
+  };
+  auto ready = [&]() {  // A written, the accumulator read: the next MMA may start
+    tc::fenceProxyAsync();
     tc::fenceBeforeSync();
     __syncthreads();
+    if (tid == 0) tc::fenceAfterSync();
+  };
+  auto storeA8 = [&](int c, const float* v) {  // columns c .. c + 7 of this row as bf16
+    __align__(16) __nv_bfloat16 h[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) h[e] = __float2bfloat16_rn(v[e]);
+    *reinterpret_cast<uint4*>(sm + tA + tc::coreOffset(r, c, kHid)) = *reinterpret_cast<uint4*>(h);
+  };
+  auto store4 = [&](float* buf, int c, float a, float b, float d, float e) {
+    *reinterpret_cast<float4*>(buf + r * kLd + c) = make_float4(a, b, d, e);
+  };
+
+  // ---- forward, layers 1 and 2
+#pragma unroll 1
+  for (int layer = 0; layer < 2; ++layer) {
+    issue(layer == 0 ? bW1 : bW2, layer == 0 ? kIn : kHid);
+    await();
+    float* const H = layer == 0 ? H1 : H2;
+    float* const D = layer == 0 ? D1 : D2;
+    const float* bias = F + layer * kHid + c0;
+#pragma unroll
+    for (int c = 0; c < 32; c += 16) {
+      float z[16], d[16];
+      tc::ld16(tRow + c, z);
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        const float a = z[e] + bias[c + e];
+        const float s = sigm(a);
+        z[e] = __bfloat162float(__float2bfloat16_rn(a * s));
+        d[e] = s * (1.f + a * (1.f - s));
+      }
+      storeA8(c0 + c, z);
+      storeA8(c0 + c + 8, z + 8);
+#pragma unroll
+      for (int e = 0; e < 16; e += 4) {
+        store4(H, c0 + c + e, z[e], z[e + 1], z[e + 2], z[e + 3]);
+        store4(D, c0 + c + e, d[e], d[e + 1], d[e + 2], d[e + 3]);
+      }
+    }
+    ready();
   }
-  // layer 1: dW1 = dz1^T x (x as bf16, the network's input precision)
+  // ---- forward, layer 3 and the output; h3 and silu'(z3) stay in registers
+  issue(bW3, kHid);
+  await();
+  float h3[32], dz[32];
+  {
+    const float* bias = F + 2 * kHid + c0;
+    const float* w4 = F + 3 * kHid + c0;
+    float y = 0.f;
+#pragma unroll
+    for (int c = 0; c < 32; c += 16) {
+      float z[16];
+      tc::ld16(tRow + c, z);
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        const float a = z[e] + bias[c + e];
+        const float s = sigm(a);
+        h3[c + e] = a * s;
+        dz[c + e] = s * (1.f + a * (1.f - s));
+        y += h3[c + e] * w4[c + e];
+      }
+    }
+    red[half * kRows + r] = y;
+  }
+  tc::fenceBeforeSync();
   __syncthreads();
-  for (int j = 0; j < kHid; ++j) dz[tid * kHid + j] = dzr[j];
-  for (int k = 0; k < kIn; ++k)
-    h[tid * kHid + k] = valid ? __bfloat162float(__float2bfloat16_rn(X[(size_t)row * kIn + k])) : 0.f;
-  __syncthreads();
-  wgradPartial(dz, h, kIn, nvalid, P + oW1, P + oB1);
+  const float e = red[r] + red[kRows + r] + F[4 * kHid] - target;
+  const float dy = valid ? 2.f * e / (float)rows : 0.f;
+#pragma unroll
+  for (int c = 0; c < 32; ++c) {
+    dz[c] = dy * F[3 * kHid + c0 + c] * dz[c];
+    h3[c] = valid ? dy * h3[c] : 0.f;  // w4's gradient sums these
+  }
+  // squared error and b4's gradient over the rows
+  float se = valid ? e * e : 0.f, sd = dy;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    se += __shfl_xor_sync(0xffffffffu, se, o);
+    sd += __shfl_xor_sync(0xffffffffu, sd, o);
+  }
+  const float w4sum = columnSums(h3);
+  __syncthreads();  // red is free
+  red[(warp & 3) * kHid + c0 + lane] = w4sum;
+  if (half == 0 && lane == 0) {
+    red[256 + warp] = se;
+    red[260 + warp] = sd;
+  }
+  // ---- backward, layers 3 and 2: dz -> dW, db; the previous layer's dz
+#pragma unroll 1
+  for (int layer = 2; layer >= 1; --layer) {
+#pragma unroll
+    for (int c = 0; c < 32; c += 8) {
+      storeA8(c0 + c, dz + c);
+      store4(DZ, c0 + c, dz[c], dz[c + 1], dz[c + 2], dz[c + 3]);
+      store4(DZ, c0 + c + 4, dz[c + 4], dz[c + 5], dz[c + 6], dz[c + 7]);
+    }
+    ready();
+    issue(layer == 2 ? bW3T : bW2T, kHid);
+    if (layer == 2 && tid < kHid) {
+      P[oW4 + tid] = (red[tid] + red[kHid + tid]) + (red[2 * kHid + tid] + red[3 * kHid + tid]);
+      if (tid == 0) {
+        sqerr[blockIdx.x] = (red[256] + red[257]) + (red[258] + red[259]);
+        P[oB4] = (red[260] + red[261]) + (red[262] + red[263]);
+      }
+    }
+    const float bsum = columnSums(dz);
+    float* const H = layer == 2 ? H2 : H1;
+    wgrad64(DZ, H, DZ, H, P + (layer == 2 ? oW3 : oW2));
+    red[(warp & 3) * kHid + c0 + lane] = bsum;  // the sums read above are behind wgrad64's barriers
+    await();
+    const float* D = layer == 2 ? D2 : D1;
+#pragma unroll
+    for (int c = 0; c < 32; c += 16) {
+      float g[16];
+      tc::ld16(tRow + c, g);
+#pragma unroll
+      for (int q = 0; q < 16; q += 4) {
+        const float4 d = *reinterpret_cast<const float4*>(D + r * kLd + c0 + c + q);
+        dz[c + q] = g[q] * d.x;
+        dz[c + q + 1] = g[q + 1] * d.y;
+        dz[c + q + 2] = g[q + 2] * d.z;
+        dz[c + q + 3] = g[q + 3] * d.w;
+      }
+    }
+    tc::fenceBeforeSync();
+    __syncthreads();  // red written; DZ and H, read for the group sums, are free
+    if (tid < kHid)
+      P[(layer == 2 ? oB3 : oB2) + tid] = (red[tid] + red[kHid + tid]) + (red[2 * kHid + tid] + red[3 * kHid + tid]);
+  }
+  // ---- layer 1: dW1 = dz1^T x (x as bf16, the network's input precision)
+#pragma unroll
+  for (int c = 0; c < 32; c += 4) store4(DZ, c0 + c, dz[c], dz[c + 1], dz[c + 2], dz[c + 3]);
+  {
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+    if (valid) {
+      const float4* xr = reinterpret_cast<const float4*>(X + (size_t)row * kIn + 8 * half);
+      a = __ldg(xr);
+      b = __ldg(xr + 1);
+    }
+    auto rnd = [](float v) { return __bfloat162float(__float2bfloat16_rn(v)); };
+    store4(H1, 8 * half, rnd(a.x), rnd(a.y), rnd(a.z), rnd(a.w));
+    store4(H1, 8 * half + 4, rnd(b.x), rnd(b.y), rnd(b.z), rnd(b.w));
+  }
+  const float bsum = columnSums(dz);
+  __syncthreads();  // red's readers are done, DZ and x are written
+  red[(warp & 3) * kHid + c0 + lane] = bsum;
+  {
+    const int grp = tid >> 6, u = tid & 63, j0 = (u >> 2) * 4, i0 = (u & 3) * 4;
+    F2 acc[4][2] = {};
+#pragma unroll 4
+    for (int q = grp * 32; q < grp * 32 + 32; ++q) {
+      const float4 d = *reinterpret_cast<const float4*>(DZ + q * kLd + j0);
+      const ulonglong2 h = *reinterpret_cast<const ulonglong2*>(H1 + q * kLd + i0);
+      const float dd[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        const F2 w = f2(dd[a], dd[a]);
+        acc[a][0] = fma2(w, h.x, acc[a][0]);
+        acc[a][1] = fma2(w, h.y, acc[a][1]);
+      }
+    }
+    float* scratch = H2 + grp * kHid * kIn;  // H2 is free
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+      *reinterpret_cast<ulonglong2*>(scratch + (j0 + a) * kIn + i0) = make_ulonglong2(acc[a][0], acc[a][1]);
+    __syncthreads();
+    const int o = tid * 4;
+    const float4 a = *reinterpret_cast<const float4*>(H2 + o), b = *reinterpret_cast<const float4*>(H2 + 1024 + o),
+                 c = *reinterpret_cast<const float4*>(H2 + 2048 + o),
+                 d = *reinterpret_cast<const float4*>(H2 + 3072 + o);
+    *reinterpret_cast<float4*>(P + oW1 + o) = make_float4((a.x + b.x) + (c.x + d.x), (a.y + b.y) + (c.y + d.y),
+                                                          (a.z + b.z) + (c.z + d.z), (a.w + b.w) + (c.w + d.w));
+    if (tid < kHid)
+      P[oB1 + tid] = (red[tid] + red[kHid + tid]) + (red[2 * kHid + tid] + red[3 * kHid + tid]);
+  }
   tc::fenceBeforeSync();
   __syncthreads();
   tc::fenceAfterSync();
   if (warp == 0) tc::tmemDealloc(tmem, 64);
 }
 
-// grad[p] = sum over CTAs of partial[cta][p] (fixed order); loss likewise.
-__global__ void k_mlp_reduce(const float* __restrict__ partial, uint32_t nparts, const float* __restrict__ sqerr,
-                             uint32_t rows, float* __restrict__ grad, float* __restrict__ loss) {
-  const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+// The gradient, grad[p] = sum over CTAs of partial[cta][p] in a fixed order
+// (four interleaved sums per parameter), and the mean squared error. With w:
+// the Adam update of the parameter and its bf16 copy in the blob follow in the
+// same thread.
+struct Adam {
+  float *w, *m, *v;
+  float lr, b1, b2, eps, c1, c2;
+};
+constexpr int kReduceParams = 64;
+__global__ void __launch_bounds__(4 * kReduceParams) k_mlp_reduce(const float* __restrict__ partial, uint32_t nparts,
+                                                                  const float* __restrict__ sqerr, uint32_t rows,
+                                                                  float* __restrict__ grad, float* __restrict__ loss,
+                                                                  Adam A, uint8_t* __restrict__ blob) {
+  __shared__ float sum[4][kReduceParams];
+  const uint32_t q = threadIdx.x % kReduceParams, g = threadIdx.x / kReduceParams;
+  const uint32_t p = blockIdx.x * kReduceParams + q;
+  float acc = 0.f;
   if (p < (uint32_t)kParams) {
-    float acc = 0.f;
-    for (uint32_t c = 0; c < nparts; ++c) acc += partial[(size_t)c * kParams + p];
-    grad[p] = acc;
+#pragma unroll 8
+    for (uint32_t c = g; c < nparts; c += 4) acc += partial[(size_t)c * kPartStride + p];
   }
-  if (p == 0) {
+  sum[g][q] = acc;
+  __syncthreads();
+  if (g == 0 && p < (uint32_t)kParams) {
+    const float gi = (sum[0][q] + sum[1][q]) + (sum[2][q] + sum[3][q]);
+    if (grad) grad[p] = gi;
+    if (A.w) {
+      const float mi = A.b1 * A.m[p] + (1.f - A.b1) * gi;
+      const float vi = A.b2 * A.v[p] + (1.f - A.b2) * gi * gi;
+      A.m[p] = mi;
+      A.v[p] = vi;
+      const float wi = A.w[p] - A.lr * (mi / A.c1) / (sqrtf(vi / A.c2) + A.eps);
+      A.w[p] = wi;
+      packParam(blob, (int)p, wi);
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x >= 4 * kReduceParams - 32) {  // the last warp: the loss
+    const uint32_t lane = threadIdx.x & 31u;
     float se = 0.f;
-    for (uint32_t c = 0; c < nparts; ++c) se += sqerr[c];
-    *loss = se / (float)rows;
+    for (uint32_t c = lane; c < nparts; c += 32) se += sqerr[c];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) se += __shfl_xor_sync(0xffffffffu, se, o);
+    if (lane == 0) *loss = se / (float)rows;
   }
-}
-
-__global__ void k_adam(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
-                       float* __restrict__ v, float lr, float b1, float b2, float eps, float c1, float c2) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= kParams) return;
-  const float gi = g[p];
-  const float mi = b1 * m[p] + (1.f - b1) * gi;
-  const float vi = b2 * v[p] + (1.f - b2) * gi * gi;
-  m[p] = mi;
-  v[p] = vi;
-  w[p] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
 }
 
 }  // namespace
@@ -429,12 +621,14 @@ __global__ void k_adam(float* __restrict__ w, const float* __restrict__ g, float
 int mlp_param_count() { return kParams; }
 size_t mlp_blob_bytes() { return kBlobBytes; }
 
+size_t mlp_partial_floats(uint32_t rows) { return (size_t)((rows + kRows - 1) / kRows) * kPartStride; }
+
 void mlp_pack(const float* dParams, void* dBlob, cudaStream_t st) {
-  k_mlp_pack<<<1, 256, 0, st>>>(dParams, static_cast<uint8_t*>(dBlob));
+  k_mlp_pack<<<(kParams + 255) / 256, 256, 0, st>>>(dParams, static_cast<uint8_t*>(dBlob));
 }
 
-cudaError_t mlp_forward(const float* dX, uint32_t rows, const void* dBlob, float* dY, float* dZ, int* dErr,
-                        cudaStream_t st, bool skipZero) {
+cudaError_t mlp_forward(const float* dX, uint32_t rows, const void* dBlob, float* dY, int* dErr, cudaStream_t st,
+                        bool skipZero) {
   static bool attr = false;
   if (!attr) {
     cudaError_t e = cudaFuncSetAttribute(k_mlp_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem);
@@ -445,35 +639,45 @@ cudaError_t mlp_forward(const float* dX, uint32_t rows, const void* dBlob, float
   const uint32_t ntiles = (rows + kRows - 1) / kRows;
   // 48 registers and 37 KB of shared memory: six CTAs per SM (384 TMEM columns)
   const uint32_t grid = ntiles < 152u * 6u ? ntiles : 152u * 6u;
-  k_mlp_fwd<<<grid, kRows, kFwdSmem, st>>>(dX, rows, static_cast<const uint8_t*>(dBlob), FwdOut{dY, dZ}, dErr,
-                                           skipZero ? 1 : 0);
+  k_mlp_fwd<<<grid, kRows, kFwdSmem, st>>>(dX, rows, static_cast<const uint8_t*>(dBlob), dY, dErr, skipZero ? 1 : 0);
   return cudaGetLastError();
 }
 
-// One training step's gradient (and mean squared error) on rows X, targets T.
-// Scratch: dY [rows], dZ [3 rows 64], dPartial [ceil(rows/128) * params],
-// dSq [ceil(rows/128)].
-cudaError_t mlp_grad(const float* dX, const float* dT, uint32_t rows, const void* dBlob, float* dY, float* dZ,
-                     float* dPartial, float* dSq, float* dGrad, float* dLoss, int* dErr, cudaStream_t st) {
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(k_mlp_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
-  cudaError_t e = mlp_forward(dX, rows, dBlob, dY, dZ, dErr, st);
-  if (e != cudaSuccess || rows == 0) return e;
-  const uint32_t ntiles = (rows + kRows - 1) / kRows;
-  k_mlp_bwd<<<ntiles, kRows, kBwdSmem, st>>>(dX, dT, rows, static_cast<const uint8_t*>(dBlob), dY, dZ, dPartial,
-                                            dSq, dErr);
-  k_mlp_reduce<<<(kParams + 255) / 256, 256, 0, st>>>(dPartial, ntiles, dSq, rows, dGrad, dLoss);
+namespace {
+cudaError_t stepKernel(const float* dX, const float* dT, uint32_t rows, const void* dBlob, float* dPartial, float* dSq,
+                       int* dErr, cudaStream_t st) {
+  cudaError_t e = cudaFuncSetAttribute(k_mlp_step, cudaFuncAttributeMaxDynamicSharedMemorySize, kStepSmem);
+  if (e != cudaSuccess) return e;
+  k_mlp_step<<<(rows + kRows - 1) / kRows, kStepThreads, kStepSmem, st>>>(
+      dX, dT, rows, static_cast<const uint8_t*>(dBlob), dPartial, dSq, dErr);
+  return cudaGetLastError();
+}
+}  // namespace
+
+// The gradient (and mean squared error) on rows X, targets T. Scratch:
+// dPartial [mlp_partial_floats(rows)], dSq [ceil(rows / 128)].
+cudaError_t mlp_grad(const float* dX, const float* dT, uint32_t rows, const void* dBlob, float* dPartial, float* dSq,
+                     float* dGrad, float* dLoss, int* dErr, cudaStream_t st) {
+  if (rows == 0) return cudaSuccess;
+  cudaError_t e = stepKernel(dX, dT, rows, dBlob, dPartial, dSq, dErr, st);
+  if (e != cudaSuccess) return e;
+  k_mlp_reduce<<<(kParams + kReduceParams - 1) / kReduceParams, 4 * kReduceParams, 0, st>>>(
+      dPartial, (rows + kRows - 1) / kRows, dSq, rows, dGrad, dLoss, Adam{}, nullptr);
   return cudaGetLastError();
 }
 
-void mlp_adam(float* dW, const float* dG, float* dM, float* dV, float lr, int step, cudaStream_t st) {
+// One Adam step on the parameters dW (moments dM, dV) and their packed copy.
+cudaError_t mlp_train_step(const float* dX, const float* dT, uint32_t rows, float* dW, float* dM, float* dV,
+                           void* dBlob, float* dPartial, float* dSq, float* dLoss, float lr, int step, int* dErr,
+                           cudaStream_t st) {
+  cudaError_t e = stepKernel(dX, dT, rows, dBlob, dPartial, dSq, dErr, st);
+  if (e != cudaSuccess) return e;
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.f - powf(b1, (float)step), c2 = 1.f - powf(b2, (float)step);
-  k_adam<<<(kParams + 255) / 256, 256, 0, st>>>(dW, dG, dM, dV, lr, b1, b2, 1e-8f, c1, c2);
+  k_mlp_reduce<<<(kParams + kReduceParams - 1) / kReduceParams, 4 * kReduceParams, 0, st>>>(
+      dPartial, (rows + kRows - 1) / kRows, dSq, rows, nullptr, dLoss, Adam{dW, dM, dV, lr, b1, b2, 1e-8f, c1, c2},
+      static_cast<uint8_t*>(dBlob));
+  return cudaGetLastError();
 }
 
 }  // namespace xpbi
