@@ -263,6 +263,7 @@ void buildSceneDev(const SceneHost& s, uint32_t sceneIdx, SceneDev& d, MatDev* m
       d.massS = md[i].mass;
     }
   if (nWater != 1) d.waterMpd = 0.f;
+  d.onePhase = nWater == 0 || nOther == 0 ? 1 : 0;
   d.twoMasses = nWater == 1 && nOther <= 1 ? 1 : 0;
 }
 
@@ -450,7 +451,9 @@ struct Schedule {
   bool features = false; // network features at iteration 0
   bool keepLam = false;  // carry the final multipliers into the next substep
   int varA = 0, varB = 0; // solveA / solveB variants
-  int lanes = 1;          // lanes per slot in solveA / solveB
+  int lanesA = 1, lanesB = 1;        // lanes per slot in solveA, solveB
+  int lanesAll = 1;                  // in computeL, xsph and the update
+  int lanesPbfA = 1, lanesPbfB = 1;  // in pbfA, pbfB
   bool active = false;    // active set (work skipping) in the iterations
   bool fallback = false;  // scenes an early-stopped solve fails are re-solved plainly
   std::string key() const {
@@ -458,7 +461,8 @@ struct Schedule {
     for (char c : pbf) k += c ? '1' : '0';
     k += ":" + std::to_string(mode) + (track ? "t" : "") + (reduce ? "r" : "") + (features ? "f" : "") +
          (keepLam ? "l" : "") + (active ? "a" : "") + (fallback ? "j" : "") + ":v" + std::to_string(varA) + std::to_string(varB) + ":g" +
-         std::to_string(lanes);
+         std::to_string(lanesA) + std::to_string(lanesB) + std::to_string(lanesAll) + std::to_string(lanesPbfA) +
+         std::to_string(lanesPbfB);
     return k;
   }
 };
@@ -472,19 +476,24 @@ Schedule schedule(const xpbi_sim* s) {
   sch.keepLam = s->mode != 0 || sch.features;
   sch.varA = s->tuneA;
   sch.varB = s->tuneB;
-  if (s->lanesMode) {
-    sch.lanes = s->lanesMode;
-  } else {
-    // the constraint kernels' work is the solid particles (water threads
-    // leave at once): few of them leave the GPU idle with one lane each
-    uint64_t solids = 0;
-    for (const SceneHost& h : s->sc)
-      for (uint32_t m = 0; m < h.nMats; ++m)
-        if (h.mats[m].kind != XPBI_WATER) solids += h.matCount[m];
-    sch.lanes = solids <= kFourLaneSolids ? 4 : (solids <= kTwoLaneSolids ? 2 : 1);
-  }
+  // the constraint kernels' work is the solid particles (water threads leave
+  // at once), the other passes' every particle
+  uint64_t solids = 0;
+  for (const SceneHost& h : s->sc)
+    for (uint32_t m = 0; m < h.nMats; ++m)
+      if (h.mats[m].kind != XPBI_WATER) solids += h.matCount[m];
+  auto lanes = [&](const LaneLimits& lim, uint64_t n) {
+    return s->lanesMode ? s->lanesMode : (n <= lim.four ? 4 : (n <= lim.two ? 2 : 1));
+  };
+  sch.lanesA = lanes(kLanesA, solids);
+  sch.lanesB = lanes(kLanesB, solids);
+  sch.lanesAll = lanes(kLanesAll, s->b.N);
+  sch.lanesPbfA = lanes(kLanesPbfA, s->b.N);
+  sch.lanesPbfB = lanes(kLanesPbfB, s->b.N);
   // the active set needs the early stop's residual sums and one lane per slot
-  sch.active = s->activeShare > 0.f && s->residTol > 0.f && sch.lanes == 1;
+  sch.active = s->activeShare > 0.f && s->residTol > 0.f &&
+               (s->lanesMode ? s->lanesMode == 1 : solids > kActiveSolids);
+  if (sch.active) sch.lanesA = sch.lanesB = 1;
   // an early-stopped solve that differs from the reference (a warm start or
   // the active set) is judged against the plain tolerances it was given
   sch.fallback = s->residTol > 0.f && (s->mode != 0 || sch.active);
@@ -580,15 +589,15 @@ void enqueuePlainResolve(xpbi_sim* s, const Schedule& sch, int in, cudaStream_t 
   for (const SceneHost& h : s->sc) K = std::max(K, h.iterations);
   for (int k = 0; k < K; ++k) {
     const bool pbf = k < (int)sch.pbf.size() && sch.pbf[k];
-    launch_solveA(b, k, b.velS[cur], kRerun, sch.varA, sch.lanes, st);
+    launch_solveA(b, k, b.velS[cur], kRerun, sch.varA, sch.lanesA, st);
     R.mark(st, "solveA");
-    launch_solveB(b, k, b.velS[cur], b.velS[cur ^ 1], pbf, kRerun, sch.varB, sch.lanes, st);
+    launch_solveB(b, k, b.velS[cur], b.velS[cur ^ 1], pbf, kRerun, sch.varB, sch.lanesB, st);
     R.mark(st, "solveB");
     cur ^= 1;
     if (pbf) {
-      launch_pbfA(b, k, b.velS[cur], kRerun, st);
+      launch_pbfA(b, k, kRerun, sch.lanesPbfA, st);
       R.mark(st, "pbfA");
-      launch_pbfB(b, k, b.velS[cur], b.velS[cur ^ 1], kRerun, st);
+      launch_pbfB(b, k, b.velS[cur], b.velS[cur ^ 1], kRerun, sch.lanesPbfB, st);
       R.mark(st, "pbfB");
       cur ^= 1;
     }
@@ -653,7 +662,8 @@ cudaError_t enqueueSubstep(xpbi_sim* s, const Schedule& sch, cudaStream_t st, Re
   // the velocity-free sums are read by the one-lane constraint sweeps; with
   // features (the learned solve, or features logged) the same pass also
   // stores iteration 0's constraint and the network's features
-  launch_computeL(b, sch.features, st);
+  // (with the sums of solveA's one-lane sweep for the constraint it stores)
+  launch_computeL(b, sch.features, sch.features && sch.lanesA == 1 ? 1 : sch.lanesAll, st);
   R.mark(st, "computeL");
   if (sch.mode == 1) {
     mlp_forward(b.feat, b.N, b.netBlob, b.netOut, s->netErr, st, true);
@@ -699,7 +709,7 @@ cudaError_t enqueueSubstep(xpbi_sim* s, const Schedule& sch, cudaStream_t st, Re
     // iteration 0 after computeL with features: it already evaluated the
     // constraint at these velocities, with one lane per slot (several lanes
     // sum in another order, so they evaluate it again)
-    const int stored = k == 0 && sch.features && sch.lanes == 1 ? kStoredC : 0;
+    const int stored = k == 0 && sch.features && sch.lanesA == 1 ? kStoredC : 0;
     // active set: iteration 0 visits every slot and marks what moved; later
     // ones visit the marked slots; velocities update in place (solveB and
     // pbfB read no neighbour's velocity), so there is no ping-pong
@@ -719,10 +729,10 @@ cudaError_t enqueueSubstep(xpbi_sim* s, const Schedule& sch, cudaStream_t st, Re
         R.mark(st, "predict");
       }
     } else {
-      launch_solveA(b, k, b.velS[in], aflags | stored | (act & kActive), sch.varA, sch.lanes, st);
+      launch_solveA(b, k, b.velS[in], aflags | stored | (act & kActive), sch.varA, sch.lanesA, st);
       R.mark(st, "solveA");
       launch_solveB(b, k, b.velS[in], b.velS[in ^ (sch.active ? 0 : 1)], sch.pbf[k] != 0,
-                    (sch.reduce ? kTrackResid : 0) | act, sch.varB, sch.lanes, st);
+                    (sch.reduce ? kTrackResid : 0) | act, sch.varB, sch.lanesB, st);
       R.mark(st, "solveB");
       if (sch.reduce) {
         launch_resid_reduce(b, k, (aflags & kWarm) != 0, st);
@@ -731,10 +741,10 @@ cudaError_t enqueueSubstep(xpbi_sim* s, const Schedule& sch, cudaStream_t st, Re
     }
     if (!sch.active) in ^= 1;
     if (sch.pbf[k]) {
-      launch_pbfA(b, k, b.velS[in], 0, st);
+      launch_pbfA(b, k, 0, sch.lanesPbfA, st);
       R.mark(st, "pbfA");
       launch_pbfB(b, k, b.velS[in], b.velS[in ^ (sch.active ? 0 : 1)],
-                  sch.active ? (kInPlace | (k >= 1 ? kMarkMoved : 0)) : 0, st);
+                  sch.active ? (kInPlace | (k >= 1 ? kMarkMoved : 0)) : 0, sch.lanesPbfB, st);
       R.mark(st, "pbfB");
       if (!sch.active) in ^= 1;
     }
@@ -757,14 +767,14 @@ cudaError_t enqueueSubstep(xpbi_sim* s, const Schedule& sch, cudaStream_t st, Re
     }
   }
   if (sch.track) {  // residual of the state the iterations leave behind
-    launch_solveA(b, sch.K, b.velS[in], kTrackResid | kMeasureOnly, sch.varA, sch.lanes, st);
+    launch_solveA(b, sch.K, b.velS[in], kTrackResid | kMeasureOnly, sch.varA, sch.lanesA, st);
     R.mark(st, "solveA(measure)");
-    launch_solveB(b, sch.K, b.velS[in], nullptr, false, kTrackResid | kMeasureOnly, sch.varB, sch.lanes, st);
+    launch_solveB(b, sch.K, b.velS[in], nullptr, false, kTrackResid | kMeasureOnly, sch.varB, sch.lanesB, st);
     R.mark(st, "solveB(measure)");
     launch_resid_reduce(b, -1, false, st);
     R.mark(st, "residual");
   }
-  launch_xsph(b, b.velS[in], b.velS[in ^ 1], st);
+  launch_xsph(b, b.velS[in], b.velS[in ^ 1], sch.lanesAll, st);
   R.mark(st, "xsph");
   in ^= 1;
   // the update moves the particles: asynchronous read-backs of the previous
@@ -775,7 +785,7 @@ cudaError_t enqueueSubstep(xpbi_sim* s, const Schedule& sch, cudaStream_t st, Re
     cudaStreamIsCapturing(st, &cs);
     cudaStreamWaitEvent(st, s->evCopy, cs == cudaStreamCaptureStatusActive ? cudaEventWaitExternal : 0);
   }
-  launch_updateF_integrate(b, b.velS[in], st);
+  launch_updateF_integrate(b, b.velS[in], sch.lanesAll, st);
   R.mark(st, "updateF+integrate");
   if (sch.keepLam) {
     launch_keep_lambda(b, st);
@@ -1424,7 +1434,7 @@ int xpbi_autotune(xpbi_sim* sim, int32_t iterations, int32_t has_water, int32_t 
     launch_scan(b, st);
     launch_scatter(b, st);
     launch_reorder(b, false, st);
-    launch_computeL(b, false, st);
+    launch_computeL(b, false, 1, st);
     cudaMemsetAsync(b.done, 0, sizeof(int) * b.S, st);  // no scene counts as converged here
     cudaMemsetAsync(b.solidDisp, 0, sizeof(uint32_t) * 2 * b.S, st);
     // iteration 0 of each variant from lambda = 0, then solveB on its record

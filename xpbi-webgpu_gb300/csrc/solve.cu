@@ -38,30 +38,20 @@ namespace xpbi {
 namespace {
 
 constexpr int kThreads = 128;
-#ifndef A_AHEAD
-#define A_AHEAD false
-#endif
-#ifndef L_AHEAD
-#define L_AHEAD false
-#endif
 
-
-// Launch bounds of the stencil kernels: defining XPBI_MINB_<KERNEL> at build
-// time asks the register allocator for that many resident CTAs per SM
-// (trading registers for occupancy); otherwise only the block size is fixed.
-#define XPBI_LB_DEFAULT __launch_bounds__(kThreads)
-#ifdef XPBI_MINB_COMPUTEL
-#define XPBI_LB_COMPUTEL __launch_bounds__(kThreads, XPBI_MINB_COMPUTEL)
-#else
-#define XPBI_LB_COMPUTEL __launch_bounds__(kThreads, 8)
-#endif
-// computeL with the stored constraint and features (the learned solve) at
-// 7 CTAs per SM (72 registers): 1.36 ms per 4M-particle substep against
-// 1.56 ms with the allocator's choice (5 CTAs).
-#ifndef XPBI_MINB_COMPUTEL_FEATURES
-#define XPBI_MINB_COMPUTEL_FEATURES 7
-#endif
-#define XPBI_LB_COMPUTEL_FEATURES __launch_bounds__(kThreads, XPBI_MINB_COMPUTEL_FEATURES)
+// Launch bounds of the stencil kernels: resident CTAs of kThreads threads per
+// SM asked of the register allocator, with one lane per slot and with several
+// (ms per launch; one lane on the 4M-particle dam-breach mix, several on the
+// 113k snowball and a 100k dam breach): computeL 9 CTAs 1.09 (8: 1.11, 7: 1.17,
+// 6: 1.27), several lanes 7: 0.054 (8: 0.059, 9: 0.065); computeL with the
+// stored constraint and features (the learned solve) 7; pbfA 10: 0.62 (8:
+// 0.66, 9: 0.64, 11: 0.63), pbfB 0.213 (8: 0.225, 11: 0.240), several lanes 8:
+// 0.0416 (10: 0.0449); the update 7: 0.303 (8: 0.337, 6: 0.332, the
+// allocator's choice 0.370).
+constexpr int minComputeL(int lanes) { return lanes == 1 ? 9 : 7; }
+constexpr int kMinComputeLFeatures = 7;
+constexpr int minPbf(int lanes) { return lanes == 1 ? 10 : 8; }
+constexpr int kMinUpdate = 7;
 // solveA and solveB are compiled in several launch shapes — the block size
 // and the minimum resident CTAs per SM asked of the register allocator (0 =
 // its own choice) — and xpbi_autotune picks one per handle by timing them on
@@ -76,17 +66,6 @@ constexpr int kSolveAMinB[kSolveAVariants] = {8, 9, 10, 7, 16, 6};
 constexpr int kSolveABlock[kSolveAVariants] = {128, 128, 128, 128, 64, 128};
 constexpr int kSolveBMinB[kSolveBVariants] = {9, 8, 7, 10, 6};
 constexpr int kSolveBBlock[kSolveBVariants] = {128, 128, 128, 128, 128};
-#ifdef XPBI_MINB_PBF
-#define XPBI_LB_PBF __launch_bounds__(kThreads, XPBI_MINB_PBF)
-#else
-#define XPBI_LB_PBF XPBI_LB_DEFAULT
-#endif
-#ifdef XPBI_MINB_UPDATE
-#define XPBI_LB_UPDATE __launch_bounds__(kThreads, XPBI_MINB_UPDATE)
-#else
-#define XPBI_LB_UPDATE XPBI_LB_DEFAULT
-#endif
-
 struct Ctx {
   const SceneDev* __restrict__ scene;
   const MatDev* __restrict__ mats;  // this scene's 8 materials
@@ -126,25 +105,38 @@ __device__ __forceinline__ T ldg(const T* p) {
 }
 
 // Stencil walk over the 9 row-merged ranges (simkernels.js:62-74):
-// row(beg, end) is called per in-range row.
-template <class Row>
-__device__ __forceinline__ void forRows(const SceneDev& S, const uint32_t* __restrict__ cellStart, V3 x, Row&& row) {
+// row(beg, end) is called per in-range row. With G lanes per slot, lane
+// `lane` takes the rows r with r % G == lane.
+template <int G = 1, class Row>
+__device__ __forceinline__ void forRows(const SceneDev& S, const uint32_t* __restrict__ cellStart, V3 x, Row&& row,
+                                        uint32_t lane = 0) {
   const I3 cc = cellCoord(S, x);
   const int x0 = max(cc.x - 1, 0);
   const int x1 = min(cc.x + 1, S.dims[0] - 1);
+  auto one = [&](int y, int z) {
+    const uint32_t c0 = S.cellBase + cellIndex(S, x0, y, z);
+    const uint32_t c2 = S.cellBase + cellIndex(S, x1, y, z);
+    const uint32_t beg = __ldg(cellStart + c0);
+    const uint32_t end = min(__ldg(cellStart + c2 + 1), beg + kRowCap);
+    row(beg, end);
+  };
+  if constexpr (G == 1) {
 #pragma unroll 1
-  for (int dz = -1; dz <= 1; ++dz) {
-    const int z = cc.z + dz;
-    if (z < 0 || z >= S.dims[2]) continue;
+    for (int dz = -1; dz <= 1; ++dz) {
+      const int z = cc.z + dz;
+      if (z < 0 || z >= S.dims[2]) continue;
 #pragma unroll 1
-    for (int dy = -1; dy <= 1; ++dy) {
-      const int y = cc.y + dy;
-      if (y < 0 || y >= S.dims[1]) continue;
-      const uint32_t c0 = S.cellBase + cellIndex(S, x0, y, z);
-      const uint32_t c2 = S.cellBase + cellIndex(S, x1, y, z);
-      const uint32_t beg = __ldg(cellStart + c0);
-      const uint32_t end = min(__ldg(cellStart + c2 + 1), beg + kRowCap);
-      row(beg, end);
+      for (int dy = -1; dy <= 1; ++dy) {
+        const int y = cc.y + dy;
+        if (y < 0 || y >= S.dims[1]) continue;
+        one(y, z);
+      }
+    }
+  } else {
+#pragma unroll 1
+    for (int r = (int)lane; r < 9; r += G) {
+      const int z = cc.z + r / 3 - 1, y = cc.y + r % 3 - 1;
+      if (z >= 0 && z < S.dims[2] && y >= 0 && y < S.dims[1]) one(y, z);
     }
   }
 }
@@ -175,72 +167,12 @@ __device__ __forceinline__ uint32_t otherCount(uint32_t c) { return (c >> 8) & 0
 __device__ __forceinline__ bool dryCount(uint32_t c) { return (c >> 16) == 1u; }
 
 // Two neighbours at a time over `groups` groups: body(j0, j1, d0, d1) with
-// d = gather(j). The gathers of a pair are issued before the arithmetic of
-// the pair before it, the list's groups one group ahead.
+// d = gather(j); the list's groups are loaded one group ahead. (Keeping the
+// next pair's gathers in flight as well costs 16 registers or more, and the
+// resident warps they displace hide more latency: solveA 0.320 ms per launch
+// without, 0.331 with, on the 4M-particle mix.)
 template <class Gather, class Body>
 __device__ __forceinline__ void forPairs(const uint4* L, uint32_t groups, Gather&& gather, Body&& body) {
-  if (groups == 0u) return;
-  uint4 cur = *(L);
-  uint4 nxt = *(L + kGroupStride * min(1u, groups - 1u));
-  auto a0 = gather(cur.x), a1 = gather(cur.y);
-#pragma unroll 1
-  for (uint32_t q = 1u; q < groups; ++q) {
-    const auto b0 = gather(cur.z), b1 = gather(cur.w);
-    const uint4 nn = *(L + kGroupStride * min(q + 1u, groups - 1u));
-    body(cur.x, cur.y, a0, a1);
-    a0 = gather(nxt.x);
-    a1 = gather(nxt.y);
-    body(cur.z, cur.w, b0, b1);
-    cur = nxt;
-    nxt = nn;
-  }
-  const auto b0 = gather(cur.z), b1 = gather(cur.w);
-  body(cur.x, cur.y, a0, a1);
-  body(cur.z, cur.w, b0, b1);
-}
-
-// One entry at a time: body(j, d) with d = gather(j), the gather of an entry
-// issued before the arithmetic of the one before it (kAhead).
-#ifndef EACH_AHEAD
-#define EACH_AHEAD 0
-#endif
-template <bool kAhead = true, class Gather, class Body>
-__device__ __forceinline__ void forSingles(const uint4* L, uint32_t groups, Gather&& gather, Body&& body) {
-  if (groups == 0u) return;
-  uint4 cur = *(L);
-  if constexpr (kAhead) {
-    uint4 nxt = *(L + kGroupStride * min(1u, groups - 1u));
-    auto d = gather(cur.x);
-#pragma unroll 1
-    for (uint32_t q = 1u; q <= groups; ++q) {
-      auto e = gather(cur.y);
-      body(cur.x, d);
-      d = gather(cur.z);
-      body(cur.y, e);
-      e = gather(cur.w);
-      body(cur.z, d);
-      const uint4 nn = *(L + kGroupStride * min(q + 1u, groups - 1u));
-      d = gather(nxt.x);
-      body(cur.w, e);
-      cur = nxt;
-      nxt = nn;
-    }
-  } else {
-#pragma unroll 1
-    for (uint32_t q = 1u; q <= groups; ++q) {
-      const uint4 nxt = *(L + kGroupStride * min(q, groups - 1u));
-      body(cur.x, gather(cur.x));
-      body(cur.y, gather(cur.y));
-      body(cur.z, gather(cur.z));
-      body(cur.w, gather(cur.w));
-      cur = nxt;
-    }
-  }
-}
-// The same without gathers in flight over a pair's arithmetic (records of
-// many registers).
-template <class Gather, class Body>
-__device__ __forceinline__ void forPairsNow(const uint4* L, uint32_t groups, Gather&& gather, Body&& body) {
   if (groups == 0u) return;
   uint4 cur = *(L);
 #pragma unroll 1
@@ -249,6 +181,38 @@ __device__ __forceinline__ void forPairsNow(const uint4* L, uint32_t groups, Gat
     body(cur.x, cur.y, gather(cur.x), gather(cur.y));
     body(cur.z, cur.w, gather(cur.z), gather(cur.w));
     cur = nxt;
+  }
+}
+// One neighbour at a time: body(j, d) (records of many registers).
+template <class Gather, class Body>
+__device__ __forceinline__ void forSingles(const uint4* L, uint32_t groups, Gather&& gather, Body&& body) {
+  if (groups == 0u) return;
+  uint4 cur = *(L);
+#pragma unroll 1
+  for (uint32_t q = 1u; q <= groups; ++q) {
+    const uint4 nxt = *(L + kGroupStride * min(q, groups - 1u));
+    body(cur.x, gather(cur.x));
+    body(cur.y, gather(cur.y));
+    body(cur.z, gather(cur.z));
+    body(cur.w, gather(cur.w));
+    cur = nxt;
+  }
+}
+
+// A list of `cnt` entries two at a time; with G lanes per slot, lane `lane`
+// takes the pairs p with p % G == lane.
+template <int G, class Gather, class Body>
+__device__ __forceinline__ void forListPairs(const uint4* L, uint32_t cnt, uint32_t lane, Gather&& gather,
+                                             Body&& body) {
+  if constexpr (G == 1) {
+    forPairs(L, (cnt + 3u) >> 2, gather, body);
+  } else {
+    const uint32_t pairs = (cnt + 1u) >> 1;
+#pragma unroll 2
+    for (uint32_t p = lane; p < pairs; p += G) {
+      const uint2 e = *(reinterpret_cast<const uint2*>(L + kGroupStride * (p >> 1)) + (p & 1u));
+      body(e.x, e.y, gather(e.x), gather(e.y));
+    }
   }
 }
 
@@ -260,26 +224,13 @@ __device__ __forceinline__ void forPairsNow(const uint4* L, uint32_t groups, Gat
 // consecutive in the warp; lane `lane` visits the pairs p with p % G == lane
 // (on the walk every G-th candidate of each row) and accumulates a partial
 // sum; laneSum adds them over the group.
-template <int G, bool kAhead = true, class Gather, class Body>
+template <int G, class Gather, class Body>
 __device__ __forceinline__ void forSame(const Bufs& b, const Ctx& cx, uint32_t i, V3 xi, bool iWater, uint32_t lane,
                                         Gather&& gather, Body&& body) {
   static_assert(G == 1 || G == 2 || G == 4, "one, two or four lanes per slot");
   const uint32_t c = b.nbrCount[i];
   if (c != kNbrOverflow) {
-    const uint4* L = nbrGroups(b.nbr, i);
-    if constexpr (G == 1) {
-      if constexpr (kAhead)
-        forPairs(L, (sameCount(c) + 3u) >> 2, gather, body);
-      else
-        forPairsNow(L, (sameCount(c) + 3u) >> 2, gather, body);
-    } else {
-      const uint32_t pairs = (sameCount(c) + 1u) >> 1;
-#pragma unroll 2
-      for (uint32_t p = lane; p < pairs; p += G) {
-        const uint2 e = *(reinterpret_cast<const uint2*>(L + kGroupStride * (p >> 1)) + (p & 1u));
-        body(e.x, e.y, gather(e.x), gather(e.y));
-      }
-    }
+    forListPairs<G>(nbrGroups(b.nbr, i), sameCount(c), lane, gather, body);
   } else {
     const SceneDev& S = *cx.scene;
     uint32_t first = i;  // a neighbour waiting for its partner
@@ -303,14 +254,14 @@ __device__ __forceinline__ void forSame(const Bufs& b, const Ctx& cx, uint32_t i
 }
 
 // A solid's solid neighbours one at a time.
-template <int G, bool kAhead, class Gather, class Body>
+template <int G, class Gather, class Body>
 __device__ __forceinline__ void forSameSingles(const Bufs& b, const Ctx& cx, uint32_t i, V3 xi, uint32_t lane,
                                                Gather&& gather, Body&& body) {
   const uint32_t c = b.nbrCount[i];
   if (c != kNbrOverflow) {
     const uint4* L = nbrGroups(b.nbr, i);
     if constexpr (G == 1) {
-      forSingles<kAhead>(L, (sameCount(c) + 3u) >> 2, gather, body);
+      forSingles(L, (sameCount(c) + 3u) >> 2, gather, body);
     } else {
       const uint32_t pairs = (sameCount(c) + 1u) >> 1;
 #pragma unroll 2
@@ -391,11 +342,11 @@ struct Planes {
 __device__ __forceinline__ Planes planesOf(const float* p, uint32_t stride) {
   return Planes{p, p + stride, p + 2 * (size_t)stride};
 }
-template <class Hit>
+template <int G = 1, class Hit>
 __device__ __forceinline__ void walkCandidates(const SceneDev& S, const uint32_t* __restrict__ cellStart, V3 x,
-                                               uint32_t i, Planes P, V3 c, float s2, Hit&& hit) {
+                                               uint32_t i, Planes P, V3 c, float s2, Hit&& hit, uint32_t lane = 0) {
   const F2 cx = f2(-c.x, -c.x), cy = f2(-c.y, -c.y), cz = f2(-c.z, -c.z), ns2 = f2(-s2, -s2);
-  forRows(S, cellStart, x, [&](uint32_t beg, uint32_t end) {
+  forRows<G>(S, cellStart, x, [&](uint32_t beg, uint32_t end) {
 #pragma unroll 1
     for (uint32_t b0 = beg & ~3u; b0 < end; b0 += 32u) {
       const uint32_t n = min(32u, end - b0);
@@ -426,8 +377,49 @@ __device__ __forceinline__ void walkCandidates(const SceneDev& S, const uint32_t
         hit(b0 + t);
       }
     }
-  });
+  }, lane);
 }
+
+// What a walk with several lanes per slot records before the lists are
+// written: each lane's hits in a column of shared memory, `same` from the top
+// and `other` from the bottom. A lane with more than the column holds loses
+// them (the list then counts as overflowed).
+template <int G>
+struct SubList {
+  static constexpr uint32_t kCap = kNbrCap;
+  uint32_t* col;  // this thread's column, stride kThreads
+  uint32_t same = 0, other = 0;
+  bool lost = false;  // of any of the slot's lanes, after totals()
+  uint32_t sameAll = 0, otherAll = 0, sameBefore = 0, otherBefore = 0;
+  __device__ __forceinline__ uint32_t at(uint32_t e) const { return col[e * kThreads]; }
+  __device__ __forceinline__ uint32_t otherAt(uint32_t e) const { return col[(kCap - 1u - e) * kThreads]; }
+  __device__ __forceinline__ void add(uint32_t j, bool own) {
+    if (same + other >= kCap) {
+      lost = true;
+      return;
+    }
+    col[(own ? same : kCap - 1u - other) * kThreads] = j;
+    same += own ? 1u : 0u;
+    other += own ? 0u : 1u;
+  }
+  // every lane of the slot together
+  __device__ __forceinline__ void totals(uint32_t lane) {
+    const uint32_t warpLane = threadIdx.x & 31u, first = warpLane & ~(uint32_t)(G - 1);
+    const unsigned group = ((1u << G) - 1u) << first;
+#pragma unroll
+    for (uint32_t o = 0; o < (uint32_t)G; ++o) {
+      const uint32_t v = __shfl_sync(group, same | other << 8 | (lost ? 1u << 16 : 0u), (int)(first + o));
+      const uint32_t sv = v & 0xffu, ov = (v >> 8) & 0xffu;
+      sameBefore += o < lane ? sv : 0u;
+      otherBefore += o < lane ? ov : 0u;
+      sameAll += sv;
+      otherAll += ov;
+      anyLost |= v >> 16;
+    }
+    lost = anyLost != 0u;
+  }
+  uint32_t anyLost = 0;
+};
 
 // The offsets of two neighbours from xi and what the sums weigh them by:
 // (dx, dy, dz) = xi - x_b, w = V_b g (dx, dy, dz), so that V_b gradW_b = c w.
@@ -485,15 +477,16 @@ struct VelSum {
 // ---------------------------------------------------------------- computeL
 // L of slot i (simkernels.js:198-220) over its recorded neighbours: the
 // SVD pseudo-inverse of sum V_b (grad W_b) (x_b - x_i)^T, which is symmetric
-// (the gradient points along the offset). For a solid (kSolid) the same sweep
+// (the gradient points along the offset), so its eigenvectors serve. For a solid (kSolid) the same sweep
 // also forms the sums of the constraint passes that no velocity enters —
 // s = sum V_b g_b, P = sum (V_b^2 / m_b) g_b g_b^T and the solid neighbour
 // count, over the solid neighbours — and stores them in sgP for every
 // iteration of the substep. With kVel (a solid, at the velocities iteration 0
 // starts from) the sweep also forms that iteration's velocity sum
 // Av = sum V_b (v_b - v_i) g_b^T — the constraint sweep's own operations.
-template <bool kSolid, bool kVel = false>
-__device__ __forceinline__ void bonetLok(const Bufs& b, const Ctx& cx, uint32_t i, V3 xi, M3* velSum = nullptr) {
+template <bool kSolid, bool kVel = false, int G = 1>
+__device__ __forceinline__ void bonetLok(const Bufs& b, const Ctx& cx, uint32_t i, V3 xi, M3* velSum = nullptr,
+                                         uint32_t lane = 0, const SubList<G>* sub = nullptr) {
   static_assert(kSolid || !kVel, "the velocity sum is a solid's");
   const SceneDev& S = *cx.scene;
   const float4* __restrict__ posS = b.posS;
@@ -515,7 +508,7 @@ __device__ __forceinline__ void bonetLok(const Bufs& b, const Ctx& cx, uint32_t 
     a02 = fma2(r.wx, r.dz, a02);
     a12 = fma2(r.wy, r.dz, a12);
   };
-  forSame<1, L_AHEAD>(b, cx, i, xi, !kSolid, 0u, gather, [&](uint32_t j0, uint32_t j1, const PV& d0, const PV& d1) {
+  auto own = [&](uint32_t j0, uint32_t j1, const PV& d0, const PV& d1) {
     const Pair r = pairOf(S, xi, d0, d1);
     addA(r);
     if constexpr (kSolid) {
@@ -533,54 +526,76 @@ __device__ __forceinline__ void bonetLok(const Bufs& b, const Ctx& cx, uint32_t 
       p12 = fma2(uy, r.wz, p12);
       cnt += (j0 != i ? 1.f : 0.f) + (j1 != i ? 1.f : 0.f);
     }
-  });
-  // the other phase's neighbours enter L alone
-  const uint32_t c = b.nbrCount[i];
-  if (c != kNbrOverflow) {
-    const uint32_t other = (otherCount(c) + 3u) >> 2;
-    if (other)
-      forPairs(nbrGroups(b.nbr, i) + kGroupStride * (kNbrCap / 4u - other), other, gather,
-               [&](uint32_t, uint32_t, const PV& d0, const PV& d1) { addA(pairOf(S, xi, d0, d1)); });
-  } else {
+  };
+  // own phase; the other phase's neighbours enter L alone
+  const uint32_t c = G == 1 ? b.nbrCount[i] : (sub->lost ? kNbrOverflow : 0u);
+  if (c == kNbrOverflow) {
     const PV self = gather(i);
-    forRows(S, b.cellStart, xi, [&](uint32_t beg, uint32_t end) {
+    forRows<G>(S, b.cellStart, xi, [&](uint32_t beg, uint32_t end) {
 #pragma unroll 1
       for (uint32_t j = beg; j < end; ++j) {
         if (j == i) continue;
         const float4 pj = ldg(posS + j);
         const V3 d = xi - xyz(pj);
-        if (dot(d, d) < S.support2 && waterW(pj.w) == kSolid) addA(pairOf(S, xi, gather(j), self));
+        if (!(dot(d, d) < S.support2)) continue;
+        if (waterW(pj.w) == kSolid)
+          addA(pairOf(S, xi, gather(j), self));
+        else
+          own(j, i, gather(j), self);
       }
-    });
+    }, lane);
+  } else if constexpr (G == 1) {
+    forPairs(nbrGroups(b.nbr, i), (sameCount(c) + 3u) >> 2, gather, own);
+    const uint32_t other = (otherCount(c) + 3u) >> 2;
+    if (other)
+      forPairs(nbrGroups(b.nbr, i) + kGroupStride * (kNbrCap / 4u - other), other, gather,
+                  [&](uint32_t, uint32_t, const PV& d0, const PV& d1) { addA(pairOf(S, xi, d0, d1)); });
+  } else {
+#pragma unroll 2
+    for (uint32_t e = 0; e < sub->same; e += 2u) {
+      const uint32_t j0 = sub->at(e), j1 = e + 1u < sub->same ? sub->at(e + 1u) : i;
+      own(j0, j1, gather(j0), gather(j1));
+    }
+    for (uint32_t e = 0; e < sub->other; e += 2u) {
+      const uint32_t j0 = sub->otherAt(e), j1 = e + 1u < sub->other ? sub->otherAt(e + 1u) : i;
+      addA(pairOf(S, xi, gather(j0), gather(j1)));
+    }
   }
   const float gc = S.gradC;
-  const V3 sg = v3(sum2(sx) * gc, sum2(sy) * gc, sum2(sz) * gc);
-  const float c2 = gc * gc;
-  const float q00 = sum2(p00) * c2, q11 = sum2(p11) * c2, q22 = sum2(p22) * c2;
-  const float q01 = sum2(p01) * c2, q02 = sum2(p02) * c2, q12 = sum2(p12) * c2;
-  if constexpr (kSolid) {
-    float4* __restrict__ R = b.sgP + i;
-    const size_t N = b.N;
-    R[0] = make_float4(sg.x, sg.y, sg.z, cnt);
-    R[N] = make_float4(q00, q11, q22, q01);
-    R[2 * N] = make_float4(q02, q12, 0.f, 0.f);
-  }
+  auto total = [&](F2 v) { return laneSum<G>(sum2(v)); };
   // x_b - x_i = -(dx, dy, dz)
-  const float b01 = -gc * sum2(a01), b02 = -gc * sum2(a02), b12 = -gc * sum2(a12);
-  const M3 A = {{v3(-gc * sum2(a00), b01, b02), v3(b01, -gc * sum2(a11), b12), v3(b02, b12, -gc * sum2(a22))}};
-  const SVD s = svd3Fast(A);
+  const float b00 = -gc * total(a00), b11 = -gc * total(a11), b22 = -gc * total(a22);
+  const float b01 = -gc * total(a01), b02 = -gc * total(a02), b12 = -gc * total(a12);
+  if constexpr (kVel) *velSum = Av.template total<G>(gc);
+  if constexpr (kSolid) {
+    const V3 sg = v3(total(sx) * gc, total(sy) * gc, total(sz) * gc);
+    const float c2 = gc * gc;
+    const float q00 = total(p00) * c2, q11 = total(p11) * c2, q22 = total(p22) * c2;
+    const float q01 = total(p01) * c2, q02 = total(p02) * c2, q12 = total(p12) * c2;
+    cnt = laneSum<G>(cnt);
+    if (lane == 0) {
+      float4* __restrict__ R = b.sgP + i;
+      const size_t N = b.N;
+      R[0] = make_float4(sg.x, sg.y, sg.z, cnt);
+      R[N] = make_float4(q00, q11, q22, q01);
+      R[2 * N] = make_float4(q02, q12, 0.f, 0.f);
+    }
+  }
+  if (G > 1 && lane != 0) return;  // lane 0 finishes the slot
+  // the pseudo-inverse of the symmetric moment matrix
+  V3 d;
+  M3 V;
+  eigSym(Sym3{b00, b11, b22, b01, b02, b12}, d, V);
   const float tol = 0.2f;
   V3 inv = splat(0.f);
-  if (fabsf(s.sig.x) > tol) inv.x = __frcp_rn(s.sig.x);
-  if (fabsf(s.sig.y) > tol) inv.y = __frcp_rn(s.sig.y);
-  if (fabsf(s.sig.z) > tol) inv.z = __frcp_rn(s.sig.z);
-  const M3 L = diagMul(s.V, inv, s.U);
-  storeM(b.L, b.N, i, L);
-  if constexpr (kVel) *velSum = Av.total<1>(gc);
+  if (fabsf(d.x) > tol) inv.x = __frcp_rn(d.x);
+  if (fabsf(d.y) > tol) inv.y = __frcp_rn(d.y);
+  if (fabsf(d.z) > tol) inv.z = __frcp_rn(d.z);
+  storeM(b.L, b.N, i, diagMul(V, inv, V));
 }
 // The water particles' L of the last substep, from the same positions,
 // neighbour lists and V^n as k_computeL would have used.
-__global__ void XPBI_LB_COMPUTEL k_computeL_water(Bufs b) {
+__global__ void __launch_bounds__(kThreads, 8) k_computeL_water(Bufs b) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= b.N) return;
   const float4 pi = b.posS[i];
@@ -604,16 +619,18 @@ __device__ __forceinline__ void storeSp(const Bufs& b, uint32_t i, const M3& m, 
   b.SpSelf[i] = make_float4(self.x, self.y, self.z, 0.f);
 }
 
-// velocityGradient (simkernels.js:224-245) of a solid over its solid neighbours.
-__device__ __forceinline__ M3 velocityGradient(const Bufs& b, const Ctx& cx, uint32_t i, V3 xi, V3 vi,
-                                               const float4* __restrict__ velIn) {
+// velocityGradient (simkernels.js:224-245) of a solid over its solid
+// neighbours, without its factor L^T.
+template <int G>
+__device__ __forceinline__ M3 velocitySum(const Bufs& b, const Ctx& cx, uint32_t i, V3 xi, V3 vi,
+                                          const float4* __restrict__ velIn, uint32_t lane) {
   const SceneDev& S = *cx.scene;
   const float4* __restrict__ posS = b.posS;
-  // sum dv_b (L g_b)^T = (sum dv_b g_b^T) L^T: L applied once, after the loop
+  // sum dv_b (L g_b)^T = (sum dv_b g_b^T) L^T: L applied once, by the caller
   VelSum A;
-  forSame<1>(b, cx, i, xi, false, 0u, [&](uint32_t j) { return PV{ldg(posS + j), ldg(velIn + j)}; },
+  forSame<G>(b, cx, i, xi, false, lane, [&](uint32_t j) { return PV{ldg(posS + j), ldg(velIn + j)}; },
              [&](uint32_t, uint32_t, const PV& d0, const PV& d1) { A.add(pairOf(S, xi, d0, d1), vi, d0.v, d1.v); });
-  return mul(A.total<1>(S.gradC), transpose(loadM(b.L, b.N, i)));
+  return A.template total<G>(S.gradC);
 }
 
 // ---------------------------------------------------------------- solveA
@@ -669,7 +686,7 @@ __device__ __forceinline__ Constraint evalConstraint(const Bufs& b, const Ctx& c
   // products factored out of the pair loop). s, P and the count do not depend
   // on the velocities: computeL formed them, so the sweep only accumulates A.
   VelSum A;
-  forSame<NL, A_AHEAD>(b, cx, i, xi, false, lane, [&](uint32_t j) { return PV{ldg(posS + j), ldg(velIn + j)}; },
+  forSame<NL>(b, cx, i, xi, false, lane, [&](uint32_t j) { return PV{ldg(posS + j), ldg(velIn + j)}; },
               [&](uint32_t, uint32_t, const PV& d0, const PV& d1) { A.add(pairOf(S, xi, d0, d1), vi, d0.v, d1.v); });
   const M3 At = A.template total<NL>(S.gradC);
   if (NL > 1 && lane != 0) return Constraint{};  // lane 0 finishes the slot
@@ -688,12 +705,16 @@ __device__ __noinline__ Constraint constraintTail(M3 A, TailIn in, const SceneDe
   const float4* __restrict__ R = in.sgP + in.i;
   const float hard = hardening(m, st);
   const float mu = m.mu * hard, lam = m.lam * hard;
-  const M3 Ftr = madd(Fn, mscale(mul(mul(A, transpose(Li)), Fn), S.dt));
-  const SVD sd = svd3Fast(Ftr);
+  // the trial F minus the identity, which keeps the digits of a small strain
+  const M3 Htr = madd(minusIdent(Fn), mscale(mul(mul(A, transpose(Li)), Fn), S.dt));
+  V3 eTr;
+  const SVD sd = strainSVD(Htr, eTr);
   Constraint out;
-  out.logSigTr = vlog(safeSig(sd.sig));
+  out.logSigTr = v3(fmaxf(fmaxf(eTr.x, eTr.y), eTr.z),
+                    fmaxf(fminf(eTr.x, eTr.y), fminf(fmaxf(eTr.x, eTr.y), eTr.z)),
+                    fminf(fminf(eTr.x, eTr.y), eTr.z));  // descending
   float stOut;
-  const Mapped mp2 = returnMap(sd.sig, out.logSigTr, m, mu, lam, st, S.dt, stOut);
+  const Mapped mp2 = returnMap(sd.sig, eTr, m, mu, lam, st, S.dt, stOut);
   const V3 e = mp2.e;
   const float tr = e.x + e.y + e.z;
   out.C = sqrtf(fmaxf(2.f * stvkPsi(e, mu, lam), 0.f));
@@ -1118,11 +1139,15 @@ __device__ __forceinline__ void storeFeatures(const Bufs& b, uint32_t i, const f
 // k_solveA_stored here, with the network's features (fillFeatures; zeros
 // for water and for scenes without iterations), without a second sweep of
 // every solid's neighbours.
-template <bool kFeatures>
+// G lanes per slot (small handles): the lanes split the stencil's rows and the
+// sums over what they find, lane 0 finishes the slot.
+template <bool kFeatures, int G>
 __device__ __forceinline__ void computeL(const Bufs& b) {
+  __shared__ uint32_t column[G == 1 ? 1 : SubList<G>::kCap * kThreads];
   // blocks run last to first: the pass starts where the reorder ended, on
   // slots whose data is still in L2
-  const uint32_t i = (gridDim.x - 1u - blockIdx.x) * blockDim.x + threadIdx.x;
+  const uint32_t t = (gridDim.x - 1u - blockIdx.x) * blockDim.x + threadIdx.x;
+  const uint32_t i = t / G, lane = t % G;
   if (i >= b.N) return;
   const Ctx cx = ctxOf(b, i);
   const SceneDev& S = *cx.scene;
@@ -1131,39 +1156,62 @@ __device__ __forceinline__ void computeL(const Bufs& b) {
   const V3 xi = xyz(pi);
   const float s2 = S.support2;
   // own phase from the front, the other one from the back (the water flag is
-  // the sign bit of pos.w); a list past the capacity is marked as overflowed
-  // and never read, its last entries land anywhere in it
+  // the sign bit of pos.w; no load for it in a scene of one phase); a list past
+  // the capacity is marked as overflowed and never read, its last entries land
+  // anywhere in it
+  auto isOwn = [&](uint32_t j) {
+    return S.onePhase || ((__float_as_uint(ldg(&posS[j].w)) ^ __float_as_uint(pi.w)) & kWaterBit) == 0u;
+  };
+  SubList<G> sub;
   uint32_t same = 0, other = 0;
-  walkCandidates(S, b.cellStart, xi, i, planesOf(b.posP, b.planeN), xi, s2, [&](uint32_t j) {
-    const bool own = ((__float_as_uint(ldg(&posS[j].w)) ^ __float_as_uint(pi.w)) & kWaterBit) == 0u;
-    const uint32_t e = own ? same : ~other;
-    *nbrEntry(b.nbr, i, e & (kNbrCap - 1u)) = j;
-    same += own ? 1u : 0u;
-    other += own ? 0u : 1u;
-  });
+  if constexpr (G == 1) {
+    walkCandidates(S, b.cellStart, xi, i, planesOf(b.posP, b.planeN), xi, s2, [&](uint32_t j) {
+      const bool own = isOwn(j);
+      const uint32_t e = own ? same : ~other;
+      *nbrEntry(b.nbr, i, e & (kNbrCap - 1u)) = j;
+      same += own ? 1u : 0u;
+      other += own ? 0u : 1u;
+    });
+  } else {
+    sub.col = column + threadIdx.x;
+    walkCandidates<G>(S, b.cellStart, xi, i, planesOf(b.posP, b.planeN), xi, s2,
+                      [&](uint32_t j) { sub.add(j, isOwn(j)); }, lane);
+    sub.totals(lane);
+    same = sub.sameAll;
+    other = sub.otherAll;
+  }
   const uint32_t same4 = (same + 3u) & ~3u, other4 = (other + 3u) & ~3u;
-  const bool fits = same4 + other4 <= kNbrCap;
+  const bool fits = same4 + other4 <= kNbrCap && !sub.lost;
   if (fits) {
-    for (uint32_t e = same; e < same4; ++e) *nbrEntry(b.nbr, i, e) = i;
-    for (uint32_t e = other; e < other4; ++e) *nbrEntry(b.nbr, i, kNbrCap - 1u - e) = i;
+    if constexpr (G > 1) {
+      for (uint32_t e = 0; e < sub.same; ++e) *nbrEntry(b.nbr, i, sub.sameBefore + e) = sub.at(e);
+      for (uint32_t e = 0; e < sub.other; ++e)
+        *nbrEntry(b.nbr, i, kNbrCap - 1u - sub.otherBefore - e) = sub.otherAt(e);
+    }
+    if (lane == 0) {
+      for (uint32_t e = same; e < same4; ++e) *nbrEntry(b.nbr, i, e) = i;
+      for (uint32_t e = other; e < other4; ++e) *nbrEntry(b.nbr, i, kNbrCap - 1u - e) = i;
+    }
   }
-  uint32_t dry = 0u;
-  if (S.hasWater && !waterW(pi.w) && fits) {  // for the PBF passes
-    const I3 cc = cellCoord(S, xi);
-    dry = 1u;
+  if (lane == 0) {
+    uint32_t dry = 0u;
+    if (S.hasWater && !waterW(pi.w) && fits && other == 0u) {  // for the PBF passes
+      const I3 cc = cellCoord(S, xi);
+      dry = 1u;
 #pragma unroll
-    for (int dz = -1; dz <= 1; ++dz)
+      for (int dz = -1; dz <= 1; ++dz)
 #pragma unroll
-      for (int dy = -1; dy <= 1; ++dy)
+        for (int dy = -1; dy <= 1; ++dy)
 #pragma unroll
-        for (int dx = -1; dx <= 1; ++dx) {
-          const int x = cc.x + dx, y = cc.y + dy, z = cc.z + dz;
-          if (x >= 0 && x < S.dims[0] && y >= 0 && y < S.dims[1] && z >= 0 && z < S.dims[2] &&
-              __ldg(b.cellWater + S.cellBase + cellIndex(S, x, y, z)) != 0)
-            dry = 0u;
-        }
+          for (int dx = -1; dx <= 1; ++dx) {
+            const int x = cc.x + dx, y = cc.y + dy, z = cc.z + dz;
+            if (x >= 0 && x < S.dims[0] && y >= 0 && y < S.dims[1] && z >= 0 && z < S.dims[2] &&
+                __ldg(b.cellWater + S.cellBase + cellIndex(S, x, y, z)) != 0)
+              dry = 0u;
+          }
+    }
+    b.nbrCount[i] = fits ? same | other << 8 | dry << 16 : kNbrOverflow;
   }
-  b.nbrCount[i] = fits ? same | other << 8 | dry << 16 : kNbrOverflow;
   // no pass of the substep reads a water particle's correction (every
   // velocity gradient is a solid's): k_computeL_water forms it when the state
   // is read
@@ -1173,7 +1221,8 @@ __device__ __forceinline__ void computeL(const Bufs& b) {
     for (int q = 0; q < kFeat; ++q) f[q] = 0.f;
     if (!waterW(pi.w)) {
       M3 Av;
-      bonetLok<true, true>(b, cx, i, xi, &Av);
+      bonetLok<true, true, G>(b, cx, i, xi, &Av, lane, &sub);
+      if (G > 1 && lane != 0) return;
       if (S.iterations > 0) {
         const uint32_t mi = matOfW(pi.w);
         const float st = b.stateS[i];
@@ -1183,13 +1232,20 @@ __device__ __forceinline__ void computeL(const Bufs& b) {
         fillFeatures(f, S, c, b.lamPrev[i], m.kind, m.mu * hardening(m, st));
       }
     }
+    if (G > 1 && lane != 0) return;
     storeFeatures(b, i, f);
   } else {
-    if (!waterW(pi.w)) bonetLok<true>(b, cx, i, xi);
+    if (!waterW(pi.w)) bonetLok<true, false, G>(b, cx, i, xi, nullptr, lane, &sub);
   }
 }
-__global__ void XPBI_LB_COMPUTEL k_computeL(Bufs b) { computeL<false>(b); }
-__global__ void XPBI_LB_COMPUTEL_FEATURES k_computeL_features(Bufs b) { computeL<true>(b); }
+template <int G>
+__global__ void __launch_bounds__(kThreads, minComputeL(G)) k_computeL(Bufs b) {
+  computeL<false, G>(b);
+}
+template <int G>
+__global__ void __launch_bounds__(kThreads, kMinComputeLFeatures) k_computeL_features(Bufs b) {
+  computeL<true, G>(b);
+}
 
 // lambda_warm = previous multiplier + network output / alphaT (the network
 // predicts alphaT times the increment over the previous substep's multiplier)
@@ -1416,8 +1472,18 @@ __device__ __forceinline__ V3 applyBoundary(const SceneDev& S, V3 xcIn, V3 vIn, 
 struct SBData {
   float4 r0, r1, r2;  // a neighbour's dlam G L columns with its position in .w (the record's first planes)
 };
-__device__ __forceinline__ SBData gatherSp(const float4* __restrict__ R, size_t N) {
-  return SBData{ldg(R), ldg(R + N), ldg(R + 2 * N)};
+// ... and, with several lanes per slot (small scenes, where a dependent load
+// costs more than its bytes), its predicted position and mass
+struct SBData4 : SBData {
+  float4 r3;
+};
+template <int G>
+__device__ __forceinline__ auto gatherSp(const float4* __restrict__ R, size_t N) {
+  if constexpr (G == 1) {
+    return SBData{ldg(R), ldg(R + N), ldg(R + 2 * N)};
+  } else {
+    return SBData4{{ldg(R), ldg(R + N), ldg(R + 2 * N)}, ldg(R + 3 * N)};
+  }
 }
 
 // sum over the neighbours b of S_b g_b (S_b = dlam G L of b, the kernel
@@ -1501,10 +1567,14 @@ __global__ void __launch_bounds__(kBlock, kMinB) k_solveB(Bufs b, int k, const f
                         1.01f;
     const float reach2 = reach * reach;
     ImpulseSum sum;
-    auto body = [&](uint32_t j, const SBData& d) {
+    auto body = [&](uint32_t j, const auto& d) {
       const float r2 = sum.add(S, xi, d);
       if (!(r2 < reach2) || j == i) return;
-      const float4 r3 = ldg(Sp + 3 * N + j);
+      float4 r3;
+      if constexpr (G == 1)
+        r3 = ldg(Sp + 3 * N + j);
+      else
+        r3 = d.r3;
       const V3 dxc = xci - xyz(r3);
       const float d2 = dot(dxc, dxc);
       if (d2 < minD * minD && d2 > 1e-18f) {
@@ -1515,7 +1585,7 @@ __global__ void __launch_bounds__(kBlock, kMinB) k_solveB(Bufs b, int k, const f
         corr = corr + dxc * (rinv * ((minD - dist) * w));
       }
     };
-    forSameSingles<G, EACH_AHEAD>(b, cx, i, xi, lane, [&](uint32_t j) { return gatherSp(Sp + j, N); }, body);
+    forSameSingles<G>(b, cx, i, xi, lane, [&](uint32_t j) { return gatherSp<G>(Sp + j, N); }, body);
     const V3 self = xyz(b.SpSelf[i]);
     const float k = Vi * S.gradC;
     if constexpr (G > 1) {
@@ -1731,28 +1801,30 @@ __device__ __forceinline__ bool pbfActive(const SceneDev& S, int k) {
   return S.hasWater && k < S.pbfUntil;
 }
 
-// The PBF pair sums, two predicted neighbours per packed instruction: offset,
-// r^2, the poly6 argument x = H^2 - r^2 cubed, and the radial factor of the
-// spiky gradient, t^2 / r with t = H - r (0 below r = 1e-9, the reference's
-// zero-distance guard). The kernels' constants multiply the sums after the
-// loop.
+// The PBF pair terms of two predicted neighbours per packed instruction: the
+// offset, the poly6 kernel of r^2 and the spiky gradient (0 below r = 1e-9,
+// the reference's zero-distance guard).
+//
+// The density solve amplifies rounding: each pass feeds its positions to the
+// next, through fourth powers. Sums packed in another order left the
+// velocities of a 1M-particle dam with 15 density passes 2.8e-5 (2-norm) from
+// the scalar sums after two substeps. So every rounding here is written out,
+// and the sums add their terms one neighbour after the other in stencil order
+// (with one lane per slot): packing changes no bit. It costs pbfB nothing and
+// pbfA 1% against packed accumulators.
 struct PbfPair {
-  F2 dx, dy, dz, x3, f;
+  F2 w6, gx, gy, gz;
 };
 __device__ __forceinline__ float invDist(float r2) { return r2 < 1e-18f ? 0.f : rsqrtf(r2); }
 __device__ __forceinline__ PbfPair pbfPair(const SceneDev& S, V3 c, const float4& p, const float4& q) {
-  PbfPair r;
-  r.dx = f2(c.x - p.x, c.x - q.x);
-  r.dy = f2(c.y - p.y, c.y - q.y);
-  r.dz = f2(c.z - p.z, c.z - q.z);
-  const F2 r2 = fma2(r.dz, r.dz, fma2(r.dy, r.dy, mul2(r.dx, r.dx)));
+  const F2 dx = f2(c.x - p.x, c.x - q.x), dy = f2(c.y - p.y, c.y - q.y), dz = f2(c.z - p.z, c.z - q.z);
+  const F2 r2 = fma2(dz, dz, fma2(dx, dx, mul2(dy, dy)));
   const F2 minus = f2(-1.f, -1.f);
   const F2 x = fma2(r2, minus, f2(S.support2, S.support2));
-  r.x3 = mul2(mul2(x, x), x);
   const F2 rinv = f2(invDist(lo2(r2)), invDist(hi2(r2)));
   const F2 t = fma2(mul2(r2, rinv), minus, f2(S.support, S.support));
-  r.f = mul2(mul2(t, t), rinv);
-  return r;
+  const F2 s = mul2(mul2(mul2(f2(S.spikyC, S.spikyC), t), t), rinv);
+  return PbfPair{mul2(mul2(mul2(f2(S.poly6C, S.poly6C), x), x), x), mul2(dx, s), mul2(dy, s), mul2(dz, s)};
 }
 
 // ---------------------------------------------------------------- pbfA
@@ -1760,8 +1832,13 @@ __device__ __forceinline__ PbfPair pbfPair(const SceneDev& S, V3 c, const float4
 // the current cell with predicted positions and records, in order, the
 // predicted neighbours of this pass: all of them for water, the water ones
 // for solids (the pairs pbfB uses, simkernels.js:457-458).
-__global__ void XPBI_LB_PBF k_pbfA(Bufs b, int k, int flags) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+// G lanes per slot (small handles): the lanes split the stencil's rows and the
+// density sums over what they find, lane 0 finishes the slot.
+template <int G>
+__global__ void __launch_bounds__(kThreads, minPbf(G)) k_pbfA(Bufs b, int k, int flags) {
+  __shared__ uint32_t column[G == 1 ? 1 : SubList<G>::kCap * kThreads];
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t i = t / G, lane = t % G;
   if (i >= b.N) return;
   const Ctx cx = ctxOf(b, i);
   const SceneDev& S = *cx.scene;
@@ -1773,7 +1850,7 @@ __global__ void XPBI_LB_PBF k_pbfA(Bufs b, int k, int flags) {
     // a solid only pairs with water here; its candidates come from its 27
     // cells, and computeL found no water particle in them: nothing to record
     // in any pass of the substep (no water particle pairs with it either)
-    if (k == 0) {
+    if (k == 0 && lane == 0) {
       b.nbrPCount[i] = 0u;
       b.pbfLam[i] = 0.f;
     }
@@ -1783,73 +1860,107 @@ __global__ void XPBI_LB_PBF k_pbfA(Bufs b, int k, int flags) {
   const float s2 = S.support2;
   // water pairs with everything, a solid with water only (the water flag is
   // the sign bit of xc.w, the sorted pos.w)
+  SubList<G> sub;
+  sub.col = column + threadIdx.x;
   uint32_t cnt = 0;
   auto record = [&](uint32_t j) {
-    *nbrEntry(b.nbrP, i, min(cnt, kNbrCap - 1u)) = j;
-    ++cnt;
+    if constexpr (G == 1) {
+      *nbrEntry(b.nbrP, i, min(cnt, kNbrCap - 1u)) = j;
+      ++cnt;
+    } else {
+      sub.add(j, true);
+    }
   };
+  const Planes P = planesOf(b.xcP, b.planeN);
   if (iWater)
-    walkCandidates(S, b.cellStart, xyz(pi), i, planesOf(b.xcP, b.planeN), xci, s2, record);
+    walkCandidates<G>(S, b.cellStart, xyz(pi), i, P, xci, s2, record, lane);
   else
-    walkCandidates(S, b.cellStart, xyz(pi), i, planesOf(b.xcP, b.planeN), xci, s2, [&](uint32_t j) {
+    walkCandidates<G>(S, b.cellStart, xyz(pi), i, P, xci, s2, [&](uint32_t j) {
       if (waterW(ldg(&xcS[j].w))) record(j);
-    });
-  const uint32_t stored = cnt <= kNbrCap ? cnt : kNbrOverflow;
-  if (stored != kNbrOverflow)  // whole groups
-    for (uint32_t e = cnt; e & 3u; ++e) *nbrEntry(b.nbrP, i, e) = i;
-  b.nbrPCount[i] = stored;
+    }, lane);
+  if constexpr (G > 1) {
+    sub.totals(lane);
+    cnt = sub.sameAll;
+  }
+  const uint32_t stored = cnt <= kNbrCap && !sub.lost ? cnt : kNbrOverflow;
+  if (stored != kNbrOverflow) {
+    if constexpr (G > 1)
+      for (uint32_t e = 0; e < sub.same; ++e) *nbrEntry(b.nbrP, i, sub.sameBefore + e) = sub.at(e);
+    if (lane == 0)  // whole groups
+      for (uint32_t e = cnt; e & 3u; ++e) *nbrEntry(b.nbrP, i, e) = i;
+  }
+  if (lane == 0) b.nbrPCount[i] = stored;
   if (!iWater) {
-    b.pbfLam[i] = 0.f;
-    b.pbfRec[i] = make_float4(xci.x, xci.y, xci.z, 0.f);
+    if (lane == 0) {
+      b.pbfLam[i] = 0.f;
+      b.pbfRec[i] = make_float4(xci.x, xci.y, xci.z, 0.f);
+    }
     return;
   }
   const MatDev& m = cx.mats[matOfW(pi.w)];
   const float rho0 = m.density;
   const float invRho0 = __frcp_rn(rho0);
-  // sums of m_b x^3, m_b f dx and their squares; a padding entry (i itself)
-  // and, on the stencil walk, the second of each pair weigh 0
-  F2 rho = 0ull, gx = 0ull, gy = 0ull, gz = 0ull, g2 = 0ull;
-  auto add = [&](const float4& p, const float4& q, F2 mass) {
+  // a padding entry (i itself) and, on the stencil walk, the second of each
+  // pair weigh 0
+  float rho = G == 1 || lane == 0 ? m.mass * S.w00 : 0.f;
+  V3 gradSum = splat(0.f);
+  float grad2 = 0.f;
+  auto add = [&](const float4& p, const float4& q, float m0, float m1) {
     const PbfPair r = pbfPair(S, xci, p, q);
-    rho = fma2(r.x3, mass, rho);
-    const F2 f = mul2(r.f, mass);
-    const F2 ux = mul2(r.dx, f), uy = mul2(r.dy, f), uz = mul2(r.dz, f);
-    gx = add2(gx, ux);
-    gy = add2(gy, uy);
-    gz = add2(gz, uz);
-    g2 = fma2(ux, ux, fma2(uy, uy, fma2(uz, uz, g2)));
+    rho = __fmaf_rn(m0, lo2(r.w6), rho);
+    rho = __fmaf_rn(m1, hi2(r.w6), rho);
+    const F2 k = f2(__fmul_rn(m0, invRho0), __fmul_rn(m1, invRho0));
+    const F2 ux = mul2(r.gx, k), uy = mul2(r.gy, k), uz = mul2(r.gz, k);
+    gradSum.x = __fadd_rn(__fadd_rn(gradSum.x, lo2(ux)), hi2(ux));
+    gradSum.y = __fadd_rn(__fadd_rn(gradSum.y, lo2(uy)), hi2(uy));
+    gradSum.z = __fadd_rn(__fadd_rn(gradSum.z, lo2(uz)), hi2(uz));
+    const F2 u2 = fma2(uz, uz, fma2(ux, ux, mul2(uy, uy)));
+    grad2 = __fadd_rn(__fadd_rn(grad2, lo2(u2)), hi2(u2));
   };
   auto massOf = [&](float w) { return cx.mats[matOfW(w)].mass; };
   auto gather = [&](uint32_t j) { return ldg(xcS + j); };
+  // the pairs of the list (with several lanes, of this lane's part of it)
+  auto pairs = [&](auto&& body) {
+    if constexpr (G == 1) {
+      forPairs(nbrGroups(b.nbrP, i), (stored + 3u) >> 2, gather, body);
+    } else {
+#pragma unroll 2
+      for (uint32_t e = 0; e < sub.same; e += 2u) {
+        const uint32_t j0 = sub.at(e), j1 = e + 1u < sub.same ? sub.at(e + 1u) : i;
+        body(j0, j1, gather(j0), gather(j1));
+      }
+    }
+  };
   if (stored != kNbrOverflow) {
-    const uint4* L = nbrGroups(b.nbrP, i);
-    const uint32_t groups = (stored + 3u) >> 2;
     if (S.twoMasses) {  // one water and at most one solid material: the sign of xc.w tells a neighbour's mass
       const float mW = S.massW, mS = S.massS;
-      forPairsNow(L, groups, gather, [&](uint32_t j0, uint32_t j1, const float4& p, const float4& q) {
-        add(p, q, f2(j0 == i ? 0.f : (waterW(p.w) ? mW : mS), j1 == i ? 0.f : (waterW(q.w) ? mW : mS)));
+      pairs([&](uint32_t j0, uint32_t j1, const float4& p, const float4& q) {
+        add(p, q, j0 == i ? 0.f : (waterW(p.w) ? mW : mS), j1 == i ? 0.f : (waterW(q.w) ? mW : mS));
       });
     } else {
-      forPairsNow(L, groups, gather, [&](uint32_t j0, uint32_t j1, const float4& p, const float4& q) {
-        add(p, q, f2(j0 == i ? 0.f : massOf(p.w), j1 == i ? 0.f : massOf(q.w)));
+      pairs([&](uint32_t j0, uint32_t j1, const float4& p, const float4& q) {
+        add(p, q, j0 == i ? 0.f : massOf(p.w), j1 == i ? 0.f : massOf(q.w));
       });
     }
   } else {
-    forRows(S, b.cellStart, xyz(pi), [&](uint32_t beg, uint32_t end) {
+    forRows<G>(S, b.cellStart, xyz(pi), [&](uint32_t beg, uint32_t end) {
 #pragma unroll 1
       for (uint32_t j = beg; j < end; ++j) {
         if (j == i) continue;
         const float4 c = ldg(xcS + j);
         const V3 d = xci - xyz(c);
-        if (dot(d, d) < s2) add(c, c, f2(massOf(c.w), 0.f));
+        if (dot(d, d) < s2) add(c, c, massOf(c.w), 0.f);
       }
-    });
+    }, lane);
   }
-  const float k6 = S.poly6C, kg = S.spikyC * invRho0;
-  const V3 gradSum = v3(sum2(gx), sum2(gy), sum2(gz)) * kg;
-  const float dens = m.mass * S.w00 + k6 * sum2(rho);
-  const float C = fmaxf(dens * invRho0 - 1.f, 0.f);
-  const float lam = -C / (kg * kg * sum2(g2) + dot(gradSum, gradSum) + S.pbfEps);
+  if constexpr (G > 1) {
+    rho = laneSum<G>(rho);
+    gradSum = laneSum<G>(gradSum);
+    grad2 = laneSum<G>(grad2);
+    if (lane != 0) return;
+  }
+  const float C = fmaxf(__fmaf_rn(rho, invRho0, -1.f), 0.f);
+  const float lam = -C / (grad2 + dot(gradSum, gradSum) + S.pbfEps);
   b.pbfLam[i] = lam;
   b.pbfRec[i] = make_float4(xci.x, xci.y, xci.z, lam);
 }
@@ -1857,10 +1968,12 @@ __global__ void XPBI_LB_PBF k_pbfA(Bufs b, int k, int flags) {
 // ---------------------------------------------------------------- pbfB
 // PBF position correction with s_corr (simkernels.js:441-477) over pbfA's
 // record of predicted neighbours.
-__global__ void XPBI_LB_PBF k_pbfB(Bufs b, int k, const float4* velIn, float4* velOut, int flags) {
+template <int G>
+__global__ void __launch_bounds__(kThreads, minPbf(G)) k_pbfB(Bufs b, int k, const float4* velIn, float4* velOut, int flags) {
   // blocks run last to first: the pass starts where pbfA ended, on
   // slots whose data is still in L2
-  const uint32_t i = (gridDim.x - 1u - blockIdx.x) * blockDim.x + threadIdx.x;
+  const uint32_t t = (gridDim.x - 1u - blockIdx.x) * blockDim.x + threadIdx.x;
+  const uint32_t i = t / G, lane = t % G;
   if (i >= b.N) return;
   const Ctx cx = ctxOf(b, i);
   const SceneDev& S = *cx.scene;
@@ -1870,7 +1983,7 @@ __global__ void XPBI_LB_PBF k_pbfB(Bufs b, int k, const float4* velIn, float4* v
   const bool iWater = waterW(pi.w);
   // no pass, or a solid without pairs: nothing moves it
   if (!pbfActive(S, k) || ((flags & kRerun) && !b.rerun[sceneIndex(b, cx)]) || (cnt == 0u && !iWater)) {
-    velOut[i] = vi4;
+    if (lane == 0) velOut[i] = vi4;
     return;
   }
   const float4* __restrict__ xcS = b.xc;
@@ -1878,44 +1991,48 @@ __global__ void XPBI_LB_PBF k_pbfB(Bufs b, int k, const float4* velIn, float4* v
   const V3 xci = xyz(xcS[i]);
   const float li = b.pbfLam[i];
   const MatDev& mWi = cx.mats[mi];
-  // sum of (lambda_i + lambda_b + s_corr) mpd_b f dx, s_corr = -k (W / W0)^4
-  F2 px = 0ull, py = 0ull, pz = 0ull;
-  const float rel = S.poly6C * S.invW0, nk = -S.sCorrK;
-  auto add = [&](const float4& p, const float4& q, F2 lb, F2 mpd) {
+  // sum of (lambda_i + lambda_b + s_corr) gradW mpd_b, s_corr = -k (W / W0)^4
+  V3 dp = splat(0.f);
+  const float nk = -S.sCorrK;
+  auto add = [&](const float4& p, const float4& q, F2 lb, float mpd0, float mpd1) {
     const PbfPair r = pbfPair(S, xci, p, q);
-    const F2 w = mul2(r.x3, f2(rel, rel));
+    const F2 w = mul2(r.w6, f2(S.invW0, S.invW0));
     const F2 w2 = mul2(w, w);
-    const F2 s = mul2(mul2(fma2(mul2(w2, w2), f2(nk, nk), add2(lb, f2(li, li))), r.f), mpd);
-    px = fma2(r.dx, s, px);
-    py = fma2(r.dy, s, py);
-    pz = fma2(r.dz, s, pz);
+    const F2 f = fma2(mul2(w2, w2), f2(nk, nk), add2(f2(li, li), lb));
+    const F2 ux = mul2(f, r.gx), uy = mul2(f, r.gy), uz = mul2(f, r.gz);
+    dp.x = __fmaf_rn(hi2(ux), mpd1, __fmaf_rn(lo2(ux), mpd0, dp.x));
+    dp.y = __fmaf_rn(hi2(uy), mpd1, __fmaf_rn(lo2(uy), mpd0, dp.y));
+    dp.z = __fmaf_rn(hi2(uz), mpd1, __fmaf_rn(lo2(uz), mpd0, dp.z));
   };
   // a pair weighs by its water particle's mass / density
   auto mpdOf = [&](float w) { return waterW(w) ? cx.mats[matOfW(w)].massPerDensity : mWi.massPerDensity; };
   if (cnt != kNbrOverflow && S.waterMpd > 0.f) {
     // one water material: every pair weighs by its mass / density, and one
     // gather of pbfA's record (predicted position, multiplier) serves a pair
-    const F2 mpd = f2(S.waterMpd, S.waterMpd);
-    forPairsNow(nbrGroups(b.nbrP, i), (cnt + 3u) >> 2, [&](uint32_t j) { return ldg(b.pbfRec + j); },
-                [&](uint32_t, uint32_t, const float4& p, const float4& q) { add(p, q, f2(p.w, q.w), mpd); });
+    const float mpd = S.waterMpd;
+    forListPairs<G>(nbrGroups(b.nbrP, i), cnt, lane, [&](uint32_t j) { return ldg(b.pbfRec + j); },
+                    [&](uint32_t, uint32_t, const float4& p, const float4& q) { add(p, q, f2(p.w, q.w), mpd, mpd); });
   } else if (cnt != kNbrOverflow) {
-    forPairsNow(nbrGroups(b.nbrP, i), (cnt + 3u) >> 2, [&](uint32_t j) { return ldg(xcS + j); },
-                [&](uint32_t j0, uint32_t j1, const float4& p, const float4& q) {
-                  add(p, q, f2(ldg(b.pbfLam + j0), ldg(b.pbfLam + j1)), f2(mpdOf(p.w), mpdOf(q.w)));
-                });
+    forListPairs<G>(nbrGroups(b.nbrP, i), cnt, lane, [&](uint32_t j) { return ldg(xcS + j); },
+                    [&](uint32_t j0, uint32_t j1, const float4& p, const float4& q) {
+                      add(p, q, f2(ldg(b.pbfLam + j0), ldg(b.pbfLam + j1)), mpdOf(p.w), mpdOf(q.w));
+                    });
   } else {
-    forRows(S, b.cellStart, xyz(pi), [&](uint32_t beg, uint32_t end) {
+    forRows<G>(S, b.cellStart, xyz(pi), [&](uint32_t beg, uint32_t end) {
 #pragma unroll 1
       for (uint32_t j = beg; j < end; ++j) {
         if (j == i) continue;
         const float4 c = ldg(xcS + j);
         if (!(iWater || waterW(c.w))) continue;
         const V3 d = xci - xyz(c);
-        if (dot(d, d) < S.support2) add(c, c, f2(ldg(b.pbfLam + j), 0.f), f2(mpdOf(c.w), 0.f));
+        if (dot(d, d) < S.support2) add(c, c, f2(ldg(b.pbfLam + j), 0.f), mpdOf(c.w), 0.f);
       }
-    });
+    }, lane);
   }
-  const V3 dp = v3(sum2(px), sum2(py), sum2(pz)) * S.spikyC;
+  if constexpr (G > 1) {
+    dp = laneSum<G>(dp);
+    if (lane != 0) return;
+  }
   const float scale = iWater ? 1.f : 0.5f;
   V3 v = xyz(vi4) + dp * (scale / S.dt);
   // active set: a water particle's boundary, which the next solveB would
@@ -1937,9 +2054,10 @@ __global__ void XPBI_LB_PBF k_pbfB(Bufs b, int k, const float4* velIn, float4* v
 
 // ---------------------------------------------------------------- xsph
 // simkernels.js:480-507
-__global__ void XPBI_LB_UPDATE k_xsph(Bufs b, const float4* __restrict__ velIn,
-                                                    float4* __restrict__ velOut) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+template <int G>
+__global__ void __launch_bounds__(kThreads) k_xsph(Bufs b, const float4* __restrict__ velIn, float4* __restrict__ velOut) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t i = t / G, lane = t % G;
   if (i >= b.N) return;
   const Ctx cx = ctxOf(b, i);
   const SceneDev& S = *cx.scene;
@@ -1949,21 +2067,29 @@ __global__ void XPBI_LB_UPDATE k_xsph(Bufs b, const float4* __restrict__ velIn,
   const float4 vi4 = velIn[i];
   const V3 vi = xyz(vi4);
   const bool iWater = waterW(pi.w);
-  // W = sigW t^4 (2 q + 1) with t = 1 - q / 2, so 2 q + 1 = 5 - 4 t
-  F2 ax = 0ull, ay = 0ull, az = 0ull;
-  forSame<1>(b, cx, i, xi, iWater, 0u, [&](uint32_t j) { return PV{ldg(posS + j), ldg(velIn + j)}; },
+  // W = sigW t^4 (2 q + 1) with t = 1 - q / 2. The two neighbours' terms are
+  // formed together and added one after the other, every rounding fixed:
+  // the water's next substep amplifies what differs here.
+  V3 acc = splat(0.f);
+  forSame<G>(b, cx, i, xi, iWater, lane, [&](uint32_t j) { return PV{ldg(posS + j), ldg(velIn + j)}; },
              [&](uint32_t, uint32_t, const PV& d0, const PV& d1) {
                const F2 dx = f2(xi.x - d0.p.x, xi.x - d1.p.x), dy = f2(xi.y - d0.p.y, xi.y - d1.p.y),
                         dz = f2(xi.z - d0.p.z, xi.z - d1.p.z);
-               const F2 r2 = fma2(dz, dz, fma2(dy, dy, mul2(dx, dx)));
-               const F2 t = falloff2(S, r2);
-               const F2 t2 = mul2(t, t);
-               const F2 w = mul2(mul2(mul2(t2, t2), fma2(t, f2(-4.f, -4.f), f2(5.f, 5.f))), f2(d0.v.w, d1.v.w));
-               ax = fma2(w, f2(d0.v.x - vi.x, d1.v.x - vi.x), ax);
-               ay = fma2(w, f2(d0.v.y - vi.y, d1.v.y - vi.y), ay);
-               az = fma2(w, f2(d0.v.z - vi.z, d1.v.z - vi.z), az);
+               const F2 r2 = fma2(dz, dz, fma2(dx, dx, mul2(dy, dy)));
+               // (a padding entry is the slot itself: r = 0, dv = 0)
+               const F2 rinv = f2(rsqrtf(fmaxf(lo2(r2), 1e-30f)), rsqrtf(fmaxf(hi2(r2), 1e-30f)));
+               const F2 q = mul2(mul2(r2, rinv), f2(S.invH, S.invH));
+               const F2 t = fma2(q, f2(-0.5f, -0.5f), f2(1.f, 1.f));
+               const F2 w = mul2(mul2(mul2(mul2(mul2(f2(S.sigW, S.sigW), t), t), t), t), fma2(q, f2(2.f, 2.f), f2(1.f, 1.f)));
+               const F2 vol = f2(d0.v.w, d1.v.w);
+               const F2 ux = mul2(vol, f2(d0.v.x - vi.x, d1.v.x - vi.x)), uy = mul2(vol, f2(d0.v.y - vi.y, d1.v.y - vi.y)),
+                        uz = mul2(vol, f2(d0.v.z - vi.z, d1.v.z - vi.z));
+               acc.x = __fmaf_rn(hi2(ux), hi2(w), __fmaf_rn(lo2(ux), lo2(w), acc.x));
+               acc.y = __fmaf_rn(hi2(uy), hi2(w), __fmaf_rn(lo2(uy), lo2(w), acc.y));
+               acc.z = __fmaf_rn(hi2(uz), hi2(w), __fmaf_rn(lo2(uz), lo2(w), acc.z));
              });
-  const V3 acc = v3(sum2(ax), sum2(ay), sum2(az)) * S.sigW;
+  acc = laneSum<G>(acc);
+  if (G > 1 && lane != 0) return;
   float c = S.xsphC;
   if (iWater) c = S.xsphC * 10.f;
   const V3 v = vi + c * acc;
@@ -1980,30 +2106,36 @@ __global__ void XPBI_LB_UPDATE k_xsph(Bufs b, const float4* __restrict__ velIn,
 // 4M-particle substep, the same bits).
 __device__ __noinline__ M3 plasticUpdate(const SceneDev& S, const M3& gradV, const M3& F0, const MatDev& m, float st,
                                          float& stOut) {
-  const M3 Ftr = madd(F0, mscale(mul(gradV, F0), S.dt));
-  const SVD sv = svd3Fast(Ftr);
+  const M3 Htr = madd(minusIdent(F0), mscale(mul(gradV, F0), S.dt));
+  V3 e;
+  const SVD sv = strainSVD(Htr, e);
   const float hard = hardening(m, st);
-  const Mapped mp = returnMap(sv.sig, vlog(safeSig(sv.sig)), m, m.mu * hard, m.lam * hard, st, S.dt, stOut);
-  return diagMul(sv.U, safeSig(mp.sig), sv.V);
+  const Mapped mp = returnMap(sv.sig, e, m, m.mu * hard, m.lam * hard, st, S.dt, stOut);
+  // the trial F, changed by what the map and the clamp changed
+  const M3 D = diagMul(sv.U, safeSig(mp.sig) - sv.sig, sv.V);
+  return madd(madd(Htr, D), mident());
 }
-__global__ void XPBI_LB_UPDATE k_updateF_integrate(Bufs b, const float4* __restrict__ velIn) {
+template <int G>
+__global__ void __launch_bounds__(kThreads, kMinUpdate) k_updateF_integrate(Bufs b, const float4* __restrict__ velIn) {
   // blocks run last to first: the pass starts where xsph ended, on
   // slots whose data is still in L2
-  const uint32_t i = (gridDim.x - 1u - blockIdx.x) * blockDim.x + threadIdx.x;
+  const uint32_t t = (gridDim.x - 1u - blockIdx.x) * blockDim.x + threadIdx.x;
+  const uint32_t i = t / G, lane = t % G;
   if (i >= b.N) return;
   const Ctx cx = ctxOf(b, i);
   const SceneDev& S = *cx.scene;
   const float4 pi = b.posS[i];
   const uint32_t mi = matOfW(pi.w);
   const float4 vi4 = velIn[i];
+  const bool iWater = waterW(pi.w);
+  M3 A = mzero();
+  if (!iWater) A = velocitySum<G>(b, cx, i, xyz(pi), xyz(vi4), velIn, lane);
+  if (G > 1 && lane != 0) return;
   const float st = b.stateS[i];
   M3 Fn = loadM(b.FS, b.N, i);
   float stOut = st;
-  if (!waterW(pi.w)) {
-    const MatDev& m = cx.mats[mi];
-    const M3 gradV = velocityGradient(b, cx, i, xyz(pi), xyz(vi4), velIn);
-    Fn = plasticUpdate(S, gradV, Fn, m, st, stOut);
-  }
+  if (!iWater)
+    Fn = plasticUpdate(S, mul(A, transpose(loadM(b.L, b.N, i))), Fn, cx.mats[mi], st, stOut);
   storeM(b.F, b.N, i, Fn);
   b.state[i] = stOut;
   V3 v = xyz(vi4);
@@ -2086,11 +2218,17 @@ inline unsigned gridOf(uint32_t n, int block) { return (unsigned)((n + (uint32_t
 
 }  // namespace
 
-void launch_computeL(const Bufs& b, bool features, cudaStream_t st) {
-  if (features)
-    k_computeL_features<<<grid(b.N), kThreads, 0, st>>>(b);
-  else
-    k_computeL<<<grid(b.N), kThreads, 0, st>>>(b);
+void launch_computeL(const Bufs& b, bool features, int lanes, cudaStream_t st) {
+  const unsigned g = grid((uint32_t)lanes * b.N);
+  if (features) {
+    if (lanes == 4) k_computeL_features<4><<<g, kThreads, 0, st>>>(b);
+    else if (lanes == 2) k_computeL_features<2><<<g, kThreads, 0, st>>>(b);
+    else k_computeL_features<1><<<g, kThreads, 0, st>>>(b);
+  } else {
+    if (lanes == 4) k_computeL<4><<<g, kThreads, 0, st>>>(b);
+    else if (lanes == 2) k_computeL<2><<<g, kThreads, 0, st>>>(b);
+    else k_computeL<1><<<g, kThreads, 0, st>>>(b);
+  }
 }
 void launch_computeL_water(const Bufs& b, cudaStream_t st) { k_computeL_water<<<grid(b.N), kThreads, 0, st>>>(b); }
 template <int V>
@@ -2226,9 +2364,12 @@ void launch_solveB_list(const Bufs& b, int k, float4* vel, int flags, int varian
     default: solveBActiveVariant<0>(b, k, vel, 0, flags, true, st); break;
   }
 }
-void launch_pbfA(const Bufs& b, int k, const float4* velIn, int flags, cudaStream_t st) {
-  (void)velIn;  // predicted positions were stored by the preceding solveB
-  k_pbfA<<<grid(b.N), kThreads, 0, st>>>(b, k, flags);
+void launch_pbfA(const Bufs& b, int k, int flags, int lanes, cudaStream_t st) {
+  // predicted positions were stored by the preceding solveB
+  const unsigned g = grid((uint32_t)lanes * b.N);
+  if (lanes == 4) k_pbfA<4><<<g, kThreads, 0, st>>>(b, k, flags);
+  else if (lanes == 2) k_pbfA<2><<<g, kThreads, 0, st>>>(b, k, flags);
+  else k_pbfA<1><<<g, kThreads, 0, st>>>(b, k, flags);
 }
 void launch_judge(const Bufs& b, cudaGraphConditionalHandle h, bool setCond, cudaStream_t st) {
   k_judge<<<1, 256, 0, st>>>(b, h, setCond ? 1 : 0);
@@ -2238,14 +2379,23 @@ void launch_predict(const Bufs& b, const float4* vel, cudaStream_t st) { k_predi
 void launch_copy_vel(const Bufs& b, const float4* src, float4* dst, cudaStream_t st) {
   k_copy_vel<<<grid(b.N), kThreads, 0, st>>>(b.N, src, dst);
 }
-void launch_pbfB(const Bufs& b, int k, const float4* velIn, float4* velOut, int flags, cudaStream_t st) {
-  k_pbfB<<<grid(b.N), kThreads, 0, st>>>(b, k, velIn, velOut, flags);
+void launch_pbfB(const Bufs& b, int k, const float4* velIn, float4* velOut, int flags, int lanes, cudaStream_t st) {
+  const unsigned g = grid((uint32_t)lanes * b.N);
+  if (lanes == 4) k_pbfB<4><<<g, kThreads, 0, st>>>(b, k, velIn, velOut, flags);
+  else if (lanes == 2) k_pbfB<2><<<g, kThreads, 0, st>>>(b, k, velIn, velOut, flags);
+  else k_pbfB<1><<<g, kThreads, 0, st>>>(b, k, velIn, velOut, flags);
 }
-void launch_xsph(const Bufs& b, const float4* velIn, float4* velOut, cudaStream_t st) {
-  k_xsph<<<grid(b.N), kThreads, 0, st>>>(b, velIn, velOut);
+void launch_xsph(const Bufs& b, const float4* velIn, float4* velOut, int lanes, cudaStream_t st) {
+  const unsigned g = grid((uint32_t)lanes * b.N);
+  if (lanes == 4) k_xsph<4><<<g, kThreads, 0, st>>>(b, velIn, velOut);
+  else if (lanes == 2) k_xsph<2><<<g, kThreads, 0, st>>>(b, velIn, velOut);
+  else k_xsph<1><<<g, kThreads, 0, st>>>(b, velIn, velOut);
 }
-void launch_updateF_integrate(const Bufs& b, const float4* velIn, cudaStream_t st) {
-  k_updateF_integrate<<<grid(b.N), kThreads, 0, st>>>(b, velIn);
+void launch_updateF_integrate(const Bufs& b, const float4* velIn, int lanes, cudaStream_t st) {
+  const unsigned g = grid((uint32_t)lanes * b.N);
+  if (lanes == 4) k_updateF_integrate<4><<<g, kThreads, 0, st>>>(b, velIn);
+  else if (lanes == 2) k_updateF_integrate<2><<<g, kThreads, 0, st>>>(b, velIn);
+  else k_updateF_integrate<1><<<g, kThreads, 0, st>>>(b, velIn);
 }
 
 }  // namespace xpbi

@@ -13,11 +13,23 @@ constexpr uint32_t kKindWater = 6u;
 constexpr uint32_t kNbrCap = 64u;      // neighbour-list capacity per particle
 constexpr int kSolveAVariants = 6;      // launch-shape variants (autotuner): block size, register cap
 constexpr int kSolveBVariants = 5;
-// Lanes per slot of solveA / solveB by the handle's solid particle count:
-// four up to 24k solids, two up to 48k, else one (measured on sand columns,
-// dam breaches of 8k-120k solids and the 113k-solid snowball)
-constexpr uint64_t kFourLaneSolids = 24576;
-constexpr uint64_t kTwoLaneSolids = 49152;
+// Lanes per slot by the handle's size: few slots leave most of the GPU idle
+// with one lane each, and several split a slot's neighbours; many slots fill
+// it, and the lanes only add their sums' shuffles. Measured us per launch
+// (four / two / one lanes): solveA 8k solids 11.1 / 12.1 / 14.9, 16k 13.5 /
+// 12.5 / 14.8, 28k 20 / 16 / 18, 40k 23 / 21 / 20; solveB 16k 11.7 / 13.6 /
+// 18.2, 28k 18 / 16 / 22, 80k 33 / 29 / 33, 112k 43 / 38 / 37; computeL 30k
+// particles 27 / 29 / 35, 70k 49 / 37 / 45, 100k 64 / 53 / 51; pbfA 100k 36 /
+// 37 / 46, 140k 44 / 44 / 54, 280k 77 / 68 / 74; pbfB 70k 12 / 13 / 14, 100k
+// 15 / 13 / 15.
+struct LaneLimits {
+  uint64_t four, two;  // up to so many particles: four lanes, two lanes
+};
+constexpr LaneLimits kLanesA = {12288, 32768}, kLanesB = {24576, 81920};  // by solids
+constexpr LaneLimits kLanesAll = {40960, 81920};                         // computeL, xsph, the update
+constexpr LaneLimits kLanesPbfA = {131072, 327680}, kLanesPbfB = {81920, 114688};
+// the active set needs more solids than this (its kernels take one lane per slot)
+constexpr uint64_t kActiveSolids = 49152;
 constexpr int kResidBlocks = 256;      // at most this many partial sums of the residual per scene
 constexpr int kMaxResid = 129;         // residual slots per scene (iterations + 1)
 constexpr int kFeat = 16;              // network features per particle
@@ -85,6 +97,7 @@ struct SceneDev {
   float residTol;           // early stop at |r_k| <= residTol |C(v_pred)|; <= 0: never
   float residTolC;          // ... and |contact_k| <= residTolC |contact_0|
   float waterMpd;           // mass / density of the scene's one water material; 0: none or several
+  int onePhase;             // the scene's materials are all water or all solid
   int twoMasses;            // one water and at most one solid material: their masses
   float massW, massS;
   uint32_t nSolid;          // solid particles of the scene
@@ -195,7 +208,7 @@ uint32_t scan_tiles(uint32_t cells);
 
 // ---- launchers (solve.cu) ----
 // features: also iteration 0's constraint (cons0) and the network features
-void launch_computeL(const Bufs& b, bool features, cudaStream_t st);
+void launch_computeL(const Bufs& b, bool features, int lanes, cudaStream_t st);
 // the water particles' L of the last substep (computeL forms the solids' only)
 void launch_computeL_water(const Bufs& b, cudaStream_t st);
 void launch_solveA(const Bufs& b, int k, const float4* velIn, int flags, int variant, int lanes, cudaStream_t st);
@@ -211,7 +224,7 @@ cudaError_t mlp_forward(const float* dX, uint32_t rows, const void* dBlob, float
                         bool skipZero = false);
 void launch_solveB(const Bufs& b, int k, const float4* velIn, float4* velOut, bool writeXc, int flags, int variant,
                    int lanes, cudaStream_t st);
-void launch_pbfA(const Bufs& b, int k, const float4* velIn, int flags, cudaStream_t st);
+void launch_pbfA(const Bufs& b, int k, int flags, int lanes, cudaStream_t st);
 // the plain re-solve: judge marks the scenes whose early-stopped solve did
 // not stop (sets the graph's condition when setCond), restore resets their
 // velocities in `vel` to vel0, copy moves every slot's velocity src -> dst
@@ -232,8 +245,8 @@ void launch_solveB_list(const Bufs& b, int k, float4* vel, int flags, int varian
 // iterating (not stopped, below its cap)
 void launch_loop_begin(const Bufs& b, int k0, cudaGraphConditionalHandle h, cudaStream_t st);
 void launch_loop_next(const Bufs& b, cudaGraphConditionalHandle h, cudaStream_t st);
-void launch_pbfB(const Bufs& b, int k, const float4* velIn, float4* velOut, int flags, cudaStream_t st);
-void launch_xsph(const Bufs& b, const float4* velIn, float4* velOut, cudaStream_t st);
-void launch_updateF_integrate(const Bufs& b, const float4* velIn, cudaStream_t st);
+void launch_pbfB(const Bufs& b, int k, const float4* velIn, float4* velOut, int flags, int lanes, cudaStream_t st);
+void launch_xsph(const Bufs& b, const float4* velIn, float4* velOut, int lanes, cudaStream_t st);
+void launch_updateF_integrate(const Bufs& b, const float4* velIn, int lanes, cudaStream_t st);
 
 }  // namespace xpbi

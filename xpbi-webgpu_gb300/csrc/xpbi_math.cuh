@@ -73,6 +73,10 @@ struct M3 {
 };
 __device__ __forceinline__ M3 mzero() { return {{splat(0.f), splat(0.f), splat(0.f)}}; }
 __device__ __forceinline__ M3 mident() { return {{v3(1.f, 0.f, 0.f), v3(0.f, 1.f, 0.f), v3(0.f, 0.f, 1.f)}}; }
+__device__ __forceinline__ M3 minusIdent(const M3& A) {
+  return {{v3(A.c[0].x - 1.f, A.c[0].y, A.c[0].z), v3(A.c[1].x, A.c[1].y - 1.f, A.c[1].z),
+           v3(A.c[2].x, A.c[2].y, A.c[2].z - 1.f)}};
+}
 __device__ __forceinline__ V3 mul(const M3& A, V3 v) { return A.c[0] * v.x + A.c[1] * v.y + A.c[2] * v.z; }
 __device__ __forceinline__ M3 mul(const M3& A, const M3& B) {
   return {{mul(A, B.c[0]), mul(A, B.c[1]), mul(A, B.c[2])}};
@@ -186,6 +190,10 @@ __device__ __forceinline__ float rsqrtNewton(float d) {
 }
 __device__ __forceinline__ V3 normalizeFast(V3 a) { return a * rsqrtNewton(dot(a, a)); }
 
+// A vector whose length is 1 up to the rounding of approximate cosines, with
+// the error's first order taken off.
+__device__ __forceinline__ V3 renormalize(V3 a) { return a * fmaf(-0.5f, dot(a, a), 1.5f); }
+
 // SVD with the reference's conventions (common.js:105-184: sigma descending,
 // the last one negative if det F < 0, U and V rotations) by one-sided Jacobi
 // sweeps: the columns of F V are made orthogonal instead of diagonalising
@@ -246,6 +254,52 @@ __device__ __forceinline__ SVD svd3Fast(const M3& F) {
   return out;
 }
 
+// Eigenvalues d and eigenvectors (the columns a) of a symmetric 3x3 matrix by
+// Jacobi rotations, in no particular order. A rotation zeroes one off-diagonal
+// exactly, moves its diagonals by t apq and turns the other two off-diagonals
+// and the vectors; off-diagonals below 1e-9 of the largest entry are left.
+struct Sym3 {
+  float xx, yy, zz, xy, xz, yz;
+};
+__device__ __forceinline__ void eigRot(float& dp, float& dq, float& apq, float& arp, float& arq, V3& vp, V3& vq,
+                                       float small, bool& more) {
+  if (!(fabsf(apq) > small)) return;
+  const float tau = __fdividef(dq - dp, 2.f * apq);
+  const float h2 = 1.f + tau * tau;
+  const float root = h2 * rsqrtf(h2);
+  const float t = __fdividef(1.f, tau >= 0.f ? tau + root : tau - root);
+  more |= fabsf(t) > 2e-4f;
+  const float c = rsqrtf(1.f + t * t);
+  const float s = t * c;
+  dp -= t * apq;
+  dq += t * apq;
+  apq = 0.f;
+  const float x = arp, y = arq;
+  arp = c * x - s * y;
+  arq = s * x + c * y;
+  const V3 p = vp, q = vq;
+  vp = c * p - s * q;
+  vq = s * p + c * q;
+}
+__device__ __forceinline__ float maxAbs(const Sym3& S) {
+  return fmaxf(fmaxf(fmaxf(fabsf(S.xx), fabsf(S.yy)), fabsf(S.zz)),
+               fmaxf(fmaxf(fabsf(S.xy), fabsf(S.xz)), fabsf(S.yz)));
+}
+__device__ __forceinline__ void eigSym(Sym3 S, V3& d, M3& V) {
+  V3 a0 = v3(1.f, 0.f, 0.f), a1 = v3(0.f, 1.f, 0.f), a2 = v3(0.f, 0.f, 1.f);
+  const float small = 1e-9f * maxAbs(S);
+#pragma unroll 1
+  for (int sweep = 0; sweep < 6; ++sweep) {
+    bool more = false;
+    eigRot(S.xx, S.yy, S.xy, S.xz, S.yz, a0, a1, small, more);
+    eigRot(S.xx, S.zz, S.xz, S.xy, S.yz, a0, a2, small, more);
+    eigRot(S.yy, S.zz, S.yz, S.xy, S.xz, a1, a2, small, more);
+    if (!more) break;
+  }
+  d = v3(S.xx, S.yy, S.zz);
+  V = {{renormalize(a0), renormalize(a1), renormalize(a2)}};
+}
+
 // U diag(d) V^T (common.js:182-184)
 __device__ __forceinline__ M3 diagMul(const M3& U, V3 d, const M3& V) {
   M3 Ud = {{U.c[0] * d.x, U.c[1] * d.y, U.c[2] * d.z}};
@@ -255,6 +309,32 @@ __device__ __forceinline__ M3 diagMul(const M3& U, V3 d, const M3& V) {
 // ----------------------------------------------------------------- StVK-Hencky
 // common.js:186-201
 __device__ __forceinline__ V3 safeSig(V3 s) { return vclamp(s, 1e-3f, 1e3f); }
+// The SVD of F = I + H and the logs of its (clamped) singular values. Near the
+// identity, where a granular body flows, f32 singular values of 1 + O(1e-4)
+// keep three digits of the strain; there the eigenvalues x of
+// F^T F - I = H + H^T + H^T H are taken instead, which H's own digits carry,
+// with log sigma = log(1 + x) / 2. (The singular values then come in no
+// particular order: the material models do not depend on it.) Beyond
+// |F^T F - I| = 0.5 the SVD of F itself keeps the small singular values.
+__device__ __forceinline__ SVD strainSVD(const M3& H, V3& e) {
+  const V3 x = H.c[0], y = H.c[1], z = H.c[2];
+  const Sym3 S = {fmaf(2.f, x.x, dot(x, x)), fmaf(2.f, y.y, dot(y, y)), fmaf(2.f, z.z, dot(z, z)),
+                  (x.y + y.x) + dot(x, y),   (x.z + z.x) + dot(x, z),   (y.z + z.y) + dot(y, z)};
+  if (maxAbs(S) < 0.5f) {
+    SVD out;
+    V3 d;
+    eigSym(S, d, out.V);
+    e = v3(0.5f * log1pf(d.x), 0.5f * log1pf(d.y), 0.5f * log1pf(d.z));
+    const V3 r = v3(rsqrtNewton(1.f + d.x), rsqrtNewton(1.f + d.y), rsqrtNewton(1.f + d.z));
+    out.sig = v3((1.f + d.x) * r.x, (1.f + d.y) * r.y, (1.f + d.z) * r.z);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) out.U.c[k] = (out.V.c[k] + mul(H, out.V.c[k])) * r[k];
+    return out;
+  }
+  const SVD out = svd3Fast(M3{{v3(1.f + x.x, x.y, x.z), v3(y.x, 1.f + y.y, y.z), v3(z.x, z.y, 1.f + z.z)}});
+  e = vlog(safeSig(out.sig));
+  return out;
+}
 // energy from the logs e of the clamped singular values; its gradient is
 // (2 mu e + lam tr e) / safeSig(sig)
 __device__ __forceinline__ float stvkPsi(V3 e, float mu, float lam) {
