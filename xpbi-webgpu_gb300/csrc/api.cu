@@ -774,7 +774,7 @@ cudaError_t enqueueSubstep(xpbi_sim* s, const Schedule& sch, cudaStream_t st, Re
     launch_resid_reduce(b, -1, false, st);
     R.mark(st, "residual");
   }
-  launch_xsph(b, b.velS[in], b.velS[in ^ 1], sch.lanesAll, st);
+  launch_xsph(b, b.velS[in], b.velS[in ^ 1], aflags, sch.lanesAll, st);
   R.mark(st, "xsph");
   in ^= 1;
   // the update moves the particles: asynchronous read-backs of the previous
@@ -795,6 +795,7 @@ cudaError_t enqueueSubstep(xpbi_sim* s, const Schedule& sch, cudaStream_t st, Re
 }
 
 int kernelsPerSubstep(const Schedule& sch) {
+  // the clearing of the sort's counters is part of the count
   int n = 5 /* count, scan, fill, bigcells, reorder */ + 1 /* computeL */ + 2 /* xsph, updateF+integrate */;
   for (int k = 0; k < sch.K; ++k) {
     const bool list = sch.active && k >= 2;  // two compactions; before a PBF pass, the predicted positions

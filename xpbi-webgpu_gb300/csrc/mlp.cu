@@ -21,6 +21,7 @@
 // stops issuing work and still releases its TMEM.
 #include <cuda_bf16.h>
 
+#include "chain.cuh"
 #include "tc.cuh"
 #include "xpbi_math.cuh"
 
@@ -335,13 +336,6 @@ __global__ void __launch_bounds__(kStepThreads) k_mlp_step(const float* __restri
   float* const DZ = reinterpret_cast<float*>(sm + tDZ);
   float* const red = reinterpret_cast<float*>(sm + tRed);
   float* const P = partial + (size_t)blockIdx.x * kPartStride;
-  {
-    const uint4* src = reinterpret_cast<const uint4*>(blob);
-    uint4* dst = reinterpret_cast<uint4*>(sm + tW);
-    for (uint32_t q = tid; q < bF32 / 16u; q += kStepThreads) dst[q] = src[q];
-    const float* fs = reinterpret_cast<const float*>(blob + bF32);
-    for (uint32_t q = tid; q < 4 * kHid + 1; q += kStepThreads) F[q] = fs[q];
-  }
   if (warp == 0) tc::tmemAlloc(&tbase, 64);
   if (tid == 0) tc::mbarInit(&bar, 1);
   // the inputs as bf16, 8 columns per thread
@@ -359,6 +353,16 @@ __global__ void __launch_bounds__(kStepThreads) k_mlp_step(const float* __restri
     *reinterpret_cast<uint4*>(sm + tA + tc::coreOffset(r, 8 * half, kIn)) = *reinterpret_cast<uint4*>(x);
   }
   const float target = valid ? T[row] : 0.f;
+  // all of the above, the batch included, does not depend on the preceding
+  // step; the weights do
+  const uint32_t w0 = afterPrevious((uint32_t)tid);
+  {
+    const uint4* src = reinterpret_cast<const uint4*>(blob);
+    uint4* dst = reinterpret_cast<uint4*>(sm + tW);
+    for (uint32_t q = w0; q < bF32 / 16u; q += kStepThreads) dst[q] = src[q];
+    const float* fs = reinterpret_cast<const float*>(blob + bF32);
+    for (uint32_t q = w0; q < 4 * kHid + 1; q += kStepThreads) F[q] = fs[q];
+  }
   tc::fenceProxyAsync();
   tc::fenceBeforeSync();
   __syncthreads();
@@ -585,7 +589,7 @@ __global__ void __launch_bounds__(4 * kReduceParams) k_mlp_reduce(const float* _
                                                                   Adam A, uint8_t* __restrict__ blob) {
   __shared__ float sum[4][kReduceParams];
   const uint32_t q = threadIdx.x % kReduceParams, g = threadIdx.x / kReduceParams;
-  const uint32_t p = blockIdx.x * kReduceParams + q;
+  const uint32_t p = afterPreviousEager(blockIdx.x * kReduceParams + q);
   float acc = 0.f;
   if (p < (uint32_t)kParams) {
 #pragma unroll 8
@@ -648,8 +652,8 @@ cudaError_t stepKernel(const float* dX, const float* dT, uint32_t rows, const vo
                        int* dErr, cudaStream_t st) {
   cudaError_t e = cudaFuncSetAttribute(k_mlp_step, cudaFuncAttributeMaxDynamicSharedMemorySize, kStepSmem);
   if (e != cudaSuccess) return e;
-  k_mlp_step<<<(rows + kRows - 1) / kRows, kStepThreads, kStepSmem, st>>>(
-      dX, dT, rows, static_cast<const uint8_t*>(dBlob), dPartial, dSq, dErr);
+  launchChained(k_mlp_step, (rows + kRows - 1) / kRows, kStepThreads, kStepSmem, st, dX, dT, rows,
+                static_cast<const uint8_t*>(dBlob), dPartial, dSq, dErr);
   return cudaGetLastError();
 }
 }  // namespace
@@ -661,8 +665,8 @@ cudaError_t mlp_grad(const float* dX, const float* dT, uint32_t rows, const void
   if (rows == 0) return cudaSuccess;
   cudaError_t e = stepKernel(dX, dT, rows, dBlob, dPartial, dSq, dErr, st);
   if (e != cudaSuccess) return e;
-  k_mlp_reduce<<<(kParams + kReduceParams - 1) / kReduceParams, 4 * kReduceParams, 0, st>>>(
-      dPartial, (rows + kRows - 1) / kRows, dSq, rows, dGrad, dLoss, Adam{}, nullptr);
+  launchChained(
+      k_mlp_reduce, (kParams + kReduceParams - 1) / kReduceParams, 4 * kReduceParams, 0, st, dPartial, (rows + kRows - 1) / kRows, dSq, rows, dGrad, dLoss, Adam{}, nullptr);
   return cudaGetLastError();
 }
 
@@ -674,8 +678,8 @@ cudaError_t mlp_train_step(const float* dX, const float* dT, uint32_t rows, floa
   if (e != cudaSuccess) return e;
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.f - powf(b1, (float)step), c2 = 1.f - powf(b2, (float)step);
-  k_mlp_reduce<<<(kParams + kReduceParams - 1) / kReduceParams, 4 * kReduceParams, 0, st>>>(
-      dPartial, (rows + kRows - 1) / kRows, dSq, rows, nullptr, dLoss, Adam{dW, dM, dV, lr, b1, b2, 1e-8f, c1, c2},
+  launchChained(
+      k_mlp_reduce, (kParams + kReduceParams - 1) / kReduceParams, 4 * kReduceParams, 0, st, dPartial, (rows + kRows - 1) / kRows, dSq, rows, nullptr, dLoss, Adam{dW, dM, dV, lr, b1, b2, 1e-8f, c1, c2},
       static_cast<uint8_t*>(dBlob));
   return cudaGetLastError();
 }

@@ -34,12 +34,12 @@
 #include <mutex>
 #include <string>
 
+#include "chain.cuh"
 #include "xpbi.h"
 #include "xpbi_internal.h"
 
 namespace xpbi {
 int setError(int code, const std::string& msg);
-uint32_t launch_bigcells(const Bufs& b, uint32_t* scratch, cudaStream_t st);
 }  // namespace xpbi
 
 using namespace xpbi;
@@ -77,7 +77,7 @@ uint32_t* g_addr[kMaxDevices] = {nullptr};
 __global__ void k_rank_only(const uint32_t* __restrict__ tmp, const uint32_t* __restrict__ key,
                             const uint32_t* __restrict__ cellStart, uint32_t n, uint32_t big,
                             uint32_t* __restrict__ sortedIdx) {
-  const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t p = afterPrevious(blockIdx.x * blockDim.x + threadIdx.x);
   if (p >= n) return;
   const uint32_t i = tmp[p];
   const uint32_t c = key[i];
@@ -92,13 +92,16 @@ __global__ void k_rank_only(const uint32_t* __restrict__ tmp, const uint32_t* __
 }
 
 // Writes the grid description, clears the material table (no material is
-// water, so no cell is flagged) and the error word.
-__global__ void k_setup(SceneDev sd, SceneDev* scene, uint32_t* matWords, uint32_t nMatWords, int* err) {
-  if (threadIdx.x == 0) {
-    *scene = sd;
-    *err = 0;
+// water, so no cell is flagged), the error word and what the sort starts from.
+__global__ void k_setup(SceneDev sd, Bufs b, uint32_t* matWords, uint32_t nMatWords) {
+  const uint32_t t = afterPreviousEager(blockIdx.x * blockDim.x + threadIdx.x);
+  sortClear(b, t);
+  if (blockIdx.x != 0) return;
+  if (t == 0) {
+    *b.scenes = sd;
+    *b.err = 0;
   }
-  for (uint32_t w = threadIdx.x; w < nMatWords; w += blockDim.x) matWords[w] = 0u;
+  for (uint32_t w = t; w < nMatWords; w += blockDim.x) matWords[w] = 0u;
 }
 
 int scratchAddress(uint32_t** out) {
@@ -177,12 +180,13 @@ extern "C" int xpbi_sort_cells_noalloc(const float* pos4, uint32_t n, const floa
   b.S = 1;
   b.scanTiles = scan_tiles(b.C);
 
-  k_setup<<<1, 128, 0, st>>>(sd, b.scenes, base + wMats, (uint32_t)((kMaxMats * sizeof(MatDev) + 3) / 4), b.err);
-  launch_count(b, st);    // clears the cell counters and water flags first
-  launch_scan(b, st);     // clears the look-back descriptors first
+  k_setup<<<(sortClearThreads(b) + 255) / 256, 256, 0, st>>>(sd, b, base + wMats,
+                                                             (uint32_t)((kMaxMats * sizeof(MatDev) + 3) / 4));
+  launch_count_cleared(b, st);
+  launch_scan(b, st);
   launch_scatter(b, st);
   const uint32_t big = launch_bigcells(b, base + wBigScratch, st);
-  k_rank_only<<<(n + 255) / 256, 256, 0, st>>>(b.tmp, b.key, b.cellStart, n, big, sorted_idx);
+  launchChained(k_rank_only, (n + 255) / 256, 256, 0, st, b.tmp, b.key, b.cellStart, n, big, sorted_idx);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return setError(XPBI_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
   return XPBI_OK;

@@ -31,6 +31,7 @@
 // parity stays consistent for every scene.
 #include <algorithm>
 
+#include "chain.cuh"
 #include "xpbi_math.cuh"
 
 namespace xpbi {
@@ -956,7 +957,7 @@ __device__ __forceinline__ void solveAUpdate(const Bufs& b, const Ctx& cx, uint3
 template <bool kTrack, int kMinB, int G, int kBlock = kThreads>
 __global__ void __launch_bounds__(kBlock, kMinB) k_solveA(Bufs b, int k, const float4* __restrict__ velIn,
                                                             int flags) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t t = afterPrevious(blockIdx.x * blockDim.x + threadIdx.x);
   const uint32_t i = t / G, lane = t % G;
   if (i >= b.N) return;
   const Ctx cx = ctxOf(b, i);
@@ -1146,7 +1147,7 @@ __device__ __forceinline__ void computeL(const Bufs& b) {
   __shared__ uint32_t column[G == 1 ? 1 : SubList<G>::kCap * kThreads];
   // blocks run last to first: the pass starts where the reorder ended, on
   // slots whose data is still in L2
-  const uint32_t t = (gridDim.x - 1u - blockIdx.x) * blockDim.x + threadIdx.x;
+  const uint32_t t = afterPrevious((gridDim.x - 1u - blockIdx.x) * blockDim.x + threadIdx.x);
   const uint32_t i = t / G, lane = t % G;
   if (i >= b.N) return;
   const Ctx cx = ctxOf(b, i);
@@ -1522,7 +1523,7 @@ __global__ void __launch_bounds__(kBlock, kMinB) k_solveB(Bufs b, int k, const f
                                                       float4* __restrict__ velOut, int writeXc, int flags) {
   // blocks run last to first: the pass starts where solveA ended, on slots
   // whose data is still in L2
-  const uint32_t t = (gridDim.x - 1u - blockIdx.x) * blockDim.x + threadIdx.x;
+  const uint32_t t = afterPrevious((gridDim.x - 1u - blockIdx.x) * blockDim.x + threadIdx.x);
   const uint32_t i = t / G, lane = t % G;
   for (uint32_t q = t; q < b.S; q += gridDim.x * blockDim.x)  // the next iteration's slot
     b.solidDisp[(size_t)((k + 1) & 1) * b.S + q] = 0u;
@@ -1837,7 +1838,7 @@ __device__ __forceinline__ PbfPair pbfPair(const SceneDev& S, V3 c, const float4
 template <int G>
 __global__ void __launch_bounds__(kThreads, minPbf(G)) k_pbfA(Bufs b, int k, int flags) {
   __shared__ uint32_t column[G == 1 ? 1 : SubList<G>::kCap * kThreads];
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t t = afterPrevious(blockIdx.x * blockDim.x + threadIdx.x);
   const uint32_t i = t / G, lane = t % G;
   if (i >= b.N) return;
   const Ctx cx = ctxOf(b, i);
@@ -1972,7 +1973,7 @@ template <int G>
 __global__ void __launch_bounds__(kThreads, minPbf(G)) k_pbfB(Bufs b, int k, const float4* velIn, float4* velOut, int flags) {
   // blocks run last to first: the pass starts where pbfA ended, on
   // slots whose data is still in L2
-  const uint32_t t = (gridDim.x - 1u - blockIdx.x) * blockDim.x + threadIdx.x;
+  const uint32_t t = afterPrevious((gridDim.x - 1u - blockIdx.x) * blockDim.x + threadIdx.x);
   const uint32_t i = t / G, lane = t % G;
   if (i >= b.N) return;
   const Ctx cx = ctxOf(b, i);
@@ -2056,7 +2057,7 @@ __global__ void __launch_bounds__(kThreads, minPbf(G)) k_pbfB(Bufs b, int k, con
 // simkernels.js:480-507
 template <int G>
 __global__ void __launch_bounds__(kThreads) k_xsph(Bufs b, const float4* __restrict__ velIn, float4* __restrict__ velOut) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t t = afterPrevious(blockIdx.x * blockDim.x + threadIdx.x);
   const uint32_t i = t / G, lane = t % G;
   if (i >= b.N) return;
   const Ctx cx = ctxOf(b, i);
@@ -2218,27 +2219,37 @@ inline unsigned gridOf(uint32_t n, int block) { return (unsigned)((n + (uint32_t
 
 }  // namespace
 
+// The reference schedule's launches are chained (its flags are 0). Those of
+// the learned solve stay plain: they follow memsets and conditional nodes or
+// form the bodies of conditional nodes.
+template <class... P, class... Q>
+inline void launchIn(int flags, void (*fn)(P...), unsigned g, unsigned block, cudaStream_t st, Q... q) {
+  if (flags == 0)
+    launchChained(fn, g, block, 0, st, q...);
+  else
+    fn<<<g, block, 0, st>>>(q...);
+}
 void launch_computeL(const Bufs& b, bool features, int lanes, cudaStream_t st) {
   const unsigned g = grid((uint32_t)lanes * b.N);
   if (features) {
-    if (lanes == 4) k_computeL_features<4><<<g, kThreads, 0, st>>>(b);
-    else if (lanes == 2) k_computeL_features<2><<<g, kThreads, 0, st>>>(b);
-    else k_computeL_features<1><<<g, kThreads, 0, st>>>(b);
+    if (lanes == 4) launchChained(k_computeL_features<4>, g, kThreads, 0, st, b);
+    else if (lanes == 2) launchChained(k_computeL_features<2>, g, kThreads, 0, st, b);
+    else launchChained(k_computeL_features<1>, g, kThreads, 0, st, b);
   } else {
-    if (lanes == 4) k_computeL<4><<<g, kThreads, 0, st>>>(b);
-    else if (lanes == 2) k_computeL<2><<<g, kThreads, 0, st>>>(b);
-    else k_computeL<1><<<g, kThreads, 0, st>>>(b);
+    if (lanes == 4) launchChained(k_computeL<4>, g, kThreads, 0, st, b);
+    else if (lanes == 2) launchChained(k_computeL<2>, g, kThreads, 0, st, b);
+    else launchChained(k_computeL<1>, g, kThreads, 0, st, b);
   }
 }
 void launch_computeL_water(const Bufs& b, cudaStream_t st) { k_computeL_water<<<grid(b.N), kThreads, 0, st>>>(b); }
 template <int V>
 void solveAVariant(const Bufs& b, int k, const float4* velIn, int flags, cudaStream_t st) {
   if (flags & kTrackResid)
-    k_solveA<true, kSolveAMinB[V], 1, kSolveABlock[V]><<<gridOf(b.N, kSolveABlock[V]), kSolveABlock[V], 0, st>>>(
-        b, k, velIn, flags);
+    launchIn(flags, k_solveA<true, kSolveAMinB[V], 1, kSolveABlock[V]>, gridOf(b.N, kSolveABlock[V]), kSolveABlock[V],
+             st, b, k, velIn, flags);
   else
-    k_solveA<false, kSolveAMinB[V], 1, kSolveABlock[V]><<<gridOf(b.N, kSolveABlock[V]), kSolveABlock[V], 0, st>>>(
-        b, k, velIn, flags);
+    launchIn(flags, k_solveA<false, kSolveAMinB[V], 1, kSolveABlock[V]>, gridOf(b.N, kSolveABlock[V]), kSolveABlock[V],
+             st, b, k, velIn, flags);
 }
 void launch_solveA(const Bufs& b, int k, const float4* velIn, int flags, int variant, int lanes, cudaStream_t st) {
   if (flags & kStoredC) {  // iteration 0 after computeL with features (one lane per slot)
@@ -2251,17 +2262,17 @@ void launch_solveA(const Bufs& b, int k, const float4* velIn, int flags, int var
   if (lanes == 4) {  // small scenes: four lanes per slot, the allocator's register choice
     const uint32_t threads = 4u * b.N;
     if (flags & kTrackResid)
-      k_solveA<true, 0, 4><<<grid(threads), kThreads, 0, st>>>(b, k, velIn, flags);
+      launchIn(flags, k_solveA<true, 0, 4>, grid(threads), kThreads, st, b, k, velIn, flags);
     else
-      k_solveA<false, 0, 4><<<grid(threads), kThreads, 0, st>>>(b, k, velIn, flags);
+      launchIn(flags, k_solveA<false, 0, 4>, grid(threads), kThreads, st, b, k, velIn, flags);
     return;
   }
   if (lanes == 2) {
     const uint32_t threads = 2u * b.N;
     if (flags & kTrackResid)
-      k_solveA<true, 0, 2><<<grid(threads), kThreads, 0, st>>>(b, k, velIn, flags);
+      launchIn(flags, k_solveA<true, 0, 2>, grid(threads), kThreads, st, b, k, velIn, flags);
     else
-      k_solveA<false, 0, 2><<<grid(threads), kThreads, 0, st>>>(b, k, velIn, flags);
+      launchIn(flags, k_solveA<false, 0, 2>, grid(threads), kThreads, st, b, k, velIn, flags);
     return;
   }
   switch (variant) {
@@ -2281,8 +2292,8 @@ void launch_resid_reduce(const Bufs& b, int k, bool warm, cudaStream_t st) {
 void launch_keep_lambda(const Bufs& b, cudaStream_t st) { k_keep_lambda<<<grid(b.N), kThreads, 0, st>>>(b); }
 template <int V>
 void solveBVariant(const Bufs& b, int k, const float4* velIn, float4* velOut, int wx, int flags, cudaStream_t st) {
-  k_solveB<kSolveBMinB[V], 1, kSolveBBlock[V]><<<gridOf(b.N, kSolveBBlock[V]), kSolveBBlock[V], 0, st>>>(
-      b, k, velIn, velOut, wx, flags);
+  launchIn(flags, k_solveB<kSolveBMinB[V], 1, kSolveBBlock[V]>, gridOf(b.N, kSolveBBlock[V]), kSolveBBlock[V], st, b, k,
+           velIn, velOut, wx, flags);
 }
 // A grid that fills the GPU once with this kernel's resident blocks (the
 // list launches loop over their lists).
@@ -2320,11 +2331,11 @@ void launch_solveB(const Bufs& b, int k, const float4* velIn, float4* velOut, bo
     return;
   }
   if (lanes == 4) {
-    k_solveB<0, 4><<<grid(4u * b.N), kThreads, 0, st>>>(b, k, velIn, velOut, wx, flags);
+    launchIn(flags, k_solveB<0, 4>, grid(4u * b.N), kThreads, st, b, k, velIn, velOut, wx, flags);
     return;
   }
   if (lanes == 2) {
-    k_solveB<0, 2><<<grid(2u * b.N), kThreads, 0, st>>>(b, k, velIn, velOut, wx, flags);
+    launchIn(flags, k_solveB<0, 2>, grid(2u * b.N), kThreads, st, b, k, velIn, velOut, wx, flags);
     return;
   }
   switch (variant) {
@@ -2367,9 +2378,9 @@ void launch_solveB_list(const Bufs& b, int k, float4* vel, int flags, int varian
 void launch_pbfA(const Bufs& b, int k, int flags, int lanes, cudaStream_t st) {
   // predicted positions were stored by the preceding solveB
   const unsigned g = grid((uint32_t)lanes * b.N);
-  if (lanes == 4) k_pbfA<4><<<g, kThreads, 0, st>>>(b, k, flags);
-  else if (lanes == 2) k_pbfA<2><<<g, kThreads, 0, st>>>(b, k, flags);
-  else k_pbfA<1><<<g, kThreads, 0, st>>>(b, k, flags);
+  if (lanes == 4) launchIn(flags, k_pbfA<4>, g, kThreads, st, b, k, flags);
+  else if (lanes == 2) launchIn(flags, k_pbfA<2>, g, kThreads, st, b, k, flags);
+  else launchIn(flags, k_pbfA<1>, g, kThreads, st, b, k, flags);
 }
 void launch_judge(const Bufs& b, cudaGraphConditionalHandle h, bool setCond, cudaStream_t st) {
   k_judge<<<1, 256, 0, st>>>(b, h, setCond ? 1 : 0);
@@ -2381,15 +2392,15 @@ void launch_copy_vel(const Bufs& b, const float4* src, float4* dst, cudaStream_t
 }
 void launch_pbfB(const Bufs& b, int k, const float4* velIn, float4* velOut, int flags, int lanes, cudaStream_t st) {
   const unsigned g = grid((uint32_t)lanes * b.N);
-  if (lanes == 4) k_pbfB<4><<<g, kThreads, 0, st>>>(b, k, velIn, velOut, flags);
-  else if (lanes == 2) k_pbfB<2><<<g, kThreads, 0, st>>>(b, k, velIn, velOut, flags);
-  else k_pbfB<1><<<g, kThreads, 0, st>>>(b, k, velIn, velOut, flags);
+  if (lanes == 4) launchIn(flags, k_pbfB<4>, g, kThreads, st, b, k, velIn, velOut, flags);
+  else if (lanes == 2) launchIn(flags, k_pbfB<2>, g, kThreads, st, b, k, velIn, velOut, flags);
+  else launchIn(flags, k_pbfB<1>, g, kThreads, st, b, k, velIn, velOut, flags);
 }
-void launch_xsph(const Bufs& b, const float4* velIn, float4* velOut, int lanes, cudaStream_t st) {
+void launch_xsph(const Bufs& b, const float4* velIn, float4* velOut, int flags, int lanes, cudaStream_t st) {
   const unsigned g = grid((uint32_t)lanes * b.N);
-  if (lanes == 4) k_xsph<4><<<g, kThreads, 0, st>>>(b, velIn, velOut);
-  else if (lanes == 2) k_xsph<2><<<g, kThreads, 0, st>>>(b, velIn, velOut);
-  else k_xsph<1><<<g, kThreads, 0, st>>>(b, velIn, velOut);
+  if (lanes == 4) launchIn(flags, k_xsph<4>, g, kThreads, st, b, velIn, velOut);
+  else if (lanes == 2) launchIn(flags, k_xsph<2>, g, kThreads, st, b, velIn, velOut);
+  else launchIn(flags, k_xsph<1>, g, kThreads, st, b, velIn, velOut);
 }
 void launch_updateF_integrate(const Bufs& b, const float4* velIn, int lanes, cudaStream_t st) {
   const unsigned g = grid((uint32_t)lanes * b.N);

@@ -3,6 +3,7 @@
 // Replaces clearBuffer + countParticles + scanBlocks + scanApply + scatter +
 // stagePVA/applyPVA/stageF/applyF (web/js/shaders/simkernels.js:78-186,
 // dispatched by web/js/sim.js:223-236) with:
+//   k_clear    zeroes the cell counters, water flags and scan descriptors
 //   k_count    cell key per particle + warp-aggregated histogram atomics
 //   k_scan     single-pass decoupled-lookback exclusive scan of the histogram
 //   k_fill     warp-aggregated slot reservation: each cell's members land in
@@ -15,6 +16,7 @@
 // in invocation order: within a cell, particles are listed by descending
 // previous index. Counts, cell starts and the permutation are therefore
 // deterministic and bit-identical to that serial order.
+#include "chain.cuh"
 #include "xpbi_math.cuh"
 
 namespace xpbi {
@@ -40,9 +42,13 @@ __device__ __forceinline__ uint32_t cellKey(const SceneDev& S, float4 p) {
   return S.cellBase + cellIndex(S, c.x, c.y, c.z);
 }
 
+__global__ void __launch_bounds__(kThreads) k_clear(Bufs b) {
+  sortClear(b, afterPreviousEager(blockIdx.x * blockDim.x + threadIdx.x));
+}
+
 // cursor[] was cleared before this launch; on exit it holds cell counts.
 __global__ void __launch_bounds__(kThreads) k_count(Bufs b) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t i = afterPreviousEager(blockIdx.x * blockDim.x + threadIdx.x);
   bool active = i < b.N;
   uint32_t key = 0;
   if (active) {
@@ -74,7 +80,7 @@ __device__ __forceinline__ unsigned long long waitDescriptor(const volatile unsi
       atomicOr(err, kErrLookback);
       return 0ull;
     }
-    __nanosleep(64);
+    if (spins > 16u) __nanosleep(64);
   }
 }
 
@@ -86,6 +92,7 @@ __device__ __forceinline__ unsigned long long waitDescriptor(const volatile unsi
 __global__ void __launch_bounds__(kScanThreads) k_scan(Bufs b) {
   __shared__ uint32_t s_tile, s_excl;
   __shared__ uint32_t s_warp[kScanThreads / 32];
+  afterPreviousEager(0u);
   if (threadIdx.x == 0) s_tile = atomicAdd(b.tileTicket, 1u);
   __syncthreads();
   const uint32_t tile = s_tile;
@@ -127,28 +134,26 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(Bufs b) {
       if (lane >= off) wi += n;
     }
     if (lane < kScanThreads / 32) s_warp[lane] = wi - w;  // exclusive warp offsets
-    if (lane == kScanThreads / 32 - 1) {
-      const uint32_t agg = wi;  // tile aggregate
-      volatile unsigned long long* status = b.tileStatus;
-      uint32_t excl = 0;
-      if (tile == 0) {
-        atomicExch(b.tileStatus + tile, (2ull << 32) | agg);
-      } else {
-        atomicExch(b.tileStatus + tile, (1ull << 32) | agg);
-        int pred = (int)tile - 1;
-        while (pred >= 0) {
-          const unsigned long long w64 = waitDescriptor(status + pred, kLookbackSpinLimit, b.err);
-          const uint32_t flag = (uint32_t)(w64 >> 32);
-          if (flag == 0u) break;  // the wait expired (error word raised)
-          excl += (uint32_t)w64;
-          if (flag == 2u) break;
-          --pred;
-        }
-        __threadfence();
-        atomicExch(b.tileStatus + tile, (2ull << 32) | (excl + agg));
+    const uint32_t agg = __shfl_sync(0xffffffffu, wi, kScanThreads / 32 - 1);  // tile aggregate
+    if (lane == 0) atomicExch(b.tileStatus + tile, ((tile == 0 ? 2ull : 1ull) << 32) | agg);
+    uint32_t excl = 0;
+    if (tile > 0) {
+      // 32 earlier tiles a step, a lane each (a walk of one tile at a time is
+      // a chain of L2 round trips): the nearest one that has its prefix, or
+      // whose wait expired (error word raised), ends it
+      const volatile unsigned long long* status = b.tileStatus;
+      for (int last = (int)tile - 1;; last -= 32) {
+        const int pred = last - lane;
+        const unsigned long long w64 = pred >= 0 ? waitDescriptor(status + pred, kLookbackSpinLimit, b.err) : 2ull << 32;
+        const unsigned ends = __ballot_sync(0xffffffffu, (uint32_t)(w64 >> 32) != 1u);
+        const int stop = ends ? __ffs((int)ends) - 1 : 31;
+        excl += __reduce_add_sync(0xffffffffu, lane <= stop ? (uint32_t)w64 : 0u);
+        if (ends) break;
       }
-      s_excl = excl;
+      __threadfence();
+      if (lane == 0) atomicExch(b.tileStatus + tile, (2ull << 32) | (excl + agg));
     }
+    if (lane == 0) s_excl = excl;
   }
   __syncthreads();
   uint32_t run = s_excl + s_warp[warp] + (incl - sum);
@@ -176,7 +181,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(Bufs b) {
 
 // Unordered bucket fill: tmp[cellStart[key] .. +count) receives the members.
 __global__ void __launch_bounds__(kThreads) k_fill(Bufs b) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t i = afterPreviousEager(blockIdx.x * blockDim.x + threadIdx.x);
   bool active = i < b.N;
   uint32_t key = active ? b.key[i] : 0u;
   unsigned mask = __ballot_sync(0xffffffffu, active);
@@ -214,6 +219,7 @@ __device__ __forceinline__ void bitonic_sort_asc(uint32_t* a, uint32_t n2) {
 
 __global__ void __launch_bounds__(kBigThreads) k_bigcells(Bufs b, uint32_t* scratch) {
   extern __shared__ uint32_t sm[];
+  afterPreviousEager(0u);
   const uint32_t nBig = *b.bigCount;
   for (uint32_t j = blockIdx.x; j < nBig; j += gridDim.x) {
     uint32_t cell = b.bigList[j];
@@ -232,7 +238,7 @@ __global__ void __launch_bounds__(kBigThreads) k_bigcells(Bufs b, uint32_t* scra
 // Final slot + physical reorder with the scatter pass's predictor fused in
 // (simkernels.js:137-146 and 154-186).
 __global__ void __launch_bounds__(kThreads) k_reorder(Bufs b, int keepLam) {
-  uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t p = afterPrevious(blockIdx.x * blockDim.x + threadIdx.x);
   // both slots of the substep's largest-solid-displacement ring start at 0
   for (uint32_t q = p; q < 2u * b.S; q += gridDim.x * blockDim.x) b.solidDisp[q] = 0u;
   if (p >= b.N) return;
@@ -284,35 +290,32 @@ __global__ void k_wait_expiry(Bufs b, const unsigned long long* slot, uint32_t p
 
 uint32_t scan_tiles(uint32_t cells) { return (cells + 1 + kScanTile - 1) / kScanTile; }
 
+// clears what the whole sort starts from, then counts
 void launch_count(const Bufs& b, cudaStream_t st) {
-  cudaMemsetAsync(b.cursor, 0, sizeof(uint32_t) * b.C, st);
-  cudaMemsetAsync(b.cellWater, 0, b.C, st);
-  k_count<<<grid(b.N, kThreads), kThreads, 0, st>>>(b);
+  k_clear<<<grid(sortClearThreads(b), kThreads), kThreads, 0, st>>>(b);
+  launch_count_cleared(b, st);
+}
+void launch_count_cleared(const Bufs& b, cudaStream_t st) {
+  launchChained(k_count, grid(b.N, kThreads), kThreads, 0, st, b);
 }
 void launch_wait_expiry(const Bufs& b, const unsigned long long* slot, uint32_t polls, cudaStream_t st) {
   k_wait_expiry<<<1, 1, 0, st>>>(b, slot, polls);
 }
-void launch_scan(const Bufs& b, cudaStream_t st) {
-  // ticket, crowded-cell count and tile descriptors are contiguous: one
-  // memset resets all three
-  cudaMemsetAsync(b.tileTicket, 0, sizeof(unsigned long long) * (b.scanTiles + 1), st);
-  k_scan<<<b.scanTiles, kScanThreads, 0, st>>>(b);
-}
+void launch_scan(const Bufs& b, cudaStream_t st) { launchChained(k_scan, b.scanTiles, kScanThreads, 0, st, b); }
 void launch_scatter(const Bufs& b, cudaStream_t st) {
-  k_fill<<<grid(b.N, kThreads), kThreads, 0, st>>>(b);
+  launchChained(k_fill, grid(b.N, kThreads), kThreads, 0, st, b);
 }
 void launch_reorder(const Bufs& b, bool keepLam, cudaStream_t st) {
   // scratch for buckets too large for shared memory lives in the Sp buffer
   // (16 floats per particle >= 2 words per particle), unused until solveA
-  uint32_t* scratch = reinterpret_cast<uint32_t*>(b.Sp);
-  k_bigcells<<<kBigGrid, kBigThreads, kSmemSortCap * sizeof(uint32_t), st>>>(b, scratch);
-  k_reorder<<<grid(b.N, kThreads), kThreads, 0, st>>>(b, keepLam ? 1 : 0);
+  launch_bigcells(b, reinterpret_cast<uint32_t*>(b.Sp), st);
+  launchChained(k_reorder, grid(b.N, kThreads), kThreads, 0, st, b, keepLam ? 1 : 0);
 }
 
 // The crowded-bucket sort alone, with caller-provided scratch of at least
 // 2N words; buckets above the returned member count are left sorted.
 uint32_t launch_bigcells(const Bufs& b, uint32_t* scratch, cudaStream_t st) {
-  k_bigcells<<<kBigGrid, kBigThreads, kSmemSortCap * sizeof(uint32_t), st>>>(b, scratch);
+  launchChained(k_bigcells, kBigGrid, kBigThreads, kSmemSortCap * sizeof(uint32_t), st, b, scratch);
   return kBigCell;
 }
 

@@ -199,10 +199,12 @@ struct Bufs {
 
 // ---- launchers (sort.cu) ----
 void launch_count(const Bufs& b, cudaStream_t st);
+void launch_count_cleared(const Bufs& b, cudaStream_t st);
 void launch_scan(const Bufs& b, cudaStream_t st);
 void launch_wait_expiry(const Bufs& b, const unsigned long long* slot, uint32_t polls, cudaStream_t st);
 void launch_scatter(const Bufs& b, cudaStream_t st);
 void launch_reorder(const Bufs& b, bool keepLam, cudaStream_t st);
+uint32_t launch_bigcells(const Bufs& b, uint32_t* scratch, cudaStream_t st);
 void launch_warm_from_prev(const Bufs& b, cudaStream_t st);
 uint32_t scan_tiles(uint32_t cells);
 
@@ -246,7 +248,7 @@ void launch_solveB_list(const Bufs& b, int k, float4* vel, int flags, int varian
 void launch_loop_begin(const Bufs& b, int k0, cudaGraphConditionalHandle h, cudaStream_t st);
 void launch_loop_next(const Bufs& b, cudaGraphConditionalHandle h, cudaStream_t st);
 void launch_pbfB(const Bufs& b, int k, const float4* velIn, float4* velOut, int flags, int lanes, cudaStream_t st);
-void launch_xsph(const Bufs& b, const float4* velIn, float4* velOut, int lanes, cudaStream_t st);
+void launch_xsph(const Bufs& b, const float4* velIn, float4* velOut, int flags, int lanes, cudaStream_t st);
 void launch_updateF_integrate(const Bufs& b, const float4* velIn, int lanes, cudaStream_t st);
 
 }  // namespace xpbi
