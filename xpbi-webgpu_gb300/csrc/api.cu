@@ -1192,52 +1192,26 @@ int xpbi_read_state(xpbi_sim* sim, uint32_t scene, float* pos4, float* vel4, flo
     XPBI_CK(cudaGetLastError());
     sim->waterLPending = false;
   }
-  XPBI_TRY(xpbi_synchronize(sim));
   const SceneHost& h = sim->sc[scene];
   const Bufs& b = sim->b;
-  const size_t n = h.n, o = h.pBase, N = b.N;
-  if (n == 0) {
-    if (cell_tab) XPBI_CK(cudaMemcpy(cell_tab, b.cellStart + h.cellBase, 4 * (size_t)h.numCells, cudaMemcpyDeviceToHost));
-    return XPBI_OK;
+  const size_t n = h.n, o = h.pBase;
+  if (cell_tab || n > 0) {
+    launch_stage_state(b, h.pBase, (uint32_t)n, h.cellBase, (uint32_t)h.numCells, F12 != nullptr, L12 != nullptr,
+                       aux4 != nullptr, sorted_idx != nullptr, cell_tab != nullptr, sim->fresh ? (float)h.V0 : -1.f,
+                       sim->stream);
+    XPBI_CK(cudaGetLastError());
   }
-  std::vector<float4> v(n);
-  if (pos4) XPBI_CK(cudaMemcpy(pos4, b.pos + o, 16 * n, cudaMemcpyDeviceToHost));
-  XPBI_CK(cudaMemcpy(v.data(), b.vel + o, 16 * n, cudaMemcpyDeviceToHost));
-  if (vel4) std::memcpy(vel4, v.data(), 16 * n);
-  auto planes = [&](const float* src, float* dst12) -> int {
-    std::vector<float> t(9 * n);
-    for (int p = 0; p < 9; ++p)
-      XPBI_CK(cudaMemcpy(t.data() + p * n, src + p * N + o, 4 * n, cudaMemcpyDeviceToHost));
-    for (size_t i = 0; i < n; ++i)
-      for (int c = 0; c < 3; ++c) {
-        for (int r = 0; r < 3; ++r) dst12[12 * i + 4 * c + r] = t[(3 * c + r) * n + i];
-        dst12[12 * i + 4 * c + 3] = 0.f;
-      }
-    return XPBI_OK;
+  XPBI_TRY(xpbi_synchronize(sim));
+  auto copy = [](void* dst, const void* src, size_t bytes) {
+    return dst && bytes ? cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost) : cudaSuccess;
   };
-  if (F12) XPBI_TRY(planes(b.F, F12));
-  if (L12) XPBI_TRY(planes(b.L, L12));
-  if (aux4) {
-    std::vector<float> lam(n), st(n), pl(n);
-    XPBI_CK(cudaMemcpy(lam.data(), b.lam + o, 4 * n, cudaMemcpyDeviceToHost));
-    XPBI_CK(cudaMemcpy(st.data(), b.state + o, 4 * n, cudaMemcpyDeviceToHost));
-    XPBI_CK(cudaMemcpy(pl.data(), b.pbfLam + o, 4 * n, cudaMemcpyDeviceToHost));
-    const float V0 = (float)h.V0;
-    for (size_t i = 0; i < n; ++i) {
-      aux4[4 * i] = sim->fresh ? V0 : v[i].w;  // aux.x = V^n (== vel.w after a substep)
-      aux4[4 * i + 1] = lam[i];
-      aux4[4 * i + 2] = st[i];
-      aux4[4 * i + 3] = pl[i];
-    }
-  }
-  if (sorted_idx) {
-    XPBI_CK(cudaMemcpy(sorted_idx, b.sortedIdx + o, 4 * n, cudaMemcpyDeviceToHost));
-    for (size_t i = 0; i < n; ++i) sorted_idx[i] -= (uint32_t)o;
-  }
-  if (cell_tab) {
-    XPBI_CK(cudaMemcpy(cell_tab, b.cellStart + h.cellBase, 4 * (size_t)h.numCells, cudaMemcpyDeviceToHost));
-    for (size_t c = 0; c < h.numCells; ++c) cell_tab[c] -= (uint32_t)o;
-  }
+  XPBI_CK(copy(pos4, b.pos + o, 16 * n));
+  XPBI_CK(copy(vel4, b.vel + o, 16 * n));
+  XPBI_CK(copy(F12, b.Sp, 48 * n));
+  XPBI_CK(copy(L12, b.cons0, 48 * n));
+  XPBI_CK(copy(aux4, b.SpSelf, 16 * n));
+  XPBI_CK(copy(sorted_idx, b.tmp, 4 * n));
+  XPBI_CK(copy(cell_tab, b.cursor, 4 * (size_t)h.numCells));
   return XPBI_OK;
 }
 

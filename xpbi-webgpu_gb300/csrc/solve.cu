@@ -2214,6 +2214,31 @@ __global__ void k_copy_vel(uint32_t n, const float4* __restrict__ src, float4* _
   if (i < n) dst[i] = src[i];
 }
 
+// One scene's state in the reference layouts, staged in working buffers that
+// the next substep rewrites: F in Sp, L in cons0 (12 floats a particle, a zero
+// behind each column), aux in SpSelf, the permutation in tmp, the cell
+// offsets in cursor, both relative to the scene. A read of the state is then
+// one copy per array: it was 26 copies and the transposes on the host, 430 us
+// for 10k particles.
+__global__ void __launch_bounds__(256) k_stage_state(Bufs b, uint32_t first, uint32_t n, uint32_t firstCell, uint32_t cells,
+                                                     uint32_t base, bool F, bool L, bool aux, bool idx, bool tab,
+                                                     float volume) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (tab && t < cells) b.cursor[t] = b.cellStart[firstCell + t] - base;
+  if (t >= n) return;
+  const uint32_t i = first + t;
+  auto columns = [&](const float* src, float4* dst) {
+    const M3 m = loadM(src, b.N, i);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) dst[3 * (size_t)t + c] = make_float4(m.c[c].x, m.c[c].y, m.c[c].z, 0.f);
+  };
+  if (F) columns(b.F, b.Sp);
+  if (L) columns(b.L, b.cons0);
+  if (aux)  // V^n is vel.w after a substep, V0 before the first
+    b.SpSelf[t] = make_float4(volume >= 0.f ? volume : b.vel[i].w, b.lam[i], b.state[i], b.pbfLam[i]);
+  if (idx) b.tmp[t] = b.sortedIdx[i] - base;
+}
+
 inline unsigned grid(uint32_t n) { return (unsigned)((n + kThreads - 1) / kThreads); }
 inline unsigned gridOf(uint32_t n, int block) { return (unsigned)((n + (uint32_t)block - 1) / (uint32_t)block); }
 
@@ -2384,6 +2409,11 @@ void launch_pbfA(const Bufs& b, int k, int flags, int lanes, cudaStream_t st) {
 }
 void launch_judge(const Bufs& b, cudaGraphConditionalHandle h, bool setCond, cudaStream_t st) {
   k_judge<<<1, 256, 0, st>>>(b, h, setCond ? 1 : 0);
+}
+void launch_stage_state(const Bufs& b, uint32_t first, uint32_t n, uint32_t firstCell, uint32_t cells, bool F, bool L,
+                        bool aux, bool idx, bool tab, float volume, cudaStream_t st) {
+  k_stage_state<<<gridOf(std::max(n, tab ? cells : 0u), 256), 256, 0, st>>>(
+      b, first, n, firstCell, cells, n ? first : 0u, F, L, aux, idx, tab, volume);
 }
 void launch_restore(const Bufs& b, float4* vel, cudaStream_t st) { k_restore<<<grid(b.N), kThreads, 0, st>>>(b, vel); }
 void launch_predict(const Bufs& b, const float4* vel, cudaStream_t st) { k_predict<<<grid(b.N), kThreads, 0, st>>>(b, vel); }

@@ -209,6 +209,9 @@ void launch_warm_from_prev(const Bufs& b, cudaStream_t st);
 uint32_t scan_tiles(uint32_t cells);
 
 // ---- launchers (solve.cu) ----
+// volume: aux.x of every particle if >= 0, else vel.w
+void launch_stage_state(const Bufs& b, uint32_t first, uint32_t n, uint32_t firstCell, uint32_t cells, bool F, bool L,
+                        bool aux, bool idx, bool tab, float volume, cudaStream_t st);
 // features: also iteration 0's constraint (cons0) and the network features
 void launch_computeL(const Bufs& b, bool features, int lanes, cudaStream_t st);
 // the water particles' L of the last substep (computeL forms the solids' only)
