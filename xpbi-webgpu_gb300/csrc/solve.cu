@@ -56,14 +56,15 @@ constexpr int kMinUpdate = 7;
 // solveA and solveB are compiled in several launch shapes — the block size
 // and the minimum resident CTAs per SM asked of the register allocator (0 =
 // its own choice) — and xpbi_autotune picks one per handle by timing them on
-// its data. Entry 0 is the default: for solveA 8 CTAs of 128 per SM (64
+// its data. Entry 0 is the default. solveA: 7 CTAs of 128 per SM (72
 // registers; the constraint's per-particle tail is a separately compiled
-// function) — 0.396 ms per launch on the 4M-particle dam-breach mix against
-// 0.417 at 7 CTAs, 0.421 at 9, 0.438 at 10 and 0.58 at 5, and the best or
-// within 1% on the 256-scene batch, the snowball and the sand column; for
-// solveB the allocator's choice (80 registers) beat every cap. The 64- and
-// 256-thread shapes keep an entry's occupancy with other block sizes.
-constexpr int kSolveAMinB[kSolveAVariants] = {8, 9, 10, 7, 16, 6};
+// function): per launch 0.649 ms on the 256-scene batch against 0.681 at 8
+// CTAs, 0.724 at 9 and 0.695 at 6; 0.0205 on 113k solids against 0.0229 and
+// 0.0241 (one wave: registers beat warps); 0.308 on the 4M-particle
+// dam-breach mix against 0.305 and 0.325. solveB: 9 CTAs, 0.333 on that mix
+// against 0.354 at 8, 0.351 at 7 and 10; on the batch all of them within 2%.
+// The 64-thread shape keeps entry 1's occupancy with blocks of half the size.
+constexpr int kSolveAMinB[kSolveAVariants] = {7, 8, 9, 10, 16, 6};
 constexpr int kSolveABlock[kSolveAVariants] = {128, 128, 128, 128, 64, 128};
 constexpr int kSolveBMinB[kSolveBVariants] = {9, 8, 7, 10, 6};
 constexpr int kSolveBBlock[kSolveBVariants] = {128, 128, 128, 128, 128};
