@@ -201,21 +201,71 @@ __device__ __forceinline__ void forSingles(const uint4* L, uint32_t groups, Gath
   }
 }
 
-// A list of `cnt` entries two at a time; with G lanes per slot, lane `lane`
-// takes the pairs p with p % G == lane.
-template <int G, class Gather, class Body>
-__device__ __forceinline__ void forListPairs(const uint4* L, uint32_t cnt, uint32_t lane, Gather&& gather,
-                                             Body&& body) {
-  if constexpr (G == 1) {
-    forPairs(L, (cnt + 3u) >> 2, gather, body);
-  } else {
-    const uint32_t pairs = (cnt + 1u) >> 1;
-#pragma unroll 2
-    for (uint32_t p = lane; p < pairs; p += G) {
-      const uint2 e = *(reinterpret_cast<const uint2*>(L + kGroupStride * (p >> 1)) + (p & 1u));
-      body(e.x, e.y, gather(e.x), gather(e.y));
-    }
+// Several lanes per slot run on scenes too small to hide a chain of loads
+// behind other warps. What the chain needs and no earlier load decides is
+// fetched first: the list's count word and the first two pairs of entries a
+// lane visits (the storage holds kNbrCap entries whatever the count; entries
+// beyond it are not used).
+struct ListHead {
+  uint32_t count;
+  uint2 e0, e1;
+};
+__device__ __forceinline__ uint2 pairAt(const uint4* L, uint32_t p) {
+  return *(reinterpret_cast<const uint2*>(L + kGroupStride * (p >> 1)) + (p & 1u));
+}
+// (volatile: not moved behind the branches that follow)
+__device__ __forceinline__ uint2 pairNow(const uint4* L, uint32_t p) {
+  uint2 e;
+  asm volatile("ld.global.v2.u32 {%0, %1}, [%2];"
+               : "=r"(e.x), "=r"(e.y)
+               : "l"(reinterpret_cast<const uint2*>(L + kGroupStride * (p >> 1)) + (p & 1u)));
+  return e;
+}
+template <int G>
+__device__ __forceinline__ ListHead listHead(const uint4* L, const uint32_t* count, uint32_t i, uint32_t lane) {
+  ListHead h;
+  if constexpr (G > 1) {
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(h.count) : "l"(count + i));
+    h.e0 = pairNow(L, lane);
+    h.e1 = pairNow(L, lane + G);
   }
+  return h;
+}
+// Lane `lane` takes the pairs p with p % G == lane of slot i's list, and
+// visit(e, d0, d1) gets them in order; kTwo: two pairs in flight.
+template <int G, bool kTwo, class Gather, class Visit>
+__device__ __forceinline__ void forLanePairs(const uint4* L, const ListHead& h, uint32_t cnt, uint32_t i, uint32_t lane,
+                                             Gather&& gather, Visit&& visit) {
+  const uint32_t pairs = (cnt + 1u) >> 1;
+  uint2 e0 = h.e0, e1 = h.e1;
+#pragma unroll 1
+  for (uint32_t p = lane; p < pairs; p += 2u * G) {
+    const uint2 n0 = pairAt(L, min(p + 2u * G, kNbrCap / 2u - 1u)), n1 = pairAt(L, min(p + 3u * G, kNbrCap / 2u - 1u));
+    const bool two = p + G < pairs;
+    const auto a0 = gather(e0.x), a1 = gather(e0.y);
+    if constexpr (kTwo) {
+      if (!two) e1 = make_uint2(i, i);
+      const auto b0 = gather(e1.x), b1 = gather(e1.y);
+      visit(e0, a0, a1);
+      if (two) visit(e1, b0, b1);
+    } else {
+      visit(e0, a0, a1);
+      if (two) visit(e1, gather(e1.x), gather(e1.y));
+    }
+    e0 = n0;
+    e1 = n1;
+  }
+}
+
+// A list of `cnt` entries two at a time.
+template <int G, class Gather, class Body>
+__device__ __forceinline__ void forListPairs(const uint4* L, const ListHead& h, uint32_t cnt, uint32_t i, uint32_t lane,
+                                             Gather&& gather, Body&& body) {
+  if constexpr (G == 1)
+    forPairs(L, (cnt + 3u) >> 2, gather, body);
+  else
+    forLanePairs<G, true>(L, h, cnt, i, lane, gather,
+                          [&](uint2 e, const auto& d0, const auto& d1) { body(e.x, e.y, d0, d1); });
 }
 
 // Slot i's neighbours of its own phase, two at a time, over the recorded
@@ -227,12 +277,12 @@ __device__ __forceinline__ void forListPairs(const uint4* L, uint32_t cnt, uint3
 // (on the walk every G-th candidate of each row) and accumulates a partial
 // sum; laneSum adds them over the group.
 template <int G, class Gather, class Body>
-__device__ __forceinline__ void forSame(const Bufs& b, const Ctx& cx, uint32_t i, V3 xi, bool iWater, uint32_t lane,
-                                        Gather&& gather, Body&& body) {
+__device__ __forceinline__ void forSame(const Bufs& b, const Ctx& cx, const ListHead& h, uint32_t i, V3 xi, bool iWater,
+                                        uint32_t lane, Gather&& gather, Body&& body) {
   static_assert(G == 1 || G == 2 || G == 4, "one, two or four lanes per slot");
-  const uint32_t c = b.nbrCount[i];
+  const uint32_t c = G == 1 ? b.nbrCount[i] : h.count;
   if (c != kNbrOverflow) {
-    forListPairs<G>(nbrGroups(b.nbr, i), sameCount(c), lane, gather, body);
+    forListPairs<G>(nbrGroups(b.nbr, i), h, sameCount(c), i, lane, gather, body);
   } else {
     const SceneDev& S = *cx.scene;
     uint32_t first = i;  // a neighbour waiting for its partner
@@ -257,22 +307,20 @@ __device__ __forceinline__ void forSame(const Bufs& b, const Ctx& cx, uint32_t i
 
 // A solid's solid neighbours one at a time.
 template <int G, class Gather, class Body>
-__device__ __forceinline__ void forSameSingles(const Bufs& b, const Ctx& cx, uint32_t i, V3 xi, uint32_t lane,
-                                               Gather&& gather, Body&& body) {
-  const uint32_t c = b.nbrCount[i];
+__device__ __forceinline__ void forSameSingles(const Bufs& b, const Ctx& cx, const ListHead& h, uint32_t i, V3 xi,
+                                               uint32_t lane, Gather&& gather, Body&& body) {
+  const uint32_t c = G == 1 ? b.nbrCount[i] : h.count;
   if (c != kNbrOverflow) {
     const uint4* L = nbrGroups(b.nbr, i);
     if constexpr (G == 1) {
       forSingles(L, (sameCount(c) + 3u) >> 2, gather, body);
     } else {
-      const uint32_t pairs = (sameCount(c) + 1u) >> 1;
-#pragma unroll 2
-      for (uint32_t p = lane; p < pairs; p += G) {
-        const uint2 e = *(reinterpret_cast<const uint2*>(L + kGroupStride * (p >> 1)) + (p & 1u));
-        const auto d0 = gather(e.x), d1 = gather(e.y);
+      // records of 16 floats: two pairs of them only where the scene needs
+      // few blocks per SM
+      forLanePairs<G, G == 4>(L, h, sameCount(c), i, lane, gather, [&](uint2 e, const auto& d0, const auto& d1) {
         body(e.x, d0);
         body(e.y, d1);
-      }
+      });
     }
   } else {
     const SceneDev& S = *cx.scene;
@@ -624,13 +672,13 @@ __device__ __forceinline__ void storeSp(const Bufs& b, uint32_t i, const M3& m, 
 // velocityGradient (simkernels.js:224-245) of a solid over its solid
 // neighbours, without its factor L^T.
 template <int G>
-__device__ __forceinline__ M3 velocitySum(const Bufs& b, const Ctx& cx, uint32_t i, V3 xi, V3 vi,
+__device__ __forceinline__ M3 velocitySum(const Bufs& b, const Ctx& cx, const ListHead& h, uint32_t i, V3 xi, V3 vi,
                                           const float4* __restrict__ velIn, uint32_t lane) {
   const SceneDev& S = *cx.scene;
   const float4* __restrict__ posS = b.posS;
   // sum dv_b (L g_b)^T = (sum dv_b g_b^T) L^T: L applied once, by the caller
   VelSum A;
-  forSame<G>(b, cx, i, xi, false, lane, [&](uint32_t j) { return PV{ldg(posS + j), ldg(velIn + j)}; },
+  forSame<G>(b, cx, h, i, xi, false, lane, [&](uint32_t j) { return PV{ldg(posS + j), ldg(velIn + j)}; },
              [&](uint32_t, uint32_t, const PV& d0, const PV& d1) { A.add(pairOf(S, xi, d0, d1), vi, d0.v, d1.v); });
   return A.template total<G>(S.gradC);
 }
@@ -676,7 +724,7 @@ __device__ __noinline__ Constraint constraintTail(M3 A, TailIn in, const SceneDe
 template <int NL = 1>
 __device__ __forceinline__ Constraint evalConstraint(const Bufs& b, const Ctx& cx, uint32_t i, float4 pi,
                                                      const float4* __restrict__ velIn, const MatDev* m, float st,
-                                                     uint32_t lane = 0) {
+                                                     const ListHead& head = ListHead{}, uint32_t lane = 0) {
   const SceneDev& S = *cx.scene;
   const float4* __restrict__ posS = b.posS;
   const V3 xi = xyz(pi);
@@ -688,7 +736,7 @@ __device__ __forceinline__ Constraint evalConstraint(const Bufs& b, const Ctx& c
   // products factored out of the pair loop). s, P and the count do not depend
   // on the velocities: computeL formed them, so the sweep only accumulates A.
   VelSum A;
-  forSame<NL>(b, cx, i, xi, false, lane, [&](uint32_t j) { return PV{ldg(posS + j), ldg(velIn + j)}; },
+  forSame<NL>(b, cx, head, i, xi, false, lane, [&](uint32_t j) { return PV{ldg(posS + j), ldg(velIn + j)}; },
               [&](uint32_t, uint32_t, const PV& d0, const PV& d1) { A.add(pairOf(S, xi, d0, d1), vi, d0.v, d1.v); });
   const M3 At = A.template total<NL>(S.gradC);
   if (NL > 1 && lane != 0) return Constraint{};  // lane 0 finishes the slot
@@ -961,6 +1009,7 @@ __global__ void __launch_bounds__(kBlock, kMinB) k_solveA(Bufs b, int k, const f
   const uint32_t t = afterPrevious(blockIdx.x * blockDim.x + threadIdx.x);
   const uint32_t i = t / G, lane = t % G;
   if (i >= b.N) return;
+  const ListHead head = listHead<G>(nbrGroups(b.nbr, i), b.nbrCount, i, lane);
   const Ctx cx = ctxOf(b, i);
   const SceneDev& S = *cx.scene;
   constexpr bool track = kTrack;
@@ -987,7 +1036,7 @@ __global__ void __launch_bounds__(kBlock, kMinB) k_solveA(Bufs b, int k, const f
   }
   const uint32_t mi = matOfW(pi.w);
   const float st = b.stateS[i];
-  const Constraint c = evalConstraint<G>(b, cx, i, pi, velIn, cx.mats + mi, st, lane);
+  const Constraint c = evalConstraint<G>(b, cx, i, pi, velIn, cx.mats + mi, st, head, lane);
   if (G > 1 && lane != 0) return;
   solveAUpdate<kTrack>(b, cx, i, pi, velIn, mi, c, k, warm0, measure, act);
 }
@@ -1073,7 +1122,7 @@ __global__ void __launch_bounds__(kBlock, kMinB) k_solveA_list(Bufs b, int k, co
     recordSolidDisp(b, i, k, S.dt * length(xyz(velIn[i])));
     const uint32_t mi = matOfW(pi.w);
     const float st = b.stateS[i];
-    const Constraint c = evalConstraint<1>(b, cx, i, pi, velIn, cx.mats + mi, st, 0);
+    const Constraint c = evalConstraint<1>(b, cx, i, pi, velIn, cx.mats + mi, st);
     solveAUpdate<true>(b, cx, i, pi, velIn, mi, c, k, false, false, true);
   }
   (void)flags;
@@ -1529,6 +1578,7 @@ __global__ void __launch_bounds__(kBlock, kMinB) k_solveB(Bufs b, int k, const f
   for (uint32_t q = t; q < b.S; q += gridDim.x * blockDim.x)  // the next iteration's slot
     b.solidDisp[(size_t)((k + 1) & 1) * b.S + q] = 0u;
   if (i >= b.N) return;
+  const ListHead head = listHead<G>(nbrGroups(b.nbr, i), b.nbrCount, i, lane);
   const Ctx cx = ctxOf(b, i);
   const SceneDev& S = *cx.scene;
   const float4* __restrict__ posS = b.posS;
@@ -1587,7 +1637,7 @@ __global__ void __launch_bounds__(kBlock, kMinB) k_solveB(Bufs b, int k, const f
         corr = corr + dxc * (rinv * ((minD - dist) * w));
       }
     };
-    forSameSingles<G>(b, cx, i, xi, lane, [&](uint32_t j) { return gatherSp<G>(Sp + j, N); }, body);
+    forSameSingles<G>(b, cx, head, i, xi, lane, [&](uint32_t j) { return gatherSp<G>(Sp + j, N); }, body);
     const V3 self = xyz(b.SpSelf[i]);
     const float k = Vi * S.gradC;
     if constexpr (G > 1) {
@@ -1977,10 +2027,11 @@ __global__ void __launch_bounds__(kThreads, minPbf(G)) k_pbfB(Bufs b, int k, con
   const uint32_t t = afterPrevious((gridDim.x - 1u - blockIdx.x) * blockDim.x + threadIdx.x);
   const uint32_t i = t / G, lane = t % G;
   if (i >= b.N) return;
+  const ListHead head = listHead<G>(nbrGroups(b.nbrP, i), b.nbrPCount, i, lane);
   const Ctx cx = ctxOf(b, i);
   const SceneDev& S = *cx.scene;
   const float4 vi4 = velIn[i];
-  const uint32_t cnt = b.nbrPCount[i];
+  const uint32_t cnt = G == 1 ? b.nbrPCount[i] : head.count;
   const float4 pi = b.posS[i];
   const bool iWater = waterW(pi.w);
   // no pass, or a solid without pairs: nothing moves it
@@ -2012,10 +2063,10 @@ __global__ void __launch_bounds__(kThreads, minPbf(G)) k_pbfB(Bufs b, int k, con
     // one water material: every pair weighs by its mass / density, and one
     // gather of pbfA's record (predicted position, multiplier) serves a pair
     const float mpd = S.waterMpd;
-    forListPairs<G>(nbrGroups(b.nbrP, i), cnt, lane, [&](uint32_t j) { return ldg(b.pbfRec + j); },
+    forListPairs<G>(nbrGroups(b.nbrP, i), head, cnt, i, lane, [&](uint32_t j) { return ldg(b.pbfRec + j); },
                     [&](uint32_t, uint32_t, const float4& p, const float4& q) { add(p, q, f2(p.w, q.w), mpd, mpd); });
   } else if (cnt != kNbrOverflow) {
-    forListPairs<G>(nbrGroups(b.nbrP, i), cnt, lane, [&](uint32_t j) { return ldg(xcS + j); },
+    forListPairs<G>(nbrGroups(b.nbrP, i), head, cnt, i, lane, [&](uint32_t j) { return ldg(xcS + j); },
                     [&](uint32_t j0, uint32_t j1, const float4& p, const float4& q) {
                       add(p, q, f2(ldg(b.pbfLam + j0), ldg(b.pbfLam + j1)), mpdOf(p.w), mpdOf(q.w));
                     });
@@ -2061,6 +2112,7 @@ __global__ void __launch_bounds__(kThreads) k_xsph(Bufs b, const float4* __restr
   const uint32_t t = afterPrevious(blockIdx.x * blockDim.x + threadIdx.x);
   const uint32_t i = t / G, lane = t % G;
   if (i >= b.N) return;
+  const ListHead head = listHead<G>(nbrGroups(b.nbr, i), b.nbrCount, i, lane);
   const Ctx cx = ctxOf(b, i);
   const SceneDev& S = *cx.scene;
   const float4* __restrict__ posS = b.posS;
@@ -2073,7 +2125,7 @@ __global__ void __launch_bounds__(kThreads) k_xsph(Bufs b, const float4* __restr
   // formed together and added one after the other, every rounding fixed:
   // the water's next substep amplifies what differs here.
   V3 acc = splat(0.f);
-  forSame<G>(b, cx, i, xi, iWater, lane, [&](uint32_t j) { return PV{ldg(posS + j), ldg(velIn + j)}; },
+  forSame<G>(b, cx, head, i, xi, iWater, lane, [&](uint32_t j) { return PV{ldg(posS + j), ldg(velIn + j)}; },
              [&](uint32_t, uint32_t, const PV& d0, const PV& d1) {
                const F2 dx = f2(xi.x - d0.p.x, xi.x - d1.p.x), dy = f2(xi.y - d0.p.y, xi.y - d1.p.y),
                         dz = f2(xi.z - d0.p.z, xi.z - d1.p.z);
@@ -2124,6 +2176,7 @@ __global__ void __launch_bounds__(kThreads, kMinUpdate) k_updateF_integrate(Bufs
   const uint32_t t = (gridDim.x - 1u - blockIdx.x) * blockDim.x + threadIdx.x;
   const uint32_t i = t / G, lane = t % G;
   if (i >= b.N) return;
+  const ListHead head = listHead<G>(nbrGroups(b.nbr, i), b.nbrCount, i, lane);
   const Ctx cx = ctxOf(b, i);
   const SceneDev& S = *cx.scene;
   const float4 pi = b.posS[i];
@@ -2131,7 +2184,7 @@ __global__ void __launch_bounds__(kThreads, kMinUpdate) k_updateF_integrate(Bufs
   const float4 vi4 = velIn[i];
   const bool iWater = waterW(pi.w);
   M3 A = mzero();
-  if (!iWater) A = velocitySum<G>(b, cx, i, xyz(pi), xyz(vi4), velIn, lane);
+  if (!iWater) A = velocitySum<G>(b, cx, head, i, xyz(pi), xyz(vi4), velIn, lane);
   if (G > 1 && lane != 0) return;
   const float st = b.stateS[i];
   M3 Fn = loadM(b.FS, b.N, i);
