@@ -898,6 +898,8 @@ int createImpl(const xpbi_scene_desc* scenes, uint32_t nScenes, xpbi_sim** out) 
   A(b.xc, n);
   A(b.posP, 3 * (size_t)b.planeN);
   A(b.xcP, 3 * (size_t)b.planeN);
+  A(b.xcRef, n);
+  A(b.pbfMoved, nScenes);
   A(b.pbfRec, n);
   A(b.lamOut, n);
   A(b.lamPrev, n);

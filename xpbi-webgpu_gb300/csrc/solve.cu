@@ -46,12 +46,13 @@ constexpr int kThreads = 128;
 // 113k snowball and a 100k dam breach): computeL 9 CTAs 1.09 (8: 1.11, 7: 1.17,
 // 6: 1.27), several lanes 7: 0.054 (8: 0.059, 9: 0.065); computeL with the
 // stored constraint and features (the learned solve) 7; pbfA 10: 0.62 (8:
-// 0.66, 9: 0.64, 11: 0.63), pbfB 0.213 (8: 0.225, 11: 0.240), several lanes 8:
-// 0.0416 (10: 0.0449); the update 7: 0.303 (8: 0.337, 6: 0.332, the
+// 0.66, 9: 0.64, 11: 0.63), several lanes 8: 0.0416 (10: 0.0449); pbfB 7: 0.047
+// on the 1M-particle dam breach (8: 0.048, 9: 0.050, 10: 0.054), several lanes 8; the update 7: 0.303 (8: 0.337, 6: 0.332, the
 // allocator's choice 0.370).
 constexpr int minComputeL(int lanes) { return lanes == 1 ? 9 : 7; }
 constexpr int kMinComputeLFeatures = 7;
-constexpr int minPbf(int lanes) { return lanes == 1 ? 10 : 8; }
+constexpr int minPbfA(int lanes) { return lanes == 1 ? 10 : 8; }
+constexpr int minPbfB(int lanes) { return lanes == 1 ? 7 : 8; }
 constexpr int kMinUpdate = 7;
 // solveA and solveB are compiled in several launch shapes — the block size
 // and the minimum resident CTAs per SM asked of the register allocator (0 =
@@ -94,11 +95,31 @@ struct PV {
 
 // The predicted position of slot i for the PBF passes: the record their pair
 // loops gather and the coordinate planes pbfA's candidate walk reads.
-__device__ __forceinline__ void storeXc(const Bufs& b, uint32_t i, V3 xc, float w) {
+// The share of the support by which a PBF walk looks further than the pass
+// needs: 0.1 against 0.05 (too little for moving water: lists of an 80k dam
+// breach rebuilt in most passes) and 0.15 (more pairs to no effect): 3733,
+// 3754 and 3768 us per substep of 1M particles, 329, 332 and 328 of 80k.
+constexpr float kPbfSkin = 0.1f;
+constexpr float kNoRef = 1e30f;  // no slot's pos.w
+// The predicted position of a PBF pass. moved: also how far it lies from where
+// the last stencil walk saw it, as the scene's maximum (pbfA decides by it
+// whether the lists still hold every neighbour).
+__device__ __forceinline__ void storeXc(const Bufs& b, uint32_t i, V3 xc, float w, bool moved) {
   b.xc[i] = make_float4(xc.x, xc.y, xc.z, w);
   b.xcP[i] = xc.x;
   b.xcP[i + b.planeN] = xc.y;
   b.xcP[i + 2 * (size_t)b.planeN] = xc.z;
+  if (!moved) return;
+  const float4 ref = b.xcRef[i];
+  if (ref.w == kNoRef) return;  // a solid that no pass pairs
+  const float dx = xc.x - ref.x, dy = xc.y - ref.y, dz = xc.z - ref.z;
+  const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+  const unsigned act = __activemask();
+  const uint32_t sc = b.S > 1 ? (uint32_t)b.sceneOf[i] : 0u;
+  const unsigned peers = b.S > 1 ? __match_any_sync(act, sc) : act;
+  // (bits of d2 >= 0 order like its values; NaN, whose bits are larger, forces a walk)
+  const unsigned mx = __reduce_max_sync(peers, __float_as_uint(d2) & 0x7fffffffu);
+  if ((threadIdx.x & 31u) == (unsigned)(__ffs((int)peers) - 1) && mx > b.pbfMoved[sc]) atomicMax(b.pbfMoved + sc, mx);
 }
 
 template <class T>
@@ -166,6 +187,8 @@ __device__ __forceinline__ uint32_t lane4(const uint4& q, uint32_t s) {
 // a solid whether its 27 cells hold no water (never set on an overflow)
 __device__ __forceinline__ uint32_t sameCount(uint32_t c) { return c & 0xffu; }
 __device__ __forceinline__ uint32_t otherCount(uint32_t c) { return (c >> 8) & 0xffu; }
+// a PBF list of the neighbours within the support alone
+constexpr uint32_t kNbrExact = 0x100u;
 __device__ __forceinline__ bool dryCount(uint32_t c) { return (c >> 16) == 1u; }
 
 // Two neighbours at a time over `groups` groups: body(j0, j1, d0, d1) with
@@ -454,6 +477,7 @@ struct SubList {
   }
   // every lane of the slot together
   __device__ __forceinline__ void totals(uint32_t lane) {
+    sameAll = otherAll = sameBefore = otherBefore = anyLost = 0u;
     const uint32_t warpLane = threadIdx.x & 31u, first = warpLane & ~(uint32_t)(G - 1);
     const unsigned group = ((1u << G) - 1u) << first;
 #pragma unroll
@@ -1592,7 +1616,7 @@ __global__ void __launch_bounds__(kBlock, kMinB) k_solveB(Bufs b, int k, const f
       velOut[i] = vi4;
       if (writeXc) {
         const V3 xc = xyz(pi) + S.dt * xyz(vi4);
-        storeXc(b, i, xc, pi.w);
+        storeXc(b, i, xc, pi.w, k > 0);
       }
     }
     return;
@@ -1657,7 +1681,7 @@ __global__ void __launch_bounds__(kBlock, kMinB) k_solveB(Bufs b, int k, const f
   velOut[i] = make_float4(v.x, v.y, v.z, vi4.w);
   if (writeXc) {
     const V3 xc = xi + S.dt * v;
-    storeXc(b, i, xc, pi.w);
+    storeXc(b, i, xc, pi.w, k > 0);
   }
 }
 
@@ -1685,7 +1709,7 @@ __device__ __forceinline__ void solveBActiveSlot(const Bufs& b, int k, float4* _
     if (writeXc) {
       const float4 vi4 = vel[i];
       const V3 xc = xyz(pi) + S.dt * xyz(vi4);
-      storeXc(b, i, xc, pi.w);
+      storeXc(b, i, xc, pi.w, k > 0);
     }
     return;
   }
@@ -1695,7 +1719,7 @@ __device__ __forceinline__ void solveBActiveSlot(const Bufs& b, int k, float4* _
     if (writeXc) {
       const float4 vi4 = vel[i];
       const V3 xc = xyz(pi) + S.dt * xyz(vi4);
-      storeXc(b, i, xc, pi.w);
+      storeXc(b, i, xc, pi.w, k > 0);
     }
     return;
   }
@@ -1711,7 +1735,7 @@ __device__ __forceinline__ void solveBActiveSlot(const Bufs& b, int k, float4* _
       if (writeXc) {
         const float4 vi4 = vel[i];
         const V3 xc = xyz(pi) + S.dt * xyz(vi4);
-        storeXc(b, i, xc, pi.w);
+        storeXc(b, i, xc, pi.w, k > 0);
       }
       return;
     }
@@ -1802,7 +1826,7 @@ __device__ __forceinline__ void solveBActiveSlot(const Bufs& b, int k, float4* _
   vel[i] = make_float4(v.x, v.y, v.z, vi4.w);
   if (writeXc) {
     const V3 xc = xi + S.dt * v;
-    storeXc(b, i, xc, pi.w);
+    storeXc(b, i, xc, pi.w, k > 0);
   }
   const V3 dvel = v - xyz(vi4);
   const float dv2 = dot(dvel, dvel);
@@ -1872,9 +1896,12 @@ __device__ __forceinline__ PbfPair pbfPair(const SceneDev& S, V3 c, const float4
   const F2 dx = f2(c.x - p.x, c.x - q.x), dy = f2(c.y - p.y, c.y - q.y), dz = f2(c.z - p.z, c.z - q.z);
   const F2 r2 = fma2(dz, dz, fma2(dx, dx, mul2(dy, dy)));
   const F2 minus = f2(-1.f, -1.f);
-  const F2 x = fma2(r2, minus, f2(S.support2, S.support2));
+  // 0 past the support: the lists also hold neighbours that may come into it
+  const F2 x0 = fma2(r2, minus, f2(S.support2, S.support2));
+  const F2 x = f2(fmaxf(lo2(x0), 0.f), fmaxf(hi2(x0), 0.f));
   const F2 rinv = f2(invDist(lo2(r2)), invDist(hi2(r2)));
-  const F2 t = fma2(mul2(r2, rinv), minus, f2(S.support, S.support));
+  const F2 t0 = fma2(mul2(r2, rinv), minus, f2(S.support, S.support));
+  const F2 t = f2(fmaxf(lo2(t0), 0.f), fmaxf(hi2(t0), 0.f));
   const F2 s = mul2(mul2(mul2(f2(S.spikyC, S.spikyC), t), t), rinv);
   return PbfPair{mul2(mul2(mul2(f2(S.poly6C, S.poly6C), x), x), x), mul2(dx, s), mul2(dy, s), mul2(dz, s)};
 }
@@ -1886,8 +1913,53 @@ __device__ __forceinline__ PbfPair pbfPair(const SceneDev& S, V3 c, const float4
 // for solids (the pairs pbfB uses, simkernels.js:457-458).
 // G lanes per slot (small handles): the lanes split the stencil's rows and the
 // density sums over what they find, lane 0 finishes the slot.
+// The stencil walk of a PBF pass: slot i's neighbours by predicted position
+// within the support (exact) or the support and its skin, recorded in order;
+// the count word. Water pairs with everything, a solid with water only (the
+// water flag is the sign bit of xc.w, the sorted pos.w).
 template <int G>
-__global__ void __launch_bounds__(kThreads, minPbf(G)) k_pbfA(Bufs b, int k, int flags) {
+__device__ __forceinline__ uint32_t pbfWalk(const Bufs& b, const SceneDev& S, uint32_t i, V3 x, const float4& xc4, bool exact,
+                                            SubList<G>& sub, uint32_t lane) {
+  const float4* __restrict__ xcS = b.xc;
+  const V3 xci = xyz(xc4);
+  const bool iWater = waterW(xc4.w);
+  const Planes P = planesOf(b.xcP, b.planeN);
+#pragma unroll 1
+  for (;;) {
+    const float s2 = exact ? S.support2 : S.support2 * ((1.f + kPbfSkin) * (1.f + kPbfSkin));
+    uint32_t cnt = 0;
+    sub.same = 0;
+    sub.lost = false;
+    auto record = [&](uint32_t j) {
+      if constexpr (G == 1) {
+        *nbrEntry(b.nbrP, i, min(cnt, kNbrCap - 1u)) = j;
+        ++cnt;
+      } else {
+        sub.add(j, true);
+      }
+    };
+    walkCandidates<G>(S, b.cellStart, x, i, P, xci, s2, [&](uint32_t j) {
+      if (iWater || waterW(ldg(&xcS[j].w))) record(j);
+    }, lane);
+    if constexpr (G > 1) {
+      sub.totals(lane);
+      cnt = sub.sameAll;
+    }
+    const bool fits = cnt <= kNbrCap && !sub.lost;
+    if (!fits && !exact) {
+      exact = true;
+      continue;
+    }
+    if (!fits) return kNbrOverflow;
+    if constexpr (G > 1)
+      for (uint32_t e = 0; e < sub.same; ++e) *nbrEntry(b.nbrP, i, sub.sameBefore + e) = sub.at(e);
+    if (lane == 0)  // whole groups
+      for (uint32_t e = cnt; e & 3u; ++e) *nbrEntry(b.nbrP, i, e) = i;
+    return exact ? cnt | kNbrExact : cnt;
+  }
+}
+template <int G>
+__global__ void __launch_bounds__(kThreads, minPbfA(G)) k_pbfA(Bufs b, int k, int flags) {
   __shared__ uint32_t column[G == 1 ? 1 : SubList<G>::kCap * kThreads];
   const uint32_t t = afterPrevious(blockIdx.x * blockDim.x + threadIdx.x);
   const uint32_t i = t / G, lane = t % G;
@@ -1905,43 +1977,36 @@ __global__ void __launch_bounds__(kThreads, minPbf(G)) k_pbfA(Bufs b, int k, int
     if (k == 0 && lane == 0) {
       b.nbrPCount[i] = 0u;
       b.pbfLam[i] = 0.f;
+      b.xcRef[i].w = kNoRef;
     }
     return;
   }
-  const V3 xci = xyz(xcS[i]);
+  const float4 xc4 = xcS[i];
+  const V3 xci = xyz(xc4);
   const float s2 = S.support2;
-  // water pairs with everything, a solid with water only (the water flag is
-  // the sign bit of xc.w, the sorted pos.w)
   SubList<G> sub;
   sub.col = column + threadIdx.x;
-  uint32_t cnt = 0;
-  auto record = [&](uint32_t j) {
-    if constexpr (G == 1) {
-      *nbrEntry(b.nbrP, i, min(cnt, kNbrCap - 1u)) = j;
-      ++cnt;
-    } else {
-      sub.add(j, true);
-    }
-  };
-  const Planes P = planesOf(b.xcP, b.planeN);
-  if (iWater)
-    walkCandidates<G>(S, b.cellStart, xyz(pi), i, P, xci, s2, record, lane);
-  else
-    walkCandidates<G>(S, b.cellStart, xyz(pi), i, P, xci, s2, [&](uint32_t j) {
-      if (waterW(ldg(&xcS[j].w))) record(j);
-    }, lane);
-  if constexpr (G > 1) {
-    sub.totals(lane);
-    cnt = sub.sameAll;
+  // One walk serves several passes: it records the neighbours within
+  // (1 + skin) times the support, and as long as no particle of the scene has
+  // moved half the skin from where that walk saw it (less 2% for rounding),
+  // every neighbour within the support is among them. The terms of the others
+  // are 0 and the sums add in the same order, so the bits are those of a walk
+  // in every pass. A slot with too many of those neighbours keeps to its exact
+  // ones and walks in every pass. The walk was two thirds of the kernel: 0.62
+  // ms with it and 0.29 without on the 4M-particle mix (pbfB, over a third
+  // more pairs, 0.21 -> 0.28); 15 passes of 100k particles 680 -> 524 us.
+  const bool still = k > 0 && __uint_as_float(b.pbfMoved[sceneIndex(b, cx)]) <=
+                                  S.support2 * (0.49f * 0.49f * kPbfSkin * kPbfSkin);
+  const uint32_t before = still ? b.nbrPCount[i] : kNbrOverflow;
+  const bool reuse = still && (before & kNbrExact) == 0u;
+  uint32_t stored;
+  if (reuse) {
+    stored = before;
+  } else {
+    stored = pbfWalk<G>(b, S, i, xyz(pi), xc4, still, sub, lane);
+    if (lane == 0) b.nbrPCount[i] = stored;
   }
-  const uint32_t stored = cnt <= kNbrCap && !sub.lost ? cnt : kNbrOverflow;
-  if (stored != kNbrOverflow) {
-    if constexpr (G > 1)
-      for (uint32_t e = 0; e < sub.same; ++e) *nbrEntry(b.nbrP, i, sub.sameBefore + e) = sub.at(e);
-    if (lane == 0)  // whole groups
-      for (uint32_t e = cnt; e & 3u; ++e) *nbrEntry(b.nbrP, i, e) = i;
-  }
-  if (lane == 0) b.nbrPCount[i] = stored;
+  if (!still && lane == 0) b.xcRef[i] = xc4;
   if (!iWater) {
     if (lane == 0) {
       b.pbfLam[i] = 0.f;
@@ -1973,8 +2038,12 @@ __global__ void __launch_bounds__(kThreads, minPbf(G)) k_pbfA(Bufs b, int k, int
   auto gather = [&](uint32_t j) { return ldg(xcS + j); };
   // the pairs of the list (with several lanes, of this lane's part of it)
   auto pairs = [&](auto&& body) {
+    const uint32_t cnt = stored & 0xffu;
     if constexpr (G == 1) {
-      forPairs(nbrGroups(b.nbrP, i), (stored + 3u) >> 2, gather, body);
+      forPairs(nbrGroups(b.nbrP, i), (cnt + 3u) >> 2, gather, body);
+    } else if (reuse) {
+      forListPairs<G>(nbrGroups(b.nbrP, i), listHead<G>(nbrGroups(b.nbrP, i), b.nbrPCount, i, lane), cnt, i, lane, gather,
+                      body);
     } else {
 #pragma unroll 2
       for (uint32_t e = 0; e < sub.same; e += 2u) {
@@ -2021,17 +2090,19 @@ __global__ void __launch_bounds__(kThreads, minPbf(G)) k_pbfA(Bufs b, int k, int
 // PBF position correction with s_corr (simkernels.js:441-477) over pbfA's
 // record of predicted neighbours.
 template <int G>
-__global__ void __launch_bounds__(kThreads, minPbf(G)) k_pbfB(Bufs b, int k, const float4* velIn, float4* velOut, int flags) {
+__global__ void __launch_bounds__(kThreads, minPbfB(G)) k_pbfB(Bufs b, int k, const float4* velIn, float4* velOut, int flags) {
   // blocks run last to first: the pass starts where pbfA ended, on
   // slots whose data is still in L2
   const uint32_t t = afterPrevious((gridDim.x - 1u - blockIdx.x) * blockDim.x + threadIdx.x);
   const uint32_t i = t / G, lane = t % G;
+  for (uint32_t q = t; q < b.S; q += gridDim.x * blockDim.x) b.pbfMoved[q] = 0u;  // the next pass's maximum
   if (i >= b.N) return;
   const ListHead head = listHead<G>(nbrGroups(b.nbrP, i), b.nbrPCount, i, lane);
   const Ctx cx = ctxOf(b, i);
   const SceneDev& S = *cx.scene;
   const float4 vi4 = velIn[i];
-  const uint32_t cnt = G == 1 ? b.nbrPCount[i] : head.count;
+  const uint32_t word = G == 1 ? b.nbrPCount[i] : head.count;
+  const uint32_t cnt = word == kNbrOverflow ? word : word & 0xffu;
   const float4 pi = b.posS[i];
   const bool iWater = waterW(pi.w);
   // no pass, or a solid without pairs: nothing moves it
@@ -2047,8 +2118,10 @@ __global__ void __launch_bounds__(kThreads, minPbf(G)) k_pbfB(Bufs b, int k, con
   // sum of (lambda_i + lambda_b + s_corr) gradW mpd_b, s_corr = -k (W / W0)^4
   V3 dp = splat(0.f);
   const float nk = -S.sCorrK;
-  auto add = [&](const float4& p, const float4& q, F2 lb, float mpd0, float mpd1) {
+  float reach = 0.f;  // a solid's: > 0 if any of its recorded neighbours is within the support
+  auto add = [&](uint32_t j0, uint32_t j1, const float4& p, const float4& q, F2 lb, float mpd0, float mpd1) {
     const PbfPair r = pbfPair(S, xci, p, q);
+    if (!iWater) reach = fmaxf(reach, fmaxf(j0 != i ? lo2(r.w6) : 0.f, j1 != i ? hi2(r.w6) : 0.f));
     const F2 w = mul2(r.w6, f2(S.invW0, S.invW0));
     const F2 w2 = mul2(w, w);
     const F2 f = fma2(mul2(w2, w2), f2(nk, nk), add2(f2(li, li), lb));
@@ -2064,11 +2137,13 @@ __global__ void __launch_bounds__(kThreads, minPbf(G)) k_pbfB(Bufs b, int k, con
     // gather of pbfA's record (predicted position, multiplier) serves a pair
     const float mpd = S.waterMpd;
     forListPairs<G>(nbrGroups(b.nbrP, i), head, cnt, i, lane, [&](uint32_t j) { return ldg(b.pbfRec + j); },
-                    [&](uint32_t, uint32_t, const float4& p, const float4& q) { add(p, q, f2(p.w, q.w), mpd, mpd); });
+                    [&](uint32_t j0, uint32_t j1, const float4& p, const float4& q) {
+                      add(j0, j1, p, q, f2(p.w, q.w), mpd, mpd);
+                    });
   } else if (cnt != kNbrOverflow) {
     forListPairs<G>(nbrGroups(b.nbrP, i), head, cnt, i, lane, [&](uint32_t j) { return ldg(xcS + j); },
                     [&](uint32_t j0, uint32_t j1, const float4& p, const float4& q) {
-                      add(p, q, f2(ldg(b.pbfLam + j0), ldg(b.pbfLam + j1)), mpdOf(p.w), mpdOf(q.w));
+                      add(j0, j1, p, q, f2(ldg(b.pbfLam + j0), ldg(b.pbfLam + j1)), mpdOf(p.w), mpdOf(q.w));
                     });
   } else {
     forRows<G>(S, b.cellStart, xyz(pi), [&](uint32_t beg, uint32_t end) {
@@ -2078,13 +2153,18 @@ __global__ void __launch_bounds__(kThreads, minPbf(G)) k_pbfB(Bufs b, int k, con
         const float4 c = ldg(xcS + j);
         if (!(iWater || waterW(c.w))) continue;
         const V3 d = xci - xyz(c);
-        if (dot(d, d) < S.support2) add(c, c, f2(ldg(b.pbfLam + j), 0.f), mpdOf(c.w), 0.f);
+        if (dot(d, d) < S.support2) add(j, i, c, c, f2(ldg(b.pbfLam + j), 0.f), mpdOf(c.w), 0.f);
       }
     }, lane);
   }
   if constexpr (G > 1) {
     dp = laneSum<G>(dp);
+    reach = laneSum<G>(reach);
     if (lane != 0) return;
+  }
+  if (!iWater && reach == 0.f) {  // no pair within the support
+    velOut[i] = vi4;
+    return;
   }
   const float scale = iWater ? 1.f : 0.5f;
   V3 v = xyz(vi4) + dp * (scale / S.dt);
@@ -2261,7 +2341,7 @@ __global__ void k_predict(Bufs b, const float4* __restrict__ vel) {
   const SceneDev& S = *ctxOf(b, i).scene;
   const float4 pi = b.posS[i];
   const V3 xc = xyz(pi) + S.dt * xyz(vel[i]);
-  storeXc(b, i, xc, pi.w);
+  storeXc(b, i, xc, pi.w, true);  // (from iteration 2 on)
 }
 __global__ void k_copy_vel(uint32_t n, const float4* __restrict__ src, float4* __restrict__ dst) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;

@@ -151,6 +151,8 @@ struct Bufs {
   uint32_t* nbrP;       // the same layout: predicted-position neighbours of the current PBF pass
   uint32_t* nbrPCount;  // [N] entries, kNbrOverflow if they did not fit
   float4* xc;           // [N] predicted positions x + dt v of the current PBF pass, w = pos.w
+  float4* xcRef;        // [N] the predicted positions of the last pass that walked the stencil
+  uint32_t* pbfMoved;   // [S] largest squared distance from them since (float bits)
   float4* pbfRec;       // [N] the same predicted position with the pass's PBF multiplier in .w (written by pbfA)
   // solver instrumentation and warm start
   float* lamOut;        // [N] final multiplier of the last substep, current order
