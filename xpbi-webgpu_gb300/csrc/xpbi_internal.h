@@ -15,19 +15,21 @@ constexpr int kSolveAVariants = 6;      // launch-shape variants (autotuner): bl
 constexpr int kSolveBVariants = 5;
 // Lanes per slot by the handle's size: few slots leave most of the GPU idle
 // with one lane each, and several split a slot's neighbours; many slots fill
-// it, and the lanes only add their sums' shuffles. Measured us per launch
-// (four / two / one lanes): solveA 8k solids 11.1 / 12.1 / 14.9, 16k 13.5 /
-// 12.5 / 14.8, 28k 20 / 16 / 18, 40k 23 / 21 / 20; solveB 16k 11.7 / 13.6 /
-// 18.2, 28k 18 / 16 / 22, 80k 33 / 29 / 33, 112k 43 / 38 / 37; computeL 30k
-// particles 27 / 29 / 35, 70k 49 / 37 / 45, 100k 64 / 53 / 51; pbfA 100k 36 /
-// 37 / 46, 140k 44 / 44 / 54, 280k 77 / 68 / 74; pbfB 70k 12 / 13 / 14, 100k
-// 15 / 13 / 15.
+// it, and the lanes only add their sums' shuffles. Each line lies where us per
+// substep of settled columns and moving dams (one / two / four lanes in the
+// one kernel, the others as set here) crossed: solveA 9k solids 185 / 166 /
+// 162, 14k 195 / 180 / 182, 36k 262 / 259 / 314, 48k 280 / 281 / 335, 64k 398 /
+// 443 / 484; solveB 14k 247 / 196 / 180, 20k 259 / 209 / 223, 48k 320 / 281 /
+// 335, 70k 378 / 413 / 427; computeL, xsph and the update 14k particles 202 /
+// 186 / 181, 28k 241 / 223 / 225 (27k of a dam breach - / 164 / 156), 64k 402 / 398 / 416; pbfA (8 passes) 40k 315 /
+// 297 / 301, 90k 429 / 428 / 439, 140k 563 / 580 / 599; pbfB 40k 308 / 303 /
+// 301, 90k 436 / 439 / 441.
 struct LaneLimits {
   uint64_t four, two;  // up to so many particles: four lanes, two lanes
 };
-constexpr LaneLimits kLanesA = {12288, 32768}, kLanesB = {24576, 81920};  // by solids
-constexpr LaneLimits kLanesAll = {40960, 81920};                         // computeL, xsph, the update
-constexpr LaneLimits kLanesPbfA = {131072, 327680}, kLanesPbfB = {81920, 114688};
+constexpr LaneLimits kLanesA = {12288, 45056}, kLanesB = {16384, 57344};  // by solids
+constexpr LaneLimits kLanesAll = {32768, 65536};                         // computeL, xsph, the update
+constexpr LaneLimits kLanesPbfA = {32768, 81920}, kLanesPbfB = {49152, 65536};
 // the active set needs more solids than this (its kernels take one lane per slot)
 constexpr uint64_t kActiveSolids = 49152;
 constexpr int kResidBlocks = 256;      // at most this many partial sums of the residual per scene
