@@ -232,12 +232,15 @@ __global__ void __launch_bounds__(kRows) k_mlp_fwd(const float* __restrict__ X, 
 // bf16 values the next layer sees, as f32) and the derivatives silu'(z1),
 // silu'(z2) stay in shared memory between the passes, rows padded to 68 floats
 // so that 16-byte accesses of a row per lane meet every bank once. The weight
-// gradients dW = dz^T h are f32 products (dz is not rounded): four groups of
-// 64 threads take 32 rows each, 8 x 8 outputs per thread in packed f32x2, and
-// the four sums are added in a fixed order. One CTA per SM; a step is bound by
-// the chain of layers and the weight gradients' shared-memory reads. (8192
-// rows: 20 us against 159 us for the forward and backward kernels it
-// replaces, whose per-thread arrays lived in local memory.)
+// gradients dW = dz^T h are f32 products (dz is not rounded), 16 outputs per
+// thread in packed f32x2. Every sum over rows or CTAs adds its terms in
+// order, one after the other: a step rounds weights and activations to bf16,
+// so sums in another order, 1e-7 apart, are 1e-4 apart after some 20 steps
+// (four partial sums of 32 rows took 2 us less). One CTA per SM; a step is
+// bound by the chain of layers and the weight gradients' shared-memory reads.
+// (A call of 24 steps of 8192 rows: 1.02 ms against 4.7 with the forward and
+// backward kernels it replaces, whose per-thread arrays lived in local
+// memory; the same bits.)
 constexpr int kStepThreads = 256;
 constexpr int kLd = 68;  // row stride of the f32 buffers
 constexpr uint32_t tA = 0;                              // A tile, bf16
@@ -246,73 +249,60 @@ constexpr uint32_t tF = tW + bF32;                      // f32 vectors
 constexpr uint32_t tH1 = tF + (4 * kHid + 4) * 4;
 constexpr uint32_t kBuf = kRows * kLd * 4;
 constexpr uint32_t tH2 = tH1 + kBuf, tD1 = tH2 + kBuf, tD2 = tD1 + kBuf, tDZ = tD2 + kBuf;
-constexpr uint32_t tRed = tDZ + kBuf;                   // [2][128] and [4][64] f32 scratch
-constexpr uint32_t kStepSmem = tRed + 512 * 4;
+constexpr uint32_t tRed = tDZ + kBuf;                   // [3][128] f32 scratch
+constexpr uint32_t kStepSmem = tRed + 3 * kRows * 4;
 static_assert(kStepSmem <= 227 * 1024, "one CTA's shared memory");
 static_assert(tH1 % 16 == 0 && bF32 % 16 == 0, "16-byte aligned buffers");
 constexpr int kPartStride = (kParams + 31) & ~31;       // floats per CTA's partial
 
-// Column sums of v[c] over the warp's 32 lanes: lane c returns column c's, in
-// 31 exchanges (each halves the columns a lane still adds up).
-__device__ __forceinline__ float columnSums(float (&v)[32]) {
-  const uint32_t lane = threadIdx.x & 31u;
+// out[j * nin + i] = sum over the CTA's rows of dz[r][j] h[r][i] and outB[j] =
+// sum of dz[r][j], for h with nin = kCols columns; each sum adds its rows in
+// order (rows past the batch hold dz = 0). 2 x kCols / 8 outputs per thread.
+template <int kCols>
+__device__ __forceinline__ void wgrad(const float* dz, const float* h, float* __restrict__ out, float* __restrict__ outB) {
+  constexpr int kV = kCols / 32;  // 16-byte groups of h per thread
+  constexpr int kAcross = kCols / (4 * (kV ? kV : 1));
+  const int tid = threadIdx.x, j0 = (tid / kAcross) * (kHid * kAcross / kStepThreads), i0 = (tid % kAcross) * 4;
+  constexpr int kJ = kHid * kAcross / kStepThreads;
+  constexpr int kN = kV ? kV : 1;
+  F2 acc[kJ][2 * kN];
+  float bias[kJ];
 #pragma unroll
-  for (int w = 16; w > 0; w >>= 1) {
-    const bool up = (lane & (uint32_t)w) != 0u;
+  for (int a = 0; a < kJ; ++a) {
+    bias[a] = 0.f;
 #pragma unroll
-    for (int c = 0; c < w; ++c) {
-      const float give = up ? v[c] : v[c + w];
-      const float keep = up ? v[c + w] : v[c];
-      v[c] = keep + __shfl_xor_sync(0xffffffffu, give, w);
-    }
+    for (int q = 0; q < 2 * kN; ++q) acc[a][q] = 0ull;
   }
-  return v[0];
-}
-
-// out[j * nin + i] = sum over the CTA's rows of dz[r][j] h[r][i], h with
-// nin = 64 columns. The group partials go through `scratch0` (groups 0, 1) and
-// `scratch1` (2, 3), which may be dz and h themselves.
-__device__ __forceinline__ void wgrad64(const float* dz, const float* h, float* scratch0, float* scratch1,
-                                        float* __restrict__ out) {
-  const int tid = threadIdx.x, grp = tid >> 6, u = tid & 63, j0 = (u >> 3) * 8, i0 = (u & 7) * 4;
-  F2 acc[8][4];
+#pragma unroll 4
+  for (int r = 0; r < kRows; ++r) {
+    float d[kJ];
+    if constexpr (kJ == 2) {
+      const float2 v = *reinterpret_cast<const float2*>(dz + r * kLd + j0);
+      d[0] = v.x;
+      d[1] = v.y;
+    } else {
+      d[0] = dz[r * kLd + j0];
+    }
+    ulonglong2 x[kN];
 #pragma unroll
-  for (int a = 0; a < 8; ++a)
+    for (int q = 0; q < kN; ++q) x[q] = *reinterpret_cast<const ulonglong2*>(h + r * kLd + i0 + 32 * q);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) acc[a][q] = 0ull;
-#pragma unroll 2
-  for (int r = grp * 32; r < grp * 32 + 32; ++r) {
-    const float4 d0 = *reinterpret_cast<const float4*>(dz + r * kLd + j0);
-    const float4 d1 = *reinterpret_cast<const float4*>(dz + r * kLd + j0 + 4);
-    const ulonglong2 h0 = *reinterpret_cast<const ulonglong2*>(h + r * kLd + i0);
-    const ulonglong2 h1 = *reinterpret_cast<const ulonglong2*>(h + r * kLd + i0 + 32);
-    const float d[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
-#pragma unroll
-    for (int a = 0; a < 8; ++a) {
+    for (int a = 0; a < kJ; ++a) {
       const F2 dd = f2(d[a], d[a]);
-      acc[a][0] = fma2(dd, h0.x, acc[a][0]);
-      acc[a][1] = fma2(dd, h0.y, acc[a][1]);
-      acc[a][2] = fma2(dd, h1.x, acc[a][2]);
-      acc[a][3] = fma2(dd, h1.y, acc[a][3]);
+      bias[a] = __fadd_rn(bias[a], d[a]);
+#pragma unroll
+      for (int q = 0; q < kN; ++q) {
+        acc[a][2 * q] = fma2(dd, x[q].x, acc[a][2 * q]);
+        acc[a][2 * q + 1] = fma2(dd, x[q].y, acc[a][2 * q + 1]);
+      }
     }
   }
-  __syncthreads();  // every read of dz and h is done
-  float* mine = (grp < 2 ? scratch0 : scratch1) + (grp & 1) * kHid * kHid;
 #pragma unroll
-  for (int a = 0; a < 8; ++a) {
-    *reinterpret_cast<ulonglong2*>(mine + (j0 + a) * kHid + i0) = make_ulonglong2(acc[a][0], acc[a][1]);
-    *reinterpret_cast<ulonglong2*>(mine + (j0 + a) * kHid + i0 + 32) = make_ulonglong2(acc[a][2], acc[a][3]);
-  }
-  __syncthreads();
+  for (int a = 0; a < kJ; ++a) {
 #pragma unroll
-  for (int q = 0; q < kHid * kHid / 4 / kStepThreads; ++q) {
-    const int o = (q * kStepThreads + tid) * 4;
-    const float4 a = *reinterpret_cast<const float4*>(scratch0 + o);
-    const float4 b = *reinterpret_cast<const float4*>(scratch0 + kHid * kHid + o);
-    const float4 c = *reinterpret_cast<const float4*>(scratch1 + o);
-    const float4 d = *reinterpret_cast<const float4*>(scratch1 + kHid * kHid + o);
-    *reinterpret_cast<float4*>(out + o) = make_float4((a.x + b.x) + (c.x + d.x), (a.y + b.y) + (c.y + d.y),
-                                                      (a.z + b.z) + (c.z + d.z), (a.w + b.w) + (c.w + d.w));
+    for (int q = 0; q < kN; ++q)
+      *reinterpret_cast<ulonglong2*>(out + (j0 + a) * kCols + i0 + 32 * q) = make_ulonglong2(acc[a][2 * q], acc[a][2 * q + 1]);
+    if (i0 == 0) outB[j0 + a] = bias[a];
   }
 }
 
@@ -441,7 +431,6 @@ __global__ void __launch_bounds__(kStepThreads) k_mlp_step(const float* __restri
   {
     const float* bias = F + 2 * kHid + c0;
     const float* w4 = F + 3 * kHid + c0;
-    float y = 0.f;
 #pragma unroll
     for (int c = 0; c < 32; c += 16) {
       float z[16];
@@ -452,34 +441,49 @@ __global__ void __launch_bounds__(kStepThreads) k_mlp_step(const float* __restri
         const float s = sigm(a);
         h3[c + e] = a * s;
         dz[c + e] = s * (1.f + a * (1.f - s));
-        y += h3[c + e] * w4[c + e];
       }
     }
-    red[half * kRows + r] = y;
+    // the output adds its 64 columns in order: the second half continues the
+    // first half's sum
+    auto output = [&](float y) {
+#pragma unroll
+      for (int c = 0; c < 32; ++c) y = __fmaf_rn(h3[c], w4[c], y);
+      red[r] = y;
+    };
+    if (half == 0) output(F[4 * kHid]);
+    __syncthreads();
+    if (half == 1) output(red[r]);
   }
   tc::fenceBeforeSync();
   __syncthreads();
-  const float e = red[r] + red[kRows + r] + F[4 * kHid] - target;
+  const float e = red[r] - target;
   const float dy = valid ? 2.f * e / (float)rows : 0.f;
 #pragma unroll
-  for (int c = 0; c < 32; ++c) {
-    dz[c] = dy * F[3 * kHid + c0 + c] * dz[c];
-    h3[c] = valid ? dy * h3[c] : 0.f;  // w4's gradient sums these
-  }
-  // squared error and b4's gradient over the rows
-  float se = valid ? e * e : 0.f, sd = dy;
+  for (int c = 0; c < 32; ++c) dz[c] = dy * F[3 * kHid + c0 + c] * dz[c];
+  // gradients of w4 and b4 and the squared error, each over the rows in order
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    se += __shfl_xor_sync(0xffffffffu, se, o);
-    sd += __shfl_xor_sync(0xffffffffu, sd, o);
+  for (int c = 0; c < 32; c += 4) store4(DZ, c0 + c, h3[c], h3[c + 1], h3[c + 2], h3[c + 3]);
+  if (half == 0) {
+    red[kRows + r] = dy;
+    red[2 * kRows + r] = valid ? __fmul_rn(e, e) : 0.f;
   }
-  const float w4sum = columnSums(h3);
-  __syncthreads();  // red is free
-  red[(warp & 3) * kHid + c0 + lane] = w4sum;
-  if (half == 0 && lane == 0) {
-    red[256 + warp] = se;
-    red[260 + warp] = sd;
+  __syncthreads();
+  if (tid < kHid) {
+    float acc = 0.f;
+#pragma unroll 16
+    for (int q = 0; q < kRows; ++q) acc = __fmaf_rn(red[kRows + q], DZ[q * kLd + tid], acc);
+    P[oW4 + tid] = acc;
+  } else if (tid == 64 || tid == 96) {
+    const float* v = red + (tid == 64 ? kRows : 2 * kRows);
+    float acc = 0.f;
+#pragma unroll 16
+    for (int q = 0; q < kRows; ++q) acc = __fadd_rn(acc, v[q]);
+    if (tid == 64)
+      P[oB4] = acc;
+    else
+      sqerr[blockIdx.x] = acc;
   }
+  __syncthreads();  // DZ is free
   // ---- backward, layers 3 and 2: dz -> dW, db; the previous layer's dz
 #pragma unroll 1
   for (int layer = 2; layer >= 1; --layer) {
@@ -491,17 +495,7 @@ __global__ void __launch_bounds__(kStepThreads) k_mlp_step(const float* __restri
     }
     ready();
     issue(layer == 2 ? bW3T : bW2T, kHid);
-    if (layer == 2 && tid < kHid) {
-      P[oW4 + tid] = (red[tid] + red[kHid + tid]) + (red[2 * kHid + tid] + red[3 * kHid + tid]);
-      if (tid == 0) {
-        sqerr[blockIdx.x] = (red[256] + red[257]) + (red[258] + red[259]);
-        P[oB4] = (red[260] + red[261]) + (red[262] + red[263]);
-      }
-    }
-    const float bsum = columnSums(dz);
-    float* const H = layer == 2 ? H2 : H1;
-    wgrad64(DZ, H, DZ, H, P + (layer == 2 ? oW3 : oW2));
-    red[(warp & 3) * kHid + c0 + lane] = bsum;  // the sums read above are behind wgrad64's barriers
+    wgrad<kHid>(DZ, layer == 2 ? H2 : H1, P + (layer == 2 ? oW3 : oW2), P + (layer == 2 ? oB3 : oB2));
     await();
     const float* D = layer == 2 ? D2 : D1;
 #pragma unroll
@@ -518,9 +512,7 @@ __global__ void __launch_bounds__(kStepThreads) k_mlp_step(const float* __restri
       }
     }
     tc::fenceBeforeSync();
-    __syncthreads();  // red written; DZ and H, read for the group sums, are free
-    if (tid < kHid)
-      P[(layer == 2 ? oB3 : oB2) + tid] = (red[tid] + red[kHid + tid]) + (red[2 * kHid + tid] + red[3 * kHid + tid]);
+    __syncthreads();  // DZ and H are free
   }
   // ---- layer 1: dW1 = dz1^T x (x as bf16, the network's input precision)
 #pragma unroll
@@ -536,69 +528,32 @@ __global__ void __launch_bounds__(kStepThreads) k_mlp_step(const float* __restri
     store4(H1, 8 * half, rnd(a.x), rnd(a.y), rnd(a.z), rnd(a.w));
     store4(H1, 8 * half + 4, rnd(b.x), rnd(b.y), rnd(b.z), rnd(b.w));
   }
-  const float bsum = columnSums(dz);
-  __syncthreads();  // red's readers are done, DZ and x are written
-  red[(warp & 3) * kHid + c0 + lane] = bsum;
-  {
-    const int grp = tid >> 6, u = tid & 63, j0 = (u >> 2) * 4, i0 = (u & 3) * 4;
-    F2 acc[4][2] = {};
-#pragma unroll 4
-    for (int q = grp * 32; q < grp * 32 + 32; ++q) {
-      const float4 d = *reinterpret_cast<const float4*>(DZ + q * kLd + j0);
-      const ulonglong2 h = *reinterpret_cast<const ulonglong2*>(H1 + q * kLd + i0);
-      const float dd[4] = {d.x, d.y, d.z, d.w};
-#pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        const F2 w = f2(dd[a], dd[a]);
-        acc[a][0] = fma2(w, h.x, acc[a][0]);
-        acc[a][1] = fma2(w, h.y, acc[a][1]);
-      }
-    }
-    float* scratch = H2 + grp * kHid * kIn;  // H2 is free
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-      *reinterpret_cast<ulonglong2*>(scratch + (j0 + a) * kIn + i0) = make_ulonglong2(acc[a][0], acc[a][1]);
-    __syncthreads();
-    const int o = tid * 4;
-    const float4 a = *reinterpret_cast<const float4*>(H2 + o), b = *reinterpret_cast<const float4*>(H2 + 1024 + o),
-                 c = *reinterpret_cast<const float4*>(H2 + 2048 + o),
-                 d = *reinterpret_cast<const float4*>(H2 + 3072 + o);
-    *reinterpret_cast<float4*>(P + oW1 + o) = make_float4((a.x + b.x) + (c.x + d.x), (a.y + b.y) + (c.y + d.y),
-                                                          (a.z + b.z) + (c.z + d.z), (a.w + b.w) + (c.w + d.w));
-    if (tid < kHid)
-      P[oB1 + tid] = (red[tid] + red[kHid + tid]) + (red[2 * kHid + tid] + red[3 * kHid + tid]);
-  }
+  __syncthreads();  // DZ and x are written
+  wgrad<kIn>(DZ, H1, P + oW1, P + oB1);
   tc::fenceBeforeSync();
   __syncthreads();
   tc::fenceAfterSync();
   if (warp == 0) tc::tmemDealloc(tmem, 64);
 }
 
-// The gradient, grad[p] = sum over CTAs of partial[cta][p] in a fixed order
-// (four interleaved sums per parameter), and the mean squared error. With w:
-// the Adam update of the parameter and its bf16 copy in the blob follow in the
-// same thread.
+// The gradient, grad[p] = sum over CTAs of partial[cta][p] in order, and the
+// mean squared error. With w: the Adam update of the parameter and its bf16
+// copy in the blob follow in the same thread. A thread per parameter; the
+// loads of 32 partials are in flight at once, their additions are a chain.
 struct Adam {
   float *w, *m, *v;
   float lr, b1, b2, eps, c1, c2;
 };
 constexpr int kReduceParams = 64;
-__global__ void __launch_bounds__(4 * kReduceParams) k_mlp_reduce(const float* __restrict__ partial, uint32_t nparts,
-                                                                  const float* __restrict__ sqerr, uint32_t rows,
-                                                                  float* __restrict__ grad, float* __restrict__ loss,
-                                                                  Adam A, uint8_t* __restrict__ blob) {
-  __shared__ float sum[4][kReduceParams];
-  const uint32_t q = threadIdx.x % kReduceParams, g = threadIdx.x / kReduceParams;
-  const uint32_t p = afterPreviousEager(blockIdx.x * kReduceParams + q);
-  float acc = 0.f;
+__global__ void __launch_bounds__(kReduceParams) k_mlp_reduce(const float* __restrict__ partial, uint32_t nparts,
+                                                              const float* __restrict__ sqerr, uint32_t rows,
+                                                              float* __restrict__ grad, float* __restrict__ loss,
+                                                              Adam A, uint8_t* __restrict__ blob) {
+  const uint32_t p = afterPreviousEager(blockIdx.x * kReduceParams + threadIdx.x);
   if (p < (uint32_t)kParams) {
-#pragma unroll 8
-    for (uint32_t c = g; c < nparts; c += 4) acc += partial[(size_t)c * kPartStride + p];
-  }
-  sum[g][q] = acc;
-  __syncthreads();
-  if (g == 0 && p < (uint32_t)kParams) {
-    const float gi = (sum[0][q] + sum[1][q]) + (sum[2][q] + sum[3][q]);
+    float gi = 0.f;
+#pragma unroll 32
+    for (uint32_t c = 0; c < nparts; ++c) gi = __fadd_rn(gi, partial[(size_t)c * kPartStride + p]);
     if (grad) grad[p] = gi;
     if (A.w) {
       const float mi = A.b1 * A.m[p] + (1.f - A.b1) * gi;
@@ -610,13 +565,11 @@ __global__ void __launch_bounds__(4 * kReduceParams) k_mlp_reduce(const float* _
       packParam(blob, (int)p, wi);
     }
   }
-  if (blockIdx.x == 0 && threadIdx.x >= 4 * kReduceParams - 32) {  // the last warp: the loss
-    const uint32_t lane = threadIdx.x & 31u;
+  if (blockIdx.x == gridDim.x - 1u && threadIdx.x == kReduceParams - 1) {
     float se = 0.f;
-    for (uint32_t c = lane; c < nparts; c += 32) se += sqerr[c];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) se += __shfl_xor_sync(0xffffffffu, se, o);
-    if (lane == 0) *loss = se / (float)rows;
+#pragma unroll 32
+    for (uint32_t c = 0; c < nparts; ++c) se = __fadd_rn(se, sqerr[c]);
+    *loss = se / (float)rows;
   }
 }
 
@@ -666,7 +619,7 @@ cudaError_t mlp_grad(const float* dX, const float* dT, uint32_t rows, const void
   cudaError_t e = stepKernel(dX, dT, rows, dBlob, dPartial, dSq, dErr, st);
   if (e != cudaSuccess) return e;
   launchChained(
-      k_mlp_reduce, (kParams + kReduceParams - 1) / kReduceParams, 4 * kReduceParams, 0, st, dPartial, (rows + kRows - 1) / kRows, dSq, rows, dGrad, dLoss, Adam{}, nullptr);
+      k_mlp_reduce, (kParams + kReduceParams - 1) / kReduceParams, kReduceParams, 0, st, dPartial, (rows + kRows - 1) / kRows, dSq, rows, dGrad, dLoss, Adam{}, nullptr);
   return cudaGetLastError();
 }
 
@@ -679,7 +632,7 @@ cudaError_t mlp_train_step(const float* dX, const float* dT, uint32_t rows, floa
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.f - powf(b1, (float)step), c2 = 1.f - powf(b2, (float)step);
   launchChained(
-      k_mlp_reduce, (kParams + kReduceParams - 1) / kReduceParams, 4 * kReduceParams, 0, st, dPartial, (rows + kRows - 1) / kRows, dSq, rows, nullptr, dLoss, Adam{dW, dM, dV, lr, b1, b2, 1e-8f, c1, c2},
+      k_mlp_reduce, (kParams + kReduceParams - 1) / kReduceParams, kReduceParams, 0, st, dPartial, (rows + kRows - 1) / kRows, dSq, rows, nullptr, dLoss, Adam{dW, dM, dV, lr, b1, b2, 1e-8f, c1, c2},
       static_cast<uint8_t*>(dBlob));
   return cudaGetLastError();
 }

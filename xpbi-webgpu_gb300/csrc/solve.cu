@@ -246,7 +246,7 @@ __device__ __forceinline__ uint2 pairNow(const uint4* L, uint32_t p) {
 }
 template <int G>
 __device__ __forceinline__ ListHead listHead(const uint4* L, const uint32_t* count, uint32_t i, uint32_t lane) {
-  ListHead h;
+  ListHead h{};
   if constexpr (G > 1) {
     asm volatile("ld.global.u32 %0, [%1];" : "=r"(h.count) : "l"(count + i));
     h.e0 = pairNow(L, lane);
