@@ -1,5 +1,5 @@
-// Neighbour-gather kernels of the XPBI substep, one thread per particle slot
-// in cell order. Each restates one compute entry point of
+// Neighbour-gather kernels of the XPBI substep, one thread (on small handles
+// two or four) per particle slot in cell order. Each restates one compute entry point of
 // web/js/shaders/simkernels.js (cited per kernel).
 //
 // Neighbour lists. Positions do not move between the reorder and the final
@@ -8,18 +8,21 @@
 // and updateF. computeL walks the reference stencil once (dz outer, dy inner,
 // candidates ascending over the row-merged range of three x-adjacent cells,
 // capped at 384, simkernels.js:62-74) and records the in-support neighbours in
-// that order, so every later pass sums over exactly the reference's terms in
-// the reference's order without rescanning ~216 candidates per particle.
-// Lists that do not fit kNbrCap fall back to the stencil walk.
+// that order, the slot's own phase (solid or water) from the front of its
+// list and the other one from the back, so every later pass sums over exactly
+// the reference's terms without rescanning ~216 candidates per particle. A
+// warp's 32 lists are interleaved in groups of four entries; loops take two
+// neighbours at a time in packed f32x2 arithmetic, and a last odd one is
+// paired with the slot itself, whose terms are 0. Lists that do not fit
+// kNbrCap fall back to the stencil walk.
 //
 // PBF passes test predicted positions x + dt v, which change every
-// iteration: pbfA walks the stencil once per pass, records the predicted
-// neighbours, and both PBF kernels then iterate that record.
+// iteration: pbfA records the predicted neighbours with a margin, walks the
+// stencil again only after particles moved past it, and both PBF kernels
+// iterate that record.
 //
-// Scans are two-phase: a branch-light candidate test that only records
-// indices, then a uniform pass over the record; list loops issue the gathers
-// of entry k+1 before the arithmetic of entry k. (The candidate-scan
-// versions ran with ~14 of 32 lanes active and stalled on gathers.)
+// Scans are two-phase: a branch-light candidate test that only sets bits of a
+// mask, then a pass over the hits.
 //
 // Sorted records carry the water flag in the sign bit of pos.w (pos.w is
 // material index + colour seed >= 0, so fabsf restores it exactly).
