@@ -795,8 +795,7 @@ cudaError_t enqueueSubstep(xpbi_sim* s, const Schedule& sch, cudaStream_t st, Re
 }
 
 int kernelsPerSubstep(const Schedule& sch) {
-  // the clearing of the sort's counters is part of the count
-  int n = 5 /* count, scan, fill, bigcells, reorder */ + 1 /* computeL */ + 2 /* xsph, updateF+integrate */;
+  int n = 5 /* clear, count, scan, fill, reorder */ + 1 /* computeL */ + 2 /* xsph, updateF+integrate */;
   for (int k = 0; k < sch.K; ++k) {
     const bool list = sch.active && k >= 2;  // two compactions; before a PBF pass, the predicted positions
     n += 2 + (sch.pbf[k] ? 2 : 0) + (sch.reduce ? 1 : 0) + (list ? 2 + (sch.pbf[k] ? 1 : 0) : 0);
@@ -887,9 +886,7 @@ int createImpl(const xpbi_scene_desc* scenes, uint32_t nScenes, xpbi_sim** out) 
   unsigned long long* ctl = nullptr;
   A(ctl, (size_t)b.scanTiles + 1);
   b.tileTicket = reinterpret_cast<uint32_t*>(ctl);
-  b.bigCount = reinterpret_cast<uint32_t*>(ctl) + 1;
   b.tileStatus = ctl + 1;
-  A(b.bigList, n / 64 + 2);
   A(b.sceneOf, n);
   A(b.nbr, (size_t)kNbrCap * ((n + 31) & ~size_t(31)));  // whole warps of interleaved lists
   A(b.nbrCount, n);

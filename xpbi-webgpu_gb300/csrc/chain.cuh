@@ -53,6 +53,23 @@ inline void launchChained(void (*fn)(P...), dim3 grid, unsigned block, size_t sm
   cudaLaunchKernelEx(&c, fn, std::forward<Q>(q)...);
 }
 
+// Number of members of the bucket tmp[s0, s1) with a larger index than i: i's
+// place in it. Counting is O(L) a member whatever the bucket's size L; four
+// members a load where it pays (9,000 in one cell take 20 us more).
+__device__ __forceinline__ uint32_t rankInBucket(const uint32_t* __restrict__ tmp, uint32_t s0, uint32_t s1, uint32_t i) {
+  uint32_t rank = 0, q = s0;
+  if (s1 - s0 > 32u) {
+    for (; q & 3u; ++q) rank += tmp[q] > i ? 1u : 0u;
+#pragma unroll 4
+    for (; q + 4u <= s1; q += 4u) {
+      const uint4 m = *reinterpret_cast<const uint4*>(tmp + q);
+      rank += (m.x > i ? 1u : 0u) + (m.y > i ? 1u : 0u) + (m.z > i ? 1u : 0u) + (m.w > i ? 1u : 0u);
+    }
+  }
+  for (; q < s1; ++q) rank += tmp[q] > i ? 1u : 0u;
+  return rank;
+}
+
 // Thread t's share of clearing what a sort starts from: cell counters, water
 // flags and the scan's control block, in whole 16-byte groups (the buffers
 // are padded to them). sortClearThreads() threads clear all of it.

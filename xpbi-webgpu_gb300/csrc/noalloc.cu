@@ -7,12 +7,12 @@
 // let a library call cudaMalloc at an arbitrary moment (a pool owner may
 // forbid it, and a malloc inside stream capture breaks the capture). For
 // them, xpbi_sort_cells_noalloc runs the uniform-grid counting sort (cell
-// histogram, decoupled-lookback scan, bucket fill, crowded-bucket sort,
-// deterministic ranks) with all of its scratch in one statically sized
-// device array of this library, and allocates nothing.
+// histogram, decoupled-lookback scan, bucket fill, deterministic ranks) with
+// all of its scratch in one statically sized device array of this library, and
+// allocates nothing.
 //
 // The array is a file-scope __device__ variable: every GPU that loads the
-// library holds it (about 10 MB) until the process exits. Its device address
+// library holds it (about 7 MB) until the process exits. Its device address
 // is looked up with cudaGetSymbolAddress the first time the entry point runs
 // on a device (with that device current); that first call should therefore
 // happen before any stream capture. All calls share the array and it keeps
@@ -48,16 +48,14 @@ namespace {
 
 constexpr uint32_t kMaxParticles = XPBI_NOALLOC_MAX_PARTICLES;
 constexpr uint32_t kMaxCells = XPBI_NOALLOC_MAX_CELLS;
-constexpr uint32_t kMaxTiles = (kMaxCells + 1 + 4095) / 4096;
+constexpr uint32_t kMaxTiles = (kMaxCells + kScanTile) / kScanTile;
 
 // Scratch layout in 4-byte words (each region 64-word aligned).
 constexpr uint32_t al(uint32_t w) { return (w + 63u) & ~63u; }
 constexpr uint32_t wKey = 0;
 constexpr uint32_t wTmp = wKey + al(kMaxParticles);
 constexpr uint32_t wCursor = wTmp + al(kMaxParticles);
-constexpr uint32_t wBigList = wCursor + al(kMaxCells + 4);
-constexpr uint32_t wBigScratch = wBigList + al(kMaxParticles / 64 + 2);
-constexpr uint32_t wCtl = wBigScratch + al(2 * kMaxParticles);        // ticket, count, tile descriptors (u64)
+constexpr uint32_t wCtl = wCursor + al(kMaxCells + 4);                // ticket, tile descriptors (u64)
 constexpr uint32_t wScene = wCtl + al(2 * (kMaxTiles + 1));
 constexpr uint32_t wMats = wScene + al((sizeof(SceneDev) + 3) / 4);
 constexpr uint32_t wCellWater = wMats + al((kMaxMats * sizeof(MatDev) + 3) / 4);
@@ -72,23 +70,14 @@ std::mutex g_lock;
 uint32_t* g_addr[kMaxDevices] = {nullptr};
 
 // Deterministic slot of every bucket member (same rule as the substep's
-// reorder): bucket start + number of members with a larger index; buckets
-// above `big` members were already sorted in place.
+// reorder): bucket start + number of members with a larger index.
 __global__ void k_rank_only(const uint32_t* __restrict__ tmp, const uint32_t* __restrict__ key,
-                            const uint32_t* __restrict__ cellStart, uint32_t n, uint32_t big,
-                            uint32_t* __restrict__ sortedIdx) {
-  const uint32_t p = afterPrevious(blockIdx.x * blockDim.x + threadIdx.x);
-  if (p >= n) return;
-  const uint32_t i = tmp[p];
+                            const uint32_t* __restrict__ cellStart, uint32_t n, uint32_t* __restrict__ sortedIdx) {
+  const uint32_t i = afterPrevious(blockIdx.x * blockDim.x + threadIdx.x);
+  if (i >= n) return;
   const uint32_t c = key[i];
   const uint32_t s0 = cellStart[c], s1 = cellStart[c + 1];
-  uint32_t s = p;
-  if (s1 - s0 <= big) {
-    uint32_t rank = 0;
-    for (uint32_t q = s0; q < s1; ++q) rank += (tmp[q] > i) ? 1u : 0u;
-    s = s0 + rank;
-  }
-  sortedIdx[s] = i;
+  sortedIdx[s0 + rankInBucket(tmp, s0, s1, i)] = i;
 }
 
 // Writes the grid description, clears the material table (no material is
@@ -167,9 +156,7 @@ extern "C" int xpbi_sort_cells_noalloc(const float* pos4, uint32_t n, const floa
   b.tmp = base + wTmp;
   b.cursor = base + wCursor;
   b.cellStart = cell_start;
-  b.bigList = base + wBigList;
   b.tileTicket = base + wCtl;
-  b.bigCount = base + wCtl + 1;
   b.tileStatus = reinterpret_cast<unsigned long long*>(base + wCtl) + 1;
   b.scenes = reinterpret_cast<SceneDev*>(base + wScene);
   b.mats = reinterpret_cast<MatDev*>(base + wMats);  // zeroed: no material is water
@@ -185,8 +172,7 @@ extern "C" int xpbi_sort_cells_noalloc(const float* pos4, uint32_t n, const floa
   launch_count_cleared(b, st);
   launch_scan(b, st);
   launch_scatter(b, st);
-  const uint32_t big = launch_bigcells(b, base + wBigScratch, st);
-  launchChained(k_rank_only, (n + 255) / 256, 256, 0, st, b.tmp, b.key, b.cellStart, n, big, sorted_idx);
+  launchChained(k_rank_only, (n + 255) / 256, 256, 0, st, b.tmp, b.key, b.cellStart, n, sorted_idx);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return setError(XPBI_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
   return XPBI_OK;

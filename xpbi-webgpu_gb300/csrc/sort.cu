@@ -8,7 +8,6 @@
 //   k_scan     single-pass decoupled-lookback exclusive scan of the histogram
 //   k_fill     warp-aggregated slot reservation: each cell's members land in
 //              its bucket in arbitrary order
-//   k_bigcells deterministic sort of crowded buckets (bounded cost)
 //   k_reorder  final slot = bucket start + number of bucket members with a
 //              larger previous index, then moves pos/vel/F/state into the
 //              slot with the scatter pass's predictor fused in
@@ -25,13 +24,8 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kScanThreads = 256;
-constexpr int kScanItems = 16;
-constexpr int kScanTile = kScanThreads * kScanItems;
-constexpr uint32_t kBigCell = 64u;          // buckets above this use k_bigcells
-constexpr uint32_t kSmemSortCap = 8192u;    // bitonic in shared memory up to this size
+constexpr int kScanItems = (int)kScanTile / kScanThreads;
 constexpr uint32_t kLookbackSpinLimit = 1u << 22;
-constexpr int kBigThreads = 256;
-constexpr unsigned kBigGrid = 152;
 
 __device__ __forceinline__ uint32_t sceneOfSlot(const Bufs& b, uint32_t i) {
   return b.S > 1 ? (uint32_t)b.sceneOf[i] : 0u;
@@ -112,10 +106,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(Bufs b) {
   }
   uint32_t sum = 0;
 #pragma unroll
-  for (int k = 0; k < kScanItems; ++k) {
-    sum += v[k];
-    if (v[k] > kBigCell) b.bigList[atomicAdd(b.bigCount, 1u)] = base + k;
-  }
+  for (int k = 0; k < kScanItems; ++k) sum += v[k];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t incl = sum;
 #pragma unroll
@@ -196,67 +187,26 @@ __global__ void __launch_bounds__(kThreads) k_fill(Bufs b) {
   b.tmp[base + rank] = i;
 }
 
-// Buckets with more than kBigCell members (listed by k_scan) are sorted
-// here, descending, by one CTA each: a bitonic network on ~index ascending, in
-// shared memory up to kSmemSortCap entries, otherwise in the scratch region
-// [2*start, 2*start + 2*len) of `scratch`, which is disjoint between buckets.
-// Cost is O(L log^2 L) per bucket, so even a pile-up of every particle in one
-// cell stays bounded. With no crowded cell every CTA exits at once.
-__device__ __forceinline__ void bitonic_sort_asc(uint32_t* a, uint32_t n2) {
-  for (uint32_t size = 2; size <= n2; size <<= 1) {
-    for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-      for (uint32_t t = threadIdx.x; t < n2 / 2; t += blockDim.x) {
-        uint32_t lo = 2 * stride * (t / stride) + (t % stride);
-        uint32_t hi = lo + stride;
-        bool up = ((lo & size) == 0);
-        uint32_t x = a[lo], y = a[hi];
-        if ((x > y) == up) { a[lo] = y; a[hi] = x; }
-      }
-      __syncthreads();
-    }
-  }
-}
-
-__global__ void __launch_bounds__(kBigThreads) k_bigcells(Bufs b, uint32_t* scratch) {
-  extern __shared__ uint32_t sm[];
-  afterPreviousEager(0u);
-  const uint32_t nBig = *b.bigCount;
-  for (uint32_t j = blockIdx.x; j < nBig; j += gridDim.x) {
-    uint32_t cell = b.bigList[j];
-    uint32_t s0 = b.cellStart[cell], len = b.cellStart[cell + 1] - s0;
-    uint32_t n2 = 1;
-    while (n2 < len) n2 <<= 1;
-    uint32_t* a = n2 <= kSmemSortCap ? sm : scratch + 2ull * s0;
-    for (uint32_t q = threadIdx.x; q < n2; q += blockDim.x) a[q] = q < len ? ~b.tmp[s0 + q] : 0xffffffffu;
-    __syncthreads();
-    bitonic_sort_asc(a, n2);
-    for (uint32_t q = threadIdx.x; q < len; q += blockDim.x) b.tmp[s0 + q] = ~a[q];
-    __syncthreads();
-  }
-}
-
 // Final slot + physical reorder with the scatter pass's predictor fused in
-// (simkernels.js:137-146 and 154-186).
+// (simkernels.js:137-146 and 154-186). A thread per particle in previous
+// order: everything it moves is loaded at once, and only its slot waits for
+// the chain key -> bucket -> members. (By slot, the chain was one load longer
+// and the moved data hung on its end, and crowded buckets had a kernel of
+// their own, a block's bitonic sort: the sort of 250k keys 21.3 us.)
 __global__ void __launch_bounds__(kThreads) k_reorder(Bufs b, int keepLam) {
-  const uint32_t p = afterPrevious(blockIdx.x * blockDim.x + threadIdx.x);
+  const uint32_t i = afterPrevious(blockIdx.x * blockDim.x + threadIdx.x);
   // both slots of the substep's largest-solid-displacement ring start at 0
-  for (uint32_t q = p; q < 2u * b.S; q += gridDim.x * blockDim.x) b.solidDisp[q] = 0u;
-  if (p >= b.N) return;
-  uint32_t i = b.tmp[p];
-  uint32_t key = b.key[i];
-  uint32_t s0 = b.cellStart[key], s1 = b.cellStart[key + 1];
-  uint32_t s;
-  if (s1 - s0 > kBigCell) {
-    s = p;  // bucket already sorted by k_bigcells
-  } else {
-    uint32_t rank = 0;
-    for (uint32_t q = s0; q < s1; ++q) rank += (b.tmp[q] > i) ? 1u : 0u;
-    s = s0 + rank;
-  }
+  for (uint32_t q = i; q < 2u * b.S; q += gridDim.x * blockDim.x) b.solidDisp[q] = 0u;
+  if (i >= b.N) return;
+  const uint32_t key = b.key[i];
+  const float4 pp = b.pos[i], v = b.vel[i];
+  const M3 F = loadM(b.F, b.N, i);
+  const float st = b.state[i];
+  const uint32_t s0 = b.cellStart[key], s1 = b.cellStart[key + 1];
+  const uint32_t s = s0 + rankInBucket(b.tmp, s0, s1, i);
   b.sortedIdx[s] = i;
   const SceneDev& S = b.scenes[sceneOfSlot(b, i)];
   // sorted records carry the water flag in the sign bit of pos.w (>= 0)
-  const float4 pp = b.pos[i];
   uint32_t mi = 0u;
   if (pp.w > 0.f) mi = min((uint32_t)pp.w, 7u);
   const bool water = b.mats[S.matBase + mi].kind == kKindWater;
@@ -264,14 +214,12 @@ __global__ void __launch_bounds__(kThreads) k_reorder(Bufs b, int keepLam) {
   b.posP[s] = pp.x;
   b.posP[s + b.planeN] = pp.y;
   b.posP[s + 2 * (size_t)b.planeN] = pp.z;
-  M3 F = loadM(b.F, b.N, i);
   storeM(b.FS, b.N, s, F);
   float Vn = S.V0 * clampf(det(F), 0.1f, 10.f);
-  float4 v = b.vel[i];
   V3 g = v3(S.grav[0], S.grav[1], S.grav[2]);
   V3 vn = xyz(v) + g * S.dt;
   b.velS[0][s] = make_float4(vn.x, vn.y, vn.z, Vn);
-  b.stateS[s] = b.state[i];
+  b.stateS[s] = st;
   b.lam[s] = 0.f;
   if (keepLam) b.lamPrev[s] = b.lamOut[i];
 }
@@ -306,17 +254,7 @@ void launch_scatter(const Bufs& b, cudaStream_t st) {
   launchChained(k_fill, grid(b.N, kThreads), kThreads, 0, st, b);
 }
 void launch_reorder(const Bufs& b, bool keepLam, cudaStream_t st) {
-  // scratch for buckets too large for shared memory lives in the Sp buffer
-  // (16 floats per particle >= 2 words per particle), unused until solveA
-  launch_bigcells(b, reinterpret_cast<uint32_t*>(b.Sp), st);
   launchChained(k_reorder, grid(b.N, kThreads), kThreads, 0, st, b, keepLam ? 1 : 0);
-}
-
-// The crowded-bucket sort alone, with caller-provided scratch of at least
-// 2N words; buckets above the returned member count are left sorted.
-uint32_t launch_bigcells(const Bufs& b, uint32_t* scratch, cudaStream_t st) {
-  launchChained(k_bigcells, kBigGrid, kBigThreads, kSmemSortCap * sizeof(uint32_t), st, b, scratch);
-  return kBigCell;
 }
 
 }  // namespace xpbi

@@ -13,6 +13,7 @@ constexpr uint32_t kKindWater = 6u;
 constexpr uint32_t kNbrCap = 64u;      // neighbour-list capacity per particle
 constexpr int kSolveAVariants = 6;      // launch-shape variants (autotuner): block size, register cap
 constexpr int kSolveBVariants = 5;
+constexpr uint32_t kScanTile = 4096u;     // cells per block of the scan
 // Lanes per slot by the handle's size: few slots leave most of the GPU idle
 // with one lane each, and several split a slot's neighbours; many slots fill
 // it, and the lanes only add their sums' shuffles. Each line lies where us per
@@ -143,9 +144,7 @@ struct Bufs {
   uint32_t* cellStart;  // [C+1] exclusive cell starts, sentinel = N
   uint8_t* cellWater;   // [C] 1 if the cell holds a water particle this substep
   uint32_t* tileTicket;            // word 0 of the scan control block
-  uint32_t* bigCount;              // word 1: crowded cells found by the scan
   unsigned long long* tileStatus;  // [tiles] look-back descriptors (after the two words)
-  uint32_t* bigList;               // [N/64 + 2] crowded cells (> 64 members)
   uint16_t* sceneOf;    // [N] scene of each particle slot (static)
   uint32_t* nbr;        // [ceil(N / 32)][kNbrCap / 4][32][4] in-support neighbours: own phase from the front in
                         //   stencil order, the other phase from the back
@@ -208,7 +207,6 @@ void launch_scan(const Bufs& b, cudaStream_t st);
 void launch_wait_expiry(const Bufs& b, const unsigned long long* slot, uint32_t polls, cudaStream_t st);
 void launch_scatter(const Bufs& b, cudaStream_t st);
 void launch_reorder(const Bufs& b, bool keepLam, cudaStream_t st);
-uint32_t launch_bigcells(const Bufs& b, uint32_t* scratch, cudaStream_t st);
 void launch_warm_from_prev(const Bufs& b, cudaStream_t st);
 uint32_t scan_tiles(uint32_t cells);
 
