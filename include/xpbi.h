@@ -229,9 +229,9 @@ int xpbi_render(xpbi_sim* sim, uint32_t scene, const xpbi_camera* cam, uint32_t 
                 uint8_t* rgba_out, void** device_rgba);
 
 /* ---- autotuner (no counterpart in the reference) ----
- * solveA and solveB are built in several launch shapes: block size (64,
- * 128 or 256 threads) and register allocation (resident blocks per SM traded
- * against registers). xpbi_autotune runs the
+ * solveA and solveB are built in several launch shapes: block size (64 or 128
+ * threads) and register allocation (resident blocks per SM traded against
+ * registers). xpbi_autotune runs the
  * substep's preparation (sort, reorder, Bonet-Lok correction) on the current
  * state and times iteration 0 of every variant `repeats` times on this
  * handle's own data, then keeps the fastest of each for the handle (the
