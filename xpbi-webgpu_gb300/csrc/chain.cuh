@@ -25,7 +25,12 @@
 namespace xpbi {
 
 // Waits for the preceding kernel. Returns its argument: an index taken
-// through here keeps the loads it addresses behind the wait.
+// through here keeps the loads it addresses behind the wait, if they are
+// ordinary loads. Read-only-cache loads (__ldg, and any load through a kernel
+// parameter that is const and __restrict__) are not memory operations to the
+// assembler's scheduler and do move above the wait (seen in the training
+// step's weights): in a chained kernel only addresses formed from data
+// loaded behind the wait may be read that way.
 __device__ __forceinline__ uint32_t afterPrevious(uint32_t t) {
   asm volatile("griddepcontrol.wait;" : "+r"(t) : : "memory");
   return t;
@@ -56,7 +61,7 @@ inline void launchChained(void (*fn)(P...), dim3 grid, unsigned block, size_t sm
 // Number of members of the bucket tmp[s0, s1) with a larger index than i: i's
 // place in it. Counting is O(L) a member whatever the bucket's size L; four
 // members a load where it pays (9,000 in one cell take 20 us more).
-__device__ __forceinline__ uint32_t rankInBucket(const uint32_t* __restrict__ tmp, uint32_t s0, uint32_t s1, uint32_t i) {
+__device__ __forceinline__ uint32_t rankInBucket(const uint32_t* tmp, uint32_t s0, uint32_t s1, uint32_t i) {
   uint32_t rank = 0, q = s0;
   if (s1 - s0 > 32u) {
     for (; q & 3u; ++q) rank += tmp[q] > i ? 1u : 0u;

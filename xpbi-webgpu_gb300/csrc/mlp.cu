@@ -255,59 +255,70 @@ static_assert(kStepSmem <= 227 * 1024, "one CTA's shared memory");
 static_assert(tH1 % 16 == 0 && bF32 % 16 == 0, "16-byte aligned buffers");
 constexpr int kPartStride = (kParams + 31) & ~31;       // floats per CTA's partial
 
-// out[j * nin + i] = sum over the CTA's rows of dz[r][j] h[r][i] and outB[j] =
-// sum of dz[r][j], for h with nin = kCols columns; each sum adds its rows in
-// order (rows past the batch hold dz = 0). 2 x kCols / 8 outputs per thread.
+// out[j * kCols + i] = sum over the CTA's rows of dz[r][j] h[r][i] and outB[j] =
+// sum of dz[r][j], for h with kCols columns; each sum adds its rows in order
+// (rows past the batch hold dz = 0). Bound by shared-memory reads: a warp takes
+// 8 outputs j, so that its reads of dz are one address for all lanes (for 16
+// columns, one per half), and its lanes the columns, two each (16 columns: one
+// column, 4 of the warp's j). (2 x 8 outputs per thread, reading 16-byte groups
+// of h, took 9,800 cycles for 64 columns and 6,250 for 16.)
 template <int kCols>
 __device__ __forceinline__ void wgrad(const float* dz, const float* h, float* __restrict__ out, float* __restrict__ outB) {
-  constexpr int kV = kCols / 32;  // 16-byte groups of h per thread
-  constexpr int kAcross = kCols / (4 * (kV ? kV : 1));
-  const int tid = threadIdx.x, j0 = (tid / kAcross) * (kHid * kAcross / kStepThreads), i0 = (tid % kAcross) * 4;
-  constexpr int kJ = kHid * kAcross / kStepThreads;
-  constexpr int kN = kV ? kV : 1;
-  F2 acc[kJ][2 * kN];
-  float bias[kJ];
+  static_assert(kStepThreads == 256 && kHid == 64 && (kCols == 64 || kCols == 16), "8 warps of 8 outputs j");
+  constexpr int kI = kCols == 64 ? 2 : 1;  // columns per lane
+  constexpr int kP = kCols == 64 ? 4 : 2;  // pairs of j per lane
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i0 = kCols == 64 ? 2 * lane : lane & 15, j0 = warp * 8 + (kCols == 64 ? 0 : (lane >> 4) * 4);
+  F2 acc[kP][kI], bias[kP];
 #pragma unroll
-  for (int a = 0; a < kJ; ++a) {
-    bias[a] = 0.f;
+  for (int p = 0; p < kP; ++p) {
+    bias[p] = 0ull;
 #pragma unroll
-    for (int q = 0; q < 2 * kN; ++q) acc[a][q] = 0ull;
+    for (int i = 0; i < kI; ++i) acc[p][i] = 0ull;
   }
-#pragma unroll 4
+#pragma unroll 8
   for (int r = 0; r < kRows; ++r) {
-    float d[kJ];
-    if constexpr (kJ == 2) {
-      const float2 v = *reinterpret_cast<const float2*>(dz + r * kLd + j0);
-      d[0] = v.x;
-      d[1] = v.y;
-    } else {
-      d[0] = dz[r * kLd + j0];
+    F2 d[kP];
+#pragma unroll
+    for (int p = 0; p < kP; p += 2) {
+      const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(dz + r * kLd + j0 + 2 * p);
+      d[p] = v.x;
+      d[p + 1] = v.y;
     }
-    ulonglong2 x[kN];
+    float x[kI];
+    if constexpr (kI == 2) {
+      const float2 v = *reinterpret_cast<const float2*>(h + r * kLd + i0);
+      x[0] = v.x;
+      x[1] = v.y;
+    } else {
+      x[0] = h[r * kLd + i0];
+    }
 #pragma unroll
-    for (int q = 0; q < kN; ++q) x[q] = *reinterpret_cast<const ulonglong2*>(h + r * kLd + i0 + 32 * q);
+    for (int p = 0; p < kP; ++p) {
+      bias[p] = add2(bias[p], d[p]);
 #pragma unroll
-    for (int a = 0; a < kJ; ++a) {
-      const F2 dd = f2(d[a], d[a]);
-      bias[a] = __fadd_rn(bias[a], d[a]);
-#pragma unroll
-      for (int q = 0; q < kN; ++q) {
-        acc[a][2 * q] = fma2(dd, x[q].x, acc[a][2 * q]);
-        acc[a][2 * q + 1] = fma2(dd, x[q].y, acc[a][2 * q + 1]);
-      }
+      for (int i = 0; i < kI; ++i) acc[p][i] = fma2(d[p], f2(x[i], x[i]), acc[p][i]);
     }
   }
 #pragma unroll
-  for (int a = 0; a < kJ; ++a) {
-#pragma unroll
-    for (int q = 0; q < kN; ++q)
-      *reinterpret_cast<ulonglong2*>(out + (j0 + a) * kCols + i0 + 32 * q) = make_ulonglong2(acc[a][2 * q], acc[a][2 * q + 1]);
-    if (i0 == 0) outB[j0 + a] = bias[a];
+  for (int p = 0; p < kP; ++p) {
+    float* o0 = out + (j0 + 2 * p) * kCols + i0;
+    if constexpr (kI == 2) {
+      *reinterpret_cast<float2*>(o0) = make_float2(lo2(acc[p][0]), lo2(acc[p][1]));
+      *reinterpret_cast<float2*>(o0 + kCols) = make_float2(hi2(acc[p][0]), hi2(acc[p][1]));
+    } else {
+      o0[0] = lo2(acc[p][0]);
+      o0[kCols] = hi2(acc[p][0]);
+    }
+    if (i0 == 0) {
+      outB[j0 + 2 * p] = lo2(bias[p]);
+      outB[j0 + 2 * p + 1] = hi2(bias[p]);
+    }
   }
 }
 
 __global__ void __launch_bounds__(kStepThreads) k_mlp_step(const float* __restrict__ X, const float* __restrict__ T,
-                                                           uint32_t rows, const uint8_t* __restrict__ blob,
+                                                           uint32_t rows, const uint8_t* blob,
                                                            float* __restrict__ partial, float* __restrict__ sqerr,
                                                            int* err) {
   extern __shared__ __align__(1024) uint8_t sm[];
@@ -349,9 +360,19 @@ __global__ void __launch_bounds__(kStepThreads) k_mlp_step(const float* __restri
   {
     const uint4* src = reinterpret_cast<const uint4*>(blob);
     uint4* dst = reinterpret_cast<uint4*>(sm + tW);
-    for (uint32_t q = w0; q < bF32 / 16u; q += kStepThreads) dst[q] = src[q];
+    // every load before the first store: one round trip to L2 (a loop took 2.7 us)
+    constexpr uint32_t kEach = (bF32 / 16u + kStepThreads - 1u) / kStepThreads;
+    uint4 v[kEach];
+#pragma unroll
+    for (uint32_t k = 0; k < kEach; ++k)
+      if (w0 + k * kStepThreads < bF32 / 16u) v[k] = src[w0 + k * kStepThreads];
     const float* fs = reinterpret_cast<const float*>(blob + bF32);
-    for (uint32_t q = w0; q < 4 * kHid + 1; q += kStepThreads) F[q] = fs[q];
+    const float f0 = fs[w0], f1 = fs[4 * kHid];
+#pragma unroll
+    for (uint32_t k = 0; k < kEach; ++k)
+      if (w0 + k * kStepThreads < bF32 / 16u) dst[w0 + k * kStepThreads] = v[k];
+    F[w0] = f0;
+    if (w0 == 0u) F[4 * kHid] = f1;
   }
   tc::fenceProxyAsync();
   tc::fenceBeforeSync();
@@ -545,10 +566,10 @@ struct Adam {
   float lr, b1, b2, eps, c1, c2;
 };
 constexpr int kReduceParams = 64;
-__global__ void __launch_bounds__(kReduceParams) k_mlp_reduce(const float* __restrict__ partial, uint32_t nparts,
-                                                              const float* __restrict__ sqerr, uint32_t rows,
-                                                              float* __restrict__ grad, float* __restrict__ loss,
-                                                              Adam A, uint8_t* __restrict__ blob) {
+__global__ void __launch_bounds__(kReduceParams) k_mlp_reduce(const float* partial, uint32_t nparts,
+                                                              const float* sqerr, uint32_t rows,
+                                                              float* grad, float* loss,
+                                                              Adam A, uint8_t* blob) {
   const uint32_t p = afterPreviousEager(blockIdx.x * kReduceParams + threadIdx.x);
   if (p < (uint32_t)kParams) {
     float gi = 0.f;

@@ -71,8 +71,8 @@ uint32_t* g_addr[kMaxDevices] = {nullptr};
 
 // Deterministic slot of every bucket member (same rule as the substep's
 // reorder): bucket start + number of members with a larger index.
-__global__ void k_rank_only(const uint32_t* __restrict__ tmp, const uint32_t* __restrict__ key,
-                            const uint32_t* __restrict__ cellStart, uint32_t n, uint32_t* __restrict__ sortedIdx) {
+__global__ void k_rank_only(const uint32_t* tmp, const uint32_t* key, const uint32_t* cellStart, uint32_t n,
+                            uint32_t* sortedIdx) {
   const uint32_t i = afterPrevious(blockIdx.x * blockDim.x + threadIdx.x);
   if (i >= n) return;
   const uint32_t c = key[i];

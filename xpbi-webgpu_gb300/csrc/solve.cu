@@ -1031,7 +1031,7 @@ __device__ __forceinline__ void solveAUpdate(const Bufs& b, const Ctx& cx, uint3
 }
 
 template <bool kTrack, int kMinB, int G, int kBlock = kThreads>
-__global__ void __launch_bounds__(kBlock, kMinB) k_solveA(Bufs b, int k, const float4* __restrict__ velIn,
+__global__ void __launch_bounds__(kBlock, kMinB) k_solveA(Bufs b, int k, const float4* velIn,
                                                             int flags) {
   const uint32_t t = afterPrevious(blockIdx.x * blockDim.x + threadIdx.x);
   const uint32_t i = t / G, lane = t % G;
@@ -1596,8 +1596,8 @@ struct ImpulseSum {
 // flags & kMeasureOnly: the contact residual only, of every solid slot, no
 //   velocity update (the pass after the last iteration).
 template <int kMinB, int G, int kBlock = kThreads>
-__global__ void __launch_bounds__(kBlock, kMinB) k_solveB(Bufs b, int k, const float4* __restrict__ velIn,
-                                                      float4* __restrict__ velOut, int writeXc, int flags) {
+__global__ void __launch_bounds__(kBlock, kMinB) k_solveB(Bufs b, int k, const float4* velIn,
+                                                      float4* velOut, int writeXc, int flags) {
   // blocks run last to first: the pass starts where solveA ended, on slots
   // whose data is still in L2
   const uint32_t t = afterPrevious((gridDim.x - 1u - blockIdx.x) * blockDim.x + threadIdx.x);
@@ -1642,7 +1642,7 @@ __global__ void __launch_bounds__(kBlock, kMinB) k_solveB(Bufs b, int k, const f
     // the predicted positions and of the bound; the test on the pairs that
     // remain is unchanged, so the result is too.
     const float reach = (minD + S.dt * length(xyz(vi4)) +
-                         __uint_as_float(__ldg(b.solidDisp + (size_t)(k & 1) * b.S + (cx.scene - b.scenes)))) *
+                         __uint_as_float(b.solidDisp[(size_t)(k & 1) * b.S + (cx.scene - b.scenes)])) *
                         1.01f;
     const float reach2 = reach * reach;
     ImpulseSum sum;
@@ -2191,7 +2191,7 @@ __global__ void __launch_bounds__(kThreads, minPbfB(G)) k_pbfB(Bufs b, int k, co
 // ---------------------------------------------------------------- xsph
 // simkernels.js:480-507
 template <int G>
-__global__ void __launch_bounds__(kThreads) k_xsph(Bufs b, const float4* __restrict__ velIn, float4* __restrict__ velOut) {
+__global__ void __launch_bounds__(kThreads) k_xsph(Bufs b, const float4* velIn, float4* velOut) {
   const uint32_t t = afterPrevious(blockIdx.x * blockDim.x + threadIdx.x);
   const uint32_t i = t / G, lane = t % G;
   if (i >= b.N) return;
