@@ -130,6 +130,17 @@ __device__ __forceinline__ T ldg(const T* p) {
   return __ldg(p);
 }
 
+// What a slot's own index addresses in the solve kernels: through the read-only
+// cache with one lane (1% of a 4M substep), whose launches are plain; several
+// lanes are chained to the preceding kernel and need an ordinary load.
+template <int G, class T>
+__device__ __forceinline__ T loadOwn(const T* p) {
+  if constexpr (G == 1)
+    return __ldg(p);
+  else
+    return *p;
+}
+
 // Stencil walk over the 9 row-merged ranges (simkernels.js:62-74):
 // row(beg, end) is called per in-range row. With G lanes per slot, lane
 // `lane` takes the rows r with r % G == lane.
@@ -755,7 +766,7 @@ __device__ __forceinline__ Constraint evalConstraint(const Bufs& b, const Ctx& c
   const SceneDev& S = *cx.scene;
   const float4* __restrict__ posS = b.posS;
   const V3 xi = xyz(pi);
-  const V3 vi = xyz(velIn[i]);
+  const V3 vi = xyz(loadOwn<NL>(velIn + i));
   // The sum runs over the raw kernel gradients g_b; the correction L is
   // applied once afterwards: with gt_b = L g_b,
   //   G = sum dv_b gt_b^T = A L^T,  s = L sum V_b g_b,  Q = L P L^T,
@@ -1049,7 +1060,7 @@ __global__ void __launch_bounds__(kBlock, kMinB) k_solveA(Bufs b, int k, const f
   const bool act = kTrack && G == 1 && (flags & kActive) != 0 && k > 0;
   bool changed = true;
   if (act && active && !waterW(pi.w)) changed = b.dirty[k & 1][i] != 0;
-  recordSolidDisp(b, i, k, active && !waterW(pi.w) && lane == 0 && changed ? S.dt * length(xyz(velIn[i])) : 0.f);
+  recordSolidDisp(b, i, k, active && !waterW(pi.w) && lane == 0 && changed ? S.dt * length(xyz(loadOwn<G>(velIn + i))) : 0.f);
   if (!active || waterW(pi.w)) {  // water: its record is never read
     if (track && lane == 0) {
       b.rr[i] = 0.f;
@@ -1610,7 +1621,7 @@ __global__ void __launch_bounds__(kBlock, kMinB) k_solveB(Bufs b, int k, const f
   const SceneDev& S = *cx.scene;
   const float4* __restrict__ posS = b.posS;
   const float4* __restrict__ Sp = b.Sp;
-  const float4 vi4 = velIn[i];
+  const float4 vi4 = loadOwn<G>(velIn + i);
   const float4 pi = posS[i];
   const bool track = (flags & kTrackResid) != 0;
   const bool measure = (flags & kMeasureOnly) != 0;
@@ -1642,7 +1653,7 @@ __global__ void __launch_bounds__(kBlock, kMinB) k_solveB(Bufs b, int k, const f
     // the predicted positions and of the bound; the test on the pairs that
     // remain is unchanged, so the result is too.
     const float reach = (minD + S.dt * length(xyz(vi4)) +
-                         __uint_as_float(b.solidDisp[(size_t)(k & 1) * b.S + (cx.scene - b.scenes)])) *
+                         __uint_as_float(loadOwn<G>(b.solidDisp + (size_t)(k & 1) * b.S + (cx.scene - b.scenes)))) *
                         1.01f;
     const float reach2 = reach * reach;
     ImpulseSum sum;
@@ -2383,7 +2394,9 @@ inline unsigned gridOf(uint32_t n, int block) { return (unsigned)((n + (uint32_t
 
 // The reference schedule's launches are chained (its flags are 0). Those of
 // the learned solve stay plain: they follow memsets and conditional nodes or
-// form the bodies of conditional nodes.
+// form the bodies of conditional nodes. So do those of the one-lane solve, on
+// large handles, where a launch's gap does not count.
+constexpr int kPlainLaunch = -1;
 template <class... P, class... Q>
 inline void launchIn(int flags, void (*fn)(P...), unsigned g, unsigned block, cudaStream_t st, Q... q) {
   if (flags == 0)
@@ -2407,10 +2420,10 @@ void launch_computeL_water(const Bufs& b, cudaStream_t st) { k_computeL_water<<<
 template <int V>
 void solveAVariant(const Bufs& b, int k, const float4* velIn, int flags, cudaStream_t st) {
   if (flags & kTrackResid)
-    launchIn(flags, k_solveA<true, kSolveAMinB[V], 1, kSolveABlock[V]>, gridOf(b.N, kSolveABlock[V]), kSolveABlock[V],
+    launchIn(kPlainLaunch, k_solveA<true, kSolveAMinB[V], 1, kSolveABlock[V]>, gridOf(b.N, kSolveABlock[V]), kSolveABlock[V],
              st, b, k, velIn, flags);
   else
-    launchIn(flags, k_solveA<false, kSolveAMinB[V], 1, kSolveABlock[V]>, gridOf(b.N, kSolveABlock[V]), kSolveABlock[V],
+    launchIn(kPlainLaunch, k_solveA<false, kSolveAMinB[V], 1, kSolveABlock[V]>, gridOf(b.N, kSolveABlock[V]), kSolveABlock[V],
              st, b, k, velIn, flags);
 }
 void launch_solveA(const Bufs& b, int k, const float4* velIn, int flags, int variant, int lanes, cudaStream_t st) {
@@ -2454,7 +2467,7 @@ void launch_resid_reduce(const Bufs& b, int k, bool warm, cudaStream_t st) {
 void launch_keep_lambda(const Bufs& b, cudaStream_t st) { k_keep_lambda<<<grid(b.N), kThreads, 0, st>>>(b); }
 template <int V>
 void solveBVariant(const Bufs& b, int k, const float4* velIn, float4* velOut, int wx, int flags, cudaStream_t st) {
-  launchIn(flags, k_solveB<kSolveBMinB[V], 1, kSolveBBlock[V]>, gridOf(b.N, kSolveBBlock[V]), kSolveBBlock[V], st, b, k,
+  launchIn(kPlainLaunch, k_solveB<kSolveBMinB[V], 1, kSolveBBlock[V]>, gridOf(b.N, kSolveBBlock[V]), kSolveBBlock[V], st, b, k,
            velIn, velOut, wx, flags);
 }
 // A grid that fills the GPU once with this kernel's resident blocks (the
