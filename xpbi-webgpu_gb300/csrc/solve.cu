@@ -1241,7 +1241,7 @@ __device__ __forceinline__ void computeL(const Bufs& b) {
   const Ctx cx = ctxOf(b, i);
   const SceneDev& S = *cx.scene;
   const float4* __restrict__ posS = b.posS;
-  const float4 pi = posS[i];
+  const float4 pi = b.posS[i];
   const V3 xi = xyz(pi);
   const float s2 = S.support2;
   // own phase from the front, the other one from the back (the water flag is
@@ -1622,7 +1622,7 @@ __global__ void __launch_bounds__(kBlock, kMinB) k_solveB(Bufs b, int k, const f
   const float4* __restrict__ posS = b.posS;
   const float4* __restrict__ Sp = b.Sp;
   const float4 vi4 = loadOwn<G>(velIn + i);
-  const float4 pi = posS[i];
+  const float4 pi = loadOwn<G>(posS + i);
   const bool track = (flags & kTrackResid) != 0;
   const bool measure = (flags & kMeasureOnly) != 0;
   if (!measure && !iterating(b, S, i, k, flags)) {
@@ -1995,7 +1995,7 @@ __global__ void __launch_bounds__(kThreads, minPbfA(G)) k_pbfA(Bufs b, int k, in
     }
     return;
   }
-  const float4 xc4 = xcS[i];
+  const float4 xc4 = b.xc[i];
   const V3 xci = xyz(xc4);
   const float s2 = S.support2;
   SubList<G> sub;
@@ -2126,7 +2126,7 @@ __global__ void __launch_bounds__(kThreads, minPbfB(G)) k_pbfB(Bufs b, int k, co
   }
   const float4* __restrict__ xcS = b.xc;
   const uint32_t mi = matOfW(pi.w);
-  const V3 xci = xyz(xcS[i]);
+  const V3 xci = xyz(b.xc[i]);
   const float li = b.pbfLam[i];
   const MatDev& mWi = cx.mats[mi];
   // sum of (lambda_i + lambda_b + s_corr) gradW mpd_b, s_corr = -k (W / W0)^4
@@ -2210,7 +2210,7 @@ __global__ void __launch_bounds__(kThreads) k_xsph(Bufs b, const float4* velIn, 
   const Ctx cx = ctxOf(b, i);
   const SceneDev& S = *cx.scene;
   const float4* __restrict__ posS = b.posS;
-  const float4 pi = posS[i];
+  const float4 pi = b.posS[i];
   const V3 xi = xyz(pi);
   const float4 vi4 = velIn[i];
   const V3 vi = xyz(vi4);
