@@ -314,13 +314,22 @@ __device__ __forceinline__ V3 safeSig(V3 s) { return vclamp(s, 1e-3f, 1e3f); }
 // keep three digits of the strain; there the eigenvalues x of
 // F^T F - I = H + H^T + H^T H are taken instead, which H's own digits carry,
 // with log sigma = log(1 + x) / 2. (The singular values then come in no
-// particular order: the material models do not depend on it.) Beyond
-// |F^T F - I| = 0.5 the SVD of F itself keeps the small singular values.
+// particular order: the material models do not depend on it.) That needs
+// det F > 0 (the eigenvalues of F^T F do not see an inversion, whose smallest
+// singular value is negative) and a bound on x away from -1: with the entries
+// of F^T F - I below 0.5 and its absolute row sums below 0.75, |x| < 0.75 and
+// sigma lies in (0.5, 1.33), inside safeSig's bounds. (The entries alone do
+// not: flattened to nothing along (1, 1, 1), every one is -1/3 and an
+// eigenvalue is -1.) Elsewhere, NaN included, the SVD of F itself keeps the
+// small singular values and the sign.
 __device__ __forceinline__ SVD strainSVD(const M3& H, V3& e) {
   const V3 x = H.c[0], y = H.c[1], z = H.c[2];
   const Sym3 S = {fmaf(2.f, x.x, dot(x, x)), fmaf(2.f, y.y, dot(y, y)), fmaf(2.f, z.z, dot(z, z)),
                   (x.y + y.x) + dot(x, y),   (x.z + z.x) + dot(x, z),   (y.z + z.y) + dot(y, z)};
-  if (maxAbs(S) < 0.5f) {
+  const M3 F = {{v3(1.f + x.x, x.y, x.z), v3(y.x, 1.f + y.y, y.z), v3(z.x, z.y, 1.f + z.z)}};
+  const float xy = fabsf(S.xy), xz = fabsf(S.xz), yz = fabsf(S.yz);
+  const float rows = fmaxf(fmaxf(fabsf(S.xx) + xy + xz, fabsf(S.yy) + xy + yz), fabsf(S.zz) + xz + yz);
+  if (maxAbs(S) < 0.5f && rows < 0.75f && det(F) > 0.f) {
     SVD out;
     V3 d;
     eigSym(S, d, out.V);
@@ -331,7 +340,7 @@ __device__ __forceinline__ SVD strainSVD(const M3& H, V3& e) {
     for (int k = 0; k < 3; ++k) out.U.c[k] = (out.V.c[k] + mul(H, out.V.c[k])) * r[k];
     return out;
   }
-  const SVD out = svd3Fast(M3{{v3(1.f + x.x, x.y, x.z), v3(y.x, 1.f + y.y, y.z), v3(z.x, z.y, 1.f + z.z)}});
+  const SVD out = svd3Fast(F);
   e = vlog(safeSig(out.sig));
   return out;
 }
