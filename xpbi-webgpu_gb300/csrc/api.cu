@@ -887,6 +887,7 @@ int createImpl(const xpbi_scene_desc* scenes, uint32_t nScenes, xpbi_sim** out) 
   A(ctl, (size_t)b.scanTiles + 1);
   b.tileTicket = reinterpret_cast<uint32_t*>(ctl);
   b.tileStatus = ctl + 1;
+  A(b.crowd, (size_t)crowdRows(b.N) * crowdSegments(b.N) + 1);
   A(b.sceneOf, n);
   A(b.nbr, (size_t)kNbrCap * ((n + 31) & ~size_t(31)));  // whole warps of interleaved lists
   A(b.nbrCount, n);

@@ -58,10 +58,43 @@ inline void launchChained(void (*fn)(P...), dim3 grid, unsigned block, size_t sm
   cudaLaunchKernelEx(&c, fn, std::forward<Q>(q)...);
 }
 
-// Number of members of the bucket tmp[s0, s1) with a larger index than i: i's
-// place in it. Counting is O(L) a member whatever the bucket's size L; four
-// members a load where it pays (9,000 in one cell take 20 us more).
-__device__ __forceinline__ uint32_t rankInBucket(const uint32_t* tmp, uint32_t s0, uint32_t s1, uint32_t i) {
+// A particle's place in its cell's bucket is the number of members with a
+// larger index. Up to crowdLimit members, tmp[s0, s1) is counted through:
+// O(L) a member, four members a load where it pays. In a crowded cell (a
+// collapsed scene, or one whose positions are all NaN, which the grid clamps
+// into its first cell) that would be quadratic in the scene. There the fill
+// has counted the cell's members per segment of 8192 consecutive particles:
+// those of the later segments are added up, and only the rest of the
+// particle's own segment is looked through, by its keys.
+// (Everything in one cell, the reorder: 250k particles 0.24 ms against 16.2 of
+// comparing all with all, 1M 0.71 against 163, 4M 2.6. The sort of 250k spread
+// particles takes 20.5 us with and without.)
+__device__ __forceinline__ bool crowded(uint32_t n, uint32_t s0, uint32_t s1) {
+  return s1 > s0 && s1 - s0 > crowdLimit(n);
+}
+// the counts of the crowded cell that starts at s0 (they start more than crowdLimit apart)
+__device__ __forceinline__ uint32_t* crowdRow(uint32_t* crowd, uint32_t n, uint32_t s0) {
+  return crowd + (size_t)(s0 / crowdLimit(n)) * crowdSegments(n);
+}
+__device__ __forceinline__ uint32_t rankInCrowd(const uint32_t* key, const uint32_t* row, uint32_t n, uint32_t i) {
+  const uint32_t c = key[i], seg = i / kCrowdSegment;
+  uint32_t rank = 0, j = i + 1u;
+#pragma unroll 4
+  for (uint32_t q = seg + 1u; q < crowdSegments(n); ++q) rank += row[q];
+  const uint32_t end = min(n, (seg + 1u) * kCrowdSegment);
+  for (; j < end && (j & 3u); ++j) rank += key[j] == c ? 1u : 0u;
+#pragma unroll 4
+  for (; j + 4u <= end; j += 4u) {
+    const uint4 m = *reinterpret_cast<const uint4*>(key + j);
+    rank += (m.x == c ? 1u : 0u) + (m.y == c ? 1u : 0u) + (m.z == c ? 1u : 0u) + (m.w == c ? 1u : 0u);
+  }
+  for (; j < end; ++j) rank += key[j] == c ? 1u : 0u;
+  return rank;
+}
+__device__ __forceinline__ uint32_t rankInBucket(const uint32_t* tmp, const uint32_t* key, uint32_t* crowd, uint32_t n,
+                                                 uint32_t s0, uint32_t s1, uint32_t i) {
+  // (the bound only matters after an expired look-back, whose starts are wrong)
+  if (crowded(n, s0, s1)) return min(rankInCrowd(key, crowdRow(crowd, n, s0), n, i), s1 - s0 - 1u);
   uint32_t rank = 0, q = s0;
   if (s1 - s0 > 32u) {
     for (; q & 3u; ++q) rank += tmp[q] > i ? 1u : 0u;
@@ -72,7 +105,7 @@ __device__ __forceinline__ uint32_t rankInBucket(const uint32_t* tmp, uint32_t s
     }
   }
   for (; q < s1; ++q) rank += tmp[q] > i ? 1u : 0u;
-  return rank;
+  return min(rank, s1 - s0 - 1u);
 }
 
 // Thread t's share of clearing what a sort starts from: cell counters, water

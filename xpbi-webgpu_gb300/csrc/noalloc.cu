@@ -56,7 +56,8 @@ constexpr uint32_t wKey = 0;
 constexpr uint32_t wTmp = wKey + al(kMaxParticles);
 constexpr uint32_t wCursor = wTmp + al(kMaxParticles);
 constexpr uint32_t wCtl = wCursor + al(kMaxCells + 4);                // ticket, tile descriptors (u64)
-constexpr uint32_t wScene = wCtl + al(2 * (kMaxTiles + 1));
+constexpr uint32_t wCrowd = wCtl + al(2 * (kMaxTiles + 1));
+constexpr uint32_t wScene = wCrowd + al(crowdRows(kMaxParticles) * crowdSegments(kMaxParticles));
 constexpr uint32_t wMats = wScene + al((sizeof(SceneDev) + 3) / 4);
 constexpr uint32_t wCellWater = wMats + al((kMaxMats * sizeof(MatDev) + 3) / 4);
 constexpr uint32_t wErr = wCellWater + al(kMaxCells / 4 + 4);
@@ -71,13 +72,13 @@ uint32_t* g_addr[kMaxDevices] = {nullptr};
 
 // Deterministic slot of every bucket member (same rule as the substep's
 // reorder): bucket start + number of members with a larger index.
-__global__ void k_rank_only(const uint32_t* tmp, const uint32_t* key, const uint32_t* cellStart, uint32_t n,
-                            uint32_t* sortedIdx) {
+__global__ void k_rank_only(const uint32_t* tmp, const uint32_t* key, const uint32_t* cellStart, uint32_t* crowd,
+                            uint32_t n, uint32_t* sortedIdx) {
   const uint32_t i = afterPrevious(blockIdx.x * blockDim.x + threadIdx.x);
   if (i >= n) return;
   const uint32_t c = key[i];
   const uint32_t s0 = cellStart[c], s1 = cellStart[c + 1];
-  sortedIdx[s0 + rankInBucket(tmp, s0, s1, i)] = i;
+  sortedIdx[s0 + rankInBucket(tmp, key, crowd, n, s0, s1, i)] = i;
 }
 
 // Writes the grid description, clears the material table (no material is
@@ -156,6 +157,7 @@ extern "C" int xpbi_sort_cells_noalloc(const float* pos4, uint32_t n, const floa
   b.tmp = base + wTmp;
   b.cursor = base + wCursor;
   b.cellStart = cell_start;
+  b.crowd = base + wCrowd;
   b.tileTicket = base + wCtl;
   b.tileStatus = reinterpret_cast<unsigned long long*>(base + wCtl) + 1;
   b.scenes = reinterpret_cast<SceneDev*>(base + wScene);
@@ -172,7 +174,7 @@ extern "C" int xpbi_sort_cells_noalloc(const float* pos4, uint32_t n, const floa
   launch_count_cleared(b, st);
   launch_scan(b, st);
   launch_scatter(b, st);
-  launchChained(k_rank_only, (n + 255) / 256, 256, 0, st, b.tmp, b.key, b.cellStart, n, sorted_idx);
+  launchChained(k_rank_only, (n + 255) / 256, 256, 0, st, b.tmp, b.key, b.cellStart, b.crowd, n, sorted_idx);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return setError(XPBI_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
   return XPBI_OK;

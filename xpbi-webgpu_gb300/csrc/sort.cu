@@ -9,8 +9,9 @@
 //   k_fill     warp-aggregated slot reservation: each cell's members land in
 //              its bucket in arbitrary order
 //   k_reorder  final slot = bucket start + number of bucket members with a
-//              larger previous index, then moves pos/vel/F/state into the
-//              slot with the scatter pass's predictor fused in
+//              larger previous index (in a crowded cell from counts the fill
+//              made per segment of particles), then moves pos/vel/F/state into
+//              the slot with the scatter pass's predictor fused in
 // The final slot rule reproduces the reference's atomicSub scatter executed
 // in invocation order: within a cell, particles are listed by descending
 // previous index. Counts, cell starts and the permutation are therefore
@@ -38,6 +39,21 @@ __device__ __forceinline__ uint32_t cellKey(const SceneDev& S, float4 p) {
 
 __global__ void __launch_bounds__(kThreads) k_clear(Bufs b) {
   sortClear(b, afterPreviousEager(blockIdx.x * blockDim.x + threadIdx.x));
+}
+
+// The crowded ones of a scan thread's cells from `base` on, which end at `end`:
+// their counts per segment start at 0, and the mark on their cursor tells the
+// fill.
+constexpr uint32_t kCrowdMark = 0x80000000u;  // (a handle holds fewer particles)
+__device__ __noinline__ void clearCrowds(const uint32_t* cellStart, uint32_t* cursor, uint32_t* crowd, uint32_t n,
+                                         uint32_t cells, uint32_t base, uint32_t end) {
+  for (uint32_t c = base; c < cells && c < base + kScanItems; ++c) {
+    const uint32_t s0 = cellStart[c], s1 = c + 1u < base + kScanItems ? cellStart[c + 1u] : end;
+    if (!crowded(n, s0, s1)) continue;
+    uint32_t* row = crowdRow(crowd, n, s0);
+    for (uint32_t q = 0; q < crowdSegments(n); ++q) row[q] = 0u;
+    cursor[c] = s0 | kCrowdMark;
+  }
 }
 
 // cursor[] was cleared before this launch; on exit it holds cell counts.
@@ -168,6 +184,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(Bufs b) {
       if (idx < b.C) b.cursor[idx] = out[k];
     }
   }
+  if (sum > crowdLimit(b.N)) clearCrowds(b.cellStart, b.cursor, b.crowd, b.N, b.C, base, run);
 }
 
 // Unordered bucket fill: tmp[cellStart[key] .. +count) receives the members.
@@ -184,7 +201,9 @@ __global__ void __launch_bounds__(kThreads) k_fill(Bufs b) {
   if (lane == leader) base = atomicAdd(&b.cursor[key], (uint32_t)__popc(peers));
   base = __shfl_sync(mask, base, leader);
   uint32_t rank = __popc(peers & ((1u << lane) - 1u));
-  b.tmp[base + rank] = i;
+  b.tmp[(base & ~kCrowdMark) + rank] = i;
+  if ((base & kCrowdMark) && lane == leader)  // (a warp's particles lie in one segment)
+    atomicAdd(crowdRow(b.crowd, b.N, b.cellStart[key]) + i / kCrowdSegment, (uint32_t)__popc(peers));
 }
 
 // Final slot + physical reorder with the scatter pass's predictor fused in
@@ -203,7 +222,7 @@ __global__ void __launch_bounds__(kThreads) k_reorder(Bufs b, int keepLam) {
   const M3 F = loadM(b.F, b.N, i);
   const float st = b.state[i];
   const uint32_t s0 = b.cellStart[key], s1 = b.cellStart[key + 1];
-  const uint32_t s = s0 + rankInBucket(b.tmp, s0, s1, i);
+  const uint32_t s = s0 + rankInBucket(b.tmp, b.key, b.crowd, b.N, s0, s1, i);
   b.sortedIdx[s] = i;
   const SceneDev& S = b.scenes[sceneOfSlot(b, i)];
   // sorted records carry the water flag in the sign bit of pos.w (>= 0)

@@ -14,6 +14,12 @@ constexpr uint32_t kNbrCap = 64u;      // neighbour-list capacity per particle
 constexpr int kSolveAVariants = 6;      // launch-shape variants (autotuner): block size, register cap
 constexpr int kSolveBVariants = 5;
 constexpr uint32_t kScanTile = 4096u;     // cells per block of the scan
+// A crowded cell has more members than this: its members are not ranked by
+// comparing each with all others (chain.cuh)
+constexpr uint32_t kCrowdSegment = 8192u;  // consecutive particles counted together
+constexpr __host__ __device__ uint32_t crowdLimit(uint32_t n) { return n / 2048u > 8192u ? n / 2048u : 8192u; }
+constexpr __host__ __device__ uint32_t crowdRows(uint32_t n) { return n / crowdLimit(n); }
+constexpr __host__ __device__ uint32_t crowdSegments(uint32_t n) { return (n + kCrowdSegment - 1u) / kCrowdSegment; }
 // Lanes per slot by the handle's size: few slots leave most of the GPU idle
 // with one lane each, and several split a slot's neighbours; many slots fill
 // it, and the lanes only add their sums' shuffles. Each line lies where us per
@@ -144,6 +150,7 @@ struct Bufs {
   uint32_t* cellStart;  // [C+1] exclusive cell starts, sentinel = N
   uint8_t* cellWater;   // [C] 1 if the cell holds a water particle this substep
   uint32_t* tileTicket;            // word 0 of the scan control block
+  uint32_t* crowd;                 // [crowdRows(N)][crowdSegments(N)] members of a crowded cell per segment of particles
   unsigned long long* tileStatus;  // [tiles] look-back descriptors (after the two words)
   uint16_t* sceneOf;    // [N] scene of each particle slot (static)
   uint32_t* nbr;        // [ceil(N / 32)][kNbrCap / 4][32][4] in-support neighbours: own phase from the front in
