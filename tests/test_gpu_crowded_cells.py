@@ -79,11 +79,13 @@ def test_permutation(built_lib, members, mix):
 
 
 def test_cost_of_one_cell(built_lib):
-    """Eight times the members of one cell take at most 16 times as long: a cost
-    in proportion takes 8 times, comparing all with all 64."""
+    """Eight times the members of one cell take at most eight times as long, a
+    cost in proportion. (Comparing all with all makes every member's chain
+    eight times as long, and there are eight times as many of them: 0.96 and
+    14.3 ms.)"""
     rng = np.random.default_rng(0)
     small, large = (_Sort(_positions(np.full(n, 77, np.int64), rng)).best_ms() for n in (32768, 262144))
-    assert large <= 16.0 * small, (small, large)
+    assert large <= 8.0 * small, (small, large)
 
 
 def test_substep_of_a_collapsed_scene(xp, built_lib):
