@@ -274,6 +274,9 @@ template <int G, bool kTwo, class Gather, class Visit>
 __device__ __forceinline__ void forLanePairs(const uint4* L, const ListHead& h, uint32_t cnt, uint32_t i, uint32_t lane,
                                              Gather&& gather, Visit&& visit) {
   const uint32_t pairs = (cnt + 1u) >> 1;
+  // i, by way of the loaded count (whose upper bits are 0 unless it overflowed):
+  // a read-only load at i itself could move above a chained kernel's wait
+  const uint32_t self = i + (h.count >> 24);
   uint2 e0 = h.e0, e1 = h.e1;
 #pragma unroll 1
   for (uint32_t p = lane; p < pairs; p += 2u * G) {
@@ -281,7 +284,7 @@ __device__ __forceinline__ void forLanePairs(const uint4* L, const ListHead& h, 
     const bool two = p + G < pairs;
     const auto a0 = gather(e0.x), a1 = gather(e0.y);
     if constexpr (kTwo) {
-      if (!two) e1 = make_uint2(i, i);
+      if (!two) e1 = make_uint2(self, self);  // gathered (one line for neighbouring slots), not visited
       const auto b0 = gather(e1.x), b1 = gather(e1.y);
       visit(e0, a0, a1);
       if (two) visit(e1, b0, b1);
@@ -307,15 +310,16 @@ __device__ __forceinline__ void forListPairs(const uint4* L, const ListHead& h, 
 
 // Slot i's neighbours of its own phase, two at a time, over the recorded
 // list, or by the stencil walk if it overflowed (a last odd neighbour is
-// paired with i itself).
+// paired with i itself, whose data self() reads with ordinary loads: its
+// address depends on no loaded value, so a chained kernel must not gather it).
 //
 // Several lanes per slot (small scenes): the G lanes of slot i are
 // consecutive in the warp; lane `lane` visits the pairs p with p % G == lane
 // (on the walk every G-th candidate of each row) and accumulates a partial
 // sum; laneSum adds them over the group.
-template <int G, class Gather, class Body>
+template <int G, class Gather, class Self, class Body>
 __device__ __forceinline__ void forSame(const Bufs& b, const Ctx& cx, const ListHead& h, uint32_t i, V3 xi, bool iWater,
-                                        uint32_t lane, Gather&& gather, Body&& body) {
+                                        uint32_t lane, Gather&& gather, Self&& self, Body&& body) {
   static_assert(G == 1 || G == 2 || G == 4, "one, two or four lanes per slot");
   const uint32_t c = G == 1 ? b.nbrCount[i] : h.count;
   if (c != kNbrOverflow) {
@@ -338,7 +342,7 @@ __device__ __forceinline__ void forSame(const Bufs& b, const Ctx& cx, const List
         }
       }
     });
-    if (first != i) body(first, i, gather(first), gather(i));
+    if (first != i) body(first, i, gather(first), self());
   }
 }
 
@@ -577,8 +581,8 @@ __device__ __forceinline__ void bonetLok(const Bufs& b, const Ctx& cx, uint32_t 
                                          uint32_t lane = 0, const SubList<G>* sub = nullptr) {
   static_assert(kSolid || !kVel, "the velocity sum is a solid's");
   const SceneDev& S = *cx.scene;
-  const float4* __restrict__ posS = b.posS;
-  const float4* __restrict__ velIn = b.velS[0];  // V^n (.w), which no pass changes; with kVel also v
+  const float4* posS = b.posS;
+  const float4* velIn = b.velS[0];  // V^n (.w), which no pass changes; with kVel also v
   V3 vi = splat(0.f);
   if constexpr (kVel) vi = xyz(velIn[i]);
   VelSum Av;
@@ -618,7 +622,7 @@ __device__ __forceinline__ void bonetLok(const Bufs& b, const Ctx& cx, uint32_t 
   // own phase; the other phase's neighbours enter L alone
   const uint32_t c = G == 1 ? b.nbrCount[i] : (sub->lost ? kNbrOverflow : 0u);
   if (c == kNbrOverflow) {
-    const PV self = gather(i);
+    const PV self{posS[i], velIn[i]};
     forRows<G>(S, b.cellStart, xi, [&](uint32_t beg, uint32_t end) {
 #pragma unroll 1
       for (uint32_t j = beg; j < end; ++j) {
@@ -639,14 +643,23 @@ __device__ __forceinline__ void bonetLok(const Bufs& b, const Ctx& cx, uint32_t 
       forPairs(nbrGroups(b.nbr, i) + kGroupStride * (kNbrCap / 4u - other), other, gather,
                   [&](uint32_t, uint32_t, const PV& d0, const PV& d1) { addA(pairOf(S, xi, d0, d1)); });
   } else {
+    // a last odd one is paired with a copy of itself of no volume
 #pragma unroll 2
     for (uint32_t e = 0; e < sub->same; e += 2u) {
-      const uint32_t j0 = sub->at(e), j1 = e + 1u < sub->same ? sub->at(e + 1u) : i;
-      own(j0, j1, gather(j0), gather(j1));
+      const bool two = e + 1u < sub->same;
+      const uint32_t j0 = sub->at(e), j1 = two ? sub->at(e + 1u) : j0;
+      const PV d0 = gather(j0);
+      PV d1 = gather(j1);
+      if (!two) d1.v.w = 0.f;
+      own(j0, two ? j1 : i, d0, d1);
     }
     for (uint32_t e = 0; e < sub->other; e += 2u) {
-      const uint32_t j0 = sub->otherAt(e), j1 = e + 1u < sub->other ? sub->otherAt(e + 1u) : i;
-      addA(pairOf(S, xi, gather(j0), gather(j1)));
+      const bool two = e + 1u < sub->other;
+      const uint32_t j0 = sub->otherAt(e), j1 = two ? sub->otherAt(e + 1u) : j0;
+      const PV d0 = gather(j0);
+      PV d1 = gather(j1);
+      if (!two) d1.v.w = 0.f;
+      addA(pairOf(S, xi, d0, d1));
     }
   }
   const float gc = S.gradC;
@@ -711,12 +724,13 @@ __device__ __forceinline__ void storeSp(const Bufs& b, uint32_t i, const M3& m, 
 // neighbours, without its factor L^T.
 template <int G>
 __device__ __forceinline__ M3 velocitySum(const Bufs& b, const Ctx& cx, const ListHead& h, uint32_t i, V3 xi, V3 vi,
-                                          const float4* __restrict__ velIn, uint32_t lane) {
+                                          const float4* velIn, uint32_t lane) {
   const SceneDev& S = *cx.scene;
-  const float4* __restrict__ posS = b.posS;
+  const float4* posS = b.posS;
   // sum dv_b (L g_b)^T = (sum dv_b g_b^T) L^T: L applied once, by the caller
   VelSum A;
   forSame<G>(b, cx, h, i, xi, false, lane, [&](uint32_t j) { return PV{ldg(posS + j), ldg(velIn + j)}; },
+             [&] { return PV{posS[i], velIn[i]}; },
              [&](uint32_t, uint32_t, const PV& d0, const PV& d1) { A.add(pairOf(S, xi, d0, d1), vi, d0.v, d1.v); });
   return A.template total<G>(S.gradC);
 }
@@ -761,10 +775,10 @@ __device__ __noinline__ Constraint constraintTail(M3 A, TailIn in, const SceneDe
 
 template <int NL = 1>
 __device__ __forceinline__ Constraint evalConstraint(const Bufs& b, const Ctx& cx, uint32_t i, float4 pi,
-                                                     const float4* __restrict__ velIn, const MatDev* m, float st,
+                                                     const float4* velIn, const MatDev* m, float st,
                                                      const ListHead& head = ListHead{}, uint32_t lane = 0) {
   const SceneDev& S = *cx.scene;
-  const float4* __restrict__ posS = b.posS;
+  const float4* posS = b.posS;
   const V3 xi = xyz(pi);
   const V3 vi = xyz(loadOwn<NL>(velIn + i));
   // The sum runs over the raw kernel gradients g_b; the correction L is
@@ -775,6 +789,7 @@ __device__ __forceinline__ Constraint evalConstraint(const Bufs& b, const Ctx& c
   // on the velocities: computeL formed them, so the sweep only accumulates A.
   VelSum A;
   forSame<NL>(b, cx, head, i, xi, false, lane, [&](uint32_t j) { return PV{ldg(posS + j), ldg(velIn + j)}; },
+              [&] { return PV{posS[i], velIn[i]}; },
               [&](uint32_t, uint32_t, const PV& d0, const PV& d1) { A.add(pairOf(S, xi, d0, d1), vi, d0.v, d1.v); });
   const M3 At = A.template total<NL>(S.gradC);
   if (NL > 1 && lane != 0) return Constraint{};  // lane 0 finishes the slot
@@ -790,7 +805,7 @@ __device__ __noinline__ Constraint constraintTail(M3 A, TailIn in, const SceneDe
   const SceneDev& S = *Sp;
   const MatDev& m = *mp;
   const M3 Li = loadM(in.L, in.N, in.i), Fn = loadM(in.F, in.N, in.i);
-  const float4* __restrict__ R = in.sgP + in.i;
+  const float4* R = in.sgP + in.i;
   const float hard = hardening(m, st);
   const float mu = m.mu * hard, lam = m.lam * hard;
   // the trial F minus the identity, which keeps the digits of a small strain
@@ -986,10 +1001,10 @@ __device__ __forceinline__ int iterK(const Bufs& b, int k) {
 // sweep, lane 0 finishes the slot.
 //
 // The update of slot i from its constraint c (lane 0 of the slot).
-template <bool kTrack>
+template <bool kTrack, int G = 1>
 __device__ __forceinline__ void solveAUpdate(const Bufs& b, const Ctx& cx, uint32_t i, const float4& pi,
-                                             const float4* __restrict__ velIn, uint32_t mi, const Constraint& c,
-                                             int k, bool warm0, bool measure, bool act = false) {
+                                             const float4* velIn, uint32_t mi, const Constraint& c, int k, bool warm0,
+                                             bool measure, bool act = false) {
   const SceneDev& S = *cx.scene;
   constexpr bool track = kTrack;
   const float g = S.kDamp;
@@ -1011,7 +1026,7 @@ __device__ __forceinline__ void solveAUpdate(const Bufs& b, const Ctx& cx, uint3
   }
   // an inactive constraint still takes part in the contact pass
   const V3 xi = xyz(pi);
-  const V3 xci = xi + S.dt * xyz(velIn[i]);
+  const V3 xci = xi + S.dt * xyz(loadOwn<G>(velIn + i));
   const float mass = cx.mats[mi].mass;
   if (measure) {  // the contact residual of these velocities, no impulse
     storeSp(b, i, mzero(), splat(0.f), xi, xci, mass);
@@ -1076,7 +1091,7 @@ __global__ void __launch_bounds__(kBlock, kMinB) k_solveA(Bufs b, int k, const f
   const float st = b.stateS[i];
   const Constraint c = evalConstraint<G>(b, cx, i, pi, velIn, cx.mats + mi, st, head, lane);
   if (G > 1 && lane != 0) return;
-  solveAUpdate<kTrack>(b, cx, i, pi, velIn, mi, c, k, warm0, measure, act);
+  solveAUpdate<kTrack, G>(b, cx, i, pi, velIn, mi, c, k, warm0, measure, act);
 }
 
 // Active set, iterations from 2: the changed slots of the scenes still
@@ -1619,10 +1634,9 @@ __global__ void __launch_bounds__(kBlock, kMinB) k_solveB(Bufs b, int k, const f
   const ListHead head = listHead<G>(nbrGroups(b.nbr, i), b.nbrCount, i, lane);
   const Ctx cx = ctxOf(b, i);
   const SceneDev& S = *cx.scene;
-  const float4* __restrict__ posS = b.posS;
   const float4* __restrict__ Sp = b.Sp;
   const float4 vi4 = loadOwn<G>(velIn + i);
-  const float4 pi = loadOwn<G>(posS + i);
+  const float4 pi = loadOwn<G>(b.posS + i);
   const bool track = (flags & kTrackResid) != 0;
   const bool measure = (flags & kMeasureOnly) != 0;
   if (!measure && !iterating(b, S, i, k, flags)) {
@@ -2061,8 +2075,9 @@ __global__ void __launch_bounds__(kThreads, minPbfA(G)) k_pbfA(Bufs b, int k, in
     } else {
 #pragma unroll 2
       for (uint32_t e = 0; e < sub.same; e += 2u) {
-        const uint32_t j0 = sub.at(e), j1 = e + 1u < sub.same ? sub.at(e + 1u) : i;
-        body(j0, j1, gather(j0), gather(j1));
+        const bool two = e + 1u < sub.same;
+        const uint32_t j0 = sub.at(e), j1 = two ? sub.at(e + 1u) : j0;
+        body(j0, two ? j1 : i, gather(j0), gather(j1));  // (i weighs 0)
       }
     }
   };
@@ -2220,7 +2235,7 @@ __global__ void __launch_bounds__(kThreads) k_xsph(Bufs b, const float4* velIn, 
   // the water's next substep amplifies what differs here.
   V3 acc = splat(0.f);
   forSame<G>(b, cx, head, i, xi, iWater, lane, [&](uint32_t j) { return PV{ldg(posS + j), ldg(velIn + j)}; },
-             [&](uint32_t, uint32_t, const PV& d0, const PV& d1) {
+             [&] { return PV{pi, vi4}; }, [&](uint32_t, uint32_t, const PV& d0, const PV& d1) {
                const F2 dx = f2(xi.x - d0.p.x, xi.x - d1.p.x), dy = f2(xi.y - d0.p.y, xi.y - d1.p.y),
                         dz = f2(xi.z - d0.p.z, xi.z - d1.p.z);
                const F2 r2 = fma2(dz, dz, fma2(dx, dx, mul2(dy, dy)));
