@@ -45,16 +45,19 @@ constexpr int kThreads = 128;
 
 // Launch bounds of the stencil kernels: resident CTAs of kThreads threads per
 // SM asked of the register allocator, with one lane per slot and with several
-// (ms per launch; one lane on the 4M-particle dam-breach mix, several on the
-// 113k snowball and a 100k dam breach): computeL 9 CTAs 1.09 (8: 1.11, 7: 1.17,
-// 6: 1.27), several lanes 7: 0.054 (8: 0.059, 9: 0.065); computeL with the
-// stored constraint and features (the learned solve) 7; pbfA 10: 0.62 (8:
-// 0.66, 9: 0.64, 11: 0.63), several lanes 8: 0.0416 (10: 0.0449); pbfB 7: 0.047
-// on the 1M-particle dam breach (8: 0.048, 9: 0.050, 10: 0.054), several lanes 8; the update 7: 0.303 (8: 0.337, 6: 0.332, the
-// allocator's choice 0.370).
-constexpr int minComputeL(int lanes) { return lanes == 1 ? 9 : 7; }
-constexpr int kMinComputeLFeatures = 7;
-constexpr int minPbfA(int lanes) { return lanes == 1 ? 10 : 8; }
+// (ms per launch; one lane on the 4M-particle dam-breach mix): computeL 9 CTAs
+// 1.09 (8: 1.11, 7: 1.17, 6: 1.27); with the stored constraint and features
+// (the learned solve) 7; pbfA 10: 0.62 (8: 0.66, 9: 0.64, 11: 0.63); pbfB 7:
+// 0.047 on the 1M-particle dam breach (8: 0.048, 9: 0.050, 10: 0.054), several
+// lanes 8; the update 7: 0.303 (8: 0.337, 6: 0.332, the allocator's choice
+// 0.370). With several lanes computeL and pbfA hold 33 KB of shared memory a
+// block, so six fit, whatever the registers: 16k solids 199.5 us a substep and
+// 27k of a dam breach 154.3 with 6 and 6, 200.5 and 154.1 with the caps of 7
+// and 8.
+constexpr int kColumnBlocks = 6;
+constexpr int minComputeL(int lanes) { return lanes == 1 ? 9 : kColumnBlocks; }
+constexpr int minComputeLFeatures(int lanes) { return lanes == 1 ? 7 : kColumnBlocks; }
+constexpr int minPbfA(int lanes) { return lanes == 1 ? 10 : kColumnBlocks; }
 constexpr int minPbfB(int lanes) { return lanes == 1 ? 7 : 8; }
 constexpr int kMinUpdate = 7;
 // solveA and solveB are compiled in several launch shapes — the block size
@@ -1347,7 +1350,7 @@ __global__ void __launch_bounds__(kThreads, minComputeL(G)) k_computeL(Bufs b) {
   computeL<false, G>(b);
 }
 template <int G>
-__global__ void __launch_bounds__(kThreads, kMinComputeLFeatures) k_computeL_features(Bufs b) {
+__global__ void __launch_bounds__(kThreads, minComputeLFeatures(G)) k_computeL_features(Bufs b) {
   computeL<true, G>(b);
 }
 
