@@ -1909,8 +1909,9 @@ __device__ __forceinline__ bool pbfActive(const SceneDev& S, int k) {
 }
 
 // The PBF pair terms of two predicted neighbours per packed instruction: the
-// offset, the poly6 kernel of r^2 and the spiky gradient (0 below r = 1e-9,
-// the reference's zero-distance guard).
+// poly6 kernel of r^2 and the spiky gradient (common.js:81-94, H = support),
+// the latter by one reciprocal square root and 0 below r = 1e-9, the
+// reference's zero-distance guard (r^2 < 1e-18).
 //
 // The density solve amplifies rounding: each pass feeds its positions to the
 // next, through fourth powers. Sums packed in another order left the

@@ -26,7 +26,6 @@ __device__ __forceinline__ V3 operator/(V3 a, float s) { return {a.x / s, a.y / 
 __device__ __forceinline__ V3 operator/(V3 a, V3 b) { return {a.x / b.x, a.y / b.y, a.z / b.z}; }
 __device__ __forceinline__ float dot(V3 a, V3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 __device__ __forceinline__ float length(V3 a) { return sqrtf(dot(a, a)); }
-__device__ __forceinline__ V3 normalize(V3 a) { return a / length(a); }
 __device__ __forceinline__ V3 cross(V3 a, V3 b) {
   return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
 }
@@ -108,26 +107,9 @@ __device__ __forceinline__ void storeM(float* __restrict__ P, uint32_t N, uint32
   }
 }
 
-// ----------------------------------------------------------------- SPH kernels
-// The Wendland C2 kernel and its gradient (support 2h, common.js:63-79) are
-// formed in the pair loops of solve.cu. PBF kernels with H = support
-// (common.js:81-94), with the square root and the division by r replaced by
-// one reciprocal square root; r < 1e-9 (the reference's zero-distance guard)
-// is r^2 < 1e-18.
-// poly6 from the squared distance: H^2 - r^2 with r^2 taken directly
-__device__ __forceinline__ float poly6Fast(const SceneDev& S, float r2) {
-  if (r2 >= S.support2) return 0.f;
-  const float x = S.support2 - r2;
-  return S.poly6C * x * x * x;
-}
-__device__ __forceinline__ V3 spikyGradFast(const SceneDev& S, V3 dxv, float r2) {
-  if (r2 < 1e-18f) return splat(0.f);
-  const float rinv = rsqrtf(r2);
-  const float r = r2 * rinv;
-  if (r >= S.support) return splat(0.f);
-  const float t = S.support - r;
-  return dxv * (S.spikyC * t * t * rinv);
-}
+// The SPH kernels are formed in the pair loops of solve.cu: Wendland C2 and its
+// gradient (support 2h, common.js:63-79) in radial2 and xsph, the PBF kernels
+// (common.js:81-94) in pbfPair.
 
 // ----------------------------------------------------------------- grid
 // common.js:97-103. Saturating f32->i32 (NaN -> 0) before clamping.
