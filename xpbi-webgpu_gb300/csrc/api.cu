@@ -214,14 +214,12 @@ void buildSceneDev(const SceneHost& s, uint32_t sceneIdx, SceneDev& d, MatDev* m
   }
   d.invH = 1.f / h;
   // The pair sums form t = 1 - r halfInvH and multiply by gradC once, after
-  // the loop. The rounding of halfInvH (up to 6e-8) shifts t^3 the same way
-  // for every neighbour — by 5.5 times as much over a lattice's neighbours
-  // weighted as in sum t^3 r^2, the moment of every gradient sum — so gradC
-  // takes that shift out again.
-  const double half = 0.5 / (double)h;
-  d.halfInvH = (float)half;
-  d.gradC = (float)(-5.0 * 21.0 / (16.0 * 3.14159265 * (double)h * h * h * h * h) *
-                    (1.0 + 5.5 * ((double)d.halfInvH / half - 1.0)));
+  // the loop. The rounding of halfInvH (up to 6e-8) makes theirs the kernel of
+  // a support that much narrower or wider, so gradC is that kernel's own
+  // factor, not the nominal one's.
+  d.halfInvH = (float)(0.5 / (double)h);
+  const double hr = 0.5 / (double)d.halfInvH;
+  d.gradC = (float)(-5.0 * 21.0 / (16.0 * 3.14159265 * hr * hr * hr * hr * hr));
   d.invW0 = 1.f / fmaxf(d.w0, 1e-12f);
   d.alphaT = (1.f / d.V0) / (dt * dt);
   d.minD = 0.75f * h;

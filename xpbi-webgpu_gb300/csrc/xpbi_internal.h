@@ -61,9 +61,10 @@ constexpr uint32_t kWaterBit = 0x80000000u;
 // Device error word bits.
 constexpr int kErrLookback = 1;        // decoupled look-back wait expired
 
-// One scene's uniforms plus constants derived from them on the host. Every
-// derived constant is formed in f32 with the operation order of the per-call
-// WGSL expression it replaces, so it is bit-identical to recomputing it.
+// One scene's uniforms plus constants derived from them on the host. A
+// derived constant that names a reference line is formed in f32 with the
+// operation order of that per-call WGSL expression, so it is bit-identical to
+// recomputing it.
 struct SceneDev {
   float origin[3];
   float cs;                 // cell size = support
@@ -95,7 +96,7 @@ struct SceneDev {
   float vmaxCFL;            // 0.45 support / dt           simkernels.js:535
   float dvCap;              // 0.2 support / dt            simkernels.js:361
   float invH;               // 1 / h
-  float gradC;              // -5 sigW / h^2: grad W = gradC (1 - r / 2h)^3 dx
+  float gradC;              // -5 sigW / h^2 for the h of halfInvH: grad W = gradC (1 - r / 2h)^3 dx
   float halfInvH;           // 1 / (2 h)
   float invW0;              // 1 / max(w0, 1e-12)          simkernels.js:466
   int iterations;           // XPBI Jacobi iterations this substep (an early-stopped solve's cap)
