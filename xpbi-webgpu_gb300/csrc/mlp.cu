@@ -383,9 +383,10 @@ __global__ void __launch_bounds__(kStepThreads) k_mlp_step(const float* __restri
   const uint32_t aAddr = tc::smemAddr(sm + tA);
   constexpr uint32_t idesc = tc::idescBf16F32(kRows, kHid);
   uint32_t phase = 0;
+  bool ok = true;  // this thread's waits have all come back
   // D = A B^T on the tensor cores; every thread has fenced and synchronised
   auto issue = [&](uint32_t wOffset, uint32_t K) {
-    if (tid == 0) {
+    if (tid == 0 && ok) {
       const uint32_t wAddr = tc::smemAddr(sm + tW + wOffset), sbo = (K / 8) * 128;
       for (uint32_t ks = 0; ks < K / 16; ++ks)
         tc::mma(tmem, tc::smemDesc(aAddr + ks * 256, 128, sbo), tc::smemDesc(wAddr + ks * 256, 128, sbo), idesc,
@@ -393,10 +394,14 @@ __global__ void __launch_bounds__(kStepThreads) k_mlp_step(const float* __restri
       tc::commit(&bar);
     }
   };
-  // no barrier is skipped when a wait expires: the error word says so, and the
-  // CTA goes on to release its TMEM
+  // When a wait expires, the error word says so, no further MMA is issued over
+  // the one that may still run, and the later waits are not tried; no barrier
+  // is skipped, and the CTA goes on to release its TMEM.
   auto await = [&]() {
-    if (!tc::mbarWait(&bar, phase, kSpin) && tid == 0) atomicOr(err, kErrMma);
+    if (ok && !tc::mbarWait(&bar, phase, kSpin)) {
+      ok = false;
+      atomicOr(err, kErrMma);
+    }
     phase ^= 1u;
     tc::fenceAfterSync();
   };
@@ -630,6 +635,11 @@ cudaError_t stepKernel(const float* dX, const float* dT, uint32_t rows, const vo
                 static_cast<const uint8_t*>(dBlob), dPartial, dSq, dErr);
   return cudaGetLastError();
 }
+void reduceKernel(const float* dPartial, const float* dSq, uint32_t rows, float* dGrad, float* dLoss, const Adam& adam,
+                  uint8_t* blob, cudaStream_t st) {
+  launchChained(k_mlp_reduce, (kParams + kReduceParams - 1) / kReduceParams, kReduceParams, 0, st, dPartial,
+                (rows + kRows - 1) / kRows, dSq, rows, dGrad, dLoss, adam, blob);
+}
 }  // namespace
 
 // The gradient (and mean squared error) on rows X, targets T. Scratch:
@@ -639,8 +649,7 @@ cudaError_t mlp_grad(const float* dX, const float* dT, uint32_t rows, const void
   if (rows == 0) return cudaSuccess;
   cudaError_t e = stepKernel(dX, dT, rows, dBlob, dPartial, dSq, dErr, st);
   if (e != cudaSuccess) return e;
-  launchChained(
-      k_mlp_reduce, (kParams + kReduceParams - 1) / kReduceParams, kReduceParams, 0, st, dPartial, (rows + kRows - 1) / kRows, dSq, rows, dGrad, dLoss, Adam{}, nullptr);
+  reduceKernel(dPartial, dSq, rows, dGrad, dLoss, Adam{}, nullptr, st);
   return cudaGetLastError();
 }
 
@@ -652,9 +661,8 @@ cudaError_t mlp_train_step(const float* dX, const float* dT, uint32_t rows, floa
   if (e != cudaSuccess) return e;
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.f - powf(b1, (float)step), c2 = 1.f - powf(b2, (float)step);
-  launchChained(
-      k_mlp_reduce, (kParams + kReduceParams - 1) / kReduceParams, kReduceParams, 0, st, dPartial, (rows + kRows - 1) / kRows, dSq, rows, nullptr, dLoss, Adam{dW, dM, dV, lr, b1, b2, 1e-8f, c1, c2},
-      static_cast<uint8_t*>(dBlob));
+  reduceKernel(dPartial, dSq, rows, nullptr, dLoss, Adam{dW, dM, dV, lr, b1, b2, 1e-8f, c1, c2},
+               static_cast<uint8_t*>(dBlob), st);
   return cudaGetLastError();
 }
 
