@@ -51,12 +51,12 @@ ALGO_BYTES = {"solveA": (196, 16), "solveB": (128, 48), "pbfA": (36, 36), "pbfB"
               "reorder": (148, 148), "count": (20, 20), "fill": (8, 8), "scan": (8, 8)}
 
 # DRAM bytes per particle per launch (dram__bytes_read.sum +
-# dram__bytes_write.sum over particles) from an ncu --set full capture of the
-# current kernels on the 1M-particle dam breach 100 plain substeps in (the
-# bench's loaded state; profiles/stencil_kernels_full_dam_breach_1M.md); the
-# traffic of a launch grows with the particle count, so the bench scales it
-# by the workload's.
-NCU_TRAFFIC_PER_PARTICLE = {"solveB": 145.6, "solveA": 213.2, "pbfA": 107.2, "computeL": 169.7}
+# dram__bytes_write.sum over particles) from an ncu capture of the current
+# kernels on the 1M-particle dam breach 100 plain substeps in (the bench's
+# loaded state; profiles/neighbour_kernels_packed_lists.md; pbfA the mean of
+# its walking and its three other passes); the traffic of a launch grows with
+# the particle count, so the bench scales it by the workload's.
+NCU_TRAFFIC_PER_PARTICLE = {"solveB": 144.7, "solveA": 144.9, "pbfA": 108.4, "computeL": 198.1}
 
 
 def workload(name: str, rank: int = 0, world: int = 1):
@@ -506,9 +506,9 @@ def run_xpbi(args, rank: int, world: int):
     torch.cuda.synchronize()
     e2e_s = max_over_ranks(time.perf_counter() - t0, dist)
     e2e = job_throughput(n_job, args.steps, e2e_s)
-    # uniforms uploaded per step: SceneDev (244 B) + MatDev table (8 x 48 B)
+    # uniforms uploaded per step: SceneDev (268 B) + MatDev table (8 x 48 B)
     # + packed material words (8 x 64 B) per scene
-    h2d = len(scenes) * (244 + 8 * 48 + 8 * 64)
+    h2d = len(scenes) * (268 + 8 * 48 + 8 * 64)
     d2h = 16 * n_rank
 
     # ---- per-kernel times (events around each launch) for the roofline: of

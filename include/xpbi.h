@@ -419,7 +419,7 @@ int xpbi_philox4x32_10(const uint32_t counter[4], const uint32_t key[2], uint32_
  * would break the recording. It runs the substep's first stage alone (cell
  * key, histogram, scan, bucket fill, deterministic ranks: the same results
  * as xpbi_encode_substep's sort) on the caller's device buffers, with all
- * scratch in one fixed array inside this library (about 10 MB per device,
+ * scratch in one fixed array inside this library (about 7 MB per device,
  * held until the process exits). Nothing is allocated.
  *   pos4        device, n float4 (x, y, z, any w), 16-byte aligned
  *   origin, cell_size, dims   host; the grid of xpbi_read_uniforms words

@@ -458,9 +458,9 @@ struct Schedule {
     std::string k = std::to_string(K) + ":";
     for (char c : pbf) k += c ? '1' : '0';
     k += ":" + std::to_string(mode) + (track ? "t" : "") + (reduce ? "r" : "") + (features ? "f" : "") +
-         (keepLam ? "l" : "") + (active ? "a" : "") + (fallback ? "j" : "") + ":v" + std::to_string(varA) + std::to_string(varB) + ":g" +
-         std::to_string(lanesA) + std::to_string(lanesB) + std::to_string(lanesAll) + std::to_string(lanesPbfA) +
-         std::to_string(lanesPbfB);
+         (keepLam ? "l" : "") + (active ? "a" : "") + (fallback ? "j" : "") + ":v" +
+         std::to_string(varA) + std::to_string(varB) + ":g" + std::to_string(lanesA) + std::to_string(lanesB) +
+         std::to_string(lanesAll) + std::to_string(lanesPbfA) + std::to_string(lanesPbfB);
     return k;
   }
 };
@@ -972,7 +972,8 @@ int createImpl(const xpbi_scene_desc* scenes, uint32_t nScenes, xpbi_sim** out) 
             H2D(b.state, state.data(), 4 * n) && H2D(b.lam, zero.data(), 4 * n) &&
             H2D(b.pbfLam, zero.data(), 4 * n) && H2D(b.sceneOf, sceneOf.data(), 2 * n) &&
             cudaMemset(b.err, 0, sizeof(int)) == cudaSuccess &&
-            cudaMemset(b.waitProbe, 0, sizeof(unsigned long long)) == cudaSuccess && cudaMemset(b.L, 0, 36 * n) == cudaSuccess &&
+            cudaMemset(b.waitProbe, 0, sizeof(unsigned long long)) == cudaSuccess &&
+            cudaMemset(b.L, 0, 36 * n) == cudaSuccess &&
             cudaMemset(b.sortedIdx, 0, 4 * n) == cudaSuccess && cudaMemset(b.lamOut, 0, 4 * n) == cudaSuccess &&
             cudaMemset(b.lamPrev, 0, 4 * n) == cudaSuccess && cudaMemset(b.lamWarm, 0, 4 * n) == cudaSuccess &&
             cudaMemset(b.done, 0, sizeof(int) * nScenes) == cudaSuccess &&

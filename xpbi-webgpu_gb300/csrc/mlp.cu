@@ -263,7 +263,8 @@ constexpr int kPartStride = (kParams + 31) & ~31;       // floats per CTA's part
 // column, 4 of the warp's j). (2 x 8 outputs per thread, reading 16-byte groups
 // of h, took 9,800 cycles for 64 columns and 6,250 for 16.)
 template <int kCols>
-__device__ __forceinline__ void wgrad(const float* dz, const float* h, float* __restrict__ out, float* __restrict__ outB) {
+__device__ __forceinline__ void wgrad(const float* dz, const float* h, float* __restrict__ out,
+                                      float* __restrict__ outB) {
   static_assert(kStepThreads == 256 && kHid == 64 && (kCols == 64 || kCols == 16), "8 warps of 8 outputs j");
   constexpr int kI = kCols == 64 ? 2 : 1;  // columns per lane
   constexpr int kP = kCols == 64 ? 4 : 2;  // pairs of j per lane

@@ -99,17 +99,16 @@ struct PV {
   float4 p, v;
 };
 
-// The predicted position of slot i for the PBF passes: the record their pair
-// loops gather and the coordinate planes pbfA's candidate walk reads.
 // The share of the support by which a PBF walk looks further than the pass
 // needs: 0.1 against 0.05 (too little for moving water: lists of an 80k dam
 // breach rebuilt in most passes) and 0.15 (more pairs to no effect): 3733,
 // 3754 and 3768 us per substep of 1M particles, 329, 332 and 328 of 80k.
 constexpr float kPbfSkin = 0.1f;
 constexpr float kNoRef = 1e30f;  // no slot's pos.w
-// The predicted position of a PBF pass. moved: also how far it lies from where
-// the last stencil walk saw it, as the scene's maximum (pbfA decides by it
-// whether the lists still hold every neighbour).
+// The predicted position of slot i for a PBF pass: the record its pair loops
+// gather and the coordinate planes pbfA's candidate walk reads. moved: also how
+// far it lies from where the last stencil walk saw it, as the scene's maximum
+// (pbfA decides by it whether the lists still hold every neighbour).
 __device__ __forceinline__ void storeXc(const Bufs& b, uint32_t i, V3 xc, float w, bool moved) {
   b.xc[i] = make_float4(xc.x, xc.y, xc.z, w);
   b.xcP[i] = xc.x;
@@ -1000,7 +999,7 @@ __device__ __forceinline__ int iterK(const Bufs& b, int k) {
 // flags & kStoredC (iteration 0, after computeL with features, one lane per
 //   slot): the constraint is the one computeL evaluated at the same
 //   velocities; k_solveA_stored applies it without a neighbour sweep.
-// G lanes per slot (G = 4 for small scenes): the lanes split the neighbour
+// G lanes per slot (two or four on small scenes): the lanes split the neighbour
 // sweep, lane 0 finishes the slot.
 //
 // The update of slot i from its constraint c (lane 0 of the slot).
@@ -1078,7 +1077,8 @@ __global__ void __launch_bounds__(kBlock, kMinB) k_solveA(Bufs b, int k, const f
   const bool act = kTrack && G == 1 && (flags & kActive) != 0 && k > 0;
   bool changed = true;
   if (act && active && !waterW(pi.w)) changed = b.dirty[k & 1][i] != 0;
-  recordSolidDisp(b, i, k, active && !waterW(pi.w) && lane == 0 && changed ? S.dt * length(xyz(loadOwn<G>(velIn + i))) : 0.f);
+  const bool counts = active && !waterW(pi.w) && lane == 0 && changed;
+  recordSolidDisp(b, i, k, counts ? S.dt * length(xyz(loadOwn<G>(velIn + i))) : 0.f);
   if (!active || waterW(pi.w)) {  // water: its record is never read
     if (track && lane == 0) {
       b.rr[i] = 0.f;
@@ -1939,19 +1939,14 @@ __device__ __forceinline__ PbfPair pbfPair(const SceneDev& S, V3 c, const float4
 }
 
 // ---------------------------------------------------------------- pbfA
-// PBF density multiplier (simkernels.js:407-439). Walks the stencil around
-// the current cell with predicted positions and records, in order, the
-// predicted neighbours of this pass: all of them for water, the water ones
-// for solids (the pairs pbfB uses, simkernels.js:457-458).
-// G lanes per slot (small handles): the lanes split the stencil's rows and the
-// density sums over what they find, lane 0 finishes the slot.
 // The stencil walk of a PBF pass: slot i's neighbours by predicted position
 // within the support (exact) or the support and its skin, recorded in order;
 // the count word. Water pairs with everything, a solid with water only (the
-// water flag is the sign bit of xc.w, the sorted pos.w).
+// pairs pbfB uses, simkernels.js:457-458; the water flag is the sign bit of
+// xc.w, the sorted pos.w).
 template <int G>
-__device__ __forceinline__ uint32_t pbfWalk(const Bufs& b, const SceneDev& S, uint32_t i, V3 x, const float4& xc4, bool exact,
-                                            SubList<G>& sub, uint32_t lane) {
+__device__ __forceinline__ uint32_t pbfWalk(const Bufs& b, const SceneDev& S, uint32_t i, V3 x, const float4& xc4,
+                                            bool exact, SubList<G>& sub, uint32_t lane) {
   const float4* __restrict__ xcS = b.xc;
   const V3 xci = xyz(xc4);
   const bool iWater = waterW(xc4.w);
@@ -1990,6 +1985,10 @@ __device__ __forceinline__ uint32_t pbfWalk(const Bufs& b, const SceneDev& S, ui
     return exact ? cnt | kNbrExact : cnt;
   }
 }
+// PBF density multiplier (simkernels.js:407-439) over the predicted neighbours,
+// which the pass's own walk around the current cell records or an earlier one
+// left. G lanes per slot (small handles): the lanes split the stencil's rows and
+// the density sums over what they find, lane 0 finishes the slot.
 template <int G>
 __global__ void __launch_bounds__(kThreads, minPbfA(G)) k_pbfA(Bufs b, int k, int flags) {
   __shared__ uint32_t column[G == 1 ? 1 : SubList<G>::kCap * kThreads];
@@ -2074,8 +2073,8 @@ __global__ void __launch_bounds__(kThreads, minPbfA(G)) k_pbfA(Bufs b, int k, in
     if constexpr (G == 1) {
       forPairs(nbrGroups(b.nbrP, i), (cnt + 3u) >> 2, gather, body);
     } else if (reuse) {
-      forListPairs<G>(nbrGroups(b.nbrP, i), listHead<G>(nbrGroups(b.nbrP, i), b.nbrPCount, i, lane), cnt, i, lane, gather,
-                      body);
+      const uint4* L = nbrGroups(b.nbrP, i);
+      forListPairs<G>(L, listHead<G>(L, b.nbrPCount, i, lane), cnt, i, lane, gather, body);
     } else {
 #pragma unroll 2
       for (uint32_t e = 0; e < sub.same; e += 2u) {
@@ -2123,7 +2122,8 @@ __global__ void __launch_bounds__(kThreads, minPbfA(G)) k_pbfA(Bufs b, int k, in
 // PBF position correction with s_corr (simkernels.js:441-477) over pbfA's
 // record of predicted neighbours.
 template <int G>
-__global__ void __launch_bounds__(kThreads, minPbfB(G)) k_pbfB(Bufs b, int k, const float4* velIn, float4* velOut, int flags) {
+__global__ void __launch_bounds__(kThreads, minPbfB(G)) k_pbfB(Bufs b, int k, const float4* velIn, float4* velOut,
+                                                               int flags) {
   // blocks run last to first: the pass starts where pbfA ended, on
   // slots whose data is still in L2
   const uint32_t t = afterPrevious((gridDim.x - 1u - blockIdx.x) * blockDim.x + threadIdx.x);
@@ -2247,10 +2247,12 @@ __global__ void __launch_bounds__(kThreads) k_xsph(Bufs b, const float4* velIn, 
                const F2 rinv = f2(rsqrtf(fmaxf(lo2(r2), 1e-30f)), rsqrtf(fmaxf(hi2(r2), 1e-30f)));
                const F2 q = mul2(mul2(r2, rinv), f2(S.invH, S.invH));
                const F2 t = fma2(q, f2(-0.5f, -0.5f), f2(1.f, 1.f));
-               const F2 w = mul2(mul2(mul2(mul2(mul2(f2(S.sigW, S.sigW), t), t), t), t), fma2(q, f2(2.f, 2.f), f2(1.f, 1.f)));
+               const F2 w = mul2(mul2(mul2(mul2(mul2(f2(S.sigW, S.sigW), t), t), t), t),
+                                 fma2(q, f2(2.f, 2.f), f2(1.f, 1.f)));
                const F2 vol = f2(d0.v.w, d1.v.w);
-               const F2 ux = mul2(vol, f2(d0.v.x - vi.x, d1.v.x - vi.x)), uy = mul2(vol, f2(d0.v.y - vi.y, d1.v.y - vi.y)),
-                        uz = mul2(vol, f2(d0.v.z - vi.z, d1.v.z - vi.z));
+               const F2 ux = mul2(vol, f2(d0.v.x - vi.x, d1.v.x - vi.x));
+               const F2 uy = mul2(vol, f2(d0.v.y - vi.y, d1.v.y - vi.y));
+               const F2 uz = mul2(vol, f2(d0.v.z - vi.z, d1.v.z - vi.z));
                acc.x = __fmaf_rn(hi2(ux), hi2(w), __fmaf_rn(lo2(ux), lo2(w), acc.x));
                acc.y = __fmaf_rn(hi2(uy), hi2(w), __fmaf_rn(lo2(uy), lo2(w), acc.y));
                acc.z = __fmaf_rn(hi2(uz), hi2(w), __fmaf_rn(lo2(uz), lo2(w), acc.z));
@@ -2387,9 +2389,9 @@ __global__ void k_copy_vel(uint32_t n, const float4* __restrict__ src, float4* _
 // offsets in cursor, both relative to the scene. A read of the state is then
 // one copy per array: it was 26 copies and the transposes on the host, 430 us
 // for 10k particles.
-__global__ void __launch_bounds__(256) k_stage_state(Bufs b, uint32_t first, uint32_t n, uint32_t firstCell, uint32_t cells,
-                                                     uint32_t base, bool F, bool L, bool aux, bool idx, bool tab,
-                                                     float volume) {
+__global__ void __launch_bounds__(256) k_stage_state(Bufs b, uint32_t first, uint32_t n, uint32_t firstCell,
+                                                     uint32_t cells, uint32_t base, bool F, bool L, bool aux, bool idx,
+                                                     bool tab, float volume) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (tab && t < cells) b.cursor[t] = b.cellStart[firstCell + t] - base;
   if (t >= n) return;
@@ -2415,7 +2417,6 @@ inline unsigned gridOf(uint32_t n, int block) { return (unsigned)((n + (uint32_t
 // the learned solve stay plain: they follow memsets and conditional nodes or
 // form the bodies of conditional nodes. So do those of the one-lane solve, on
 // large handles, where a launch's gap does not count.
-constexpr int kPlainLaunch = -1;
 template <class... P, class... Q>
 inline void launchIn(int flags, void (*fn)(P...), unsigned g, unsigned block, cudaStream_t st, Q... q) {
   if (flags == 0)
@@ -2438,12 +2439,11 @@ void launch_computeL(const Bufs& b, bool features, int lanes, cudaStream_t st) {
 void launch_computeL_water(const Bufs& b, cudaStream_t st) { k_computeL_water<<<grid(b.N), kThreads, 0, st>>>(b); }
 template <int V>
 void solveAVariant(const Bufs& b, int k, const float4* velIn, int flags, cudaStream_t st) {
+  constexpr int kBlock = kSolveABlock[V];
   if (flags & kTrackResid)
-    launchIn(kPlainLaunch, k_solveA<true, kSolveAMinB[V], 1, kSolveABlock[V]>, gridOf(b.N, kSolveABlock[V]), kSolveABlock[V],
-             st, b, k, velIn, flags);
+    k_solveA<true, kSolveAMinB[V], 1, kBlock><<<gridOf(b.N, kBlock), kBlock, 0, st>>>(b, k, velIn, flags);
   else
-    launchIn(kPlainLaunch, k_solveA<false, kSolveAMinB[V], 1, kSolveABlock[V]>, gridOf(b.N, kSolveABlock[V]), kSolveABlock[V],
-             st, b, k, velIn, flags);
+    k_solveA<false, kSolveAMinB[V], 1, kBlock><<<gridOf(b.N, kBlock), kBlock, 0, st>>>(b, k, velIn, flags);
 }
 void launch_solveA(const Bufs& b, int k, const float4* velIn, int flags, int variant, int lanes, cudaStream_t st) {
   if (flags & kStoredC) {  // iteration 0 after computeL with features (one lane per slot)
@@ -2486,8 +2486,8 @@ void launch_resid_reduce(const Bufs& b, int k, bool warm, cudaStream_t st) {
 void launch_keep_lambda(const Bufs& b, cudaStream_t st) { k_keep_lambda<<<grid(b.N), kThreads, 0, st>>>(b); }
 template <int V>
 void solveBVariant(const Bufs& b, int k, const float4* velIn, float4* velOut, int wx, int flags, cudaStream_t st) {
-  launchIn(kPlainLaunch, k_solveB<kSolveBMinB[V], 1, kSolveBBlock[V]>, gridOf(b.N, kSolveBBlock[V]), kSolveBBlock[V], st, b, k,
-           velIn, velOut, wx, flags);
+  constexpr int kBlock = kSolveBBlock[V];
+  k_solveB<kSolveBMinB[V], 1, kBlock><<<gridOf(b.N, kBlock), kBlock, 0, st>>>(b, k, velIn, velOut, wx, flags);
 }
 // A grid that fills the GPU once with this kernel's resident blocks (the
 // list launches loop over their lists).
@@ -2585,7 +2585,9 @@ void launch_stage_state(const Bufs& b, uint32_t first, uint32_t n, uint32_t firs
       b, first, n, firstCell, cells, n ? first : 0u, F, L, aux, idx, tab, volume);
 }
 void launch_restore(const Bufs& b, float4* vel, cudaStream_t st) { k_restore<<<grid(b.N), kThreads, 0, st>>>(b, vel); }
-void launch_predict(const Bufs& b, const float4* vel, cudaStream_t st) { k_predict<<<grid(b.N), kThreads, 0, st>>>(b, vel); }
+void launch_predict(const Bufs& b, const float4* vel, cudaStream_t st) {
+  k_predict<<<grid(b.N), kThreads, 0, st>>>(b, vel);
+}
 void launch_copy_vel(const Bufs& b, const float4* src, float4* dst, cudaStream_t st) {
   k_copy_vel<<<grid(b.N), kThreads, 0, st>>>(b.N, src, dst);
 }

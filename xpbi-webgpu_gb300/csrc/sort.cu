@@ -151,7 +151,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(Bufs b) {
       const volatile unsigned long long* status = b.tileStatus;
       for (int last = (int)tile - 1;; last -= 32) {
         const int pred = last - lane;
-        const unsigned long long w64 = pred >= 0 ? waitDescriptor(status + pred, kLookbackSpinLimit, b.err) : 2ull << 32;
+        const unsigned long long w64 =
+            pred >= 0 ? waitDescriptor(status + pred, kLookbackSpinLimit, b.err) : 2ull << 32;
         const unsigned ends = __ballot_sync(0xffffffffu, (uint32_t)(w64 >> 32) != 1u);
         const int stop = ends ? __ffs((int)ends) - 1 : 31;
         excl += __reduce_add_sync(0xffffffffu, lane <= stop ? (uint32_t)w64 : 0u);

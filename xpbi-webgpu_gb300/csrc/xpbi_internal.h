@@ -151,7 +151,7 @@ struct Bufs {
   uint32_t* cellStart;  // [C+1] exclusive cell starts, sentinel = N
   uint8_t* cellWater;   // [C] 1 if the cell holds a water particle this substep
   uint32_t* tileTicket;            // word 0 of the scan control block
-  uint32_t* crowd;                 // [crowdRows(N)][crowdSegments(N)] members of a crowded cell per segment of particles
+  uint32_t* crowd;      // [crowdRows(N)][crowdSegments(N)] members of a crowded cell per segment of particles
   unsigned long long* tileStatus;  // [tiles] look-back descriptors (after the two words)
   uint16_t* sceneOf;    // [N] scene of each particle slot (static)
   uint32_t* nbr;        // [ceil(N / 32)][kNbrCap / 4][32][4] in-support neighbours: own phase from the front in
