@@ -55,3 +55,30 @@ def test_flattened_and_inverted_particles(xp, oracle, built_lib, model, path):
     planted = np.isin(s1["sortedIdx"], idx)
     assert planted.sum() == len(idx)
     assert np.linalg.det(s1["F"].reshape(-1, 3, 4)[planted][:, :, :3].astype(np.float64)).min() > 0.0
+
+
+@pytest.mark.parametrize("model", ["sand_two_blocks", "plasticine", "goo", "snow_classic"])
+def test_strongly_stretched_particles(xp, oracle, built_lib, model):
+    """Gradients of size 300, which the return maps bring back: the result is
+    as accurate as its own size, not F's."""
+    sc = getattr(xp.scenes, model)()
+    p = xp.params_for(sc)
+    F, idx = _plant(len(sc["positions"]))
+    rng = np.random.default_rng(1)
+    for i in idx:
+        F[i].reshape(3, 4)[:, :3] = 300.0 * rng.normal(size=(3, 3))
+    with xp.Simulation(sc) as sim:
+        sim.write_params(p)
+        sim.write_state(0, F=F)
+        s0 = sim.read_state()
+        pw, mw = sim.uniforms()
+        ref = oracle.substep(pw, mw, s0, 1, False, -1)
+        ref64 = oracle.substep(pw, mw, s0, 1, False, -1, f64=True)
+        sim.encode_substep(1, False)
+        s1 = sim.read_state()
+    compare(s1, ref, ref64,
+            perturbed=perturbed_runs(oracle, sc, s0, iterations=1, has_water=False, xp=xp, params=p, positions=True))
+    scale = np.abs(ref64["F"]).max(axis=1, keepdims=True)
+    far = np.isin(s1["sortedIdx"], idx)
+    err = [(np.abs(x["F"] - ref64["F"]) / scale)[far].max() for x in (s1, ref)]
+    assert err[0] <= max(1e-5, 4.0 * err[1]), err

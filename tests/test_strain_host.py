@@ -26,14 +26,15 @@ def strain(tmp_path_factory):
     assert r.returncode == 0, r.stderr
     fn = C.CDLL(lib).strain_svd
 
-    def run(F):
+    def run(F, lo=1e-3, hi=1e3):
         H = (np.asarray(F, np.float64) - np.eye(3)).astype(np.float32)
         n = len(H)
         cols = np.ascontiguousarray(np.swapaxes(H, 1, 2))
-        out = [np.zeros(s, np.float32) for s in ((n, 3), (n, 3), (n, 3, 3), (n, 3, 3))]
-        fn(cols.ctypes.data_as(C.c_void_p), n, *[a.ctypes.data_as(C.c_void_p) for a in out])
-        sig, e, U, V = [a.astype(np.float64) for a in out]
-        return H.astype(np.float64) + np.eye(3), sig, e, np.swapaxes(U, 1, 2), np.swapaxes(V, 1, 2)
+        out = [np.zeros(s, np.float32) for s in ((n, 3), (n, 3), (n, 3, 3), (n, 3, 3), (n, 3, 3))]
+        ptr = [a.ctypes.data_as(C.c_void_p) for a in out]
+        fn(cols.ctypes.data_as(C.c_void_p), n, *ptr[:4], C.c_float(lo), C.c_float(hi), ptr[4])
+        sig, e, U, V, G = [a.astype(np.float64) for a in out]
+        return H.astype(np.float64) + np.eye(3), sig, e, *(np.swapaxes(a, 1, 2) for a in (U, V, G))
     return run
 
 
@@ -44,7 +45,7 @@ TOL = 3e-6
 
 
 def _check(strain, F):
-    F, sig, e, U, V = strain(F)
+    F, sig, e, U, V, _ = strain(F)
     assert all(np.isfinite(a).all() for a in (sig, e, U, V))
     want = np.linalg.svd(F, compute_uv=False)
     want[:, 2] *= np.where(np.linalg.det(F) < 0, -1.0, 1.0)
@@ -87,5 +88,24 @@ def test_reflections_and_nan(strain):
     _check(strain, q)
     bad = np.eye(3)[None].copy()
     bad[0, 0, 0] = np.nan
-    _, sig, _, _, _ = strain(bad)  # not taken for an undeformed particle
+    _, sig, *_ = strain(bad)  # not taken for an undeformed particle
     assert not np.isfinite(sig).all()
+
+
+@pytest.mark.parametrize("size", [1e-4, 0.05, 0.3, 3.0, 30.0, 300.0])
+@pytest.mark.parametrize("hi", [1.001, 1000.0])
+def test_clamped_singular_values(strain, size, hi):
+    """F with its singular values clamped, as the return maps do: accurate to
+    the size of the result, however large F was. (Its rotation feels F's own
+    rounding over the smallest sum of two singular values; U and V are off by
+    TOL each in at most two columns.)"""
+    rng = np.random.default_rng(3)
+    F, _, _, _, _, G = strain(np.eye(3) + size * rng.normal(size=(5000, 3, 3)), 0.999, hi)
+    u, s, vt = np.linalg.svd(F)
+    sign = np.where(np.linalg.det(F) < 0, -1.0, 1.0)
+    u[:, :, 2] *= sign[:, None]
+    s[:, 2] *= sign
+    to = np.clip(s, 0.999, hi)
+    want = np.einsum("nij,nj,njk->nik", u, to, vt)
+    cond = np.maximum(s[:, 0] / np.maximum(s[:, 1] + s[:, 2], 1e-30), 1.0)
+    assert (np.abs(G - want).max(axis=(1, 2)) <= 4 * TOL * to[:, 0] * cond).all()

@@ -813,7 +813,8 @@ __device__ __noinline__ Constraint constraintTail(M3 A, TailIn in, const SceneDe
   // the trial F minus the identity, which keeps the digits of a small strain
   const M3 Htr = madd(minusIdent(Fn), mscale(mul(mul(A, transpose(Li)), Fn), S.dt));
   V3 eTr;
-  const SVD sd = strainSVD(Htr, eTr);
+  bool near;
+  const SVD sd = strainSVD(Htr, eTr, near);
   Constraint out;
   out.logSigTr = v3(fmaxf(fmaxf(eTr.x, eTr.y), eTr.z),
                     fmaxf(fminf(eTr.x, eTr.y), fminf(fmaxf(eTr.x, eTr.y), eTr.z)),
@@ -2277,12 +2278,11 @@ __device__ __noinline__ M3 plasticUpdate(const SceneDev& S, const M3& gradV, con
                                          float& stOut) {
   const M3 Htr = madd(minusIdent(F0), mscale(mul(gradV, F0), S.dt));
   V3 e;
-  const SVD sv = strainSVD(Htr, e);
+  bool near;
+  const SVD sv = strainSVD(Htr, e, near);
   const float hard = hardening(m, st);
   const Mapped mp = returnMap(sv.sig, e, m, m.mu * hard, m.lam * hard, st, S.dt, stOut);
-  // the trial F, changed by what the map and the clamp changed
-  const M3 D = diagMul(sv.U, safeSig(mp.sig) - sv.sig, sv.V);
-  return madd(madd(Htr, D), mident());
+  return withSigma(Htr, sv, safeSig(mp.sig), near);
 }
 template <int G>
 __global__ void __launch_bounds__(kThreads, kMinUpdate) k_updateF_integrate(Bufs b, const float4* __restrict__ velIn) {

@@ -303,15 +303,16 @@ __device__ __forceinline__ V3 safeSig(V3 s) { return vclamp(s, 1e-3f, 1e3f); }
 // sigma lies in (0.5, 1.33), inside safeSig's bounds. (The entries alone do
 // not: flattened to nothing along (1, 1, 1), every one is -1/3 and an
 // eigenvalue is -1.) Elsewhere, NaN included, the SVD of F itself keeps the
-// small singular values and the sign.
-__device__ __forceinline__ SVD strainSVD(const M3& H, V3& e) {
+// small singular values and the sign. near: which of the two it was.
+__device__ __forceinline__ SVD strainSVD(const M3& H, V3& e, bool& near) {
   const V3 x = H.c[0], y = H.c[1], z = H.c[2];
   const Sym3 S = {fmaf(2.f, x.x, dot(x, x)), fmaf(2.f, y.y, dot(y, y)), fmaf(2.f, z.z, dot(z, z)),
                   (x.y + y.x) + dot(x, y),   (x.z + z.x) + dot(x, z),   (y.z + z.y) + dot(y, z)};
   const M3 F = {{v3(1.f + x.x, x.y, x.z), v3(y.x, 1.f + y.y, y.z), v3(z.x, z.y, 1.f + z.z)}};
   const float xy = fabsf(S.xy), xz = fabsf(S.xz), yz = fabsf(S.yz);
   const float rows = fmaxf(fmaxf(fabsf(S.xx) + xy + xz, fabsf(S.yy) + xy + yz), fabsf(S.zz) + xz + yz);
-  if (maxAbs(S) < 0.5f && rows < 0.75f && det(F) > 0.f) {
+  near = maxAbs(S) < 0.5f && rows < 0.75f && det(F) > 0.f;
+  if (near) {
     SVD out;
     V3 d;
     eigSym(S, d, out.V);
@@ -325,6 +326,13 @@ __device__ __forceinline__ SVD strainSVD(const M3& H, V3& e) {
   const SVD out = svd3Fast(F);
   e = vlog(safeSig(out.sig));
   return out;
+}
+// F = I + H with its singular values replaced by s. Near the identity what the
+// map changed is added to F, which keeps the digits of a small strain; far from
+// it that would leave the rounding of a large F on a result that the map may
+// have brought back to sigma = 1 (F of size 30 to 2e-5, 2e-7 composed anew).
+__device__ __forceinline__ M3 withSigma(const M3& H, const SVD& sv, V3 s, bool near) {
+  return near ? madd(madd(H, diagMul(sv.U, s - sv.sig, sv.V)), mident()) : diagMul(sv.U, s, sv.V);
 }
 // energy from the logs e of the clamped singular values; its gradient is
 // (2 mu e + lam tr e) / safeSig(sig)
