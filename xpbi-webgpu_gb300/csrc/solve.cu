@@ -335,13 +335,18 @@ __device__ __forceinline__ void forSame(const Bufs& b, const Ctx& cx, const List
         if (j == i) continue;
         const float4 pj = ldg(b.posS + j);
         const V3 d = xi - xyz(pj);
-        if (!(dot(d, d) < S.support2) || waterW(pj.w) != iWater) continue;
-        if (first == i) {
+        const float d2 = dot(d, d);
+        if (!(d2 < S.support2) || waterW(pj.w) != iWater) continue;
+        const bool twin = d2 == 0.f && !iWater;  // paired with i (see coincident)
+        if (first == i && !twin) {
           first = j;
-        } else {
-          body(first, j, gather(first), gather(j));
-          first = i;
+          continue;
         }
+        const auto p = gather(twin ? j : first);
+        auto q = gather(j);
+        if (twin) q = self();
+        body(twin ? j : first, twin ? i : j, p, q);
+        if (!twin) first = i;
       }
     });
     if (first != i) body(first, i, gather(first), self());
@@ -473,6 +478,43 @@ __device__ __forceinline__ void walkCandidates(const SceneDev& S, const uint32_t
   }, lane);
 }
 
+// Exactly coincident solids. The reference's sums see a particle's twin as a
+// term of 0, so twins that start alike stay together. The packed sums add even
+// and odd neighbours apart, and the twin stands elsewhere in one list than in
+// the other: everything behind it would change halves, the sums differ in their
+// last bits, and the contact pass drives apart what a rounding separated (a
+// doubled body of 2744 particles: 2084 pairs apart after 20 substeps, none with
+// the terms in one order). So a list's coincident entries come last, and on the
+// stencil walks they are paired with the slot itself.
+__device__ __forceinline__ bool coincident(Planes P, uint32_t j, V3 x) {
+  return ldg(P.x + j) == x.x && ldg(P.y + j) == x.y && ldg(P.z + j) == x.z;
+}
+// the n entries at(0), at(1), ... with the coincident ones last, the others in
+// their order
+template <class At>
+__device__ __forceinline__ void coincidentLast(Planes P, V3 x, uint32_t n, At&& at) {
+  uint32_t last = n;
+#pragma unroll 1
+  for (uint32_t e = n; e-- > 0u;) {
+    const uint32_t j = *at(e);
+    if (!coincident(P, j, x)) continue;
+    --last;
+#pragma unroll 1
+    for (uint32_t q = e; q < last; ++q) *at(q) = *at(q + 1u);
+    *at(last) = j;
+  }
+}
+__device__ __noinline__ void coincidentLastInList(Planes P, V3 x, uint32_t n, uint32_t* nbr, uint32_t i) {
+  coincidentLast(P, x, n, [&](uint32_t e) { return nbrEntry(nbr, i, e); });
+}
+// (several lanes: the column of lane 0, whose row holds the slot's own cell and
+// whose entries the list starts with)
+__device__ __noinline__ void coincidentLastInColumn(Planes P, V3 x, uint32_t n, uint32_t* col, uint32_t* nbr,
+                                                    uint32_t i) {
+  coincidentLast(P, x, n, [&](uint32_t e) { return col + e * (uint32_t)kThreads; });
+  for (uint32_t e = 0; e < n; ++e) *nbrEntry(nbr, i, e) = col[e * (uint32_t)kThreads];
+}
+
 // What a walk with several lanes per slot records before the lists are
 // written: each lane's hits in a column of shared memory, `same` from the top
 // and `other` from the bottom. A lane with more than the column holds loses
@@ -518,14 +560,15 @@ struct SubList {
 // The offsets of two neighbours from xi and what the sums weigh them by:
 // (dx, dy, dz) = xi - x_b, w = V_b g (dx, dy, dz), so that V_b gradW_b = c w.
 struct Pair {
-  F2 dx, dy, dz, wx, wy, wz;
+  F2 dx, dy, dz, r2, wx, wy, wz;
 };
 __device__ __forceinline__ Pair pairOf(const SceneDev& S, V3 xi, const PV& p, const PV& q) {
   Pair r;
   r.dx = f2(xi.x - p.p.x, xi.x - q.p.x);
   r.dy = f2(xi.y - p.p.y, xi.y - q.p.y);
   r.dz = f2(xi.z - p.p.z, xi.z - q.p.z);
-  const F2 s = mul2(radial2(S, fma2(r.dz, r.dz, fma2(r.dy, r.dy, mul2(r.dx, r.dx)))), f2(p.v.w, q.v.w));
+  r.r2 = fma2(r.dz, r.dz, fma2(r.dy, r.dy, mul2(r.dx, r.dx)));
+  const F2 s = mul2(radial2(S, r.r2), f2(p.v.w, q.v.w));
   r.wx = mul2(r.dx, s);
   r.wy = mul2(r.dy, s);
   r.wz = mul2(r.dz, s);
@@ -592,7 +635,7 @@ __device__ __forceinline__ void bonetLok(const Bufs& b, const Ctx& cx, uint32_t 
   F2 a00 = 0ull, a11 = 0ull, a22 = 0ull, a01 = 0ull, a02 = 0ull, a12 = 0ull;
   F2 sx = 0ull, sy = 0ull, sz = 0ull;
   F2 p00 = 0ull, p11 = 0ull, p22 = 0ull, p01 = 0ull, p02 = 0ull, p12 = 0ull;
-  float cnt = 0.f;
+  uint32_t cnt = 0, zeros = 0;  // the solid neighbours; distances of 0 among them and the padding
   auto gather = [&](uint32_t j) { return PV{ldg(posS + j), ldg(velIn + j)}; };
   auto addA = [&](const Pair& r) {
     a00 = fma2(r.wx, r.dx, a00);
@@ -602,7 +645,7 @@ __device__ __forceinline__ void bonetLok(const Bufs& b, const Ctx& cx, uint32_t 
     a02 = fma2(r.wx, r.dz, a02);
     a12 = fma2(r.wy, r.dz, a12);
   };
-  auto own = [&](uint32_t j0, uint32_t j1, const PV& d0, const PV& d1) {
+  auto own = [&](uint32_t, uint32_t, const PV& d0, const PV& d1) {
     const Pair r = pairOf(S, xi, d0, d1);
     addA(r);
     if constexpr (kSolid) {
@@ -618,8 +661,14 @@ __device__ __forceinline__ void bonetLok(const Bufs& b, const Ctx& cx, uint32_t 
       p01 = fma2(ux, r.wy, p01);
       p02 = fma2(ux, r.wz, p02);
       p12 = fma2(uy, r.wz, p12);
-      cnt += (j0 != i ? 1.f : 0.f) + (j1 != i ? 1.f : 0.f);
+      zeros += (lo2(r.r2) == 0.f ? 1u : 0u) + (hi2(r.r2) == 0.f ? 1u : 0u);
     }
+  };
+  auto clear = [&] {
+    a00 = a11 = a22 = a01 = a02 = a12 = 0ull;
+    sx = sy = sz = 0ull;
+    p00 = p11 = p22 = p01 = p02 = p12 = 0ull;
+    if constexpr (kVel) Av = VelSum();
   };
   // own phase; the other phase's neighbours enter L alone
   const uint32_t c = G == 1 ? b.nbrCount[i] : (sub->lost ? kNbrOverflow : 0u);
@@ -632,28 +681,44 @@ __device__ __forceinline__ void bonetLok(const Bufs& b, const Ctx& cx, uint32_t 
         const float4 pj = ldg(posS + j);
         const V3 d = xi - xyz(pj);
         if (!(dot(d, d) < S.support2)) continue;
-        if (waterW(pj.w) == kSolid)
+        if (waterW(pj.w) == kSolid) {
           addA(pairOf(S, xi, gather(j), self));
-        else
+        } else {
           own(j, i, gather(j), self);
+          ++cnt;
+        }
       }
     }, lane);
   } else if constexpr (G == 1) {
-    forPairs(nbrGroups(b.nbr, i), (sameCount(c) + 3u) >> 2, gather, own);
+    cnt = sameCount(c);
+#pragma unroll 1
+    for (bool again = false;; again = true) {
+      forPairs(nbrGroups(b.nbr, i), (cnt + 3u) >> 2, gather, own);
+      if (!kSolid || again || zeros <= ((0u - cnt) & 3u)) break;
+      coincidentLastInList(planesOf(b.posP, b.planeN), xi, cnt, b.nbr, i);
+      clear();
+    }
     const uint32_t other = (otherCount(c) + 3u) >> 2;
     if (other)
       forPairs(nbrGroups(b.nbr, i) + kGroupStride * (kNbrCap / 4u - other), other, gather,
                   [&](uint32_t, uint32_t, const PV& d0, const PV& d1) { addA(pairOf(S, xi, d0, d1)); });
   } else {
+    cnt = sub->same;
     // a last odd one is paired with a copy of itself of no volume
+#pragma unroll 1
+    for (bool again = false;; again = true) {
 #pragma unroll 2
-    for (uint32_t e = 0; e < sub->same; e += 2u) {
-      const bool two = e + 1u < sub->same;
-      const uint32_t j0 = sub->at(e), j1 = two ? sub->at(e + 1u) : j0;
-      const PV d0 = gather(j0);
-      PV d1 = gather(j1);
-      if (!two) d1.v.w = 0.f;
-      own(j0, two ? j1 : i, d0, d1);
+      for (uint32_t e = 0; e < cnt; e += 2u) {
+        const bool two = e + 1u < cnt;
+        const uint32_t j0 = sub->at(e), j1 = two ? sub->at(e + 1u) : j0;
+        const PV d0 = gather(j0);
+        PV d1 = gather(j1);
+        if (!two) d1.v.w = 0.f;
+        own(j0, two ? j1 : i, d0, d1);
+      }
+      if (!kSolid || again || zeros == 0u || lane != 0) break;
+      coincidentLastInColumn(planesOf(b.posP, b.planeN), xi, cnt, sub->col, b.nbr, i);
+      clear();
     }
     for (uint32_t e = 0; e < sub->other; e += 2u) {
       const bool two = e + 1u < sub->other;
@@ -675,11 +740,11 @@ __device__ __forceinline__ void bonetLok(const Bufs& b, const Ctx& cx, uint32_t 
     const float c2 = gc * gc;
     const float q00 = total(p00) * c2, q11 = total(p11) * c2, q22 = total(p22) * c2;
     const float q01 = total(p01) * c2, q02 = total(p02) * c2, q12 = total(p12) * c2;
-    cnt = laneSum<G>(cnt);
+    const float count = laneSum<G>((float)cnt);
     if (lane == 0) {
       float4* __restrict__ R = b.sgP + i;
       const size_t N = b.N;
-      R[0] = make_float4(sg.x, sg.y, sg.z, cnt);
+      R[0] = make_float4(sg.x, sg.y, sg.z, count);
       R[N] = make_float4(q00, q11, q22, q01);
       R[2 * N] = make_float4(q02, q12, 0.f, 0.f);
     }
@@ -1272,8 +1337,9 @@ __device__ __forceinline__ void computeL(const Bufs& b) {
   };
   SubList<G> sub;
   uint32_t same = 0, other = 0;
+  const Planes planes = planesOf(b.posP, b.planeN);
   if constexpr (G == 1) {
-    walkCandidates(S, b.cellStart, xi, i, planesOf(b.posP, b.planeN), xi, s2, [&](uint32_t j) {
+    walkCandidates(S, b.cellStart, xi, i, planes, xi, s2, [&](uint32_t j) {
       const bool own = isOwn(j);
       const uint32_t e = own ? same : ~other;
       *nbrEntry(b.nbr, i, e & (kNbrCap - 1u)) = j;
@@ -1282,8 +1348,7 @@ __device__ __forceinline__ void computeL(const Bufs& b) {
     });
   } else {
     sub.col = column + threadIdx.x;
-    walkCandidates<G>(S, b.cellStart, xi, i, planesOf(b.posP, b.planeN), xi, s2,
-                      [&](uint32_t j) { sub.add(j, isOwn(j)); }, lane);
+    walkCandidates<G>(S, b.cellStart, xi, i, planes, xi, s2, [&](uint32_t j) { sub.add(j, isOwn(j)); }, lane);
     sub.totals(lane);
     same = sub.sameAll;
     other = sub.otherAll;
